@@ -1,4 +1,4 @@
-/* Single-pass causal attention for a prompt slice: a block of RB consecutive query rows of ONE session per CTA.
+/* Single-pass causal attention for a prompt slice: 4 x QT consecutive query rows of ONE session per CTA.
  *
  * Arithmetic per (row, head): that of the single-row kernel in prims.cu (the reference's k_attention /
  * k_attention8, src/slowar/kernels.cu:234-309 and :625-728) - tiles of 128 cached positions, per position one
@@ -6,229 +6,385 @@
  * tile max and sum by 128-wide halving trees, l = fma(l, corr, tile_sum), acc *= corr, then one fma per position in
  * ascending order - so the outputs are the same bits.
  *
- * What the row block buys.  The single-row kernel stages a K and a V tile per (row, kv head), converts every cached
- * value for that one row and crosses ~20 CTA barriers per tile: a 512-token prompt spends 13 of its 29 ms there, an
- * 8192-token prompt 2.8 of 2.9 s.  Here a tile is staged once for RB rows, a cached key or value is read and
- * converted once and feeds RB chains held side by side in registers, and the trees of the RB rows share their
- * barriers.  (RB = 4 in the product: 64 registers, two CTAs per SM.)  Rows of a block differ only in how far they may look: row i of the block sees positions below
- * len0 + i, which only matters in the block's last one or two tiles; there the chains of positions a row may not see
- * yield -inf / probability 0 and its value sum skips them, exactly as the single-row loop ends earlier.
+ * What bounds it: fp32 fma issue (the chains are fp32 by contract, 256 fma per (row, head, position)).  So the two
+ * products are laid out as register-tiled fp32 matrix products.  The queries of a CTA are its rows x the four heads of
+ * one kv head, 2 QT NW of them; consumer warp w owns queries 2 QT w .. +2 QT - 1 in BOTH phases, a thread QT of them times
+ * eight positions (score phase) or eight dimensions (value phase).  Keys and values of a tile are widened to f32 once per CTA
+ * into shared memory, keys transposed, and every chain advances on the packed fma (fma.rn.f32x2, two independent
+ * roundings; it holds the fma pipe for two cycles, so shared reads and the broadcast of the query or weight operand issue
+ * beside it).  A warp sees all 128 positions of its queries, so max, sum and weights never leave it (the sum tree's pairs: 64
+ * in the thread, 32..4 over four lane bits, 2 and 1 in the thread).  Four producer warps widen the tiles ahead of the
+ * consumers, which therefore meet no CTA barrier.
  *
- * Thread (g, t) of 512: head g of the kv head's four; t is a cached position of the tile in the score phase and a
- * head dimension in the value phase.
+ * Measured (INT8 cache, 2048 rows after 6052 positions, 119 G fma): 12.6 ms with four rows per 512-thread CTA, keys converted
+ * by every reader and trees over shared memory; 10.6 ms register-tiled 2 x 8; 6.5 ms 4 x 8; 5.7 ms with 12 warps instead of
+ * 8; 5.5 ms = 21.7 T fma/s with the producers, 0.58 of the fp32 peak.  The score phase runs at nine tenths of the fma
+ * rate; the value phase pays one multiplication per weight and group scale.  8 x 8 tiles measured the same per row with
+ * worse waves; 2 queries x 16 dimensions per thread in the value phase slower (more shared reads).
  */
 #pragma once
 #include <math.h>
 #include "common.cuh"
 #include "headops.cuh"
 #include "ops.h"
+#include "pipe.cuh"
 
 namespace s2p {
 
-template <bool KV8, int RB> struct AttnPrefillSmem {
-    static constexpr int VB = KV8 ? 128 : 256; /* payload bytes per cached vector */
-    static constexpr int TS = VB + 4;          /* staged row stride: word reads of 32 different rows hit 32 banks */
-    alignas(16) unsigned char tile[128 * TS];  /* K rows of the tile, then its V rows */
-    alignas(16) __half ssc[128 * 4];           /* group scales of the keys (INT8 cache) */
-    alignas(16) __half vssc[128 * 4];          /* ... and of the values, staged with the keys */
-    alignas(16) float sq[RB][4][128];          /* pre-scaled queries */
-    alignas(16) float red[RB][4][128];         /* tree scratch */
-    /* weights of the value sum: [row][head][value group][position] = probability x the group's scale (INT8 cache),
-     * or [row][head][0][position] = probability (bf16 cache) */
-    alignas(16) float spv[RB][4][KV8 ? 4 : 1][128];
+typedef unsigned long long f32x2; /* two f32 in a register pair, low half first */
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ void ffma2(f32x2& d, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ f32x2 ffma2_of(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 fmul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+constexpr int ATTN_PREFILL_PRODUCERS = 128; /* threads that widen the tiles */
+
+template <bool KV8, int QT, int NW> struct AttnPrefillSmem {
+    static constexpr int M = 2 * QT * NW;               /* queries of a CTA */
+    alignas(16) float q[128][M];                        /* pre-scaled queries, dimension-major */
+    alignas(16) float k[128][128];                      /* key tile, dimension-major */
+    /* value tile; the 16-byte chunk c of a row (dimensions 4c..) at slot (c & 1) * 16 + (c >> 1), which makes a thread's
+     * eight dimensions two conflict-free reads */
+    alignas(16) float v[128][128];
+    /* soft-max weights, private to a warp: [half of its queries][query][position], the second half with position bit 4
+     * flipped so that the two halves of a warp read different banks */
+    alignas(16) float p[NW][2][QT][128];
+    alignas(16) __half ksc[KV8 ? 4 : 1][128], vsc[KV8 ? 4 : 1][128]; /* group scales of the tile */
+    alignas(8) uint64_t kfull, kempty, vfull, vempty;
 };
 
-template <bool KV8, int RB>
-__global__ void __launch_bounds__(512) k_attn_prefill(AttnArgs a, int rows) {
+/* 16 payload bytes, from an address that may be aligned to 4 bytes only */
+__device__ __forceinline__ uint4 attn_prefill_load16(const unsigned char* src, int wide) {
+    if (wide) return __ldg(reinterpret_cast<const uint4*>(src));
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+/* a key tile to f32, dimension-major: a thread per position, so the transposed stores are conflict-free */
+template <bool KV8>
+__device__ __forceinline__ void attn_prefill_keys(float (*k)[128], const unsigned char* src, int r, int lim, int wide) {
+    constexpr int NCH = KV8 ? 8 : 16; /* 16-byte chunks of a cached vector */
+#pragma unroll 1
+    for (int c0 = 0; c0 < NCH; c0 += 2) {
+        uint4 x[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+            x[u] = r < lim ? attn_prefill_load16(src + (size_t)r * (NCH * 16) + (c0 + u) * 16, wide) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+            float(*d)[128] = k + (c0 + u) * (KV8 ? 16 : 8);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (KV8) {
+                    const uint32_t b = s8x4_bias(w[j]);
+                    d[4 * j][r] = s8_biased_to_f32<0>(b);
+                    d[4 * j + 1][r] = s8_biased_to_f32<1>(b);
+                    d[4 * j + 2][r] = s8_biased_to_f32<2>(b);
+                    d[4 * j + 3][r] = s8_biased_to_f32<3>(b);
+                } else {
+                    d[2 * j][r] = bf_lo(w[j]);
+                    d[2 * j + 1][r] = bf_hi(w[j]);
+                }
+            }
+        }
+    }
+}
+/* a value tile to f32, rows in the slot order of AttnPrefillSmem::v */
+template <bool KV8>
+__device__ __forceinline__ void attn_prefill_values(float (*v)[128], const unsigned char* src, int pt, int lim, int wide) {
+    constexpr int NCH = KV8 ? 8 : 16;
+    const int c = pt % NCH;
+#pragma unroll 2
+    for (int r = pt / NCH; r < 128; r += ATTN_PREFILL_PRODUCERS / NCH) {
+        const uint4 x = r < lim ? attn_prefill_load16(src + (size_t)r * (NCH * 16) + c * 16, wide) : make_uint4(0, 0, 0, 0);
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+        float4* d = reinterpret_cast<float4*>(v[r]);
+        if (KV8) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t b = s8x4_bias(w[j]);
+                d[(j & 1) * 16 + c * 2 + (j >> 1)] = make_float4(s8_biased_to_f32<0>(b), s8_biased_to_f32<1>(b), s8_biased_to_f32<2>(b), s8_biased_to_f32<3>(b));
+            }
+        } else {
+            d[c] = make_float4(bf_lo(w[0]), bf_hi(w[0]), bf_lo(w[1]), bf_hi(w[1]));
+            d[16 + c] = make_float4(bf_lo(w[2]), bf_hi(w[2]), bf_lo(w[3]), bf_hi(w[3]));
+        }
+    }
+}
+__device__ __forceinline__ void attn_prefill_scales(__half (*dst)[128], const __half* src, int r, int lim) {
+    const unsigned short* s = reinterpret_cast<const unsigned short*>(src) + (size_t)r * 4;
+#pragma unroll
+    for (int g = 0; g < 4; g++) dst[g][r] = __ushort_as_half(r < lim ? s[g] : (unsigned short)0);
+}
+__device__ __forceinline__ f32x2 half2_to_f32x2(uint32_t h) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    return pack2(f.x, f.y);
+}
+
+/* one dimension of the score phase: QT queries x eight positions */
+template <int QT>
+__device__ __forceinline__ void attn_prefill_dim(const float* krow, const float* qrow, int tx, f32x2 (&s)[QT][4]) {
+    const ulonglong2 ka = *reinterpret_cast<const ulonglong2*>(krow + tx * 4), kb = *reinterpret_cast<const ulonglong2*>(krow + 64 + tx * 4);
+    float qv[QT];
+    if (QT >= 4) {
+#pragma unroll
+        for (int i = 0; i < QT; i += 4) *reinterpret_cast<float4*>(qv + i) = *reinterpret_cast<const float4*>(qrow + i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < QT; i += 2) *reinterpret_cast<float2*>(qv + i) = *reinterpret_cast<const float2*>(qrow + i);
+    }
+#pragma unroll
+    for (int i = 0; i < QT; i++) {
+        const f32x2 qq = pack2(qv[i], qv[i]);
+        ffma2(s[i][0], qq, ka.x);
+        ffma2(s[i][1], qq, ka.y);
+        ffma2(s[i][2], qq, kb.x);
+        ffma2(s[i][3], qq, kb.y);
+    }
+}
+
+/* NW consumer warps and four producer warps.  The producers widen key tile t + 1 while the consumers are in the value
+ * phase of tile t, and value tile t + 1 under score phase t + 1; the four mbarriers let every consumer warp run at its own
+ * pace inside that window, so one warp's soft-max overlaps another's fma.  SPLIT_REGS: 512 threads at 128 registers, of
+ * which the producers give theirs up (12 x 32 x 160 + 4 x 32 x 32 = 65536 = what the block was launched with). */
+template <bool KV8, int QT, int NW>
+__global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_prefill(AttnArgs a, int rows, int wide, int* status) {
     extern __shared__ __align__(16) unsigned char attn_prefill_smem[];
-    AttnPrefillSmem<KV8, RB>& sm = *reinterpret_cast<AttnPrefillSmem<KV8, RB>*>(attn_prefill_smem);
-    constexpr int VB = AttnPrefillSmem<KV8, RB>::VB, TS = AttnPrefillSmem<KV8, RB>::TS;
+    typedef AttnPrefillSmem<KV8, QT, NW> Smem;
+    Smem& sm = *reinterpret_cast<Smem*>(attn_prefill_smem);
+    constexpr bool SPLIT_REGS = NW == 12;
+    constexpr int M = Smem::M, RB = M / 4, NC = 32 * NW, VB = KV8 ? 128 : 256;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     /* the last rows of the slice look furthest back: their blocks start first, the short ones fill in behind them */
     const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * RB, kvh = blockIdx.y;
     const int rb = min(RB, rows - r0);
-    const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
-    const int QH = a.q_heads, h = kvh * 4 + g;
     const int len0 = a.pos0 + r0 + 1;   /* positions row r0 attends over; row r0 + i: len0 + i */
     const int len_max = len0 + rb - 1;
-    const size_t plane = (size_t)kvh * a.max_seq;
-    const unsigned char* kc = kv_payload(a.kv, r0) + a.kv.k_off; /* one cache for all rows of the block */
-    const unsigned char* vc = kv_payload(a.kv, r0) + a.kv.v_off;
-    const __half* ks = KV8 ? reinterpret_cast<const __half*>(kv_scales(a.kv, r0) + a.kv.ks_off) : nullptr;
-    const __half* vs = KV8 ? reinterpret_cast<const __half*>(kv_scales(a.kv, r0) + a.kv.vs_off) : nullptr;
-
+    if (tid == 0) {
+        mbar_init(&sm.kfull, ATTN_PREFILL_PRODUCERS);
+        mbar_init(&sm.vfull, ATTN_PREFILL_PRODUCERS);
+        mbar_init(&sm.kempty, NW);
+        mbar_init(&sm.vempty, NW);
+        mbar_init_fence();
+    }
     const float scale = rsqrtf((float)a.head_dim); /* run-time value on purpose, see AttnArgs */
-#pragma unroll
-    for (int i = 0; i < RB; i++)
-        sm.sq[i][g][t] = i < rb ? __fmul_rn(bf2f(a.q[((size_t)(r0 + i) * QH + h) * 128 + t]), scale) : 0.f;
-
-    float m[RB], l[RB], acc[RB];
-#pragma unroll
-    for (int i = 0; i < RB; i++) { m[i] = -INFINITY; l[i] = 0.f; acc[i] = 0.f; }
-
-    for (int t0 = 0; t0 < len_max; t0 += 128) {
-        const int lim_max = min(128, len_max - t0);
-        __syncthreads(); /* previous tile fully consumed; sq visible */
-        for (int i = threadIdx.x; i < lim_max * (VB / 4); i += 512) {
-            const int rr = i / (VB / 4), cw = i - rr * (VB / 4);
-            *reinterpret_cast<uint32_t*>(sm.tile + rr * TS + cw * 4) =
-                __ldg(reinterpret_cast<const uint32_t*>(kc + (plane + t0 + rr) * VB + cw * 4));
-        }
-        if (KV8)
-            for (int i = threadIdx.x; i < lim_max * 4; i += 512) {
-                sm.ssc[i] = ks[(plane + t0) * 4 + i];
-                sm.vssc[i] = vs[(plane + t0) * 4 + i];
-            }
-        __syncthreads();
-
-        /* ---- scores: the key of position t, converted once, against the RB rows' queries ---- */
-        float d[RB];
-#pragma unroll
-        for (int i = 0; i < RB; i++) d[i] = 0.f;
-        if (t < lim_max) {
-            const uint32_t* kw = reinterpret_cast<const uint32_t*>(sm.tile + t * TS);
-            if (KV8) {
-#pragma unroll 1
-                for (int gi = 0; gi < 4; gi++) {
-                    float pp[RB];
-#pragma unroll
-                    for (int i = 0; i < RB; i++) pp[i] = 0.f;
-#pragma unroll
-                    for (int w = 0; w < 8; w++) {
-                        const uint32_t u = s8x4_bias(kw[gi * 8 + w]);
-                        const float k0 = s8_biased_to_f32<0>(u), k1 = s8_biased_to_f32<1>(u), k2 = s8_biased_to_f32<2>(u), k3 = s8_biased_to_f32<3>(u);
-#pragma unroll
-                        for (int i = 0; i < RB; i++) {
-                            const float4 qv = reinterpret_cast<const float4*>(sm.sq[i][g])[gi * 8 + w];
-                            pp[i] = __fmaf_rn(qv.x, k0, pp[i]);
-                            pp[i] = __fmaf_rn(qv.y, k1, pp[i]);
-                            pp[i] = __fmaf_rn(qv.z, k2, pp[i]);
-                            pp[i] = __fmaf_rn(qv.w, k3, pp[i]);
-                        }
-                    }
-                    const float ksf = __half2float(sm.ssc[t * 4 + gi]);
-#pragma unroll
-                    for (int i = 0; i < RB; i++) d[i] = __fmaf_rn(pp[i], ksf, d[i]);
-                }
+    for (int i = tid; i < M * 16; i += NC + ATTN_PREFILL_PRODUCERS) { /* 16 bytes of one query's vector each, neighbouring lanes neighbouring queries */
+        const int qi = i % M, c = i / M, row = qi >> 2;
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+        if (row < rb) {
+            const __nv_bfloat16* src = a.q + ((size_t)(r0 + row) * a.q_heads + kvh * 4 + (qi & 3)) * 128 + c * 8;
+            if (wide) {
+                const uint4 x = *reinterpret_cast<const uint4*>(src);
+                w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
             } else {
-#pragma unroll 4
-                for (int w = 0; w < 64; w += 2) { /* two words = four bf16 */
-                    const uint32_t w0 = kw[w], w1 = kw[w + 1];
-                    const float k0 = bf_lo(w0), k1 = bf_hi(w0), k2 = bf_lo(w1), k3 = bf_hi(w1);
 #pragma unroll
-                    for (int i = 0; i < RB; i++) {
-                        const float4 qv = reinterpret_cast<const float4*>(sm.sq[i][g])[w >> 1];
-                        d[i] = __fmaf_rn(qv.x, k0, d[i]);
-                        d[i] = __fmaf_rn(qv.y, k1, d[i]);
-                        d[i] = __fmaf_rn(qv.z, k2, d[i]);
-                        d[i] = __fmaf_rn(qv.w, k3, d[i]);
-                    }
-                }
+                for (int j = 0; j < 4; j++)
+                    w[j] = (uint32_t)__bfloat16_as_ushort(src[2 * j]) | ((uint32_t)__bfloat16_as_ushort(src[2 * j + 1]) << 16);
             }
         }
-        /* row i of the block sees positions below len0 + i */
-        float s[RB];
 #pragma unroll
-        for (int i = 0; i < RB; i++) s[i] = (i < rb && t0 + t < len0 + i) ? d[i] : -INFINITY;
-
-        /* ---- tile max per (row, head): the 128-wide halving tree, the rows' trees side by side ---- */
-#pragma unroll
-        for (int i = 0; i < RB; i++) sm.red[i][g][t] = s[i];
-        __syncthreads();
-        if (t < 64) {
-#pragma unroll
-            for (int i = 0; i < RB; i++) sm.red[i][g][t] = fmaxf(sm.red[i][g][t], sm.red[i][g][t + 64]);
-        }
-        __syncthreads();
-        if (t < 32) {
-#pragma unroll
-            for (int i = 0; i < RB; i++) sm.red[i][g][t] = fmaxf(sm.red[i][g][t], sm.red[i][g][t + 32]);
-        }
-        __syncthreads();
-        float corr[RB], mn[RB];
-#pragma unroll
-        for (int i = 0; i < RB; i++) {
-            const float tmax = warp_tree_max(sm.red[i][g][t & 31]);
-            mn[i] = fmaxf(m[i], tmax);
-            corr[i] = (m[i] == -INFINITY) ? 0.f : expf(m[i] - mn[i]);
-        }
-        __syncthreads();
-        {
-            float vsf[4] = {1.f, 1.f, 1.f, 1.f};
-            if (KV8 && t < lim_max) {
-                const uint2 sv = *reinterpret_cast<const uint2*>(sm.vssc + t * 4);
-                const __half2 sva = *reinterpret_cast<const __half2*>(&sv.x), svb = *reinterpret_cast<const __half2*>(&sv.y);
-                vsf[0] = __low2float(sva); vsf[1] = __high2float(sva); vsf[2] = __low2float(svb); vsf[3] = __high2float(svb);
-            }
-#pragma unroll
-            for (int i = 0; i < RB; i++) {
-                const float p = (s[i] == -INFINITY) ? 0.f : expf(s[i] - mn[i]);
-                sm.red[i][g][t] = p;
-                if (KV8) {
-#pragma unroll
-                    for (int grp = 0; grp < 4; grp++) sm.spv[i][g][grp][t] = __fmul_rn(p, vsf[grp]);
-                } else {
-                    sm.spv[i][g][0][t] = p;
-                }
-            }
-        }
-        __syncthreads();
-        if (t < 64) {
-#pragma unroll
-            for (int i = 0; i < RB; i++) sm.red[i][g][t] += sm.red[i][g][t + 64];
-        }
-        __syncthreads();
-        if (t < 32) {
-#pragma unroll
-            for (int i = 0; i < RB; i++) sm.red[i][g][t] += sm.red[i][g][t + 32];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < RB; i++) {
-            const float tsum = warp_tree_sum(sm.red[i][g][t & 31]);
-            if (i < rb && t0 < len0 + i) { /* the row reaches into this tile (uniform over the CTA) */
-                l[i] = __fmaf_rn(l[i], corr[i], tsum);
-                acc[i] = __fmul_rn(acc[i], corr[i]);
-                m[i] = mn[i];
-            }
-        }
-        __syncthreads(); /* K tile no longer needed: the buffer takes V */
-        for (int i = threadIdx.x; i < lim_max * (VB / 4); i += 512) {
-            const int rr = i / (VB / 4), cw = i - rr * (VB / 4);
-            *reinterpret_cast<uint32_t*>(sm.tile + rr * TS + cw * 4) =
-                __ldg(reinterpret_cast<const uint32_t*>(vc + (plane + t0 + rr) * VB + cw * 4));
-        }
-        __syncthreads();
-
-        /* ---- value sums: the value of (position j, dimension t), converted once, into the RB rows' chains; the
-         * weights of four positions come with one 16-byte read per row ---- */
-        const int full = min(lim_max, max(0, len0 - t0)); /* positions every row of the block sees */
-        const int grp = KV8 ? (t >> 5) : 0;
-        auto value_at = [&](int j) -> float {
-            return KV8 ? s8_to_f32(reinterpret_cast<const int8_t*>(sm.tile + j * TS)[t])
-                       : bf2f(reinterpret_cast<const __nv_bfloat16*>(sm.tile + j * TS)[t]);
-        };
-        int j = 0;
-        for (; j + 4 <= full; j += 4) {
-            const float v0 = value_at(j), v1 = value_at(j + 1), v2 = value_at(j + 2), v3 = value_at(j + 3);
-#pragma unroll
-            for (int i = 0; i < RB; i++) {
-                const float4 w = *reinterpret_cast<const float4*>(&sm.spv[i][g][grp][j]);
-                acc[i] = __fmaf_rn(w.x, v0, acc[i]);
-                acc[i] = __fmaf_rn(w.y, v1, acc[i]);
-                acc[i] = __fmaf_rn(w.z, v2, acc[i]);
-                acc[i] = __fmaf_rn(w.w, v3, acc[i]);
-            }
-        }
-        for (; j < lim_max; j++) { /* the rest, and the diagonal: row i sees position t0 + j only if it lies below len0 + i */
-            const float vf = value_at(j);
-#pragma unroll
-            for (int i = 0; i < RB; i++)
-                if (i < rb && t0 + j < len0 + i) acc[i] = __fmaf_rn(sm.spv[i][g][grp][j], vf, acc[i]);
+        for (int j = 0; j < 4; j++) {
+            sm.q[c * 8 + 2 * j][qi] = __fmul_rn(bf_lo(w[j]), scale);
+            sm.q[c * 8 + 2 * j + 1][qi] = __fmul_rn(bf_hi(w[j]), scale);
         }
     }
+    __syncthreads();
+
+    if (warp >= NW) { /* ---- producers ---- */
+        if (SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        const size_t plane = (size_t)kvh * a.max_seq;
+        const unsigned char* kc = kv_payload(a.kv, r0) + a.kv.k_off + plane * VB; /* one cache for all rows of the block */
+        const unsigned char* vc = kv_payload(a.kv, r0) + a.kv.v_off + plane * VB;
+        const __half* ks = KV8 ? reinterpret_cast<const __half*>(kv_scales(a.kv, r0) + a.kv.ks_off) + plane * 4 : nullptr;
+        const __half* vs = KV8 ? reinterpret_cast<const __half*>(kv_scales(a.kv, r0) + a.kv.vs_off) + plane * 4 : nullptr;
+        const int pt = tid - NC;
+        unsigned phase = 1; /* the buffers start empty: the first waits pass at once */
+        for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1) {
+            /* rows past the last position any query sees become zero */
+            const int lim = min(128, len_max - t0);
+            if (!mbar_wait_bounded(&sm.kempty, phase, status)) return;
+            attn_prefill_keys<KV8>(sm.k, kc + (size_t)t0 * VB, pt, lim, wide);
+            if (KV8) attn_prefill_scales(sm.ksc, ks + (size_t)t0 * 4, pt, lim);
+            mbar_arrive(&sm.kfull);
+            if (!mbar_wait_bounded(&sm.vempty, phase, status)) return;
+            attn_prefill_values<KV8>(sm.v, vc + (size_t)t0 * VB, pt, lim, wide);
+            if (KV8) attn_prefill_scales(sm.vsc, vs + (size_t)t0 * 4, pt, lim);
+            mbar_arrive(&sm.vfull);
+        }
+        return;
+    }
+    if (SPLIT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+
+    /* ---- consumers ---- */
+    const int tx = lane >> 1, qg = lane & 1; /* neighbouring lanes read the same key / value: 16-byte shared reads merge pairs */
+    const int q0 = (warp * 2 + qg) * QT;     /* this thread's queries q0 .. q0 + QT - 1; query = 4 * (row in block) + head */
+    float* const pw = &sm.p[warp][qg][0][0];
+    const int flip = qg << 4;
+    float m[QT], l[QT];
+    f32x2 acc[QT][4];
 #pragma unroll
-    for (int i = 0; i < RB; i++)
-        if (i < rb) a.out[((size_t)(r0 + i) * QH + h) * 128 + t] = f2bf(__fdiv_rn(acc[i], l[i]));
+    for (int i = 0; i < QT; i++) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[i][c] = 0ull;
+    }
+    unsigned phase = 0;
+    for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1) {
+        const int lim_max = min(128, len_max - t0);
+        if (!mbar_wait_bounded(&sm.kfull, phase, status)) return;
+        /* ---- scores of QT queries x positions {4 tx .. +3, 64 + 4 tx .. +3}, two positions per packed fma ---- */
+        f32x2 d[QT][4];
+#pragma unroll
+        for (int i = 0; i < QT; i++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) d[i][c] = 0ull;
+        if (KV8) {
+#pragma unroll 1
+            for (int gi = 0; gi < 4; gi++) {
+                f32x2 pp[QT][4];
+#pragma unroll
+                for (int i = 0; i < QT; i++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) pp[i][c] = 0ull;
+#pragma unroll 4
+                for (int e = gi * 32; e < gi * 32 + 32; e++) attn_prefill_dim<QT>(sm.k[e], sm.q[e] + q0, tx, pp);
+                const uint2 ha = *reinterpret_cast<const uint2*>(&sm.ksc[gi][tx * 4]), hb = *reinterpret_cast<const uint2*>(&sm.ksc[gi][64 + tx * 4]);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const f32x2 f = half2_to_f32x2(c == 0 ? ha.x : c == 1 ? ha.y : c == 2 ? hb.x : hb.y);
+#pragma unroll
+                    for (int i = 0; i < QT; i++) d[i][c] = ffma2_of(pp[i][c], f, d[i][c]);
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (int e = 0; e < 128; e++) attn_prefill_dim<QT>(sm.k[e], sm.q[e] + q0, tx, d);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.kempty);
+
+        /* ---- soft-max of the tile, one query after another; the query's eight weights of this thread go to shared memory ---- */
+        float corr[QT];
+#pragma unroll
+        for (int i = 0; i < QT; i++) {
+            const int row = (q0 + i) >> 2;
+            const int see = row < rb ? len0 + row - t0 : 0; /* positions of the tile this query sees (may be <= 0 or > 128) */
+            float s[8];
+#pragma unroll
+            for (int c = 0; c < 4; c++) unpack2(d[i][c], s[2 * c], s[2 * c + 1]);
+            float mx = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const int pos = (c >> 2) * 64 + tx * 4 + (c & 3);
+                if (pos >= see) s[c] = -INFINITY;
+                mx = fmaxf(mx, s[c]);
+            }
+#pragma unroll
+            for (int off = 16; off > 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(S2P_FULL_MASK, mx, off));
+            const float mn = fmaxf(m[i], mx);
+            corr[i] = (m[i] == -INFINITY) ? 0.f : expf(m[i] - mn);
+#pragma unroll
+            for (int c = 0; c < 8; c++) s[c] = (s[c] == -INFINITY) ? 0.f : expf(s[c] - mn);
+            *reinterpret_cast<float4*>(pw + i * 128 + ((tx * 4) ^ flip)) = make_float4(s[0], s[1], s[2], s[3]);
+            *reinterpret_cast<float4*>(pw + i * 128 + 64 + ((tx * 4) ^ flip)) = make_float4(s[4], s[5], s[6], s[7]);
+            /* the 128-wide halving tree: 64 in the thread; 32 (lane bit 3) and 16 (bit 2) while handing half of the
+             * four sums away each time; 8 and 4 (bits 1, 0); the last two levels pair what those lanes kept */
+            const float u0 = s[0] + s[4], u1 = s[1] + s[5], u2 = s[2] + s[6], u3 = s[3] + s[7];
+            const bool b3 = (tx & 8) != 0, b2 = (tx & 4) != 0;
+            const float g0 = __shfl_xor_sync(S2P_FULL_MASK, b3 ? u0 : u2, 16), g1 = __shfl_xor_sync(S2P_FULL_MASK, b3 ? u1 : u3, 16);
+            const float k0 = (b3 ? u2 : u0) + g0, k1 = (b3 ? u3 : u1) + g1;   /* sums 0,1 or 2,3 */
+            const float g2 = __shfl_xor_sync(S2P_FULL_MASK, b2 ? k0 : k1, 8);
+            float k = (b2 ? k1 : k0) + g2;                                    /* sum (b3, b2) */
+            k += __shfl_xor_sync(S2P_FULL_MASK, k, 4);
+            k += __shfl_xor_sync(S2P_FULL_MASK, k, 2);
+            k += __shfl_xor_sync(S2P_FULL_MASK, k, 16);                       /* level 2: sums 0 + 2, 1 + 3 */
+            k += __shfl_xor_sync(S2P_FULL_MASK, k, 8);                        /* level 1 */
+            if (see > 0) { /* the query reaches into this tile */
+                l[i] = __fmaf_rn(l[i], corr[i], k);
+                m[i] = mn;
+            } else {
+                corr[i] = 1.f;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < QT; i++) {
+            const f32x2 cc = pack2(corr[i], corr[i]);
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[i][c] = fmul2(acc[i][c], cc);
+        }
+        __syncwarp();
+
+        /* ---- value sums of QT queries x dimensions 8 tx .. +7 (one scale group), two dimensions per packed fma.
+         * Positions a query does not see have weight 0 and finite values: their fma leaves the sum as it is. ---- */
+        const int n4 = (lim_max + 3) & ~3;
+        if (!mbar_wait_bounded(&sm.vfull, phase, status)) return;
+#pragma unroll 1
+        for (int j = 0; j < n4; j += 4) {
+            f32x2 w01[QT], w23[QT];
+#pragma unroll
+            for (int i = 0; i < QT; i++) {
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(pw + i * 128 + (j ^ flip));
+                w01[i] = w.x; w23[i] = w.y;
+            }
+            if (KV8) {
+                const uint2 h = *reinterpret_cast<const uint2*>(&sm.vsc[tx >> 2][j]);
+                const f32x2 f01 = half2_to_f32x2(h.x), f23 = half2_to_f32x2(h.y);
+#pragma unroll
+                for (int i = 0; i < QT; i++) { w01[i] = fmul2(w01[i], f01); w23[i] = fmul2(w23[i], f23); }
+            }
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+                const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(&sm.v[j + jj][tx * 4]);
+                const ulonglong2 vb = *reinterpret_cast<const ulonglong2*>(&sm.v[j + jj][64 + tx * 4]);
+#pragma unroll
+                for (int i = 0; i < QT; i++) {
+                    float lo, hi;
+                    unpack2(jj < 2 ? w01[i] : w23[i], lo, hi);
+                    const float w = jj & 1 ? hi : lo;
+                    const f32x2 ww = pack2(w, w);
+                    ffma2(acc[i][0], ww, va.x);
+                    ffma2(acc[i][1], ww, va.y);
+                    ffma2(acc[i][2], ww, vb.x);
+                    ffma2(acc[i][3], ww, vb.y);
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.vempty);
+    }
+#pragma unroll
+    for (int i = 0; i < QT; i++) {
+        const int qi = q0 + i, row = qi >> 2;
+        if (row >= rb) continue;
+        uint32_t o[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            float lo, hi;
+            unpack2(acc[i][c], lo, hi);
+            o[c] = (uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(lo, l[i]))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(hi, l[i]))) << 16);
+        }
+        __nv_bfloat16* dst = a.out + ((size_t)(r0 + row) * a.q_heads + kvh * 4 + (qi & 3)) * 128 + tx * 8;
+        if (wide) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; c++) dst[c] = __ushort_as_bfloat16((unsigned short)(c & 1 ? o[c >> 1] >> 16 : o[c >> 1] & 0xffffu));
+        }
+    }
 }
 
 }  // namespace s2p

@@ -50,9 +50,6 @@ static_assert(sizeof(SamplerSmem<MEGA_WORKERS>) <= MEGA_MIN_WORK, "sampler scrat
 static_assert(sizeof(MegaCopyCmd) == 64, "one copy command per 64-byte line");
 
 __device__ __forceinline__ bool cta_sync_and(bool p) { return __syncthreads_and(p ? 1 : 0) != 0; }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 /* order-preserving arg-max key: larger value first, then lower index
  * (src/slowar/kernels.cu:1326-1357); -0 counts as +0 */

@@ -16,6 +16,8 @@
 
 namespace s2p {
 
+int device_sm_count(); /* gemv.cu */
+
 static inline int grid_for(int64_t total, int threads) {
     int64_t b = (total + threads - 1) / threads;
     if (b > 148 * 16) b = 148 * 16;
@@ -250,22 +252,63 @@ __global__ void __launch_bounds__(512) k_attn_single(AttnArgs a) {
 }
 
 /* prompt slices: consecutive rows of one session go to the row-block kernel (attn_prefill.cuh) */
-template <bool KV8, int ATTN_PREFILL_ROWS>
+static __device__ int g_attn_prefill_status; /* code of a bounded wait that gave up (pipe.cuh), 0 otherwise */
+
+template <bool KV8, int QT, int NW>
 static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, cudaStream_t st) {
-    static bool attr_set[64] = {false};
-    constexpr size_t smem = sizeof(AttnPrefillSmem<KV8, ATTN_PREFILL_ROWS>);
+    static int* status[64] = {nullptr};
+    constexpr size_t smem = sizeof(AttnPrefillSmem<KV8, QT, NW>);
+    static_assert(smem <= 227 * 1024, "shared memory of a CTA");
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!attr_set[dev]) {
-        e = cudaFuncSetAttribute(k_attn_prefill<KV8, ATTN_PREFILL_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!status[dev]) {
+        e = cudaFuncSetAttribute(k_attn_prefill<KV8, QT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        attr_set[dev] = true;
+        int* p = nullptr;
+        e = cudaGetSymbolAddress((void**)&p, g_attn_prefill_status);
+        if (e != cudaSuccess) return e;
+        status[dev] = p;
     }
-    dim3 grid((unsigned)((rows + ATTN_PREFILL_ROWS - 1) / ATTN_PREFILL_ROWS), (unsigned)a->kv_heads);
-    k_attn_prefill<KV8, ATTN_PREFILL_ROWS><<<grid, 512, smem, st>>>(*a, rows);
+    uintptr_t all = (uintptr_t)a->q | (uintptr_t)a->out | (uintptr_t)a->kv.base0 | a->kv.k_off | a->kv.v_off;
+    if (a->kv8) all |= (uintptr_t)a->kv.sbase0 | a->kv.ks_off | a->kv.vs_off;
+    constexpr int RB = QT * NW / 2;
+    dim3 grid((unsigned)((rows + RB - 1) / RB), (unsigned)a->kv_heads);
+    k_attn_prefill<KV8, QT, NW><<<grid, 32 * NW + ATTN_PREFILL_PRODUCERS, smem, st>>>(*a, rows, (all & 15) == 0, status[dev]);
     return cudaGetLastError();
+}
+
+/* A CTA fills an SM whatever its size, so a launch takes (waves of CTAs) x (time per 128-position tile): 7.5 us with blocks of
+ * 4 rows, 10.1 with 8, 15.2 with 16, 20.0 with 24 (INT8 cache; bf16 within 10 %).  Large blocks are the cheapest per row (0.83 us
+ * against 1.9), small ones fill the GPU when the slice is short.  The single-block kernel before this one: 9 us for blocks
+ * of 4.  Measured (us, before -> now): 2048 rows after 6052 positions 12595 -> 5466, 512 after none 162 -> 112, 77 after
+ * 1024 154 -> 95, 20 after 2000 157 -> 120. */
+template <bool KV8>
+static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, cudaStream_t st) {
+    static const int block_rows[4] = {24, 16, 8, 4}, tile_ns[4] = {20000, 15200, 10100, 7500};
+    int best = 0;
+    long long best_cost = 0;
+    for (int v = 0; v < 4; v++) {
+        const int ctas = (rows + block_rows[v] - 1) / block_rows[v] * a->kv_heads;
+        const long long cost = (long long)((ctas + device_sm_count() - 1) / device_sm_count()) * tile_ns[v];
+        if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
+    }
+    switch (best) {
+    case 0: return launch_attn_prefill<KV8, 4, 12>(a, rows, st);
+    case 1: return launch_attn_prefill<KV8, 4, 8>(a, rows, st);
+    case 2: return launch_attn_prefill<KV8, 2, 8>(a, rows, st);
+    default: return launch_attn_prefill<KV8, 2, 4>(a, rows, st);
+    }
+}
+
+/* copies the status word of the slices' attention to `host` (pinned) in stream order */
+cudaError_t attn_prefill_status(int* host, cudaStream_t st) {
+    return cudaMemcpyFromSymbolAsync(host, g_attn_prefill_status, sizeof(int), 0, cudaMemcpyDeviceToHost, st);
+}
+cudaError_t attn_prefill_reset(cudaStream_t st) {
+    static const int zero = 0;
+    return cudaMemcpyToSymbolAsync(g_attn_prefill_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, st);
 }
 
 cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st) {
@@ -273,10 +316,7 @@ cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st) {
     if (a->q_heads != a->kv_heads * 4 || a->head_dim != 128) return cudaErrorInvalidValue;
     if (rows >= 2 && !a->pos_arr && a->pos_row_step == 1 && !a->kv.bases && a->kv.row_stride == 0 &&
         (!a->kv8 || (!a->kv.sbases && a->kv.srow_stride == 0)))
-        /* blocks of 4 rows: 64 registers, two CTAs per SM; 8 rows amortise the tiles further but leave one CTA per
-         * SM (measured 1.15 s against 1.14 s on an 8192-token prompt, 14.6 against 14.3 ms on 512 tokens), 2 rows
-         * are 30 % slower */
-        return a->kv8 ? launch_attn_prefill<true, 4>(a, rows, st) : launch_attn_prefill<false, 4>(a, rows, st);
+        return a->kv8 ? launch_attn_prefill_rows<true>(a, rows, st) : launch_attn_prefill_rows<false>(a, rows, st);
     dim3 grid((unsigned)rows, (unsigned)a->kv_heads);
     if (a->kv8) k_attn_single<true><<<grid, 512, 0, st>>>(*a);
     else k_attn_single<false><<<grid, 512, 0, st>>>(*a);

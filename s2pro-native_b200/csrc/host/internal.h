@@ -92,6 +92,7 @@ struct s2p_model {
     void *d_up, *h_up;
     size_t out_bytes, off_sem, off_ocodes, off_eos;
     void *d_out, *h_out;
+    int* h_prefill_status;          /* pinned copy of the prompt attention's status word */
     /* one executable graph per steady batch size */
     cudaGraphExec_t gexec[S2P_MAX_BATCH + 1];
     unsigned char gready[S2P_MAX_BATCH + 1];

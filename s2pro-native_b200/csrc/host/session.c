@@ -315,7 +315,13 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
     S2P_LAUNCH(m, rms_norm(BF(m->sx) + (size_t)(n_ids - 1) * S2P_DIM, m->final_norm.data, s->pending_hidden.data, 1,
                           S2P_DIM, S2P_NORM_EPS, st));
     dump_bf16("backbone_final_norm", s->pending_hidden.data, S2P_DIM, st);
+    S2P_CUDA_TRY(attn_prefill_status(m->h_prefill_status, st));
     S2P_CUDA_TRY(cudaStreamSynchronize(st));
+    if (*m->h_prefill_status != 0) {
+        fprintf(stderr, "[s2pro] prompt attention gave up on a bounded wait (code %d); the slice is lost\n", *m->h_prefill_status);
+        S2P_CUDA_TRY(attn_prefill_reset(st));
+        return S2P_ERR_INTERNAL;
+    }
     if (n_ids > S2P_INT8_GEMV_MAX_M && m->mode == S2P_GEMM_INT8 && s2p_env_is_one("S2P_PREFILL_TC")) {
         /* the slice's linears ran on the tensor-core kernel: a bounded wait that gave up inside it left a code */
         int sk = 0;

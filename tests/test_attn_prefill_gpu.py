@@ -1,0 +1,47 @@
+"""The row-block attention of prompt slices against the single-row kernel, bit for bit."""
+import ctypes as C
+
+import pytest
+
+from _internal_abi import AttnArgs
+
+pytestmark = pytest.mark.gpu
+QH, KVH, HD = 32, 8, 128
+
+
+@pytest.mark.parametrize("kv8", [0, 1])
+@pytest.mark.parametrize("shift", [0, 4])
+@pytest.mark.parametrize("pos0,rows", [(0, 2), (0, 129), (127, 2), (126, 5), (250, 73), (128, 128), (1000, 21), (0, 300), (40, 460), (3000, 450)])
+def test_rows_of_a_slice_equal_single_rows(testlib, kv8, shift, pos0, rows):
+    """All four block sizes (their choice depends on the slice's length), ragged last blocks, tiles cut by the diagonal,
+    and caches that are aligned to 4 bytes only."""
+    import torch
+    testlib.attn_single.argtypes = [C.POINTER(AttnArgs), C.c_int, C.c_void_p]
+    g = torch.Generator(device="cuda").manual_seed(pos0 * 7 + rows)
+    max_seq = (pos0 + rows + 64) // 64 * 64
+    n = KVH * max_seq
+    raw = torch.zeros(2 * n * HD * (1 if kv8 else 2) + 64, dtype=torch.uint8, device="cuda")
+    scales = torch.full((2 * n * 4 + 32,), float("nan"), dtype=torch.float16, device="cuda")
+    body = raw[shift:shift + raw.numel() - 64]
+    if kv8:
+        body.copy_(torch.randint(-127, 128, (2 * n * HD,), dtype=torch.int8, device="cuda", generator=g).view(torch.uint8))
+        live = scales[shift // 2:shift // 2 + 2 * n * 4].view(2, KVH, max_seq, 4)
+        live[:, :, :pos0 + rows] = (torch.rand(2, KVH, pos0 + rows, 4, device="cuda", generator=g) * 0.02 + 0.001).half()
+    else:
+        v = torch.randn(2, KVH, max_seq, HD, device="cuda", generator=g).bfloat16()
+        v[:, :, pos0 + rows:] = float("nan")  # nothing past the last position may be read into a result
+        body.copy_(v.flatten().view(torch.uint8))
+    q = torch.randn(rows, QH * HD, device="cuda", generator=g).bfloat16()
+    out, ref = torch.zeros_like(q), torch.zeros_like(q)
+    a = AttnArgs()
+    a.q_heads, a.kv_heads, a.max_seq, a.kv8, a.head_dim, a.pos_row_step = QH, KVH, max_seq, kv8, HD, 1
+    a.kv.base0, a.kv.k_off, a.kv.v_off = raw.data_ptr() + shift, 0, n * HD * (1 if kv8 else 2)
+    a.kv.sbase0, a.kv.ks_off, a.kv.vs_off = scales.data_ptr() + shift, 0, n * 8
+    a.q, a.out, a.pos0 = q.data_ptr(), out.data_ptr(), pos0
+    assert testlib.attn_single(C.byref(a), rows, None) == 0
+    for r in range(rows):
+        a.q, a.out, a.pos0 = q[r].data_ptr(), ref[r].data_ptr(), pos0 + r
+        assert testlib.attn_single(C.byref(a), 1, None) == 0
+    torch.cuda.synchronize()
+    assert not torch.isnan(ref.float()).any()
+    assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
