@@ -39,6 +39,8 @@ void s2p_sampler_init(s2p_sampler* sp, const s2p_sampling_cfg* cfg, uint64_t ent
 
 typedef enum { SESS_NEW = 0, SESS_PREFILLED, SESS_DECODING, SESS_FINISHED } sess_state;
 
+#define S2P_POOL_MAX 64
+
 struct s2p_model {
     s2p_gemm_mode mode;
     int kv8, embed_i8_only, head_full;
@@ -65,6 +67,9 @@ struct s2p_model {
     unsigned long long* d_mega_trace; /* [stages][4] clock stamps, when S2P_TICK_TRACE=1 */
     int32_t* mega_types;        /* host copy of the stage kinds */
     cudaStream_t stream;
+    /* device blocks of closed sessions, for the next ones (session.c) */
+    void* pool[S2P_POOL_MAX];
+    int n_pool;
 
     /* weights */
     s2p_tensor embed, embed_i8, embed_scale;
@@ -109,14 +114,17 @@ struct s2p_session {
     s2p_model* m;
     sess_state state;
     int kv_len;
-    s2p_tensor kv;  /* [n_slow][16][ctx][128] bf16 or i8 */
-    s2p_tensor kvs; /* kv8: [n_slow][16][ctx][4] f16 */
-    s2p_tensor pending_hidden;
+    void* block;          /* the session's device memory; the pointers below lie in it */
+    void* kv;             /* [n_slow][16][ctx][128] bf16 or i8 */
+    void* kvs;            /* kv8: [n_slow][16][ctx][4] f16, else NULL */
+    void* pending_hidden; /* [2560] bf16 */
     int64_t prev_token;
     int32_t prev_codes[S2P_NUM_CODEBOOKS];
     void* dsamp; /* device SamplerState */
     s2p_sampler sampler;
 };
+
+void s2p_session_pool_clear(s2p_model* m);
 
 /* model.c helpers used by session.c */
 size_t s2p_kv_vec_bytes(const s2p_model* m);

@@ -335,6 +335,7 @@ static void free_layer(s2p_layer* L) {
 void s2p_model_free(s2p_model* m) {
     if (!m) return;
     if (m->stream) cudaStreamSynchronize(m->stream);
+    s2p_session_pool_clear(m);
     for (int b = 0; b <= S2P_MAX_BATCH; b++)
         if (m->gready[b]) cudaGraphExecDestroy(m->gexec[b]);
     for (int l = 0; l < S2P_SLOW_LAYERS; l++) free_layer(&m->slow[l]);

@@ -63,6 +63,41 @@ static void dump_bf16(const char* name, const void* dev, int64_t n, cudaStream_t
 }
 
 /* ---- sessions ---------------------------------------------------------------- */
+/* A session's device memory is one block: KV payload, KV scales, pending hidden state, sampler state.  Blocks of closed
+ * sessions are kept for the next ones, because the driver's calls cost more than a short prompt: cudaMalloc + cudaFree of
+ * the four former buffers took 1.5 ms per request at a 2048-token context and 90 ms (mostly the unmapping in cudaFree) at
+ * 9216 tokens.  The pool belongs to the model and holds at most S2P_POOL_BYTES (or one block, if a block is larger): enough
+ * for the turnover of a server, 1/64 of the GPU.  It is given back when the model is freed. */
+#define S2P_POOL_BYTES ((size_t)2816 << 20)
+
+void s2p_session_pool_clear(s2p_model* m) {
+    while (m->n_pool > 0) cudaFree(m->pool[--m->n_pool]);
+}
+
+static size_t block_align(size_t v) { return (v + 255) & ~(size_t)255; }
+
+/* byte offsets of the four parts; returns the block's size */
+static size_t session_block(const s2p_model* m, size_t* scales, size_t* hidden, size_t* samp) {
+    const size_t planes = (size_t)m->n_slow * S2P_KV_PLANES_PER_LAYER;
+    *scales = block_align(planes * s2p_kv_plane_bytes(m));
+    *hidden = *scales + block_align(m->kv8 ? planes * s2p_kvs_plane_bytes(m) : 0);
+    *samp = *hidden + block_align((size_t)S2P_DIM * 2);
+    return *samp + block_align(sizeof(SamplerState));
+}
+
+static s2p_status block_take(s2p_model* m, size_t bytes, void** out) {
+    if (m->n_pool > 0) { *out = m->pool[--m->n_pool]; return S2P_OK; }
+    const cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaSuccess) return S2P_OK;
+    fprintf(stderr, "[s2pro] cudaMalloc(%zu) for a session failed: %s\n", bytes, cudaGetErrorString(e));
+    return e == cudaErrorMemoryAllocation ? S2P_ERR_OOM : S2P_ERR_CUDA;
+}
+
+static void block_give(s2p_model* m, void* block, size_t bytes) {
+    if (m->n_pool < S2P_POOL_MAX && (m->n_pool == 0 || (size_t)(m->n_pool + 1) * bytes <= S2P_POOL_BYTES)) m->pool[m->n_pool++] = block;
+    else cudaFree(block);
+}
+
 s2p_status s2p_session_create(s2p_model* m, const s2p_sampling_cfg* cfg, s2p_session** out) {
     if (!m || !out) return S2P_ERR_INVALID;
     *out = NULL;
@@ -71,17 +106,14 @@ s2p_status s2p_session_create(s2p_model* m, const s2p_sampling_cfg* cfg, s2p_ses
     if (!s) return S2P_ERR_OOM;
     s->m = m;
     s->state = SESS_NEW;
-    const int64_t kv_shape[4] = {m->n_slow, S2P_KV_PLANES_PER_LAYER, m->ctx_len, S2P_HEAD_DIM};
-    s2p_status rc = s2p_tensor_device_alloc(&s->kv, m->kv8 ? S2P_DT_I8 : S2P_DT_BF16, 4, kv_shape);
-    if (rc == S2P_OK && m->kv8) {
-        const int64_t sc_shape[4] = {m->n_slow, S2P_KV_PLANES_PER_LAYER, m->ctx_len, S2P_HEAD_DIM / 32};
-        rc = s2p_tensor_device_alloc(&s->kvs, S2P_DT_F16, 4, sc_shape);
-    }
+    size_t o_scales, o_hidden, o_samp;
+    const size_t bytes = session_block(m, &o_scales, &o_hidden, &o_samp);
+    s2p_status rc = block_take(m, bytes, &s->block);
     if (rc == S2P_OK) {
-        const int64_t h_shape[1] = {S2P_DIM};
-        rc = s2p_tensor_device_alloc(&s->pending_hidden, S2P_DT_BF16, 1, h_shape);
-    }
-    if (rc == S2P_OK) {
+        s->kv = s->block;
+        s->kvs = m->kv8 ? (char*)s->block + o_scales : NULL;
+        s->pending_hidden = (char*)s->block + o_hidden;
+        s->dsamp = (char*)s->block + o_samp;
         struct timespec ts;
         clock_gettime(CLOCK_MONOTONIC, &ts);
         const uint64_t entropy = ((uint64_t)ts.tv_sec * 1000000000ULL + (uint64_t)ts.tv_nsec) ^ (uint64_t)(uintptr_t)s;
@@ -95,15 +127,11 @@ s2p_status s2p_session_create(s2p_model* m, const s2p_sampling_cfg* cfg, s2p_ses
         hst.window = s->sampler.window;
         hst.seeded = s->sampler.seeded;
         hst.seed31 = s->sampler.seed31;
-        if (cudaMalloc(&s->dsamp, sizeof(hst)) != cudaSuccess ||
-            cudaMemcpy(s->dsamp, &hst, sizeof(hst), cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = S2P_ERR_CUDA;
+        /* pageable source: staged by the time the call returns */
+        if (cudaMemcpyAsync(s->dsamp, &hst, sizeof(hst), cudaMemcpyHostToDevice, m->stream) != cudaSuccess) rc = S2P_ERR_CUDA;
     }
     if (rc != S2P_OK) {
-        if (s->dsamp) cudaFree(s->dsamp);
-        s2p_tensor_free(&s->kv);
-        s2p_tensor_free(&s->kvs);
-        s2p_tensor_free(&s->pending_hidden);
+        if (s->block) cudaFree(s->block);
         free(s);
         return rc;
     }
@@ -114,14 +142,10 @@ s2p_status s2p_session_create(s2p_model* m, const s2p_sampling_cfg* cfg, s2p_ses
 
 void s2p_session_destroy(s2p_session* s) {
     if (!s) return;
-    if (s->m) {
-        cudaStreamSynchronize(s->m->stream);
-        s->m->n_sessions--;
-    }
-    s2p_tensor_free(&s->kv);
-    s2p_tensor_free(&s->kvs);
-    s2p_tensor_free(&s->pending_hidden);
-    if (s->dsamp) cudaFree(s->dsamp);
+    size_t o_scales, o_hidden, o_samp;
+    cudaStreamSynchronize(s->m->stream);
+    s->m->n_sessions--;
+    block_give(s->m, s->block, session_block(s->m, &o_scales, &o_hidden, &o_samp));
     free(s);
 }
 
@@ -258,8 +282,8 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
     if (total_mask != total_t) return S2P_ERR_INVALID;
 
     cudaStream_t st = m->stream;
-    /* caller buffers are pageable: synchronous copies */
-    S2P_CUDA_TRY(cudaMemcpy(m->sids.data, ids, (size_t)n_ids * sizeof(int64_t), cudaMemcpyHostToDevice));
+    /* the caller's buffers may be pageable (staged by the time the call returns) or pinned (read until the sync below) */
+    S2P_CUDA_TRY(cudaMemcpyAsync(m->sids.data, ids, (size_t)n_ids * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     int part_start[64];
     size_t part_off[64];
     {
@@ -268,13 +292,16 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
         for (int p = 0; p < n_parts; p++) {
             while (cur < n_ids && !vq_mask[cur]) cur++;
             const int T = parts[p].T;
-            if (cur + T > n_ids) return S2P_ERR_INVALID;
-            for (int t = 0; t < T; t++)
-                if (!vq_mask[cur + t]) return S2P_ERR_INVALID; /* a part must cover one unbroken masked run */
+            int whole = cur + T <= n_ids;
+            for (int t = 0; whole && t < T; t++) whole = vq_mask[cur + t] != 0;
+            if (!whole) { /* a part must cover one unbroken masked run */
+                cudaStreamSynchronize(st);
+                return S2P_ERR_INVALID;
+            }
             part_start[p] = cur;
             part_off[p] = off;
-            S2P_CUDA_TRY(cudaMemcpy((int32_t*)m->svq.data + off, parts[p].codes,
-                                    (size_t)S2P_NUM_CODEBOOKS * T * sizeof(int32_t), cudaMemcpyHostToDevice));
+            S2P_CUDA_TRY(cudaMemcpyAsync((int32_t*)m->svq.data + off, parts[p].codes,
+                                         (size_t)S2P_NUM_CODEBOOKS * T * sizeof(int32_t), cudaMemcpyHostToDevice, st));
             off += (size_t)S2P_NUM_CODEBOOKS * T;
             cur += T;
         }
@@ -295,8 +322,8 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
     layer_ctx c;
     memset(&c, 0, sizeof(c));
     c.rows = n_ids;
-    c.kv.base0 = s->kv.data;
-    c.kv.sbase0 = s->kvs.data;
+    c.kv.base0 = s->kv;
+    c.kv.sbase0 = s->kvs;
     c.max_seq = m->ctx_len;
     c.kv8 = m->kv8;
     c.pos0 = pos0;
@@ -312,9 +339,9 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
         }
     }
     /* the final-normed LAST hidden is what frame 0 samples from and what primes the fast-AR */
-    S2P_LAUNCH(m, rms_norm(BF(m->sx) + (size_t)(n_ids - 1) * S2P_DIM, m->final_norm.data, s->pending_hidden.data, 1,
+    S2P_LAUNCH(m, rms_norm(BF(m->sx) + (size_t)(n_ids - 1) * S2P_DIM, m->final_norm.data, s->pending_hidden, 1,
                           S2P_DIM, S2P_NORM_EPS, st));
-    dump_bf16("backbone_final_norm", s->pending_hidden.data, S2P_DIM, st);
+    dump_bf16("backbone_final_norm", s->pending_hidden, S2P_DIM, st);
     S2P_CUDA_TRY(attn_prefill_status(m->h_prefill_status, st));
     S2P_CUDA_TRY(cudaStreamSynchronize(st));
     if (*m->h_prefill_status != 0) {
@@ -352,17 +379,17 @@ static s2p_status kv_blob_copy(s2p_session* s, void* blob, int n_tokens, int sav
     const size_t planes = (size_t)m->n_slow * S2P_KV_PLANES_PER_LAYER;
     const size_t width = (size_t)n_tokens * s2p_kv_vec_bytes(m), pitch = s2p_kv_plane_bytes(m);
     if (save)
-        S2P_CUDA_TRY(cudaMemcpy2DAsync(blob, width, s->kv.data, pitch, width, planes, cudaMemcpyDeviceToDevice, m->stream));
+        S2P_CUDA_TRY(cudaMemcpy2DAsync(blob, width, s->kv, pitch, width, planes, cudaMemcpyDeviceToDevice, m->stream));
     else
-        S2P_CUDA_TRY(cudaMemcpy2DAsync(s->kv.data, pitch, blob, width, width, planes, cudaMemcpyDeviceToDevice, m->stream));
+        S2P_CUDA_TRY(cudaMemcpy2DAsync(s->kv, pitch, blob, width, width, planes, cudaMemcpyDeviceToDevice, m->stream));
     if (m->kv8) {
         char* sblob = (char*)blob + planes * width;
         const size_t swidth = (size_t)n_tokens * (S2P_HEAD_DIM / 32) * 2, spitch = s2p_kvs_plane_bytes(m);
         if (save)
-            S2P_CUDA_TRY(cudaMemcpy2DAsync(sblob, swidth, s->kvs.data, spitch, swidth, planes, cudaMemcpyDeviceToDevice,
+            S2P_CUDA_TRY(cudaMemcpy2DAsync(sblob, swidth, s->kvs, spitch, swidth, planes, cudaMemcpyDeviceToDevice,
                                            m->stream));
         else
-            S2P_CUDA_TRY(cudaMemcpy2DAsync(s->kvs.data, spitch, sblob, swidth, swidth, planes, cudaMemcpyDeviceToDevice,
+            S2P_CUDA_TRY(cudaMemcpy2DAsync(s->kvs, spitch, sblob, swidth, swidth, planes, cudaMemcpyDeviceToDevice,
                                            m->stream));
     }
     S2P_CUDA_TRY(cudaStreamSynchronize(m->stream));
@@ -537,7 +564,7 @@ static s2p_status tick_general(s2p_model* m, s2p_session* const* act, int bd, in
         S2P_LAUNCH(m, rms_norm(m->sx.data, m->final_norm.data, m->shidden.data, bd, S2P_DIM, S2P_NORM_EPS, st));
     }
     for (int b = bd; b < nact; b++) /* freshly prefilled rows sample from their stashed hidden (eager only) */
-        S2P_CUDA_TRY(cudaMemcpyAsync(BF(m->shidden) + (size_t)b * S2P_DIM, act[b]->pending_hidden.data,
+        S2P_CUDA_TRY(cudaMemcpyAsync(BF(m->shidden) + (size_t)b * S2P_DIM, act[b]->pending_hidden,
                                      (size_t)S2P_DIM * 2, cudaMemcpyDeviceToDevice, st));
     S2P_TRY(head_and_sample(m, &d, nact, 1));
     S2P_TRY(fast_frame_general(m, &d, nact, 1));
@@ -580,7 +607,7 @@ static s2p_status tick_fused_b1(s2p_model* m, s2p_session* const* act, int decod
         }
         S2P_LAUNCH(m, rms_norm(m->sx.data, m->final_norm.data, m->shidden.data, 1, S2P_DIM, S2P_NORM_EPS, st));
     } else {
-        S2P_CUDA_TRY(cudaMemcpyAsync(m->shidden.data, act[0]->pending_hidden.data, (size_t)S2P_DIM * 2,
+        S2P_CUDA_TRY(cudaMemcpyAsync(m->shidden.data, act[0]->pending_hidden, (size_t)S2P_DIM * 2,
                                      cudaMemcpyDeviceToDevice, st));
         S2P_CUDA_TRY(cudaMemsetAsync(m->fkeys, 0, 9 * sizeof(unsigned long long), st));
     }
@@ -989,8 +1016,8 @@ s2p_status s2p_model_batch_next_frame(s2p_model* m, s2p_session** sess, int n, i
         for (int b = 0; b < nact; b++) {
             s2p_session* s = act[b];
             samp[b] = s->dsamp;
-            kvb[b] = s->kv.data;
-            kvsb[b] = s->kvs.data;
+            kvb[b] = s->kv;
+            kvsb[b] = s->kvs;
             if (b < bd) {
                 ids[b] = s->prev_token;
                 pos[b] = s->kv_len;
