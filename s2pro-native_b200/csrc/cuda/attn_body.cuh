@@ -104,14 +104,14 @@ __device__ void attn_decode_cta(const AttnArgs& a, const AttnPrep& pz, int row, 
         const int h = kvh * 4 + g;
         float v;
         if (PREP) {
+            float c, s; /* the angle functions run while the projection may still be on its way */
+            rope_cs(t >> 1, pos, pz.rope_base, c, s);
             v = prep_load(pz, (size_t)row * (QH + 2 * KVH) * 128 + (size_t)h * 128 + t);
             if (pz.q_norm) {
                 const float tot = head_tree_sum(__fmaf_rn(v, v, 0.f), red, g, t);
                 const float inv = rsqrtf(__fdiv_rn(tot, 128.0f) + pz.eps);
                 v = bf16_round(__fmul_rn(__fmul_rn(v, inv), bf2f(pz.q_norm[t])));
             }
-            float c, s;
-            rope_cs(t >> 1, pos, pz.rope_base, c, s);
             const float other = __shfl_xor_sync(S2P_FULL_MASK, v, 1);
             v = rope_elem(t, v, other, c, s);
         } else {
