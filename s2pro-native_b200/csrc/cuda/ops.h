@@ -288,7 +288,13 @@ cudaError_t embed_rows_i8(const void* table, const float* scales, const int64_t*
 cudaError_t vq_embed_add(const void* cb_table, const int32_t* codes_dev, int T, void* rows, cudaStream_t st);
 cudaError_t scale_div(void* x, int64_t n, float divisor, cudaStream_t st);
 cudaError_t scale_rows_masked(void* x, const uint8_t* mask, int rows, int dim, float scale, cudaStream_t st);
-cudaError_t embed_codes(const void* table, const int32_t* codes, void* out, int rows, cudaStream_t st);
+/* rows of the model width, all 16-byte aligned: x += add, then y = norm(x) with gain w (w NULL: no norm) */
+cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st);
+/* x = src, y = norm(x) */
+cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st);
+/* x = table[code], y = norm(x); the codes are given, or the arg-max of each row of `logits`, which also goes to codes_out */
+cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logits, int32_t* codes_out, void* x, const void* w,
+                       void* y, int rows, cudaStream_t st);
 cudaError_t argmax_rows(const void* logits, int32_t* ids, int rows, int vocab, cudaStream_t st);
 cudaError_t pack_frame(const int32_t* stage, int rows, int32_t* codes, cudaStream_t st);
 

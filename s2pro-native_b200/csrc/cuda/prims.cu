@@ -9,6 +9,7 @@
  */
 #include <math.h>
 #include "common.cuh"
+#include "gemv.cuh"
 #include "headops.cuh"
 #include "ops.h"
 #include "attn_prefill.cuh"
@@ -39,6 +40,95 @@ __global__ void __launch_bounds__(256) k_rms_norm(const __nv_bfloat16* __restric
     const float inv = rsqrtf(__fdiv_rn(tot, (float)width) + eps);
     for (int i = threadIdx.x; i < width; i += 256)
         y[base + i] = f2bf(__fmul_rn(__fmul_rn(bf2f(x[base + i]), inv), bf2f(w[i])));
+}
+
+/* The norm together with what precedes it: v = src row (or row code[r] of a table; the code may be the arg-max of a row of
+ * logits, found here), plus the linear output to add to it; v goes to x_out and its norm to y.  k_rms_norm's pairs and
+ * roundings, but the row crosses memory once, in 16-byte vectors that stay in registers from the load to the store (norm
+ * alone, 8 rows: 3.6 -> 2.0 us in the captured tick; it also saves the launch of the add, of the embedding and of the arg-max). */
+struct NormRowArgs {
+    const __nv_bfloat16* src;    /* [rows, width], or the table */
+    const __nv_bfloat16* add;    /* [rows, width] or NULL */
+    const int32_t* codes;        /* [rows] or NULL: row of the table, clamped to table_rows (fastar.cu:150-158) */
+    const __nv_bfloat16* logits; /* [rows, table_rows] or NULL: the code is their arg-max, also written to codes_out */
+    int32_t* codes_out;
+    __nv_bfloat16* x_out;        /* NULL: the sum is not kept */
+    const __nv_bfloat16* w;      /* NULL: no norm wanted */
+    __nv_bfloat16* y;
+    int width, table_rows;
+    float eps;
+};
+constexpr int NORM_MAX_WIDTH = 4096; /* two vectors per thread */
+__global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
+    __shared__ __align__(16) __nv_bfloat16 xs[NORM_MAX_WIDTH];
+    __shared__ float red[257];
+    __shared__ unsigned long long best[8];
+    const int tid = threadIdx.x, r = blockIdx.x, nv = a.width >> 3;
+    const int v0 = tid, v1 = tid + 256;
+    uint4 g0 = make_uint4(0, 0, 0, 0), g1 = g0;
+    if (a.w) {
+        if (v0 < nv) g0 = reinterpret_cast<const uint4*>(a.w)[v0];
+        if (v1 < nv) g1 = reinterpret_cast<const uint4*>(a.w)[v1];
+    }
+    size_t row = (size_t)r;
+    if (a.logits) { /* larger value first, then lower index (kernels.cu:1326-1357); -0 counts as +0 */
+        unsigned long long key = 0ull;
+        for (int i = tid; i < a.table_rows; i += 256) {
+            const float l = bf2f(a.logits[(size_t)r * a.table_rows + i]);
+            if (l != l) continue; /* a row of NaN gives index 0, as the reference's */
+            uint32_t u = __float_as_uint(l);
+            if (u == 0x80000000u) u = 0u;
+            u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+            const unsigned long long k = ((unsigned long long)u << 32) | (0xFFFFFFFFu - (uint32_t)i);
+            key = k > key ? k : key;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(S2P_FULL_MASK, key, off);
+            key = o > key ? o : key;
+        }
+        if ((tid & 31) == 0) best[tid >> 5] = key;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 8; k++) key = best[k] > key ? best[k] : key; /* every thread ends with the row's key */
+        row = key ? 0xFFFFFFFFu - (uint32_t)key : 0u;
+        if (tid == 0) a.codes_out[r] = (int32_t)row;
+    } else if (a.codes) {
+        row = (size_t)max(0, min(a.table_rows - 1, a.codes[r]));
+    }
+    const uint4* src = reinterpret_cast<const uint4*>(a.src + row * a.width);
+    const uint4* add = a.add ? reinterpret_cast<const uint4*>(a.add + (size_t)r * a.width) : nullptr;
+    uint4* xo = a.x_out ? reinterpret_cast<uint4*>(a.x_out + (size_t)r * a.width) : nullptr;
+    auto load = [&](int v) {
+        uint4 q = src[v];
+        if (add) {
+            const uint4 p = add[v];
+            uint32_t* qw = &q.x;
+            const uint32_t pw[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                qw[c] = (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(qw[c]), bf_lo(pw[c])))) |
+                        ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(qw[c]), bf_hi(pw[c])))) << 16);
+        }
+        if (xo) xo[v] = q;
+        reinterpret_cast<uint4*>(xs)[v] = q;
+        return q;
+    };
+    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+    if (v0 < nv) x0 = load(v0);
+    if (v1 < nv) x1 = load(v1);
+    if (!a.w) return;
+    __syncthreads();
+    float ss = 0.f;
+    for (int i = tid; i < a.width; i += 256) {
+        const float v = bf2f(xs[i]);
+        ss = __fmaf_rn(v, v, ss);
+    }
+    const float tot = tree256_sum(ss, red);
+    const float inv = rsqrtf(__fdiv_rn(tot, (float)a.width) + a.eps);
+    uint4* y = reinterpret_cast<uint4*>(a.y + (size_t)r * a.width);
+    if (v0 < nv) y[v0] = norm_vec8(x0, g0, inv);
+    if (v1 < nv) y[v1] = norm_vec8(x1, g1, inv);
 }
 
 /* ---- per-head RMSNorm, 128 partials (kernels.cu:81-101), in place ---------- */
@@ -483,13 +573,6 @@ __global__ void __launch_bounds__(256) k_scale_rows_masked(__nv_bfloat16* __rest
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
         if (mask[i / dim]) x[i] = f2bf(__fmul_rn(bf2f(x[i]), scale));
 }
-__global__ void k_embed_codes(const __nv_bfloat16* __restrict__ table, const int32_t* __restrict__ codes,
-                              __nv_bfloat16* __restrict__ out, int rows, int dim, int cbsize) {
-    /* fast-AR step input: row of the 4096-entry table, code clamped (fastar.cu:150-158) */
-    const int r = blockIdx.x;
-    const int c = max(0, min(cbsize - 1, codes[r]));
-    for (int d = threadIdx.x; d < dim; d += blockDim.x) out[(size_t)r * dim + d] = table[(size_t)c * dim + d];
-}
 __global__ void k_pack_frame(const int32_t* __restrict__ stage, int rows, int32_t* __restrict__ codes) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * 9) return;
@@ -498,9 +581,41 @@ __global__ void k_pack_frame(const int32_t* __restrict__ stage, int rows, int32_
 }
 
 /* ---- internal launchers ---------------------------------------------------- */
+static bool norm_row_serves(const NormRowArgs& a) {
+    const uintptr_t all = (uintptr_t)a.src | (uintptr_t)a.add | (uintptr_t)a.x_out | (uintptr_t)a.w | (uintptr_t)a.y;
+    return a.width % 8 == 0 && a.width <= NORM_MAX_WIDTH && !(all & 15);
+}
 cudaError_t rms_norm(const void* x, const void* w, void* y, int rows, int width, float eps, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
-    k_rms_norm<<<rows, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, width, eps);
+    NormRowArgs a = {};
+    a.src = (const __nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = width; a.eps = eps;
+    if (norm_row_serves(a)) k_norm_row<<<rows, 256, 0, st>>>(a);
+    else k_rms_norm<<<rows, 256, 0, st>>>(a.src, a.w, a.y, width, eps);
+    return cudaGetLastError();
+}
+cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    NormRowArgs a = {};
+    a.src = (const __nv_bfloat16*)x; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
+    a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
+    k_norm_row<<<rows, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    NormRowArgs a = {};
+    a.src = (const __nv_bfloat16*)src; a.x_out = (__nv_bfloat16*)x;
+    a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
+    k_norm_row<<<rows, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logits, int32_t* codes_out, void* x, const void* w, void* y, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    NormRowArgs a = {};
+    a.src = (const __nv_bfloat16*)table; a.codes = codes; a.logits = (const __nv_bfloat16*)logits; a.codes_out = codes_out;
+    a.x_out = (__nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y;
+    a.width = S2P_DIM; a.table_rows = S2P_CB_SIZE; a.eps = S2P_NORM_EPS;
+    k_norm_row<<<rows, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 cudaError_t silu_mul(const void* gu, void* h, int rows, int ffn, cudaStream_t st) {
@@ -545,11 +660,6 @@ cudaError_t scale_rows_masked(void* x, const uint8_t* mask, int rows, int dim, f
     if (rows <= 0) return cudaSuccess;
     const int64_t total = (int64_t)rows * dim;
     k_scale_rows_masked<<<grid_for(total, 256), 256, 0, st>>>((__nv_bfloat16*)x, mask, total, dim, scale);
-    return cudaGetLastError();
-}
-cudaError_t embed_codes(const void* table, const int32_t* codes, void* out, int rows, cudaStream_t st) {
-    if (rows <= 0) return cudaSuccess;
-    k_embed_codes<<<rows, 256, 0, st>>>((const __nv_bfloat16*)table, codes, (__nv_bfloat16*)out, rows, S2P_DIM, S2P_CB_SIZE);
     return cudaGetLastError();
 }
 cudaError_t argmax_rows(const void* logits, int32_t* ids, int rows, int vocab, cudaStream_t st) {

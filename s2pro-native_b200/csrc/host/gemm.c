@@ -300,6 +300,13 @@ s2p_status s2p_linear_gemv_rows(const s2p_linear* lin, const void* x_bf16, void*
     return S2P_OK;
 }
 
+s2p_status s2p_linear_dequant(const s2p_linear* lin, void* w_bf16, cudaStream_t stream) {
+    const int N = lin->out_features, K = lin->in_features;
+    if (lin->q_packed) return s2p_int4p_dequant(w_bf16, lin->w_pack.data, lin->w_iscale.data, N, K, lin->q_group, stream);
+    if (lin->q_group > 0) return s2p_intq_dequant(w_bf16, lin->w_int8.data, lin->w_iscale.data, N, K, lin->q_group, stream);
+    return s2p_int8_dequant(w_bf16, lin->w_int8.data, (const float*)lin->w_iscale.data, N, K, stream);
+}
+
 s2p_status s2p_linear_forward(const s2p_linear* lin, const void* x_bf16, void* y_bf16, int M, s2p_gemm_mode mode,
                               cudaStream_t stream) {
     if (!lin || !x_bf16 || !y_bf16 || M <= 0) return S2P_ERR_INVALID;
@@ -334,9 +341,7 @@ s2p_status s2p_linear_forward(const s2p_linear* lin, const void* x_bf16, void* y
             if (rc == S2P_OK) G.deq_bytes = need;
         }
         if (rc == S2P_OK) {
-            if (lin->q_packed) rc = s2p_int4p_dequant(G.deq, lin->w_pack.data, lin->w_iscale.data, N, K, lin->q_group, stream);
-            else if (lin->q_group > 0) rc = s2p_intq_dequant(G.deq, lin->w_int8.data, lin->w_iscale.data, N, K, lin->q_group, stream);
-            else rc = s2p_int8_dequant(G.deq, lin->w_int8.data, (const float*)lin->w_iscale.data, N, K, stream);
+            rc = s2p_linear_dequant(lin, G.deq, stream);
         }
         if (rc == S2P_OK) rc = cublas_xwT(x_bf16, G.deq, y_bf16, M, N, K, stream);
         pthread_mutex_unlock(&G.mu);

@@ -18,12 +18,16 @@ void s2p_linear_tc_disable(void);
 /* what a tensor-parallel model may do (session.c) */
 s2p_status s2p_tp_guard_tick(int tp_world, int decoding_rows, int persistent_path);
 s2p_status s2p_tp_guard_kv_save(int tp_world);
+s2p_status s2p_linear_dequant(const s2p_linear* lin, void* w_bf16, cudaStream_t stream);
 s2p_status s2p_linear_tc_add(const s2p_linear* lin, const void* x_bf16, void* y_inout_bf16, int M, cudaStream_t stream);
 s2p_status s2p_linear_tc_swiglu(const s2p_linear* lin, const void* x_bf16, void* h_bf16, int M, cudaStream_t stream);
 
 typedef struct {
     s2p_linear wqkv, wo, gate_up, w2;
     s2p_tensor attn_norm, ffn_norm, q_norm, k_norm; /* q/k_norm empty in the fast-AR */
+    /* backbone: bf16 copies of the four quantised matrices (wqkv, wo, gate_up, w2) for prompt slices, in the model's
+     * `wide_weights`; NULL where there are none */
+    void* wide[4];
 } s2p_layer;
 
 /* host sampler parameters and history mirror (reference: src/slowar/slowar_internal.h:40-55) */
@@ -75,6 +79,7 @@ struct s2p_model {
     s2p_tensor embed, embed_i8, embed_scale;
     s2p_layer slow[S2P_SLOW_LAYERS];
     s2p_tensor final_norm;
+    void* wide_weights;
     s2p_layer fast[S2P_FAST_LAYERS];
     s2p_tensor fast_norm, cb_emb, fast_emb;
     s2p_linear fast_out;

@@ -160,26 +160,35 @@ typedef struct {
     int decode;     /* decode-sized rows: GEMV in slices instead of the prefill GEMM */
 } layer_ctx;
 
-static s2p_status lin_apply(s2p_model* m, const s2p_linear* lin, const void* x, void* y, int rows, int decode) {
+/* y = x · Wᵀ; `wide`: the layer's bf16 copy, or NULL */
+static s2p_status lin_apply(s2p_model* m, const s2p_linear* lin, const void* wide, const void* x, void* y, int rows, int decode) {
+    if (wide && !decode && rows > S2P_INT8_GEMV_MAX_M && !s2p_env_is_one("S2P_PREFILL_TC")) {
+        m->tick_kernels += 1;
+        return s2p_gemm_bf16(x, wide, y, rows, lin->out_features, lin->in_features, m->stream);
+    }
     m->tick_kernels += !decode ? 2 : (m->mode == S2P_GEMM_INT8 && lin->int8_ready && s2p_linear_rows_on_tc(lin, rows))
                                          ? 1 : (rows + S2P_INT8_GEMV_MAX_M - 1) / S2P_INT8_GEMV_MAX_M;
     if (decode && m->mode == S2P_GEMM_INT8 && lin->int8_ready) return s2p_linear_gemv_rows(lin, x, y, rows, m->stream);
     return s2p_linear_forward(lin, x, y, rows, m->mode, m->stream);
 }
 
-/* CTAs per (row, kv head) of the split-K decode attention: enough CTAs in total (about 2048) that a
- * long context is walked by several workers even when the batch alone would fill the GPU */
-/* x += in · Wᵀ: one launch where the batch runs on the tensor cores, else linear into `proj` and the add kernel */
-static s2p_status lin_add(s2p_model* m, const s2p_linear* lin, const void* in, void* x, void* proj, int rows, int decode) {
+/* x += in · Wᵀ, then `out` = norm of x with `gain` (gain NULL: no norm): the residual add is part of the linear where the
+ * batch runs on the tensor cores, else of the norm */
+static s2p_status lin_add_norm(s2p_model* m, const s2p_linear* lin, const void* wide, const void* in, void* x, void* proj, const void* gain,
+                               void* out, int rows, int decode) {
     if (decode && m->mode == S2P_GEMM_INT8 && lin->int8_ready && s2p_linear_rows_on_tc(lin, rows)) {
         m->tick_kernels += 1;
-        return s2p_linear_tc_add(lin, in, x, rows, m->stream);
+        S2P_TRY(s2p_linear_tc_add(lin, in, x, rows, m->stream));
+        if (gain) S2P_LAUNCH(m, rms_norm(x, gain, out, rows, S2P_DIM, S2P_NORM_EPS, m->stream));
+        return S2P_OK;
     }
-    S2P_TRY(lin_apply(m, lin, in, proj, rows, decode));
-    S2P_LAUNCH(m, add_inplace(x, proj, (int64_t)rows * lin->out_features, m->stream));
+    S2P_TRY(lin_apply(m, lin, wide, in, proj, rows, decode));
+    S2P_LAUNCH(m, add_norm(x, proj, gain, out, rows, m->stream));
     return S2P_OK;
 }
 
+/* CTAs per (row, kv head) of the split-K decode attention: enough CTAs in total (about 2048) that a
+ * long context is walked by several workers even when the batch alone would fill the GPU */
 static int attn_workers_for(int rows) {
     static int forced = -1; /* S2P_ATTN_WORKERS=n (1..16) overrides the choice */
     if (forced < 0) {
@@ -192,14 +201,15 @@ static int attn_workers_for(int rows) {
     return w < 1 ? 1 : (w > 16 ? 16 : w);
 }
 
-/* x: residual stream [rows, 2560]; scratch tensors: norm/qkv/q/attn/proj/gu/hff */
+/* x: residual stream [rows, 2560], `norm` its norm with the layer's first gain; scratch tensors: qkv/q/attn/proj/gu/hff.
+ * Leaves the norm with the gain `next` (NULL: none) in `next_out`. */
 static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ctx* c, s2p_dev_bf16* x,
                                 s2p_dev_bf16* norm, s2p_dev_bf16* qkv, s2p_dev_bf16* q, s2p_dev_bf16* attn,
-                                s2p_dev_bf16* proj, s2p_dev_bf16* gu, s2p_dev_bf16* hff) {
+                                s2p_dev_bf16* proj, s2p_dev_bf16* gu, s2p_dev_bf16* hff, const void* next,
+                                s2p_dev_bf16* next_out) {
     cudaStream_t st = m->stream;
     const int rows = c->rows;
-    S2P_LAUNCH(m, rms_norm(x, L->attn_norm.data, norm, rows, S2P_DIM, S2P_NORM_EPS, st));
-    S2P_TRY(lin_apply(m, &L->wqkv, norm, qkv, rows, c->decode));
+    S2P_TRY(lin_apply(m, &L->wqkv, L->wide[0], norm, qkv, rows, c->decode));
     QkvPostArgs qa;
     memset(&qa, 0, sizeof(qa));
     qa.qkv = qkv; qa.q = q;
@@ -221,17 +231,16 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
     } else {
         S2P_LAUNCH(m, attn_single(&aa, rows, st));
     }
-    S2P_TRY(lin_add(m, &L->wo, attn, x, proj, rows, c->decode));
-    S2P_LAUNCH(m, rms_norm(x, L->ffn_norm.data, norm, rows, S2P_DIM, S2P_NORM_EPS, st));
+    S2P_TRY(lin_add_norm(m, &L->wo, L->wide[1], attn, x, proj, L->ffn_norm.data, norm, rows, c->decode));
     if (c->decode && m->mode == S2P_GEMM_INT8 && L->gate_up.int8_ready && s2p_linear_rows_on_tc(&L->gate_up, rows) &&
         L->gate_up.out_features == 2 * S2P_FFN_DIM) {
         m->tick_kernels += 1; /* gate/up linear and SwiGLU in one launch */
         S2P_TRY(s2p_linear_tc_swiglu(&L->gate_up, norm, hff, rows, st));
     } else {
-        S2P_TRY(lin_apply(m, &L->gate_up, norm, gu, rows, c->decode));
+        S2P_TRY(lin_apply(m, &L->gate_up, L->wide[2], norm, gu, rows, c->decode));
         S2P_LAUNCH(m, silu_mul(gu, hff, rows, S2P_FFN_DIM, st));
     }
-    S2P_TRY(lin_add(m, &L->w2, hff, x, proj, rows, c->decode));
+    S2P_TRY(lin_add_norm(m, &L->w2, L->wide[3], hff, x, proj, next, next_out, rows, c->decode));
     return S2P_OK;
 }
 
@@ -328,10 +337,12 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
     c.kv8 = m->kv8;
     c.pos0 = pos0;
     c.pos_row_step = 1;
+    S2P_LAUNCH(m, rms_norm(m->sx.data, m->slow[0].attn_norm.data, m->snorm.data, n_ids, S2P_DIM, S2P_NORM_EPS, st));
     for (int l = 0; l < m->n_slow; l++) {
         slow_kv_offsets(m, l, &c.kv);
         S2P_TRY(layer_general(m, &m->slow[l], &c, BF(m->sx), BF(m->snorm), BF(m->sqkv), BF(m->sq), BF(m->sattn),
-                              BF(m->sproj), BF(m->sgu), BF(m->sffn)));
+                              BF(m->sproj), BF(m->sgu), BF(m->sffn), l + 1 < m->n_slow ? m->slow[l + 1].attn_norm.data : NULL,
+                              BF(m->snorm)));
         if (dump_dir()) {
             char nm[32];
             snprintf(nm, sizeof(nm), "backbone_layer%02d", l);
@@ -511,20 +522,19 @@ static s2p_status fast_frame_general(s2p_model* m, const tick_dev* d, int nact, 
     layer_ctx c;
     memset(&c, 0, sizeof(c));
     c.rows = nact; c.max_seq = S2P_FAST_SEQ; c.kv8 = 0; c.pos_row_step = 0; c.decode = 1; c.split_k = 0;
-    S2P_CUDA_TRY(cudaMemcpyAsync(m->fx.data, m->shidden.data, (size_t)nact * S2P_DIM * 2, cudaMemcpyDeviceToDevice, st));
+    S2P_LAUNCH(m, copy_norm(m->shidden.data, m->fx.data, m->fast[0].attn_norm.data, m->ft.data, nact, st));
     for (int cb = 0; cb < S2P_NUM_CODEBOOKS; cb++) {
         c.pos0 = cb;
         for (int l = 0; l < S2P_FAST_LAYERS; l++) {
             fast_kv_ref(m, l, &c.kv);
             S2P_TRY(layer_general(m, &m->fast[l], &c, BF(m->fx), BF(m->ft), BF(m->fqkv), BF(m->fq), BF(m->fattn),
-                                  BF(m->fproj), BF(m->fgu), BF(m->fhff)));
+                                  BF(m->fproj), BF(m->fgu), BF(m->fhff),
+                                  l + 1 < S2P_FAST_LAYERS ? m->fast[l + 1].attn_norm.data : cb ? m->fast_norm.data : NULL, BF(m->ft)));
         }
-        const int32_t* next_codes;
-        if (cb == 0) {
-            next_codes = d->sem; /* the prime pass produces no logits; step 1 is fed embeddings[sem] */
+        if (cb == 0) { /* the prime pass produces no logits; step 1 is fed embeddings[sem] */
+            S2P_LAUNCH(m, embed_norm(m->fast_emb.data, d->sem, NULL, NULL, m->fx.data, m->fast[0].attn_norm.data, m->ft.data, nact, st));
         } else {
-            S2P_LAUNCH(m, rms_norm(m->fx.data, m->fast_norm.data, m->ft.data, nact, S2P_DIM, S2P_NORM_EPS, st));
-            S2P_TRY(lin_apply(m, &m->fast_out, m->ft.data, m->flogits.data, nact, 1));
+            S2P_TRY(lin_apply(m, &m->fast_out, NULL, m->ft.data, m->flogits.data, nact, 1));
             if (dump_ok && dump_dir() && nact == 1) {
                 static int dump_frame = 0;
                 if (cb == 1) dump_frame++;
@@ -535,10 +545,11 @@ static s2p_status fast_frame_general(s2p_model* m, const tick_dev* d, int nact, 
                 }
             }
             int32_t* dst = m->fstage + (size_t)(cb - 1) * nact;
-            S2P_LAUNCH(m, argmax_rows(m->flogits.data, dst, nact, S2P_CB_SIZE, st));
-            next_codes = dst;
+            if (cb < S2P_NUM_CODEBOOKS - 1)
+                S2P_LAUNCH(m, embed_norm(m->fast_emb.data, NULL, m->flogits.data, dst, m->fx.data, m->fast[0].attn_norm.data, m->ft.data, nact, st));
+            else
+                S2P_LAUNCH(m, argmax_rows(m->flogits.data, dst, nact, S2P_CB_SIZE, st));
         }
-        if (cb < S2P_NUM_CODEBOOKS - 1) S2P_LAUNCH(m, embed_codes(m->fast_emb.data, next_codes, m->fx.data, nact, st));
     }
     S2P_LAUNCH(m, pack_frame(m->fstage, nact, d->ocodes, st));
     return S2P_OK;
@@ -556,12 +567,14 @@ static s2p_status tick_general(s2p_model* m, s2p_session* const* act, int bd, in
         memset(&c, 0, sizeof(c));
         c.rows = bd; c.kv.bases = d.kv_bases; c.kv.sbases = d.kvs_bases;
         c.max_seq = m->ctx_len; c.kv8 = m->kv8; c.pos_arr = d.pos; c.split_k = 1; c.decode = 1;
+        S2P_LAUNCH(m, rms_norm(m->sx.data, m->slow[0].attn_norm.data, m->snorm.data, bd, S2P_DIM, S2P_NORM_EPS, st));
         for (int l = 0; l < m->n_slow; l++) {
+            const int last = l + 1 == m->n_slow;
             slow_kv_offsets(m, l, &c.kv);
             S2P_TRY(layer_general(m, &m->slow[l], &c, BF(m->sx), BF(m->snorm), BF(m->sqkv), BF(m->sq), BF(m->sattn),
-                                  BF(m->sproj), BF(m->sgu), BF(m->sffn)));
+                                  BF(m->sproj), BF(m->sgu), BF(m->sffn), last ? m->final_norm.data : m->slow[l + 1].attn_norm.data,
+                                  last ? BF(m->shidden) : BF(m->snorm)));
         }
-        S2P_LAUNCH(m, rms_norm(m->sx.data, m->final_norm.data, m->shidden.data, bd, S2P_DIM, S2P_NORM_EPS, st));
     }
     for (int b = bd; b < nact; b++) /* freshly prefilled rows sample from their stashed hidden (eager only) */
         S2P_CUDA_TRY(cudaMemcpyAsync(BF(m->shidden) + (size_t)b * S2P_DIM, act[b]->pending_hidden,
