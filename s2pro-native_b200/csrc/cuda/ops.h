@@ -87,6 +87,13 @@ typedef struct {
     int N, K, gshift;
 } LinRef;
 
+/* Output of a linear left as partials over its K range (wide.cuh) */
+typedef struct {
+    const float* partial; /* [tile of 128 outputs][piece][batch row][128] */
+    const float* scales;  /* per-output factor of the sum, or NULL */
+    int pieces, M;
+} WidePart;
+
 /* Where a [K] activation (or residual) vector comes from: a plain vector, or a
  * row of a table selected on the device by an int32 index or by the low word
  * of a packed arg-max key (index = 0xFFFFFFFF - low32). */
@@ -132,9 +139,21 @@ cudaError_t gemv_setup_all(void); /* once per device, before any stream capture 
 cudaError_t skinny_gemm_tc(const LinRef* lin, const void* x, int M, void* y, const void* resid, cudaStream_t st);
 /* h[M, N / 2] = silu(x · Wg^T) * (x · Wu^T) for W = [Wg | Wu] stacked along N (gate/up linear + SwiGLU in one launch) */
 cudaError_t skinny_gemm_tc_swiglu(const LinRef* lin, const void* x, int M, void* h, cudaStream_t st);
+/* The same products from weights converted once (skinny.cu): f16 tiles of `lin` (wide_weight_bytes bytes; ffn > 0: of a
+ * [gate | up] pair in the order its SwiGLU needs) and activations as f16 units (wide.cuh; 512 * K bytes serve any M <= 256).
+ * wide_gemm leaves x · W^T in y [M, N] or, where K is split over CTAs, as partials described in `part` (partial NULL: y was
+ * written); with ffn h = silu(gate) * up into y [M, ffn] or, as the units of a next linear of kind h_kind, into h_tiled.  The
+ * sums equal those of skinny_gemm_tc / skinny_gemm_tc_swiglu bit for bit. */
+int wide_serves(const LinRef* lin, int ffn);
+size_t wide_weight_bytes(const LinRef* lin, int ffn);
+cudaError_t wide_convert(const LinRef* lin, int ffn, void* out, cudaStream_t st);
+cudaError_t wide_pack(int kind, const void* x, int M, int K, void* xt, cudaStream_t st);
+cudaError_t wide_gemm(const LinRef* lin, const void* wide, const void* xt, int M, int ffn, void* y, void* h_tiled, int h_kind, WidePart* part,
+                      cudaStream_t st);
 /* any M >= 1: prompt slices in blocks of 256 rows, activations pre-tiled (not under stream capture) */
 cudaError_t skinny_prefill_tc(const LinRef* lin, const void* x, int M, void* y, cudaStream_t st);
 cudaError_t skinny_status(int* out);
+cudaError_t skinny_status_async(int* host, cudaStream_t st); /* to pinned memory, in stream order */
 cudaError_t skinny_reset(cudaStream_t st);            /* clears the status code and the arrival counters */
 cudaError_t skinny_set_wait_ns(unsigned long long ns); /* test hook: deadline of the kernel's bounded waits */
 cudaError_t skinny_setup(int max_rows); /* once per device, outside stream capture: scratch for split-K launches */
@@ -290,6 +309,14 @@ cudaError_t scale_div(void* x, int64_t n, float divisor, cudaStream_t st);
 cudaError_t scale_rows_masked(void* x, const uint8_t* mask, int rows, int dim, float scale, cudaStream_t st);
 /* rows of the model width, all 16-byte aligned: x += add, then y = norm(x) with gain w (w NULL: no norm) */
 cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st);
+/* The same around wide_gemm.  `part` with `alt` is its output: the partials, or alt where it wrote that.
+ * x = src (+ the output, if part is given); or, with a table, its row `codes[r]`, or the one that the arg-max of the output
+ * selects (to codes_out).  y = norm(x) with gain w (NULL: none), as bf16 and / or as the units of a linear of kind `kind`. */
+cudaError_t wide_norm(const void* src, const WidePart* part, const void* alt, void* x, const void* w, void* y, void* y_tiled, int kind, int rows,
+                      cudaStream_t st);
+cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WidePart* part, const void* alt, int32_t* codes_out, void* x, const void* w,
+                            void* y_tiled, int kind, int rows, cudaStream_t st);
+cudaError_t qkv_post_part(const QkvPostArgs* a, const WidePart* part, int rows, cudaStream_t st);
 /* x = src, y = norm(x) */
 cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st);
 /* x = table[code], y = norm(x); the codes are given, or the arg-max of each row of `logits`, which also goes to codes_out */

@@ -12,6 +12,7 @@
 #include "gemv.cuh"
 #include "headops.cuh"
 #include "ops.h"
+#include "wide.cuh"
 #include "attn_prefill.cuh"
 #include "s2p_b200_abi.h"
 
@@ -57,6 +58,10 @@ struct NormRowArgs {
     __nv_bfloat16* y;
     int width, table_rows;
     float eps;
+    WidePart part;               /* partial set: takes the place of `add`, or with part_logits of `logits` */
+    int part_logits;
+    uint4* tiled;                /* the norm also as matrix units of the next linear (wide.cuh), for a batch padded to 1 << lg rows */
+    int tiled_int4, lg;
 };
 constexpr int NORM_MAX_WIDTH = 4096; /* two vectors per thread */
 __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
@@ -71,17 +76,23 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
         if (v1 < nv) g1 = reinterpret_cast<const uint4*>(a.w)[v1];
     }
     size_t row = (size_t)r;
-    if (a.logits) { /* larger value first, then lower index (kernels.cu:1326-1357); -0 counts as +0 */
+    auto offer = [](unsigned long long& key, float l, int i) {
+        if (l != l) return; /* a row of NaN gives index 0, as the reference's */
+        uint32_t u = __float_as_uint(l);
+        if (u == 0x80000000u) u = 0u;
+        u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+        const unsigned long long k = ((unsigned long long)u << 32) | (0xFFFFFFFFu - (uint32_t)i);
+        key = k > key ? k : key;
+    };
+    if (a.logits || a.part_logits) { /* larger value first, then lower index (kernels.cu:1326-1357); -0 counts as +0 */
         unsigned long long key = 0ull;
-        for (int i = tid; i < a.table_rows; i += 256) {
-            const float l = bf2f(a.logits[(size_t)r * a.table_rows + i]);
-            if (l != l) continue; /* a row of NaN gives index 0, as the reference's */
-            uint32_t u = __float_as_uint(l);
-            if (u == 0x80000000u) u = 0u;
-            u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-            const unsigned long long k = ((unsigned long long)u << 32) | (0xFFFFFFFFu - (uint32_t)i);
-            key = k > key ? k : key;
-        }
+        if (a.part_logits)
+            for (int i = tid * 4; i < a.table_rows; i += 1024) {
+                const float4 l = wide_part4(a.part, i, r);
+                offer(key, bf16_round(l.x), i); offer(key, bf16_round(l.y), i + 1); offer(key, bf16_round(l.z), i + 2); offer(key, bf16_round(l.w), i + 3);
+            }
+        else
+            for (int i = tid; i < a.table_rows; i += 256) offer(key, bf2f(a.logits[(size_t)r * a.table_rows + i]), i);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
             const unsigned long long o = __shfl_xor_sync(S2P_FULL_MASK, key, off);
@@ -99,10 +110,15 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
     const uint4* src = reinterpret_cast<const uint4*>(a.src + row * a.width);
     const uint4* add = a.add ? reinterpret_cast<const uint4*>(a.add + (size_t)r * a.width) : nullptr;
     uint4* xo = a.x_out ? reinterpret_cast<uint4*>(a.x_out + (size_t)r * a.width) : nullptr;
+    const bool part_add = a.part.partial != nullptr && !a.part_logits;
     auto load = [&](int v) {
         uint4 q = src[v];
-        if (add) {
-            const uint4 p = add[v];
+        if (add || part_add) {
+            uint4 p;
+            if (part_add) {
+                const uint2 lo = wide_part4_bf16(a.part, v * 8, r), hi = wide_part4_bf16(a.part, v * 8 + 4, r);
+                p = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            } else p = add[v];
             uint32_t* qw = &q.x;
             const uint32_t pw[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
@@ -126,9 +142,13 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
     }
     const float tot = tree256_sum(ss, red);
     const float inv = rsqrtf(__fdiv_rn(tot, (float)a.width) + a.eps);
-    uint4* y = reinterpret_cast<uint4*>(a.y + (size_t)r * a.width);
-    if (v0 < nv) y[v0] = norm_vec8(x0, g0, inv);
-    if (v1 < nv) y[v1] = norm_vec8(x1, g1, inv);
+    uint4* y = a.y ? reinterpret_cast<uint4*>(a.y + (size_t)r * a.width) : nullptr;
+    auto put = [&](int v, const uint4& q) {
+        if (y) y[v] = q;
+        if (a.tiled) a.tiled[((size_t)v << a.lg) + r] = wide_unit(q, a.tiled_int4);
+    };
+    if (v0 < nv) put(v0, norm_vec8(x0, g0, inv));
+    if (v1 < nv) put(v1, norm_vec8(x1, g1, inv));
 }
 
 /* ---- per-head RMSNorm, 128 partials (kernels.cu:81-101), in place ---------- */
@@ -178,7 +198,7 @@ __global__ void __launch_bounds__(256) k_rope(__nv_bfloat16* __restrict__ x, int
  * heads instead of once per element, which is what bounded the thread-per-element form (512 rows: 29.9 -> 10.5 us, 2048: 107 -> 29).
  * grid (rows, (q_heads + 2 kv_heads) / 16), 512 threads. */
 constexpr int QKV_HEADS_PER_CTA = 16;
-__global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs a) {
+__global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs a, WidePart part) {
     __shared__ float2 cs[64];
     const int r = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * QKV_HEADS_PER_CTA + (threadIdx.x >> 5);
     const int QH = a.q_heads, KVH = a.kv_heads, heads = QH + 2 * KVH;
@@ -186,7 +206,7 @@ __global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs
     const bool live = h < heads, is_q = h < QH, rotated = h < QH + KVH;
     uint2 x = make_uint2(0u, 0u), nw = x;
     const __nv_bfloat16* gain = is_q ? a.q_norm : a.k_norm;
-    if (live) x = *reinterpret_cast<const uint2*>(a.qkv + ((size_t)r * heads + h) * 128 + lane * 4);
+    if (live) x = part.partial ? wide_part4_bf16(part, h * 128 + lane * 4, r) : *reinterpret_cast<const uint2*>(a.qkv + ((size_t)r * heads + h) * 128 + lane * 4);
     if (rotated && gain) nw = *reinterpret_cast<const uint2*>(gain + lane * 4);
     if (threadIdx.x < 64 && blockIdx.y * QKV_HEADS_PER_CTA < QH + KVH) rope_cs(threadIdx.x, pos, a.rope_base, cs[threadIdx.x].x, cs[threadIdx.x].y);
     __syncthreads();
@@ -241,12 +261,13 @@ __global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs
     if ((lane & 7) == 0) reinterpret_cast<__half*>(scales)[vec * 4 + (lane >> 3)] = hsc;
 }
 
-cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st) {
+cudaError_t qkv_post_part(const QkvPostArgs* a, const WidePart* part, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     dim3 grid((unsigned)rows, (unsigned)((a->q_heads + 2 * a->kv_heads + QKV_HEADS_PER_CTA - 1) / QKV_HEADS_PER_CTA));
-    k_qkv_post<<<grid, 32 * QKV_HEADS_PER_CTA, 0, st>>>(*a);
+    k_qkv_post<<<grid, 32 * QKV_HEADS_PER_CTA, 0, st>>>(*a, part ? *part : WidePart());
     return cudaGetLastError();
 }
+cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st) { return qkv_post_part(a, nullptr, rows, st); }
 
 /* ---- plain KV append (contract s2pk_kv_append, kernels.cu:172-195) --------- */
 __global__ void __launch_bounds__(256) k_kv_append(const __nv_bfloat16* __restrict__ k,
@@ -598,6 +619,33 @@ cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows,
     NormRowArgs a = {};
     a.src = (const __nv_bfloat16*)x; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
+    k_norm_row<<<rows, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+static NormRowArgs wide_norm_args(void* x, const void* w, void* y, void* y_tiled, int kind, int rows) {
+    NormRowArgs a = {};
+    a.x_out = (__nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y;
+    a.tiled = (uint4*)y_tiled; a.tiled_int4 = kind == WK_INT4_PACK; a.lg = wide_lg(rows);
+    a.width = S2P_DIM; a.table_rows = S2P_CB_SIZE; a.eps = S2P_NORM_EPS;
+    return a;
+}
+cudaError_t wide_norm(const void* src, const WidePart* part, const void* alt, void* x, const void* w, void* y, void* y_tiled, int kind, int rows,
+                      cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    NormRowArgs a = wide_norm_args(x, w, y, y_tiled, kind, rows);
+    a.src = (const __nv_bfloat16*)src;
+    if (part && part->partial) a.part = *part;
+    else if (part) a.add = (const __nv_bfloat16*)alt;
+    k_norm_row<<<rows, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WidePart* part, const void* alt, int32_t* codes_out, void* x, const void* w,
+                            void* y_tiled, int kind, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    NormRowArgs a = wide_norm_args(x, w, nullptr, y_tiled, kind, rows);
+    a.src = (const __nv_bfloat16*)table; a.codes = codes; a.codes_out = codes_out;
+    if (part && part->partial) { a.part = *part; a.part_logits = 1; }
+    else if (part) a.logits = (const __nv_bfloat16*)alt;
     k_norm_row<<<rows, 256, 0, st>>>(a);
     return cudaGetLastError();
 }

@@ -29,6 +29,7 @@
 #include "ops.h"
 #include "pipe.cuh"
 #include "s2p_b200_abi.h"
+#include "wide.cuh"
 
 namespace s2p {
 
@@ -128,22 +129,7 @@ template <int WK, int NT, int KCP> struct SkGeom {
 /* bf16 x 8 -> f16 x 8 for the B tile.  INT4 slabs keep the order their conversion produces
  * (elements 0,4,1,5,2,6,3,7 of every eight: no re-interleaving of the nibbles), and the activations
  * follow the same order: the contraction does not care as long as both operands agree. */
-template <int WK> __device__ __forceinline__ uint4 sk_x_unit(const uint4& v) {
-    __half2 h[4];
-    if (WK == WK_INT4_PACK) {
-        h[0] = __floats2half2_rn(bf_lo(v.x), bf_lo(v.z));
-        h[1] = __floats2half2_rn(bf_hi(v.x), bf_hi(v.z));
-        h[2] = __floats2half2_rn(bf_lo(v.y), bf_lo(v.w));
-        h[3] = __floats2half2_rn(bf_hi(v.y), bf_hi(v.w));
-    } else {
-        h[0] = __floats2half2_rn(bf_lo(v.x), bf_hi(v.x));
-        h[1] = __floats2half2_rn(bf_lo(v.y), bf_hi(v.y));
-        h[2] = __floats2half2_rn(bf_lo(v.z), bf_hi(v.z));
-        h[3] = __floats2half2_rn(bf_lo(v.w), bf_hi(v.w));
-    }
-    return make_uint4(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]), *reinterpret_cast<uint32_t*>(&h[2]),
-                      *reinterpret_cast<uint32_t*>(&h[3]));
-}
+template <int WK> __device__ __forceinline__ uint4 sk_x_unit(const uint4& v) { return wide_unit(v, WK == WK_INT4_PACK); }
 
 /* weight row behind row r of tile t: plain tiles are 128 consecutive rows; SwiGLU tiles (ffn > 0: the matrix is
  * [gate rows | up rows], ffn of each) pair 64 gate rows with their 64 up rows.  Rows beyond the matrix repeat its
@@ -470,7 +456,9 @@ __global__ void __launch_bounds__(NT + 32, 1) k_skinny_tc(const void* __restrict
                 uint32_t v[32];
                 sk_tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0, v);
 #pragma unroll
-                for (int j = 0; j < 32; j++) ex[(lrow - 64) * (NB + 1) + col0 + j] = bf16_round(__fmul_rn(__uint_as_float(v[j]), rs));
+                for (int j = 0; j < 32; j++)
+                    if (col0 + j < NB * NBLK) /* 32 columns are read even where the batch has 16 */
+                        ex[(lrow - 64) * (NB + 1) + col0 + j] = bf16_round(__fmul_rn(__uint_as_float(v[j]), rs));
             }
         }
         __syncthreads();
@@ -765,6 +753,329 @@ extern "C" cudaError_t skinny_gemm_tc_swiglu(const LinRef* lin, const void* x, i
     return sk_entry(lin, x, M, lin->N / 2, h, nullptr, st);
 }
 
+/* ---- weights converted once ("wide"): the same products from resident f16 tiles --------------------------------
+ * What bounds k_skinny_tc is the instruction stream of its conversion, repeated every tick (8 instructions per weight at
+ * 0.4 per cycle and scheduler).  The model therefore keeps the converted tiles: per row tile the K-major core-matrix image
+ * of its slabs, 64 k x 128 rows = 16 KB each, exactly what a stage's A operand looks like, so a stage is two bulk copies and
+ * no thread touches an operand.  16 bits per weight instead of 4.5 or 8 is what the 180 GB are for; reading them is
+ * HBM-bound, which the conversion never was.  The operands, the order of the MMAs, the split of K and the epilogue are
+ * k_skinny_tc's: the results are the same bits; up to 256 rows go in one launch instead of two.
+ * Where K is split, a piece stores its f32 accumulator and leaves: the last piece of a tile used to add up to ten of
+ * them alone (30 us of the 57 at 128 rows), now the kernel that consumes the output does it beside its own loads
+ * (wide.cuh).  SwiGLU is spread over all threads through shared memory instead of two of four lane quarters.
+ * Measured (packed INT4, us, k_skinny_tc -> now): 19456 x 2560 with SwiGLU, 32 rows 39.2 -> 31.5, 128 rows 86.5 -> 38.4, 200 rows
+ * 367 -> 46; 2560 x 9728: 23.7 -> 14.3, 57.0 -> 15.6, 115 -> 18.9; 6144 x 2560: 19.7 -> 11.6, 46.4 -> 13.1, 117 -> 15.7.  Without
+ * its epilogue the largest takes 24.6 us for 100 MB, of which 6 are launch, TMEM and barrier set-up. */
+constexpr int WD_KC = 64, WD_A_BYTES = SK_BM * WD_KC * 2;
+constexpr int WD_EPI = 256;                    /* epilogue threads; a copying and an MMA warp besides */
+constexpr int WD_MAX_STAGES = 10;
+static_assert(SK_SUPER_K % WD_KC == 0, "a piece of K is whole slabs");
+
+__host__ __device__ inline size_t wide_tiles(int N, int ffn) { return ffn ? (size_t)(ffn + 63) / 64 : (size_t)(N + SK_BM - 1) / SK_BM; }
+
+/* one 16-byte unit (8 k of a row) per thread: [tile][k / 8][row] */
+template <int WK>
+__global__ void __launch_bounds__(256) k_wide_convert(const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift,
+                                                      int ffn, uint4* __restrict__ out, size_t units) {
+    const size_t u = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (u >= units) return;
+    const int r = (int)(u & (SK_BM - 1));
+    const size_t tk = u >> 7;
+    const int k8 = (int)(tk % (size_t)(K >> 3)), tile = (int)(tk / (size_t)(K >> 3));
+    const size_t row = (size_t)min(sk_row(tile, r, ffn), N - 1);
+    __half2 sc2 = __float2half2_rn(1.f);
+    if (WK != WK_INT8_CH) sc2 = __half2half2(static_cast<const __half*>(scales)[row * (size_t)(K >> gshift) + ((k8 * 8) >> gshift)]);
+    if (WK == WK_INT4_PACK) {
+        out[u] = sk_int4_chunk(static_cast<const uint32_t*>(w)[row * (size_t)(K >> 3) + k8], sc2);
+    } else {
+        const uint2 c = static_cast<const uint2*>(w)[row * (size_t)(K >> 3) + k8];
+        out[u] = sk_int8_chunk<WK == WK_INT8_GRP>(c.x, c.y, sc2);
+    }
+}
+
+/* activations [M, K] bf16 -> f16 units [k / 8][NB rows], rows beyond M zero; a thread per unit, 8 units of 4 rows per warp */
+template <int WK>
+__global__ void __launch_bounds__(256) k_wide_pack(const __nv_bfloat16* __restrict__ x, int M, int K, int lgNB, uint4* __restrict__ out) {
+    const int u = blockIdx.x * 256 + threadIdx.x, lane = u & 31, g = u >> 5;
+    const int rg = (1 << lgNB) >> 2;                 /* groups of four rows */
+    const int slab = g / rg, row = (g - slab * rg) * 4 + (lane >> 3), k8 = slab * 8 + (lane & 7);
+    if (slab >= (K >> 6)) return;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (row < M) v = __ldg(reinterpret_cast<const uint4*>(x + (size_t)row * K) + k8);
+    out[((size_t)k8 << lgNB) + row] = sk_x_unit<WK>(v);
+}
+
+struct WideArgs {
+    const unsigned char *wide, *xt;
+    const void* scales;
+    int N, K, M, ffn, lgNB, stages;
+    int n_split_tiles, KS;  /* the last row tiles have their K range in KS pieces, which come first in the grid */
+    __nv_bfloat16* y;       /* [M, N] or [M, ffn] */
+    uint4* tiled;           /* SwiGLU: result as units of the next linear, instead of y */
+    int tiled_int4;
+    float* partial;         /* [split tile][piece][M][128] */
+};
+
+/* SwiGLU results of rows r8 .. r8 + 7 of a tile's gate half, batch row m; g(r), u(r): the two products */
+template <class G, class U>
+__device__ __forceinline__ void wide_put_swiglu(const WideArgs& a, int tile, int r8, int m, G g, U u) {
+    const int gi = tile * 64 + r8;
+    uint32_t o[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const uint32_t v = __bfloat16_as_ushort(sk_swiglu(bf16_round(g(r8 + j)), bf16_round(u(r8 + j))));
+        o[j >> 1] |= v << (16 * (j & 1));
+    }
+    const uint4 q = make_uint4(o[0], o[1], o[2], o[3]);
+    if (a.tiled) { a.tiled[((size_t)(gi >> 3) << a.lgNB) + m] = wide_unit(q, a.tiled_int4); return; }
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        if (gi + j < a.ffn) a.y[(size_t)m * a.ffn + gi + j] = __ushort_as_bfloat16((unsigned short)(o[j >> 1] >> (16 * (j & 1))));
+}
+
+/* the split tiles of a SwiGLU pair, once their pieces are there; CTA = (split tile, batch row), a group of 8 rows per thread */
+template <int WK>
+__global__ void __launch_bounds__(32) k_wide_surplus(WideArgs a) {
+    const int stile = blockIdx.x, m = blockIdx.y * 4 + (threadIdx.x >> 3), r8 = (threadIdx.x & 7) * 8;
+    const int tile = (a.ffn + 63) / 64 - a.n_split_tiles + stile;
+    if (m >= a.M || tile * 64 + r8 >= a.ffn) return;
+    const float* at = a.partial + ((size_t)stile * a.KS * a.M + m) * SK_BM;
+    float g[8], u[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) { g[j] = 0.f; u[j] = 0.f; }
+    for (int q = 0; q < a.KS; q++) {
+        const float4* pg = reinterpret_cast<const float4*>(at + (size_t)q * a.M * SK_BM + r8);
+        const float4 g0 = __ldcg(pg), g1 = __ldcg(pg + 1), u0 = __ldcg(pg + 16), u1 = __ldcg(pg + 17);
+        g[0] += g0.x; g[1] += g0.y; g[2] += g0.z; g[3] += g0.w; g[4] += g1.x; g[5] += g1.y; g[6] += g1.z; g[7] += g1.w;
+        u[0] += u0.x; u[1] += u0.y; u[2] += u0.z; u[3] += u0.w; u[4] += u1.x; u[5] += u1.y; u[6] += u1.z; u[7] += u1.w;
+    }
+    if (WK == WK_INT8_CH)
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int gi = min(tile * 64 + r8 + j, a.ffn - 1);
+            g[j] = __fmul_rn(g[j], static_cast<const float*>(a.scales)[gi]);
+            u[j] = __fmul_rn(u[j], static_cast<const float*>(a.scales)[a.ffn + gi]);
+        }
+    wide_put_swiglu(a, tile, r8, m, [&](int r) { return g[r & 7]; }, [&](int r) { return u[r & 7]; });
+}
+
+template <int WK>
+__global__ void __launch_bounds__(WD_EPI + 64, 1) k_wide_tc(WideArgs a) {
+    const int lgNB = a.lgNB, stages = a.stages, K = a.K;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int NB = 1 << lgNB, b_bytes = NB * WD_KC * 2;
+    int* status = &g_sk_status;
+    unsigned char* stage_b0 = smem + stages * WD_A_BYTES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(stage_b0 + stages * b_bytes);
+    uint64_t* done = full + WD_MAX_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + WD_MAX_STAGES);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n_tiles = (int)wide_tiles(a.N, a.ffn), n_pieces = a.n_split_tiles * a.KS;
+    const bool piece = (int)blockIdx.x < n_pieces;
+    const int stile = piece ? (int)blockIdx.x / a.KS : 0, ks = piece ? (int)blockIdx.x % a.KS : 0;
+    const int tile = piece ? n_tiles - a.n_split_tiles + stile : (int)blockIdx.x - n_pieces;
+    int ncols = 32;
+    while (ncols < NB) ncols <<= 1;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < stages; i++) { mbar_init(full + i, 1); mbar_init(done + i, 1); }
+        mbar_init_fence();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    /* the K range of this CTA, cut where k_skinny_tc cuts it */
+    const int nsup_all = K / SK_SUPER_K, ksn = piece ? a.KS : 1;
+    const int sup_first = nsup_all * ks / ksn, nsup = nsup_all * (ks + 1) / ksn - sup_first;
+    const int it_first = sup_first * (SK_SUPER_K / WD_KC), nk = nsup * (SK_SUPER_K / WD_KC);
+    bool ok = true;
+    if (warp == WD_EPI / 32) { /* ---- the copying warp (its lane 0) */
+        if (lane == 0) {
+            const unsigned char* a_src = a.wide + ((size_t)tile * (size_t)(K / WD_KC) + (size_t)it_first) * WD_A_BYTES;
+            const unsigned char* b_src = a.xt + (size_t)it_first * (size_t)b_bytes;
+            int s = 0, issued = 0;
+            unsigned parity = 1; /* the stages start free */
+            for (int it = 0; it < nk; it++) {
+                if (!mbar_wait_bounded(done + s, parity, status)) { ok = false; break; }
+                mbar_expect_tx(full + s, (unsigned)(WD_A_BYTES + b_bytes));
+                tma_load_1d(smem + s * WD_A_BYTES, a_src + (size_t)it * WD_A_BYTES, WD_A_BYTES, full + s);
+                tma_load_1d(stage_b0 + s * b_bytes, b_src + (size_t)it * (size_t)b_bytes, (unsigned)b_bytes, full + s);
+                issued = it + 1;
+                if (++s == stages) { s = 0; parity ^= 1u; }
+            }
+            if (!ok) /* nothing of this thread's may be in flight past here: the last copies, with a limit of their own */
+                for (int k = issued > stages ? issued - stages : 0; k < issued; k++) {
+                    PipeDeadline dl;
+                    for (unsigned i = 0; i < PIPE_MBAR_TRIES && !mbar_try_wait(full + k % stages, (unsigned)(k / stages) & 1u); i++)
+                        if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
+                }
+        }
+        __syncwarp();
+    } else if (warp == WD_EPI / 32 + 1) { /* ---- the MMA warp (its lane 0) */
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
+        const uint64_t desc_a0 = sk_smem_desc(smem_u32(smem), SK_BM * 16, 128);
+        const uint64_t desc_b0 = sk_smem_desc(smem_u32(stage_b0), (uint32_t)NB * 16, 128);
+        int s = 0, issued = 0;
+        unsigned parity = 0;
+        for (int it = 0; it < nk; it++) {
+            ok = mbar_wait_bounded(full + s, parity, status);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (lane == 0) {
+                const uint64_t da0 = desc_a0 + (uint64_t)((s * WD_A_BYTES) >> 4), db0 = desc_b0 + (uint64_t)((s * b_bytes) >> 4);
+#pragma unroll
+                for (int kk = 0; kk < WD_KC / 16; kk++) {
+                    const uint32_t accumulate = (it > 0 || kk > 0) ? 1u : 0u;
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                        ::"r"(tmem), "l"(da0 + (uint64_t)(kk * 2 * SK_BM)), "l"(db0 + (uint64_t)(kk * 2 * NB)), "r"(idesc), "r"(accumulate) : "memory");
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(done + s)) : "memory");
+            }
+            __syncwarp();
+            issued = it + 1;
+            if (++s == stages) { s = 0; parity ^= 1u; }
+        }
+        if (!ok && issued > 0) { /* TMEM must not be freed under MMAs in flight: the last commit, with a limit of its own */
+            PipeDeadline dl;
+            for (unsigned i = 0; i < PIPE_MBAR_TRIES && !mbar_try_wait(done + (issued - 1) % stages, (unsigned)((issued - 1) / stages) & 1u); i++)
+                if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
+        }
+    }
+    /* the last commit covers every MMA before it */
+    if (ok) ok = mbar_wait_bounded(done + (nk - 1) % stages, (unsigned)((nk - 1) / stages) & 1u, status);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const bool all_ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    /* ---- warp w of the first eight reads TMEM lanes 32 (w % 4) .. + 31 = rows of the tile, the two warps of a lane
+     * quarter alternate over groups of 32 columns = batch rows */
+    float* const ex = reinterpret_cast<float*>(smem); /* SwiGLU: both products of the tile, [row][NB + 1] (the stages are free) */
+    if (all_ok && warp < WD_EPI / 32) {
+        const int lrow = (warp & 3) * 32 + lane, grow = sk_row(tile, lrow, a.ffn);
+        const float rs = WK == WK_INT8_CH ? static_cast<const float*>(a.scales)[min(grow, a.N - 1)] : 1.f;
+        for (int col0 = (warp >> 2) * 32; col0 < NB; col0 += WD_EPI / 128 * 32) {
+            if (col0 >= a.M) break;
+            uint32_t v[32];
+            sk_tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0, v);
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                const int m = col0 + j;
+                if (m >= a.M) continue;
+                if (piece) {
+                    __stcg(a.partial + (((size_t)stile * a.KS + ks) * a.M + m) * SK_BM + lrow, __uint_as_float(v[j]));
+                } else if (a.ffn) {
+                    ex[lrow * (NB + 1) + m] = __fmul_rn(__uint_as_float(v[j]), rs);
+                } else if (grow < a.N) {
+                    a.y[(size_t)m * a.N + grow] = f2bf(__fmul_rn(__uint_as_float(v[j]), rs));
+                }
+            }
+        }
+    }
+    if (a.ffn && !piece) {
+        __syncthreads();
+        if (all_ok)
+            for (int u = tid; u < 8 * a.M; u += WD_EPI + 64) { /* eight gate rows of one batch row per thread */
+                const int m = u >> 3, r8 = (u & 7) * 8;
+                if (tile * 64 + r8 < a.ffn)
+                    wide_put_swiglu(a, tile, r8, m, [&](int r) { return ex[r * (NB + 1) + m]; }, [&](int r) { return ex[(64 + r) * (NB + 1) + m]; });
+            }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+}
+
+extern "C" size_t wide_weight_bytes(const LinRef* lin, int ffn) { return wide_tiles(lin->N, ffn) * SK_BM * (size_t)lin->K * 2; }
+extern "C" int wide_serves(const LinRef* lin, int ffn) {
+    if (lin->K % SK_SUPER_K || ((uintptr_t)lin->w & 15)) return 0;
+    if (lin->kind != WK_INT8_CH && (lin->gshift < 4 || lin->gshift > 7)) return 0;
+    if (lin->kind == WK_INT4_PACK && lin->gshift < 5) return 0;
+    return !ffn || lin->N == 2 * ffn;
+}
+extern "C" cudaError_t wide_convert(const LinRef* lin, int ffn, void* out, cudaStream_t st) {
+    if (!wide_serves(lin, ffn)) return cudaErrorInvalidValue;
+    const size_t units = wide_weight_bytes(lin, ffn) / 16;
+    const unsigned grid = (unsigned)((units + 255) / 256);
+    switch (lin->kind) {
+    case WK_INT8_CH: k_wide_convert<WK_INT8_CH><<<grid, 256, 0, st>>>(lin->w, lin->scales, lin->N, lin->K, lin->gshift, ffn, (uint4*)out, units); break;
+    case WK_INT8_GRP: k_wide_convert<WK_INT8_GRP><<<grid, 256, 0, st>>>(lin->w, lin->scales, lin->N, lin->K, lin->gshift, ffn, (uint4*)out, units); break;
+    default: k_wide_convert<WK_INT4_PACK><<<grid, 256, 0, st>>>(lin->w, lin->scales, lin->N, lin->K, lin->gshift, ffn, (uint4*)out, units); break;
+    }
+    return cudaGetLastError();
+}
+extern "C" cudaError_t wide_pack(int kind, const void* x, int M, int K, void* xt, cudaStream_t st) {
+    if (M < 1 || M > 256 || K % 64) return cudaErrorInvalidValue;
+    const int lg = wide_lg(M);
+    const unsigned grid = (unsigned)((((size_t)(K >> 3) << lg) + 255) / 256);
+    if (kind == WK_INT4_PACK) k_wide_pack<WK_INT4_PACK><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, M, K, lg, (uint4*)xt);
+    else k_wide_pack<WK_INT8_CH><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, M, K, lg, (uint4*)xt);
+    return cudaGetLastError();
+}
+
+template <int WK>
+static cudaError_t wide_launch(const WideArgs& a, int grid, cudaStream_t st) {
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!attr_set[dev]) {
+        err = cudaFuncSetAttribute(k_wide_tc<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SK_SMEM_ONE);
+        if (err != cudaSuccess) return err;
+        attr_set[dev] = true;
+    }
+    k_wide_tc<WK><<<grid, WD_EPI + 64, (size_t)a.stages * (WD_A_BYTES + (WD_KC * 2 << a.lgNB)) + 256, st>>>(a);
+    if (a.ffn && a.n_split_tiles) k_wide_surplus<WK><<<dim3((unsigned)a.n_split_tiles, (unsigned)((a.M + 3) / 4)), 32, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+extern "C" cudaError_t wide_gemm(const LinRef* lin, const void* wide, const void* xt, int M, int ffn, void* y, void* h_tiled, int h_kind, WidePart* part,
+                                 cudaStream_t st) {
+    if (!lin || !wide || !xt || M < 1 || M > 256 || !wide_serves(lin, ffn) || (h_tiled && !ffn)) return cudaErrorInvalidValue;
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    SkPlan p;
+    bool ok = false;
+    const int mp = M < 128 ? M : 128; /* k_skinny_tc takes 128 rows at a time: the split of K it would choose */
+    switch (lin->kind) {
+    case WK_INT8_CH: ok = sk_plan<WK_INT8_CH>(lin->N, lin->K, mp, g_partial_rows[dev], ffn, &p); break;
+    case WK_INT8_GRP: ok = sk_plan<WK_INT8_GRP>(lin->N, lin->K, mp, g_partial_rows[dev], ffn, &p); break;
+    case WK_INT4_PACK: ok = sk_plan<WK_INT4_PACK>(lin->N, lin->K, mp, g_partial_rows[dev], ffn, &p); break;
+    }
+    /* without SwiGLU either all tiles are split, for the consumer to add, or none */
+    if (!ok || (!ffn && p.S && (p.S != p.tiles || !part))) return cudaErrorInvalidValue;
+    if ((size_t)p.S * p.KS * M * SK_BM > (size_t)SK_SCRATCH_FLOATS_PER_ROW * g_partial_rows[dev]) return cudaErrorInvalidValue;
+    WideArgs a = {};
+    a.wide = (const unsigned char*)wide; a.xt = (const unsigned char*)xt;
+    a.scales = lin->scales;
+    a.N = lin->N; a.K = lin->K; a.M = M; a.ffn = ffn; a.lgNB = wide_lg(M); a.n_split_tiles = p.S; a.KS = p.KS;
+    a.y = (__nv_bfloat16*)y;
+    a.tiled = (uint4*)h_tiled;
+    a.tiled_int4 = h_kind == WK_INT4_PACK;
+    a.partial = g_partial[dev];
+    a.stages = (int)((SK_SMEM_ONE - 256) / (WD_A_BYTES + (WD_KC * 2 << a.lgNB)));
+    if (a.stages > WD_MAX_STAGES) a.stages = WD_MAX_STAGES;
+    if (part) {
+        *part = WidePart();
+        if (p.S && !ffn) {
+            part->partial = g_partial[dev];
+            part->scales = lin->kind == WK_INT8_CH ? (const float*)lin->scales : nullptr;
+            part->pieces = p.KS; part->M = M;
+        }
+    }
+    switch (lin->kind) {
+    case WK_INT8_CH: return wide_launch<WK_INT8_CH>(a, p.grid, st);
+    case WK_INT8_GRP: return wide_launch<WK_INT8_GRP>(a, p.grid, st);
+    default: return wide_launch<WK_INT4_PACK>(a, p.grid, st);
+    }
+}
+
 /* ---- prompt-sized inputs (prefill): M rows in blocks of 256 ------------------------------------------------
  * What this replaces: the reference dequantises the whole layer to bf16 and calls cuBLAS for M > 16
  * (src/sched/gemm.c:467-490; its own S2P_PREFILL_TC path, :458-466, serves M <= 128 only).  Here the packed
@@ -876,6 +1187,11 @@ extern "C" cudaError_t skinny_prefill_tc(const LinRef* lin, const void* x, int M
 }
 
 /* status word of the launches so far on the current device (0 = no wait ever gave up); synchronises */
+extern "C" cudaError_t skinny_status_async(int* host, cudaStream_t st) {
+    void* sp = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&sp, g_sk_status);
+    return e != cudaSuccess ? e : cudaMemcpyAsync(host, sp, sizeof(int), cudaMemcpyDeviceToHost, st);
+}
 extern "C" cudaError_t skinny_status(int* out) { return cudaMemcpyFromSymbol(out, g_sk_status, sizeof(int)); }
 
 }  // namespace s2p

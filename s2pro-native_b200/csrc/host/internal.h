@@ -28,6 +28,8 @@ typedef struct {
     /* backbone: bf16 copies of the four quantised matrices (wqkv, wo, gate_up, w2) for prompt slices, in the model's
      * `wide_weights`; NULL where there are none */
     void* wide[4];
+    /* f16 tiles of the four matrices for batches on the tensor cores (wide_gemm), in the model's `tc_weights`; NULL: none */
+    void* tc[4];
 } s2p_layer;
 
 /* host sampler parameters and history mirror (reference: src/slowar/slowar_internal.h:40-55) */
@@ -80,6 +82,8 @@ struct s2p_model {
     s2p_layer slow[S2P_SLOW_LAYERS];
     s2p_tensor final_norm;
     void* wide_weights;
+    void *tc_weights, *tc_fast_out;
+    void *xt_norm, *xt_attn, *xt_ffn; /* a batch's activations as matrix units, one buffer per linear input */
     s2p_layer fast[S2P_FAST_LAYERS];
     s2p_tensor fast_norm, cb_emb, fast_emb;
     s2p_linear fast_out;
@@ -103,6 +107,7 @@ struct s2p_model {
     size_t out_bytes, off_sem, off_ocodes, off_eos;
     void *d_out, *h_out;
     int* h_prefill_status;          /* pinned copy of the prompt attention's status word */
+    int* h_tc_status;               /* ... and of the batched tensor-core linears' */
     /* one executable graph per steady batch size */
     cudaGraphExec_t gexec[S2P_MAX_BATCH + 1];
     unsigned char gready[S2P_MAX_BATCH + 1];

@@ -187,7 +187,9 @@ static s2p_status alloc_workspace(s2p_model* m) {
     m->out_bytes = align_up(m->off_eos + (size_t)B, 16);
     S2P_CUDA_TRY(cudaMalloc(&m->d_out, m->out_bytes));
     S2P_CUDA_TRY(cudaMallocHost(&m->h_out, m->out_bytes));
-    S2P_CUDA_TRY(cudaMallocHost((void**)&m->h_prefill_status, sizeof(int)));
+    S2P_CUDA_TRY(cudaMallocHost((void**)&m->h_prefill_status, 2 * sizeof(int)));
+    m->h_tc_status = m->h_prefill_status + 1;
+    *m->h_tc_status = 0;
     return S2P_OK;
 }
 
@@ -217,6 +219,50 @@ static s2p_status widen_backbone(s2p_model* m) {
             S2P_TRY(s2p_linear_dequant(lin[i], at, m->stream));
             m->slow[l].wide[i] = at;
             at += align_up((size_t)lin[i]->in_features * lin[i]->out_features * 2, 256);
+        }
+    }
+    return S2P_OK;
+}
+
+/* f16 tiles of every linear of both stacks and of the fast head, for ticks of more than 16 rows (wide_gemm): 8.1 GB for the
+ * full model, and 8.4 MB for the activations.  Same rule as above; without them such ticks convert weights as they go. */
+static s2p_status tile_linears(s2p_model* m) {
+    size_t bytes = 0, free_b = 0, total_b = 0;
+    LinRef lr;
+    if (m->max_sessions <= S2P_INT8_GEMV_MAX_M) return S2P_OK;
+    for (int l = 0; l <= m->n_slow + S2P_FAST_LAYERS; l++) {
+        s2p_layer* L = l < m->n_slow ? &m->slow[l] : &m->fast[l - m->n_slow];
+        const s2p_linear* lin[4] = {&L->wqkv, &L->wo, &L->gate_up, &L->w2};
+        const int head = l == m->n_slow + S2P_FAST_LAYERS;
+        for (int i = 0; i < (head ? 1 : 4); i++) {
+            const s2p_linear* q = head ? &m->fast_out : lin[i];
+            s2p_lin_ref(q, &lr);
+            if (!q->int8_ready || !wide_serves(&lr, i == 2 ? S2P_FFN_DIM : 0)) return S2P_OK;
+            bytes += wide_weight_bytes(&lr, i == 2 ? S2P_FFN_DIM : 0);
+        }
+    }
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 8) return S2P_OK;
+    const size_t xb = (size_t)2 * S2P_MAX_BATCH;
+    if (cudaMalloc(&m->tc_weights, bytes) != cudaSuccess || cudaMalloc(&m->xt_norm, xb * (S2P_DIM + S2P_Q_WIDTH + S2P_FFN_DIM)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (m->tc_weights) cudaFree(m->tc_weights);
+        m->tc_weights = m->xt_norm = NULL;
+        return S2P_OK;
+    }
+    S2P_CUDA_TRY(cudaMemsetAsync(m->xt_norm, 0, xb * (S2P_DIM + S2P_Q_WIDTH + S2P_FFN_DIM), m->stream));
+    m->xt_attn = (char*)m->xt_norm + xb * S2P_DIM;
+    m->xt_ffn = (char*)m->xt_attn + xb * S2P_Q_WIDTH;
+    char* at = (char*)m->tc_weights;
+    for (int l = 0; l <= m->n_slow + S2P_FAST_LAYERS; l++) {
+        s2p_layer* L = l < m->n_slow ? &m->slow[l] : &m->fast[l - m->n_slow];
+        const s2p_linear* lin[4] = {&L->wqkv, &L->wo, &L->gate_up, &L->w2};
+        const int head = l == m->n_slow + S2P_FAST_LAYERS;
+        for (int i = 0; i < (head ? 1 : 4); i++) {
+            s2p_lin_ref(head ? &m->fast_out : lin[i], &lr);
+            S2P_CUDA_TRY(wide_convert(&lr, i == 2 ? S2P_FFN_DIM : 0, at, m->stream));
+            if (head) m->tc_fast_out = at;
+            else L->tc[i] = at;
+            at += wide_weight_bytes(&lr, i == 2 ? S2P_FFN_DIM : 0);
         }
     }
     return S2P_OK;
@@ -336,7 +382,7 @@ s2p_status s2p_model_load(const char* model_dir, const s2p_model_opts* opts, s2p
         if (rc != S2P_OK) goto fail;
     }
     if ((rc = alloc_workspace(m)) != S2P_OK) goto fail;
-    if (m->mode == S2P_GEMM_INT8 && (rc = widen_backbone(m)) != S2P_OK) goto fail;
+    if (m->mode == S2P_GEMM_INT8 && ((rc = widen_backbone(m)) != S2P_OK || (rc = tile_linears(m)) != S2P_OK)) goto fail;
     if (cudaEventCreate(&m->ev0) != cudaSuccess || cudaEventCreate(&m->ev1) != cudaSuccess) { rc = S2P_ERR_CUDA; goto fail; }
     if (cudaStreamSynchronize(m->stream) != cudaSuccess) { rc = S2P_ERR_CUDA; goto fail; }
     s2p_st_close(st);
@@ -379,6 +425,8 @@ void s2p_model_free(s2p_model* m) {
     for (size_t i = 0; i < sizeof(ts) / sizeof(ts[0]); i++) s2p_tensor_free(ts[i]);
     s2p_linear_free(&m->fast_out);
     if (m->wide_weights) cudaFree(m->wide_weights);
+    if (m->tc_weights) cudaFree(m->tc_weights);
+    if (m->xt_norm) cudaFree(m->xt_norm);
     if (m->attn_ctr) cudaFree(m->attn_ctr);
     if (m->d_mega_stages) cudaFree(m->d_mega_stages);
     if (m->d_mega_sync) cudaFree(m->d_mega_sync);

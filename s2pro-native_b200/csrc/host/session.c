@@ -201,15 +201,11 @@ static int attn_workers_for(int rows) {
     return w < 1 ? 1 : (w > 16 ? 16 : w);
 }
 
-/* x: residual stream [rows, 2560], `norm` its norm with the layer's first gain; scratch tensors: qkv/q/attn/proj/gu/hff.
- * Leaves the norm with the gain `next` (NULL: none) in `next_out`. */
-static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ctx* c, s2p_dev_bf16* x,
-                                s2p_dev_bf16* norm, s2p_dev_bf16* qkv, s2p_dev_bf16* q, s2p_dev_bf16* attn,
-                                s2p_dev_bf16* proj, s2p_dev_bf16* gu, s2p_dev_bf16* hff, const void* next,
-                                s2p_dev_bf16* next_out) {
+/* head norms, RoPE, cache append and attention of one layer; the projection is qkv, or left in partials */
+static s2p_status layer_attention(s2p_model* m, const s2p_layer* L, const layer_ctx* c, s2p_dev_bf16* qkv, const WidePart* part, s2p_dev_bf16* q,
+                                  s2p_dev_bf16* attn) {
     cudaStream_t st = m->stream;
     const int rows = c->rows;
-    S2P_TRY(lin_apply(m, &L->wqkv, L->wide[0], norm, qkv, rows, c->decode));
     QkvPostArgs qa;
     memset(&qa, 0, sizeof(qa));
     qa.qkv = qkv; qa.q = q;
@@ -217,7 +213,7 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
     qa.eps = S2P_NORM_EPS; qa.rope_base = S2P_ROPE_BASE;
     qa.q_heads = S2P_SLOW_Q_HEADS; qa.kv_heads = S2P_SLOW_KV_HEADS; qa.max_seq = c->max_seq; qa.kv8 = c->kv8;
     qa.pos0 = c->pos0; qa.pos_row_step = c->pos_row_step; qa.pos_arr = c->pos_arr; qa.kv = c->kv;
-    S2P_LAUNCH(m, qkv_post(&qa, rows, st));
+    S2P_LAUNCH(m, qkv_post_part(&qa, part, rows, st));
     AttnArgs aa;
     memset(&aa, 0, sizeof(aa));
     aa.q = q; aa.out = attn;
@@ -231,6 +227,19 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
     } else {
         S2P_LAUNCH(m, attn_single(&aa, rows, st));
     }
+    return S2P_OK;
+}
+
+/* x: residual stream [rows, 2560], `norm` its norm with the layer's first gain; scratch tensors: qkv/q/attn/proj/gu/hff.
+ * Leaves the norm with the gain `next` (NULL: none) in `next_out`. */
+static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ctx* c, s2p_dev_bf16* x,
+                                s2p_dev_bf16* norm, s2p_dev_bf16* qkv, s2p_dev_bf16* q, s2p_dev_bf16* attn,
+                                s2p_dev_bf16* proj, s2p_dev_bf16* gu, s2p_dev_bf16* hff, const void* next,
+                                s2p_dev_bf16* next_out) {
+    cudaStream_t st = m->stream;
+    const int rows = c->rows;
+    S2P_TRY(lin_apply(m, &L->wqkv, L->wide[0], norm, qkv, rows, c->decode));
+    S2P_TRY(layer_attention(m, L, c, qkv, NULL, q, attn));
     S2P_TRY(lin_add_norm(m, &L->wo, L->wide[1], attn, x, proj, L->ffn_norm.data, norm, rows, c->decode));
     if (c->decode && m->mode == S2P_GEMM_INT8 && L->gate_up.int8_ready && s2p_linear_rows_on_tc(&L->gate_up, rows) &&
         L->gate_up.out_features == 2 * S2P_FFN_DIM) {
@@ -243,6 +252,30 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
     S2P_TRY(lin_add_norm(m, &L->w2, L->wide[3], hff, x, proj, next, next_out, rows, c->decode));
     return S2P_OK;
 }
+
+/* A decode layer of a batch on the tensor cores with resident f16 tiles: the activations between the linears travel as matrix
+ * units, and outputs whose K range was split are added by the kernel that consumes them.  On entry m->xt_norm holds the norm of x
+ * with the layer's first gain; on exit, unless next is NULL, the norm with the gain `next`, as units of a linear of kind
+ * next_kind (in m->xt_norm) or, next_out given, as bf16 there. */
+static s2p_status layer_wide(s2p_model* m, const s2p_layer* L, const layer_ctx* c, s2p_dev_bf16* x, s2p_dev_bf16* qkv, s2p_dev_bf16* q,
+                             s2p_dev_bf16* attn, s2p_dev_bf16* proj, const void* next, int next_kind, void* next_out) {
+    cudaStream_t st = m->stream;
+    const int rows = c->rows;
+    LinRef wqkv, wo, gate_up, w2;
+    s2p_lin_ref(&L->wqkv, &wqkv); s2p_lin_ref(&L->wo, &wo); s2p_lin_ref(&L->gate_up, &gate_up); s2p_lin_ref(&L->w2, &w2);
+    WidePart part;
+    S2P_LAUNCH(m, wide_gemm(&wqkv, L->tc[0], m->xt_norm, rows, 0, qkv, NULL, 0, &part, st));
+    S2P_TRY(layer_attention(m, L, c, qkv, part.partial ? &part : NULL, q, attn));
+    S2P_LAUNCH(m, wide_pack(wo.kind, attn, rows, S2P_Q_WIDTH, m->xt_attn, st));
+    S2P_LAUNCH(m, wide_gemm(&wo, L->tc[1], m->xt_attn, rows, 0, proj, NULL, 0, &part, st));
+    S2P_LAUNCH(m, wide_norm(x, &part, proj, x, L->ffn_norm.data, NULL, m->xt_norm, gate_up.kind, rows, st));
+    m->tick_kernels += 1; /* the tiles of the pair whose K range is split are a launch of their own */
+    S2P_LAUNCH(m, wide_gemm(&gate_up, L->tc[2], m->xt_norm, rows, S2P_FFN_DIM, NULL, m->xt_ffn, w2.kind, NULL, st));
+    S2P_LAUNCH(m, wide_gemm(&w2, L->tc[3], m->xt_ffn, rows, 0, proj, NULL, 0, &part, st));
+    if (next) S2P_LAUNCH(m, wide_norm(x, &part, proj, x, next, next_out, next_out ? NULL : m->xt_norm, next_kind, rows, st));
+    return S2P_OK;
+}
+static int wide_rows(const s2p_model* m, int rows) { return m->tc_weights && s2p_linear_rows_on_tc(&m->slow[0].wqkv, rows); }
 
 static void slow_kv_offsets(const s2p_model* m, int layer, KvRef* kv) {
     const size_t plane = s2p_kv_plane_bytes(m), splane = s2p_kvs_plane_bytes(m);
@@ -517,6 +550,39 @@ static s2p_status head_and_sample(s2p_model* m, const tick_dev* d, int nact, int
 }
 
 /* fast-AR frame, general sequence (src/fastar/fastar.cu:726-788) */
+static s2p_status fast_frame_wide(s2p_model* m, const tick_dev* d, int nact) {
+    cudaStream_t st = m->stream;
+    layer_ctx c;
+    memset(&c, 0, sizeof(c));
+    c.rows = nact; c.max_seq = S2P_FAST_SEQ; c.kv8 = 0; c.pos_row_step = 0; c.decode = 1; c.split_k = 0;
+    LinRef first, head, lr;
+    WidePart part;
+    s2p_lin_ref(&m->fast[0].wqkv, &first);
+    s2p_lin_ref(&m->fast_out, &head);
+    S2P_LAUNCH(m, wide_norm(m->shidden.data, NULL, NULL, m->fx.data, m->fast[0].attn_norm.data, NULL, m->xt_norm, first.kind, nact, st));
+    for (int cb = 0; cb < S2P_NUM_CODEBOOKS; cb++) {
+        c.pos0 = cb;
+        for (int l = 0; l < S2P_FAST_LAYERS; l++) {
+            const int last = l + 1 == S2P_FAST_LAYERS;
+            fast_kv_ref(m, l, &c.kv);
+            if (last) lr = head;
+            else s2p_lin_ref(&m->fast[l + 1].wqkv, &lr);
+            /* the prime pass produces no logits: nothing follows its last layer */
+            S2P_TRY(layer_wide(m, &m->fast[l], &c, BF(m->fx), BF(m->fqkv), BF(m->fq), BF(m->fattn), BF(m->fproj),
+                               !last ? m->fast[l + 1].attn_norm.data : cb ? m->fast_norm.data : NULL, lr.kind, NULL));
+        }
+        if (cb == 0) { /* step 1 is fed embeddings[sem] */
+            S2P_LAUNCH(m, wide_embed_norm(m->fast_emb.data, d->sem, NULL, NULL, NULL, m->fx.data, m->fast[0].attn_norm.data, m->xt_norm, first.kind, nact, st));
+        } else {
+            S2P_LAUNCH(m, wide_gemm(&head, m->tc_fast_out, m->xt_norm, nact, 0, m->flogits.data, NULL, 0, &part, st));
+            S2P_LAUNCH(m, wide_embed_norm(m->fast_emb.data, NULL, &part, m->flogits.data, m->fstage + (size_t)(cb - 1) * nact, m->fx.data,
+                                          cb < S2P_NUM_CODEBOOKS - 1 ? m->fast[0].attn_norm.data : NULL, m->xt_norm, first.kind, nact, st));
+        }
+    }
+    S2P_LAUNCH(m, pack_frame(m->fstage, nact, d->ocodes, st));
+    return S2P_OK;
+}
+
 static s2p_status fast_frame_general(s2p_model* m, const tick_dev* d, int nact, int dump_ok) {
     cudaStream_t st = m->stream;
     layer_ctx c;
@@ -567,20 +633,32 @@ static s2p_status tick_general(s2p_model* m, s2p_session* const* act, int bd, in
         memset(&c, 0, sizeof(c));
         c.rows = bd; c.kv.bases = d.kv_bases; c.kv.sbases = d.kvs_bases;
         c.max_seq = m->ctx_len; c.kv8 = m->kv8; c.pos_arr = d.pos; c.split_k = 1; c.decode = 1;
-        S2P_LAUNCH(m, rms_norm(m->sx.data, m->slow[0].attn_norm.data, m->snorm.data, bd, S2P_DIM, S2P_NORM_EPS, st));
+        const int wide = wide_rows(m, bd);
+        LinRef lr;
+        s2p_lin_ref(&m->slow[0].wqkv, &lr);
+        if (wide) S2P_LAUNCH(m, wide_norm(m->sx.data, NULL, NULL, NULL, m->slow[0].attn_norm.data, NULL, m->xt_norm, lr.kind, bd, st));
+        else S2P_LAUNCH(m, rms_norm(m->sx.data, m->slow[0].attn_norm.data, m->snorm.data, bd, S2P_DIM, S2P_NORM_EPS, st));
         for (int l = 0; l < m->n_slow; l++) {
             const int last = l + 1 == m->n_slow;
+            const void* next = last ? m->final_norm.data : m->slow[l + 1].attn_norm.data;
             slow_kv_offsets(m, l, &c.kv);
-            S2P_TRY(layer_general(m, &m->slow[l], &c, BF(m->sx), BF(m->snorm), BF(m->sqkv), BF(m->sq), BF(m->sattn),
-                                  BF(m->sproj), BF(m->sgu), BF(m->sffn), last ? m->final_norm.data : m->slow[l + 1].attn_norm.data,
-                                  last ? BF(m->shidden) : BF(m->snorm)));
+            if (wide) {
+                if (!last) s2p_lin_ref(&m->slow[l + 1].wqkv, &lr);
+                S2P_TRY(layer_wide(m, &m->slow[l], &c, BF(m->sx), BF(m->sqkv), BF(m->sq), BF(m->sattn), BF(m->sproj), next, lr.kind,
+                                   last ? m->shidden.data : NULL));
+            } else {
+                S2P_TRY(layer_general(m, &m->slow[l], &c, BF(m->sx), BF(m->snorm), BF(m->sqkv), BF(m->sq), BF(m->sattn),
+                                      BF(m->sproj), BF(m->sgu), BF(m->sffn), next, last ? BF(m->shidden) : BF(m->snorm)));
+            }
         }
     }
     for (int b = bd; b < nact; b++) /* freshly prefilled rows sample from their stashed hidden (eager only) */
         S2P_CUDA_TRY(cudaMemcpyAsync(BF(m->shidden) + (size_t)b * S2P_DIM, act[b]->pending_hidden,
                                      (size_t)S2P_DIM * 2, cudaMemcpyDeviceToDevice, st));
     S2P_TRY(head_and_sample(m, &d, nact, 1));
-    S2P_TRY(fast_frame_general(m, &d, nact, 1));
+    if (wide_rows(m, nact)) S2P_TRY(fast_frame_wide(m, &d, nact));
+    else S2P_TRY(fast_frame_general(m, &d, nact, 1));
+    S2P_CUDA_TRY(skinny_status_async(m->h_tc_status, st));
     S2P_CUDA_TRY(cudaMemcpyAsync(m->h_out, m->d_out, m->out_bytes, cudaMemcpyDeviceToHost, st));
     return S2P_OK;
 }
@@ -1103,8 +1181,7 @@ s2p_status s2p_model_batch_next_frame(s2p_model* m, s2p_session** sess, int n, i
     if (!mega && m->n_slow > 0 && m->mode == S2P_GEMM_INT8 && m->slow[0].wqkv.int8_ready &&
         s2p_linear_rows_on_tc(&m->slow[0].wqkv, nact)) {
         /* the batched linears ran on the tensor-core kernel: a bounded wait that gave up inside it left a code */
-        int sk = 0;
-        S2P_CUDA_TRY(skinny_status(&sk));
+        const int sk = *m->h_tc_status;
         if (sk != 0) {
             fprintf(stderr, "[s2pro] batched tensor-core linear gave up on a bounded wait (code %d); the frame is lost and later "
                             "batched ticks use the exact-order kernel\n", sk);
