@@ -10,6 +10,7 @@
  */
 #include <stdio.h>
 #include "gemv.cuh"
+#include "packed.cuh"
 #include "s2p_b200_abi.h"
 
 namespace s2p {
@@ -105,231 +106,209 @@ extern "C" cudaError_t gemv_setup_all(void) {
 }
 
 /* ---- exact-order small batch (2 <= M <= 16) -------------------------------
- * One warp per output row; lane l owns k = 512 i + 16 l .. +15.  The 16 codes
- * of a tile are widened once, then each of the M activation rows runs its own
- * 16-term fma chain and tile fold, exactly as for M == 1. */
-template <int WK>
-__device__ __forceinline__ void widen16(const typename LaneTile<WK>::type& t, float* w16);
-template <>
-__device__ __forceinline__ void widen16<WK_INT4_PACK>(const uint2& t, float* w16) {
-    const uint32_t u[2] = {t.x ^ 0x88888888u, t.y ^ 0x88888888u};
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const uint32_t e = u[h] & 0x0F0F0F0Fu, o = (u[h] >> 4) & 0x0F0F0F0Fu;
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            w16[h * 8 + 2 * b] = biased_byte_to_f32(e, b, 8388616.0f);
-            w16[h * 8 + 2 * b + 1] = biased_byte_to_f32(o, b, 8388616.0f);
-        }
+ * Lane l owns k = 512 i + 16 l .. +15 of every tile i, as for M == 1; a warp carries four weight rows and MM activation
+ * rows, 4 x MM independent chains.
+ *
+ * What bounds it: fp32 fma and what surrounds one.  Two activation rows share a register pair, so a chain step is packed
+ * (fma.rn.f32x2: two independent roundings, the same bits as fmaf on either half); an activation becomes f32 with one
+ * instruction, a code (a byte planted in the mantissa of 2^23 twice and one packed subtraction, exact) once per MM activation rows.
+ * The chains of a k advance side by side, because each waits for its own previous step.  Weights go from DRAM to registers a tile
+ * ahead; the activations of a tile are shared by the SM's warps through L1.
+ *
+ * A matrix of few rows does not fill the GPU with warps of four rows, and a lone warp per scheduler waits on its own
+ * latencies.  There NS = 4 warps share four rows and take tiles in turn; the tiles' chain results meet in shared memory and each warp
+ * folds a quarter of the activation rows, tiles ascending.
+ * Measured, us for one layer's four matrices (N x K 6144 x 2560, 2560 x 4096, 19456 x 2560, 2560 x 9728), before (scalar fma, one
+ * weight row per warp for INT8; mixed bf16 fma, one to four for INT4) and now, at 2 / 4 / 8 / 16 rows:
+ *   INT8  52 / 84 / 148 / 258 -> 44 / 56 / 83 / 138      INT4  46 / 70 / 103 / 180 -> 46 / 58 / 85 / 144
+ * 16 rows of 19456 x 2560 run at 13.5 T fma/s; the pipe's rate is 36 T. */
+template <int WK> struct BatchCodes;
+template <> struct BatchCodes<WK_INT8_CH> {
+    static __device__ __forceinline__ f32x2 twice(uint32_t u, uint32_t sel, float minus) {
+        const float f = __uint_as_float(__byte_perm(u, 0x4B000000u, sel));
+        return fadd2(pack2(f, f), pack2(minus, minus));
     }
-}
-template <>
-__device__ __forceinline__ void widen16<WK_INT8_CH>(const uint4& t, float* w16) {
-    const uint32_t u[4] = {t.x ^ 0x80808080u, t.y ^ 0x80808080u, t.z ^ 0x80808080u, t.w ^ 0x80808080u};
+    /* codes k = 8 h + 0..7 of a lane as f32 pairs of equals */
+    static __device__ __forceinline__ void widen8(const uint4& a, int h, f32x2 (&w)[8]) {
+        const uint32_t u[2] = {s8x4_bias(h ? a.z : a.x), s8x4_bias(h ? a.w : a.y)};
 #pragma unroll
-    for (int h = 0; h < 4; h++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) w16[h * 4 + b] = biased_byte_to_f32(u[h], b, 8388736.0f);
-}
-template <>
-__device__ __forceinline__ void widen16<WK_INT8_GRP>(const uint4& t, float* w16) { widen16<WK_INT8_CH>(t, w16); }
-
-template <int WK, int MM>
-__global__ void __launch_bounds__(256) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
-                                                    const void* __restrict__ w, const void* __restrict__ scales,
-                                                    int M, int N, int K, int gshift) {
-    typedef typename LaneTile<WK>::type tile_t;
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const size_t row_bytes = (WK == WK_INT4_PACK) ? (size_t)(K >> 1) : (size_t)K;
-    const int T = K >> 9;
-    /* the grid's y dimension walks groups of MM activation rows (see k_gemv_batch_i4) */
-    x += (size_t)blockIdx.y * MM * K;
-    y += (size_t)blockIdx.y * MM * N;
-    M = min(MM, M - (int)blockIdx.y * MM);
-    for (int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; n < N; n += warps) {
-        const unsigned char* wrow = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes;
-        float acc[MM];
-#pragma unroll
-        for (int m = 0; m < MM; m++) acc[m] = 0.f;
-        tile_t nxt = *reinterpret_cast<const tile_t*>(wrow + (size_t)lane * sizeof(tile_t));
-        for (int i = 0; i < T; i++) {
-            const tile_t cur = nxt;
-            if (i + 1 < T)
-                nxt = *reinterpret_cast<const tile_t*>(wrow + (size_t)(i + 1) * 32 * sizeof(tile_t) +
-                                                       (size_t)lane * sizeof(tile_t));
-            const int k0 = i * 512 + lane * 16;
-            float gs = 1.f;
-            if (WK != WK_INT8_CH)
-                gs = __half2float(static_cast<const __half*>(scales)[(size_t)n * (K >> gshift) + (k0 >> gshift)]);
-            float w16[16];
-            widen16<WK>(cur, w16);
-#pragma unroll
-            for (int m = 0; m < MM; m++) {
-                if (m < M) {
-                    const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)m * K + k0);
-                    const uint4 xa = xp[0], xb = xp[1];
-                    const uint32_t xu[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-                    float s = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        s = __fmaf_rn(w16[2 * j], bf_bits_to_f32(xu[j] & 0xffffu), s);
-                        s = __fmaf_rn(w16[2 * j + 1], __uint_as_float(xu[j] & 0xffff0000u), s);
-                    }
-                    if (WK == WK_INT8_CH) acc[m] += s;
-                    else acc[m] = __fmaf_rn(s, gs, acc[m]);
-                }
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < MM; m++) {
-            float a = warp_tree_sum(acc[m]);
-            if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[n]);
-            if (lane == 0 && m < M) y[(size_t)m * N + n] = f2bf(a);
-        }
+        for (int j = 0; j < 8; j++) w[j] = twice(u[j >> 2], 0x7440u + (j & 3), -8388736.0f);
     }
-}
+};
+template <> struct BatchCodes<WK_INT8_GRP> : BatchCodes<WK_INT8_CH> {};
+template <> struct BatchCodes<WK_INT4_PACK> {
+    static __device__ __forceinline__ void widen8(const uint2& a, int h, f32x2 (&w)[8]) {
+        const uint32_t u = h ? a.y : a.x; /* two's complement nibble -> code + 8, even and odd k apart */
+        const uint32_t e = (u & 0x0F0F0F0Fu) ^ 0x08080808u, o = ((u >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+#pragma unroll
+        for (int j = 0; j < 8; j++) w[j] = BatchCodes<WK_INT8_CH>::twice(j & 1 ? o : e, 0x7440u + (j >> 1), -8388616.0f);
+    }
+};
 
-/* The same for packed INT4, R weight rows per warp: the 16 codes of each row's tile become bf16 once
- * (exact), an activation row's 16 values are loaded once for the R rows, and every (row, activation row)
- * pair runs its own chain of mixed-precision fmas (bf16 x bf16 exact, f32 accumulate: bit for bit
- * fmaf((float)w, (float)x, s)).  Loading the activations once per R rows is what matters: a lockstep
- * batch reads M x 32 bytes per lane and tile, which otherwise bounds the kernel by L1 bandwidth. */
-template <int MM, int R>
-__global__ void __launch_bounds__(256) k_gemv_batch_i4(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
-                                                       const unsigned char* __restrict__ w, const __half* __restrict__ scales,
+template <int WK, int MM, int NS>
+__global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+                                                       const void* __restrict__ w, const void* __restrict__ scales,
                                                        int M, int N, int K, int gshift) {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const size_t row_bytes = (size_t)(K >> 1);
+    typedef typename LaneTile<WK>::type tile_t;
+    constexpr int R = 4, P = MM / 2; /* weight rows of a warp, pairs of activation rows */
+    constexpr int PD = WK == WK_INT4_PACK && MM <= 4 ? 2 : 1; /* tiles of weights under way */
+    constexpr int FM = NS == 1 ? MM : (MM + NS - 1) / NS; /* activation rows whose sums this warp keeps */
+    __shared__ float part[NS == 1 ? 1 : 2 * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][m, then the scales][row][lane] */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n0 = (blockIdx.x * (4 / NS) + warp / NS) * R, ns = warp % NS;
+    if (n0 >= N) return; /* NS > 1: uniform over the CTA */
+    const size_t row_bytes = (WK == WK_INT4_PACK) ? (size_t)(K >> 1) : (size_t)K;
     const int T = K >> 9, spr = K >> gshift;
-    /* the grid's y dimension walks groups of MM activation rows: a matrix of few rows gets enough warps that way
-     * while every warp still carries R weight rows per activation load (each (m, n) chain is untouched by it) */
-    x += (size_t)blockIdx.y * MM * K;
+    /* the grid's y dimension walks groups of MM activation rows */
+    x += (size_t)blockIdx.y * MM * K + lane * 16;
     y += (size_t)blockIdx.y * MM * N;
     M = min(MM, M - (int)blockIdx.y * MM);
-    for (int n0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * R; n0 < N; n0 += warps * R) {
-        const unsigned char* wrow[R];
-        const __half* srow[R];
+    const unsigned char* wrow[R];
+    const __half* srow[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) { /* rows beyond N repeat row N - 1 and are not stored */
-            const int n = min(n0 + r, N - 1);
-            wrow[r] = w + (size_t)n * row_bytes + (size_t)lane * sizeof(uint2);
-            srow[r] = scales + (size_t)n * spr;
+    for (int r = 0; r < R; r++) { /* rows beyond N repeat row N - 1 and are not stored */
+        const int n = min(n0 + r, N - 1);
+        wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
+        srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
+    }
+    float acc[FM][R];
+#pragma unroll
+    for (int m = 0; m < FM; m++)
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[m][r] = 0.f;
+    tile_t nxt[PD][R];
+    __half gnx[PD][R];
+    auto fetch = [&](int d, int i) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            nxt[d][r] = *reinterpret_cast<const tile_t*>(wrow[r] + (size_t)i * 32 * sizeof(tile_t));
+            gnx[d][r] = WK != WK_INT8_CH ? srow[r][(i * 512 + lane * 16) >> gshift] : __half(0.f);
         }
-        float acc[R][MM];
+    };
 #pragma unroll
-        for (int r = 0; r < R; r++)
+    for (int d = 0; d < PD; d++) fetch(d, min(d * NS + ns, T - 1));
+    const int rounds = (T + NS - 1) / NS;
+    for (int rnd0 = 0; rnd0 < rounds; rnd0 += PD)
 #pragma unroll
-            for (int m = 0; m < MM; m++) acc[r][m] = 0.f;
-        /* each row's next PD tiles are in registers: with few warps per SM the loads of one tile ahead
-         * would leave the weight stream bound by DRAM latency */
-        constexpr int PD = 4;
-        uint2 pf[R][PD];
+    for (int d = 0; d < PD; d++) {
+        const int rnd = rnd0 + d, i = rnd * NS + ns;
+        if (PD > 1 && rnd >= rounds) break;
+        tile_t cur[R];
+        float gs[R];
 #pragma unroll
-        for (int r = 0; r < R; r++)
+        for (int r = 0; r < R; r++) { cur[r] = nxt[d][r]; gs[r] = __half2float(gnx[d][r]); }
+        if (i + PD * NS < T) fetch(d, i + PD * NS);
+        if (NS == 1 || i < T) {
+            f32x2 s[R][P];
 #pragma unroll
-            for (int d = 0; d < PD; d++)
-                pf[r][d] = d < T ? *reinterpret_cast<const uint2*>(wrow[r] + (size_t)d * 32 * sizeof(uint2)) : make_uint2(0, 0);
-        for (int i0 = 0; i0 < T; i0 += PD) {
+            for (int r = 0; r < R; r++)
 #pragma unroll
-          for (int d = 0; d < PD; d++) {
-            const int i = i0 + d;
-            if (i >= T) break;
-            const int k0 = i * 512 + lane * 16;
-            unsigned short wl[R][16];
-            float gs[R];
+                for (int p = 0; p < P; p++) s[r][p] = 0ull;
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                const uint2 cur = pf[r][d];
-                if (i + PD < T) pf[r][d] = *reinterpret_cast<const uint2*>(wrow[r] + (size_t)(i + PD) * 32 * sizeof(uint2));
-                gs[r] = __half2float(srow[r][k0 >> gshift]);
-                const uint32_t tw[2] = {cur.x, cur.y};
+            for (int h = 0; h < 2; h++) { /* eight k of the lane's sixteen */
+                uint4 xv[MM];
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint32_t a = tw[h] ^ 0x88888888u; /* two's complement nibble -> code + 8 */
+                for (int m = 0; m < MM; m++) xv[m] = *reinterpret_cast<const uint4*>(x + (size_t)min(m, M - 1) * K + i * 512 + h * 8);
+                f32x2 wf[R][8];
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        uint32_t mg = ((a >> (4 * k)) & 0x000F000Fu) | 0x43004300u; /* bf16x2 (128 + n_k, 128 + n_{k+4}) */
-                        __nv_bfloat162 hv = *reinterpret_cast<__nv_bfloat162*>(&mg);
-                        const uint32_t c136 = 0x43084308u;
-                        hv = __hsub2(hv, *reinterpret_cast<const __nv_bfloat162*>(&c136));
-                        const uint32_t pr = *reinterpret_cast<uint32_t*>(&hv);
-                        asm("mov.b32 {%0,%1}, %2;" : "=h"(wl[r][h * 8 + k]), "=h"(wl[r][h * 8 + 4 + k]) : "r"(pr));
+                for (int r = 0; r < R; r++) BatchCodes<WK>::widen8(cur[r], h, wf[r]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    f32x2 xx[P];
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        auto word = [&](const uint4& v) { return (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w; };
+                        const uint32_t x0 = word(xv[2 * p]), x1 = word(xv[2 * p + 1]);
+                        xx[p] = j & 1 ? pack2(bf_hi(x0), bf_hi(x1)) : pack2(bf_lo(x0), bf_lo(x1));
+                    }
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+#pragma unroll
+                        for (int p = 0; p < P; p++) ffma2(s[r][p], wf[r][j], xx[p]);
+                }
+            }
+            if (NS == 1) {
+#pragma unroll
+                for (int r = 0; r < R; r++)
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        float s0, s1;
+                        unpack2(s[r][p], s0, s1);
+                        acc[2 * p][r] = WK == WK_INT8_CH ? acc[2 * p][r] + s0 : __fmaf_rn(s0, gs[r], acc[2 * p][r]);
+                        acc[2 * p + 1][r] = WK == WK_INT8_CH ? acc[2 * p + 1][r] + s1 : __fmaf_rn(s1, gs[r], acc[2 * p + 1][r]);
+                    }
+            } else {
+                float* at = part + ((rnd & 1) * NS + ns) * ((MM + 1) * R * 32) + lane;
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        float s0, s1;
+                        unpack2(s[r][p], s0, s1);
+                        at[((2 * p) * R + r) * 32] = s0;
+                        at[((2 * p + 1) * R + r) * 32] = s1;
+                    }
+                    if (WK != WK_INT8_CH) at[(MM * R + r) * 32] = gs[r];
+                }
+            }
+        }
+        if (NS > 1) { /* the round's tiles in ascending order, for this warp's activation rows */
+            __syncthreads();
+            const int live = min(NS, T - rnd * NS);
+            for (int t = 0; t < live; t++) {
+                const float* at = part + ((rnd & 1) * NS + t) * ((MM + 1) * R * 32) + lane;
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const float g = WK != WK_INT8_CH ? at[(MM * R + r) * 32] : 1.f;
+#pragma unroll
+                    for (int m = 0; m < FM; m++) {
+                        const int mm = ns * FM + m;
+                        if (FM * NS > MM && mm >= MM) continue;
+                        const float v = at[(mm * R + r) * 32];
+                        acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + v : __fmaf_rn(v, g, acc[m][r]);
                     }
                 }
             }
-#pragma unroll
-            for (int m = 0; m < MM; m++) {
-                if (m < M) {
-                    const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)m * K + k0);
-                    const uint4 xa = xp[0], xb = xp[1];
-                    const uint32_t xu[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-                    unsigned short xh[16];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) asm("mov.b32 {%0,%1}, %2;" : "=h"(xh[2 * j]), "=h"(xh[2 * j + 1]) : "r"(xu[j]));
-#pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        float sm_ = 0.f;
-#pragma unroll
-                        for (int j = 0; j < 16; j++) sm_ = fma_bf16(wl[r][j], xh[j], sm_);
-                        acc[r][m] = __fmaf_rn(sm_, gs[r], acc[r][m]);
-                    }
-                }
-            }
-          }
         }
+    }
+    /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
+    const int r = lane >> 3, n = n0 + r;
+    const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[min(n, N - 1)] : 1.f;
 #pragma unroll
-        for (int r = 0; r < R; r++)
-#pragma unroll
-            for (int m = 0; m < MM; m++) {
-                const float a = warp_tree_sum(acc[r][m]);
-                if (lane == 0 && m < M && n0 + r < N) y[(size_t)m * N + n0 + r] = f2bf(a);
-            }
+    for (int m = 0; m < FM; m++) {
+        const int mm = NS == 1 ? m : ns * FM + m;
+        float a = warp_tree4<false>(acc[m][0], acc[m][1], acc[m][2], acc[m][3], lane);
+        if (WK == WK_INT8_CH) a = __fmul_rn(a, rs);
+        if ((lane & 7) == 0 && mm < M && n < N) y[(size_t)mm * N + n] = f2bf(a);
     }
 }
 
+template <int WK, int MM, int NS>
+static void run_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, cudaStream_t stream) {
+    constexpr int rows = 4 * (4 / NS); /* weight rows of a CTA */
+    k_gemv_batch<WK, MM, NS><<<dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, stream>>>(
+        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift);
+}
 template <int WK>
 cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K,
                               int gshift, cudaStream_t stream) {
-    const int cap = device_sm_count() * 8;
-    if (WK == WK_INT4_PACK) { /* two or four weight rows per warp, 8 warps per CTA */
-#define S2P_GB4(MM, R)                                                                                     \
-    do {                                                                                                   \
-        int g4 = (N + 8 * R - 1) / (8 * R);                                                                \
-        if (g4 > cap) g4 = cap;                                                                            \
-        k_gemv_batch_i4<MM, R><<<dim3((unsigned)g4, (unsigned)((M + MM - 1) / MM)), 256, 0, stream>>>(     \
-            (__nv_bfloat16*)y, (const __nv_bfloat16*)x, (const unsigned char*)w, (const __half*)scales, M, N, K, gshift); \
+    /* As few groups of activation rows as eight a group allow (each converts every code once), of even size.  Four warps share
+     * four rows where one warp each would leave a scheduler with less than 2.5, which do not hide each other's latencies, provided
+     * that three quarters of the rounds' turns have a tile (a CTA waits for its slowest warp: at K = 2560, five tiles
+     * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all. */
+    const int groups = (M + 7) / 8, mm = ((M + groups - 1) / groups + 1) & ~1;
+    const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
+    const int T = K >> 9, turns = (T + 3) / 4 * 4;
+    const bool shared = 2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns);
+#define S2P_GB(MM)                                                                                            \
+    do {                                                                                                      \
+        if (shared) run_gemv_batch<WK, MM, 4>(y, x, w, scales, M, N, K, gshift, stream);                      \
+        else run_gemv_batch<WK, MM, 1>(y, x, w, scales, M, N, K, gshift, stream);                             \
     } while (0)
-        /* A warp carries R weight rows and a group of MM activation rows: R x MM x 16 fmas per tile against MM
-         * 32-byte activation loads per lane, so R is what keeps the kernel off the L1 bandwidth bound (R = 1: two
-         * cycles of L1 per cycle of fma issue), and the accumulators (R x MM) are what decides how many warps an SM
-         * holds: 8 rows x 4 rows is 158 registers (8 warps per SM), 4 x 4 is 128 (16 warps), 4 x 2 is 80.  Measured on
-         * the lockstep tick: beyond 4 activation rows, groups of 4 over the grid's y dimension with R = 4 on the large
-         * matrices and R = 2 on those of few rows (2560: twice the warps) beat 8-row groups by a quarter (batch 8:
-         * 13.9 -> 10.6 ms per tick, batch 16: 23.0 -> 17.5).  With 4 rows or fewer the kernel is bound by latency and
-         * warps count for more than reuse.  Per-row results do not depend on any of this. */
-        const int sms = device_sm_count();
-        const int ctas4 = (N + 31) / 32, ctas2 = (N + 15) / 16; /* CTAs of 8 warps at R = 4 / R = 2 */
-        if (M <= 4) {
-            const int R = ctas4 >= 2 * sms ? 4 : (ctas2 >= 2 * sms ? 2 : 1);
-            if (M <= 2) { if (R == 4) S2P_GB4(2, 4); else if (R == 2) S2P_GB4(2, 2); else S2P_GB4(2, 1); }
-            else { if (R == 4) S2P_GB4(4, 4); else if (R == 2) S2P_GB4(4, 2); else S2P_GB4(4, 1); }
-        }
-        else if (ctas4 >= sms) S2P_GB4(4, 4);
-        else S2P_GB4(4, 2);
-#undef S2P_GB4
-        return cudaGetLastError();
-    }
-    int grid = (N + 7) / 8;
-    if (grid > cap) grid = cap;
-#define S2P_GB(MM)                                                                                      \
-    k_gemv_batch<WK, MM><<<dim3((unsigned)grid, (unsigned)((M + MM - 1) / MM)), 256, 0, stream>>>(      \
-        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift)
-    /* beyond four activation rows: groups of four over the grid's y dimension (twice to four times the warps at half
-     * the registers; INT8 lockstep tick at 16 rows 34.7 -> 22.9 ms, at 8 rows 15.4 -> 13.9) */
-    if (M <= 2) S2P_GB(2);
-    else S2P_GB(4);
+    if (mm == 2) S2P_GB(2);
+    else if (mm == 4) S2P_GB(4);
+    else if (mm == 6) S2P_GB(6);
+    else S2P_GB(8);
 #undef S2P_GB
     return cudaGetLastError();
 }
