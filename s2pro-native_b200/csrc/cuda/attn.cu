@@ -45,8 +45,7 @@ static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, cudaStream_t s
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    k_attn_decode_team<KV8, NT><<<grid, NT * 64, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_attn_decode_team<KV8, NT>, grid, NT * 64, smem, st, a);
 }
 constexpr int ATTN_TEAMS_KV8 = 4, ATTN_TEAMS_BF16 = 3; /* two CTAs per SM either way */
 static bool attn_team_serves(const AttnArgs& a, int rows) {

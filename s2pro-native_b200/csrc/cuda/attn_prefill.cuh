@@ -29,6 +29,7 @@
 #include "ops.h"
 #include "pipe.cuh"
 #include "packed.cuh"
+#include "launch.cuh"
 
 namespace s2p {
 
@@ -162,6 +163,8 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
         mbar_init(&sm.vempty, NW);
         mbar_init_fence();
     }
+    grid_wait();
+    grid_release();
     const float scale = rsqrtf((float)a.head_dim); /* run-time value on purpose, see AttnArgs */
     for (int i = tid; i < M * 16; i += NC + ATTN_PREFILL_PRODUCERS) { /* 16 bytes of one query's vector each, neighbouring lanes neighbouring queries */
         const int qi = i % M, c = i / M, row = qi >> 2;

@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "headops.cuh"
 #include "ops.h"
+#include "launch.cuh"
 
 namespace s2p {
 
@@ -203,8 +204,12 @@ __global__ void __launch_bounds__(NT * 64) k_attn_decode_team(AttnArgs a) {
         }
         cp_async_commit();
     };
-    fetch_k(first);
-    fetch_v(first);
+    /* the kernel in front writes this token's position, in the last split; older ones are whole */
+    const bool settled = first < n_active - 1;
+    if (settled) { fetch_k(first); fetch_v(first); }
+    grid_wait();
+    grid_release();
+    if (!settled) { fetch_k(first); fetch_v(first); }
 
     {   /* queries of the four heads sharing this kv head, pre-scaled */
         const float scale = rsqrtf(128.0f);

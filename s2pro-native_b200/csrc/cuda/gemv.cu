@@ -10,6 +10,7 @@
  */
 #include <stdio.h>
 #include "gemv.cuh"
+#include "ops.h"
 #include "packed.cuh"
 #include "s2p_b200_abi.h"
 
@@ -23,6 +24,15 @@ int device_sm_count() {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
     }
     return n;
+}
+
+/* Both kernels fetch their first weights before they wait for the kernel in front (launch.cuh).  `early` says that it is
+ * not that kernel which writes them: so inside a tick, not where a caller may have queued a quantisation just before. */
+template <class... P, class... A>
+static cudaError_t launch_gemv(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, int early, cudaStream_t st, A... args) {
+    if (early) return launch_after(kernel, grid, threads, smem, st, args...);
+    kernel<<<grid, threads, smem, st>>>(args...);
+    return cudaGetLastError();
 }
 
 template <int WK, int PRO, int EPI>
@@ -56,7 +66,7 @@ cudaError_t gemv_stage_setup() {
 }
 
 template <int WK, int PRO, int EPI>
-cudaError_t launch_gemv_stage(GemvStage g, cudaStream_t stream) {
+cudaError_t launch_gemv_stage(GemvStage g, int early, cudaStream_t stream) {
     const size_t limit = GEMV_SMEM_LIMIT;
     {
         const cudaError_t e = gemv_stage_setup<WK, PRO, EPI>();
@@ -68,19 +78,18 @@ cudaError_t launch_gemv_stage(GemvStage g, cudaStream_t stream) {
     const int rows_per_cta = (units + grid - 1) / grid;
     g.rows_per_pass = gemv_rows_per_pass(WK, rows_per_cta, g.K, g.gshift, EPI == EPI_SWIGLU, limit);
     const size_t smem = gemv_smem_bytes(WK, g.rows_per_pass * (EPI == EPI_SWIGLU ? 2 : 1), g.K, g.gshift);
-    k_gemv_stage<WK, PRO, EPI><<<grid, GEMV_THREADS, smem, stream>>>(g);
-    return cudaGetLastError();
+    return launch_gemv(k_gemv_stage<WK, PRO, EPI>, dim3((unsigned)grid), GEMV_THREADS, smem, early, stream, g);
 }
 
 /* instantiations used by the tick live here so that every kernel is compiled once */
-template cudaError_t launch_gemv_stage<WK_INT8_CH, PRO_VEC, EPI_STORE>(GemvStage, cudaStream_t);
-template cudaError_t launch_gemv_stage<WK_INT8_GRP, PRO_VEC, EPI_STORE>(GemvStage, cudaStream_t);
-template cudaError_t launch_gemv_stage<WK_INT4_PACK, PRO_VEC, EPI_STORE>(GemvStage, cudaStream_t);
+template cudaError_t launch_gemv_stage<WK_INT8_CH, PRO_VEC, EPI_STORE>(GemvStage, int, cudaStream_t);
+template cudaError_t launch_gemv_stage<WK_INT8_GRP, PRO_VEC, EPI_STORE>(GemvStage, int, cudaStream_t);
+template cudaError_t launch_gemv_stage<WK_INT4_PACK, PRO_VEC, EPI_STORE>(GemvStage, int, cudaStream_t);
 #define S2P_INST(WK)                                                                         \
-    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_STORE>(GemvStage, cudaStream_t); \
-    template cudaError_t launch_gemv_stage<WK, PRO_VEC, EPI_RESID>(GemvStage, cudaStream_t);  \
-    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_SWIGLU>(GemvStage, cudaStream_t);\
-    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_ARGMAX>(GemvStage, cudaStream_t);
+    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_STORE>(GemvStage, int, cudaStream_t); \
+    template cudaError_t launch_gemv_stage<WK, PRO_VEC, EPI_RESID>(GemvStage, int, cudaStream_t);  \
+    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_SWIGLU>(GemvStage, int, cudaStream_t);\
+    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_ARGMAX>(GemvStage, int, cudaStream_t);
 S2P_INST(WK_INT8_CH)
 S2P_INST(WK_INT8_GRP)
 S2P_INST(WK_INT4_PACK)
@@ -187,6 +196,8 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
     };
 #pragma unroll
     for (int d = 0; d < PD; d++) fetch(d, min(d * NS + ns, T - 1));
+    grid_wait();
+    grid_release();
     const int rounds = (T + NS - 1) / NS;
     for (int rnd0 = 0; rnd0 < rounds; rnd0 += PD)
 #pragma unroll
@@ -284,14 +295,14 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
 }
 
 template <int WK, int MM, int NS>
-static void run_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, cudaStream_t stream) {
+static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
     constexpr int rows = 4 * (4 / NS); /* weight rows of a CTA */
-    k_gemv_batch<WK, MM, NS><<<dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, stream>>>(
-        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift);
+    return launch_gemv(k_gemv_batch<WK, MM, NS>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, early, stream,
+                       (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift);
 }
 template <int WK>
 cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K,
-                              int gshift, cudaStream_t stream) {
+                              int gshift, int early, cudaStream_t stream) {
     /* As few groups of activation rows as eight a group allow (each converts every code once), of even size.  Four warps share
      * four rows where one warp each would leave a scheduler with less than 2.5, which do not hide each other's latencies, provided
      * that three quarters of the rounds' turns have a tile (a CTA waits for its slowest warp: at K = 2560, five tiles
@@ -302,15 +313,14 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
     const bool shared = 2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns);
 #define S2P_GB(MM)                                                                                            \
     do {                                                                                                      \
-        if (shared) run_gemv_batch<WK, MM, 4>(y, x, w, scales, M, N, K, gshift, stream);                      \
-        else run_gemv_batch<WK, MM, 1>(y, x, w, scales, M, N, K, gshift, stream);                             \
+        if (shared) return run_gemv_batch<WK, MM, 4>(y, x, w, scales, M, N, K, gshift, early, stream);        \
+        return run_gemv_batch<WK, MM, 1>(y, x, w, scales, M, N, K, gshift, early, stream);                    \
     } while (0)
     if (mm == 2) S2P_GB(2);
-    else if (mm == 4) S2P_GB(4);
-    else if (mm == 6) S2P_GB(6);
-    else S2P_GB(8);
+    if (mm == 4) S2P_GB(4);
+    if (mm == 6) S2P_GB(6);
+    S2P_GB(8);
 #undef S2P_GB
-    return cudaGetLastError();
 }
 
 int gshift_of(int G) {
@@ -322,7 +332,7 @@ int gshift_of(int G) {
 
 template <int WK>
 s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, const void* scales, int M, int N,
-                      int K, int gshift, cudaStream_t stream) {
+                      int K, int gshift, int early, cudaStream_t stream) {
     /* 16-byte loads of activations and weight tiles */
     if (((uintptr_t)x | (uintptr_t)w) & 15) return S2P_ERR_INVALID;
     cudaError_t ce;
@@ -330,9 +340,9 @@ s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, c
         GemvStage g = {};
         g.w = w; g.scales = scales; g.N = N; g.K = K; g.gshift = gshift;
         g.x = (const __nv_bfloat16*)x; g.y = (__nv_bfloat16*)y;
-        ce = launch_gemv_stage<WK, PRO_VEC, EPI_STORE>(g, stream);
+        ce = launch_gemv_stage<WK, PRO_VEC, EPI_STORE>(g, early, stream);
     } else {
-        ce = launch_gemv_batch<WK>(y, x, w, scales, M, N, K, gshift, stream);
+        ce = launch_gemv_batch<WK>(y, x, w, scales, M, N, K, gshift, early, stream);
     }
     if (ce != cudaSuccess) {
         fprintf(stderr, "[s2pro] %s launch (M=%d,N=%d,K=%d): %s\n", what, M, N, K, cudaGetErrorString(ce));
@@ -345,11 +355,23 @@ s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, c
 
 using namespace s2p;
 
+extern "C" int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t stream) {
+    if (!lin || !lin->w || !lin->scales || !x || !y || M <= 0 || M > S2P_INT8_GEMV_MAX_M || lin->N <= 0 || lin->K <= 0 || lin->K % 512 ||
+        (lin->kind != WK_INT8_CH && lin->K % (1 << lin->gshift)))
+        return S2P_ERR_INVALID;
+    switch (lin->kind) {
+    case WK_INT8_CH: return gemv_entry<WK_INT8_CH>("int8 gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, 0, early, stream);
+    case WK_INT8_GRP: return gemv_entry<WK_INT8_GRP>("intq gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
+    case WK_INT4_PACK: return gemv_entry<WK_INT4_PACK>("int4p gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
+    }
+    return S2P_ERR_INVALID;
+}
+
 extern "C" s2p_status s2p_int8_gemv(void* y_bf16, const void* x_bf16, const void* w_i8, const float* scales, int M,
                                     int N, int K, cudaStream_t stream) {
     if (!y_bf16 || !x_bf16 || !w_i8 || !scales || M <= 0 || N <= 0 || K <= 0) return S2P_ERR_INVALID;
     if (M > S2P_INT8_GEMV_MAX_M || K % 512 != 0) return S2P_ERR_INVALID;
-    return gemv_entry<WK_INT8_CH>("int8 gemv", y_bf16, x_bf16, w_i8, scales, M, N, K, 0, stream);
+    return gemv_entry<WK_INT8_CH>("int8 gemv", y_bf16, x_bf16, w_i8, scales, M, N, K, 0, 0, stream);
 }
 
 extern "C" s2p_status s2p_intq_gemv(void* y_bf16, const void* x_bf16, const void* w_i8, const void* scales_f16,
@@ -357,7 +379,7 @@ extern "C" s2p_status s2p_intq_gemv(void* y_bf16, const void* x_bf16, const void
     if (!y_bf16 || !x_bf16 || !w_i8 || !scales_f16 || M <= 0 || N <= 0 || K <= 0) return S2P_ERR_INVALID;
     const int gs = gshift_of(G);
     if (M > S2P_INT8_GEMV_MAX_M || K % 512 != 0 || gs < 0 || K % G != 0) return S2P_ERR_INVALID;
-    return gemv_entry<WK_INT8_GRP>("intq gemv", y_bf16, x_bf16, w_i8, scales_f16, M, N, K, gs, stream);
+    return gemv_entry<WK_INT8_GRP>("intq gemv", y_bf16, x_bf16, w_i8, scales_f16, M, N, K, gs, 0, stream);
 }
 
 extern "C" s2p_status s2p_int4p_gemv(void* y_bf16, const void* x_bf16, const void* w_pack, const void* scales_f16,
@@ -365,5 +387,5 @@ extern "C" s2p_status s2p_int4p_gemv(void* y_bf16, const void* x_bf16, const voi
     if (!y_bf16 || !x_bf16 || !w_pack || !scales_f16 || M <= 0 || N <= 0 || K <= 0) return S2P_ERR_INVALID;
     const int gs = gshift_of(G);
     if (M > S2P_INT8_GEMV_MAX_M || K % 512 != 0 || gs < 0 || K % G != 0) return S2P_ERR_INVALID;
-    return gemv_entry<WK_INT4_PACK>("int4p gemv", y_bf16, x_bf16, w_pack, scales_f16, M, N, K, gs, stream);
+    return gemv_entry<WK_INT4_PACK>("int4p gemv", y_bf16, x_bf16, w_pack, scales_f16, M, N, K, gs, 0, stream);
 }

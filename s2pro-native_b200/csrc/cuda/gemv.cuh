@@ -33,6 +33,7 @@
  */
 #pragma once
 #include "common.cuh"
+#include "launch.cuh"
 
 namespace s2p {
 
@@ -349,7 +350,11 @@ __device__ void gemv_stage_cta(const GemvStage& g, int row0, int cnt_total, unsi
                 sc_s[idx] = sg[(size_t)global_row(l) * sc_per_row + c];
             }
         }
-        if (done == 0) stage_activation<WK, PRO>(g, xs, red, GEMV_THREADS);
+        if (done == 0) {
+            grid_wait();
+            grid_release();
+            stage_activation<WK, PRO>(g, xs, red, GEMV_THREADS);
+        }
         S2P_CTA_SYNC();
 
         LaneX<WK> lx;

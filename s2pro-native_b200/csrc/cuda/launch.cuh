@@ -1,0 +1,37 @@
+/* Kernels of a chain that start before the one in front of them has finished.
+ *
+ * A tick is several hundred short kernels in one stream, and each pays for its launch, its set-up and its predecessor's last
+ * CTAs.  A kernel launched by launch_after may begin as soon as every CTA of its predecessor has begun (grid_release)
+ * or ended, and calls grid_wait before it reads or writes anything that an earlier kernel of the stream reads or writes;
+ * what comes before that call is index arithmetic, barrier set-up and the first loads of weights, which nothing in a stream writes.
+ * grid_wait returns when the predecessor has completed and its writes are visible; as every kernel so launched calls it in
+ * every CTA that does not leave at once, a completed predecessor implies the completion of all before it.
+ * grid_release follows grid_wait, so that what comes before a kernel's grid_wait overlaps its predecessor alone and may rely on
+ * everything older (positions, cached keys).  The exception are the short kernels in front of a wide linear: they release at
+ * once, and the linear, which reads nothing but weights before it waits, fills its stages while the linear before last drains
+ * (batch of 128: 13.43 -> 13.20 ms; the same everywhere costs the small batches 1 to 3 %).
+ *
+ * Measured, tick of the full model, before and now: batch of 3 5.88 -> 5.60 ms, 16 (INT8) 13.4 -> 12.9, 128 14.2 -> 13.2; request
+ * start on a cached voice 10.4 -> 9.3 ms.
+ *
+ * A kernel in front that never calls grid_release, or one behind that is launched the ordinary way, behaves as usual. */
+#pragma once
+#include <cuda_runtime.h>
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+static inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute early = {};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}

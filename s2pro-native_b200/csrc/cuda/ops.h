@@ -134,6 +134,8 @@ cudaError_t tick_begin(const TickBeginArgs* a, int rows, cudaStream_t st);
 cudaError_t tick_finish_keys(const unsigned long long* keys, int rows, int32_t* codes, cudaStream_t st);
 
 cudaError_t gemv_setup_all(void); /* once per device, before any stream capture */
+/* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: see launch_gemv in gemv.cu */
+int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t st);
 
 /* batched decode linear on the tensor cores (skinny.cu): y[M, N] = x[M, K] · W^T, 1 <= M <= 256 */
 cudaError_t skinny_gemm_tc(const LinRef* lin, const void* x, int M, void* y, const void* resid, cudaStream_t st);

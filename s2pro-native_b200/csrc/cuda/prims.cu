@@ -9,6 +9,7 @@
  */
 #include <math.h>
 #include "common.cuh"
+#include "launch.cuh"
 #include "gemv.cuh"
 #include "headops.cuh"
 #include "ops.h"
@@ -70,6 +71,9 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
     __shared__ unsigned long long best[8];
     const int tid = threadIdx.x, r = blockIdx.x, nv = a.width >> 3;
     const int v0 = tid, v1 = tid + 256;
+    if (a.tiled) grid_release(); /* a wide linear is next: see launch.cuh */
+    grid_wait();
+    if (!a.tiled) grid_release();
     uint4 g0 = make_uint4(0, 0, 0, 0), g1 = g0;
     if (a.w) {
         if (v0 < nv) g0 = reinterpret_cast<const uint4*>(a.w)[v0];
@@ -206,9 +210,12 @@ __global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs
     const bool live = h < heads, is_q = h < QH, rotated = h < QH + KVH;
     uint2 x = make_uint2(0u, 0u), nw = x;
     const __nv_bfloat16* gain = is_q ? a.q_norm : a.k_norm;
+    const bool turns = threadIdx.x < 64 && blockIdx.y * QKV_HEADS_PER_CTA < QH + KVH;
+    if (turns) rope_cs(threadIdx.x, pos, a.rope_base, cs[threadIdx.x].x, cs[threadIdx.x].y); /* the kernel in front writes no position */
+    grid_wait();
+    grid_release();
     if (live) x = part.partial ? wide_part4_bf16(part, h * 128 + lane * 4, r) : *reinterpret_cast<const uint2*>(a.qkv + ((size_t)r * heads + h) * 128 + lane * 4);
     if (rotated && gain) nw = *reinterpret_cast<const uint2*>(gain + lane * 4);
-    if (threadIdx.x < 64 && blockIdx.y * QKV_HEADS_PER_CTA < QH + KVH) rope_cs(threadIdx.x, pos, a.rope_base, cs[threadIdx.x].x, cs[threadIdx.x].y);
     __syncthreads();
     if (!live) return;
     float v[4] = {bf_lo(x.x), bf_hi(x.x), bf_lo(x.y), bf_hi(x.y)};
@@ -264,8 +271,7 @@ __global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs
 cudaError_t qkv_post_part(const QkvPostArgs* a, const WidePart* part, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     dim3 grid((unsigned)rows, (unsigned)((a->q_heads + 2 * a->kv_heads + QKV_HEADS_PER_CTA - 1) / QKV_HEADS_PER_CTA));
-    k_qkv_post<<<grid, 32 * QKV_HEADS_PER_CTA, 0, st>>>(*a, part ? *part : WidePart());
-    return cudaGetLastError();
+    return launch_after(k_qkv_post, grid, 32 * QKV_HEADS_PER_CTA, 0, st, *a, part ? *part : WidePart());
 }
 cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st) { return qkv_post_part(a, nullptr, rows, st); }
 
@@ -301,6 +307,8 @@ __global__ void __launch_bounds__(512) k_attn_single(AttnArgs a) {
     __shared__ float sp[4][128];
     __shared__ float red[4][128];
     __shared__ __half ssc[128 * 4];
+    grid_wait();
+    grid_release();
     const int row = blockIdx.x, kvh = blockIdx.y;
     const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
     const int QH = a.q_heads;
@@ -420,8 +428,7 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, cudaStream_t
     if (a->kv8) all |= (uintptr_t)a->kv.sbase0 | a->kv.ks_off | a->kv.vs_off;
     constexpr int RB = QT * NW / 2;
     dim3 grid((unsigned)((rows + RB - 1) / RB), (unsigned)a->kv_heads);
-    k_attn_prefill<KV8, QT, NW><<<grid, 32 * NW + ATTN_PREFILL_PRODUCERS, smem, st>>>(*a, rows, (all & 15) == 0, status[dev]);
-    return cudaGetLastError();
+    return launch_after(k_attn_prefill<KV8, QT, NW>, grid, 32 * NW + ATTN_PREFILL_PRODUCERS, smem, st, *a, rows, (int)((all & 15) == 0), status[dev]);
 }
 
 /* A CTA fills an SM whatever its size, so a launch takes (waves of CTAs) x (time per 128-position tile): 7.5 us with blocks of
@@ -463,9 +470,7 @@ cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st) {
         (!a->kv8 || (!a->kv.sbases && a->kv.srow_stride == 0)))
         return a->kv8 ? launch_attn_prefill_rows<true>(a, rows, st) : launch_attn_prefill_rows<false>(a, rows, st);
     dim3 grid((unsigned)rows, (unsigned)a->kv_heads);
-    if (a->kv8) k_attn_single<true><<<grid, 512, 0, st>>>(*a);
-    else k_attn_single<false><<<grid, 512, 0, st>>>(*a);
-    return cudaGetLastError();
+    return launch_after(a->kv8 ? k_attn_single<true> : k_attn_single<false>, grid, 512, 0, st, *a);
 }
 
 /* ---- SwiGLU (kernels.cu:1216-1229) ---------------------------------------- */
@@ -487,6 +492,8 @@ __global__ void __launch_bounds__(256) k_silu_mul(const __nv_bfloat16* __restric
  * 16-byte store, one division per eight elements instead of one 64-bit division per element */
 __global__ void __launch_bounds__(256) k_silu_mul8(const uint4* __restrict__ gu, uint4* __restrict__ h, unsigned n_units,
                                                    unsigned f8) {
+    grid_wait();
+    grid_release();
     for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
         const unsigned r = u / f8, c8 = u - r * f8;
         const uint4 gv = gu[(size_t)r * 2 * f8 + c8], uv = gu[(size_t)r * 2 * f8 + f8 + c8];
@@ -610,8 +617,8 @@ cudaError_t rms_norm(const void* x, const void* w, void* y, int rows, int width,
     if (rows <= 0) return cudaSuccess;
     NormRowArgs a = {};
     a.src = (const __nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = width; a.eps = eps;
-    if (norm_row_serves(a)) k_norm_row<<<rows, 256, 0, st>>>(a);
-    else k_rms_norm<<<rows, 256, 0, st>>>(a.src, a.w, a.y, width, eps);
+    if (norm_row_serves(a)) return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    k_rms_norm<<<rows, 256, 0, st>>>(a.src, a.w, a.y, width, eps);
     return cudaGetLastError();
 }
 cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st) {
@@ -619,8 +626,7 @@ cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows,
     NormRowArgs a = {};
     a.src = (const __nv_bfloat16*)x; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
-    k_norm_row<<<rows, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }
 static NormRowArgs wide_norm_args(void* x, const void* w, void* y, void* y_tiled, int kind, int rows) {
     NormRowArgs a = {};
@@ -636,8 +642,7 @@ cudaError_t wide_norm(const void* src, const WidePart* part, const void* alt, vo
     a.src = (const __nv_bfloat16*)src;
     if (part && part->partial) a.part = *part;
     else if (part) a.add = (const __nv_bfloat16*)alt;
-    k_norm_row<<<rows, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }
 cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WidePart* part, const void* alt, int32_t* codes_out, void* x, const void* w,
                             void* y_tiled, int kind, int rows, cudaStream_t st) {
@@ -646,16 +651,14 @@ cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WideP
     a.src = (const __nv_bfloat16*)table; a.codes = codes; a.codes_out = codes_out;
     if (part && part->partial) { a.part = *part; a.part_logits = 1; }
     else if (part) a.logits = (const __nv_bfloat16*)alt;
-    k_norm_row<<<rows, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }
 cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     NormRowArgs a = {};
     a.src = (const __nv_bfloat16*)src; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
-    k_norm_row<<<rows, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }
 cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logits, int32_t* codes_out, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
@@ -663,16 +666,14 @@ cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logi
     a.src = (const __nv_bfloat16*)table; a.codes = codes; a.logits = (const __nv_bfloat16*)logits; a.codes_out = codes_out;
     a.x_out = (__nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y;
     a.width = S2P_DIM; a.table_rows = S2P_CB_SIZE; a.eps = S2P_NORM_EPS;
-    k_norm_row<<<rows, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }
 cudaError_t silu_mul(const void* gu, void* h, int rows, int ffn, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     const int64_t total = (int64_t)rows * ffn;
     if (ffn % 8 == 0 && (((uintptr_t)gu | (uintptr_t)h) & 15) == 0 && total / 8 < 0xFFFFFFFFll)
-        k_silu_mul8<<<grid_for(total / 8, 256), 256, 0, st>>>((const uint4*)gu, (uint4*)h, (unsigned)(total / 8), (unsigned)(ffn / 8));
-    else
-        k_silu_mul<<<grid_for(total, 256), 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)h, total, ffn);
+        return launch_after(k_silu_mul8, dim3((unsigned)grid_for(total / 8, 256)), 256, 0, st, (const uint4*)gu, (uint4*)h, (unsigned)(total / 8), (unsigned)(ffn / 8));
+    k_silu_mul<<<grid_for(total, 256), 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)h, total, ffn);
     return cudaGetLastError();
 }
 cudaError_t add_inplace(void* y, const void* x, int64_t n, cudaStream_t st) {

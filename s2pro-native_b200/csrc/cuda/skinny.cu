@@ -25,6 +25,7 @@
  */
 #include <stdio.h>
 #include "common.cuh"
+#include "launch.cuh"
 #include "gemv.cuh"
 #include "ops.h"
 #include "pipe.cuh"
@@ -796,6 +797,8 @@ __global__ void __launch_bounds__(256) k_wide_convert(const void* __restrict__ w
 /* activations [M, K] bf16 -> f16 units [k / 8][NB rows], rows beyond M zero; a thread per unit, 8 units of 4 rows per warp */
 template <int WK>
 __global__ void __launch_bounds__(256) k_wide_pack(const __nv_bfloat16* __restrict__ x, int M, int K, int lgNB, uint4* __restrict__ out) {
+    grid_release(); /* a wide linear is next: see launch.cuh */
+    grid_wait();
     const int u = blockIdx.x * 256 + threadIdx.x, lane = u & 31, g = u >> 5;
     const int rg = (1 << lgNB) >> 2;                 /* groups of four rows */
     const int slab = g / rg, row = (g - slab * rg) * 4 + (lane >> 3), k8 = slab * 8 + (lane & 7);
@@ -836,6 +839,8 @@ __device__ __forceinline__ void wide_put_swiglu(const WideArgs& a, int tile, int
 /* the split tiles of a SwiGLU pair, once their pieces are there; CTA = (split tile, batch row), a group of 8 rows per thread */
 template <int WK>
 __global__ void __launch_bounds__(32) k_wide_surplus(WideArgs a) {
+    grid_release(); /* a wide linear is next: see launch.cuh */
+    grid_wait();
     const int stile = blockIdx.x, m = blockIdx.y * 4 + (threadIdx.x >> 3), r8 = (threadIdx.x & 7) * 8;
     const int tile = (a.ffn + 63) / 64 - a.n_split_tiles + stile;
     if (m >= a.M || tile * 64 + r8 >= a.ffn) return;
@@ -893,16 +898,30 @@ __global__ void __launch_bounds__(WD_EPI + 64, 1) k_wide_tc(WideArgs a) {
     const int sup_first = nsup_all * ks / ksn, nsup = nsup_all * (ks + 1) / ksn - sup_first;
     const int it_first = sup_first * (SK_SUPER_K / WD_KC), nk = nsup * (SK_SUPER_K / WD_KC);
     bool ok = true;
+    if (warp != WD_EPI / 32) {
+        grid_wait();
+        grid_release();
+    }
     if (warp == WD_EPI / 32) { /* ---- the copying warp (its lane 0) */
         if (lane == 0) {
             const unsigned char* a_src = a.wide + ((size_t)tile * (size_t)(K / WD_KC) + (size_t)it_first) * WD_A_BYTES;
             const unsigned char* b_src = a.xt + (size_t)it_first * (size_t)b_bytes;
             int s = 0, issued = 0;
             unsigned parity = 1; /* the stages start free */
-            for (int it = 0; it < nk; it++) {
-                if (!mbar_wait_bounded(done + s, parity, status)) { ok = false; break; }
+            auto fetch_a = [&](int it) {
                 mbar_expect_tx(full + s, (unsigned)(WD_A_BYTES + b_bytes));
                 tma_load_1d(smem + s * WD_A_BYTES, a_src + (size_t)it * WD_A_BYTES, WD_A_BYTES, full + s);
+            };
+            /* weights for every stage while the kernel in front still writes the activations */
+            const int ahead = min(stages, nk);
+            for (s = 0; s < ahead; s++) fetch_a(s);
+            s = 0;
+            grid_wait();
+            for (int it = 0; it < nk; it++) {
+                if (it >= ahead) {
+                    if (!mbar_wait_bounded(done + s, parity, status)) { ok = false; break; }
+                    fetch_a(it);
+                }
                 tma_load_1d(stage_b0 + s * b_bytes, b_src + (size_t)it * (size_t)b_bytes, (unsigned)b_bytes, full + s);
                 issued = it + 1;
                 if (++s == stages) { s = 0; parity ^= 1u; }
@@ -1011,9 +1030,7 @@ extern "C" cudaError_t wide_pack(int kind, const void* x, int M, int K, void* xt
     if (M < 1 || M > 256 || K % 64) return cudaErrorInvalidValue;
     const int lg = wide_lg(M);
     const unsigned grid = (unsigned)((((size_t)(K >> 3) << lg) + 255) / 256);
-    if (kind == WK_INT4_PACK) k_wide_pack<WK_INT4_PACK><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, M, K, lg, (uint4*)xt);
-    else k_wide_pack<WK_INT8_CH><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, M, K, lg, (uint4*)xt);
-    return cudaGetLastError();
+    return launch_after(kind == WK_INT4_PACK ? k_wide_pack<WK_INT4_PACK> : k_wide_pack<WK_INT8_CH>, dim3(grid), 256, 0, st, (const __nv_bfloat16*)x, M, K, lg, (uint4*)xt);
 }
 
 template <int WK>
@@ -1028,9 +1045,10 @@ static cudaError_t wide_launch(const WideArgs& a, int grid, cudaStream_t st) {
         if (err != cudaSuccess) return err;
         attr_set[dev] = true;
     }
-    k_wide_tc<WK><<<grid, WD_EPI + 64, (size_t)a.stages * (WD_A_BYTES + (WD_KC * 2 << a.lgNB)) + 256, st>>>(a);
-    if (a.ffn && a.n_split_tiles) k_wide_surplus<WK><<<dim3((unsigned)a.n_split_tiles, (unsigned)((a.M + 3) / 4)), 32, 0, st>>>(a);
-    return cudaGetLastError();
+    err = launch_after(k_wide_tc<WK>, dim3((unsigned)grid), WD_EPI + 64, (size_t)a.stages * (WD_A_BYTES + (WD_KC * 2 << a.lgNB)) + 256, st, a);
+    if (err == cudaSuccess && a.ffn && a.n_split_tiles)
+        err = launch_after(k_wide_surplus<WK>, dim3((unsigned)a.n_split_tiles, (unsigned)((a.M + 3) / 4)), 32, 0, st, a);
+    return err;
 }
 
 extern "C" cudaError_t wide_gemm(const LinRef* lin, const void* wide, const void* xt, int M, int ffn, void* y, void* h_tiled, int h_kind, WidePart* part,

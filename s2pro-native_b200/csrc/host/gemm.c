@@ -271,15 +271,15 @@ s2p_status s2p_linear_tc_swiglu(const s2p_linear* lin, const void* x_bf16, void*
     return S2P_OK;
 }
 
-s2p_status s2p_linear_gemv_rows(const s2p_linear* lin, const void* x_bf16, void* y_bf16, int M, cudaStream_t stream) {
+s2p_status s2p_linear_gemv_rows(const s2p_linear* lin, const void* x_bf16, void* y_bf16, int M, int early, cudaStream_t stream) {
     const int N = lin->out_features, K = lin->in_features;
+    LinRef lr;
+    s2p_lin_ref(lin, &lr);
     /* beyond the reference's 16-row GEMV the batch goes to the tensor cores in one launch
      * (S2P_NO_TC=1 keeps the exact-order kernel, 16 rows at a time; S2P_TC_MIN_ROWS=n, 2 <= n <= 16,
      * sends batches of n rows and more there too, giving up bit-equality with the reference's
      * batched GEMV for them) */
     if (s2p_linear_rows_on_tc(lin, M)) {
-        LinRef lr;
-        s2p_lin_ref(lin, &lr);
         const cudaError_t ce = skinny_gemm_tc(&lr, x_bf16, M, y_bf16, NULL, stream);
         if (ce != cudaSuccess) {
             fprintf(stderr, "[s2pro] batched tensor-core linear (M=%d,N=%d,K=%d): %s\n", M, N, K, cudaGetErrorString(ce));
@@ -287,14 +287,12 @@ s2p_status s2p_linear_gemv_rows(const s2p_linear* lin, const void* x_bf16, void*
         }
         return S2P_OK;
     }
+    if (lin->q_group > 0 && (lin->q_group < 16 || 1 << lr.gshift != lin->q_group)) return S2P_ERR_INVALID;
     for (int m0 = 0; m0 < M; m0 += S2P_INT8_GEMV_MAX_M) {
         const int mm = M - m0 < S2P_INT8_GEMV_MAX_M ? M - m0 : S2P_INT8_GEMV_MAX_M;
         const char* xs = (const char*)x_bf16 + (size_t)m0 * K * 2;
         char* ys = (char*)y_bf16 + (size_t)m0 * N * 2;
-        s2p_status rc;
-        if (lin->q_packed) rc = s2p_int4p_gemv(ys, xs, lin->w_pack.data, lin->w_iscale.data, mm, N, K, lin->q_group, stream);
-        else if (lin->q_group > 0) rc = s2p_intq_gemv(ys, xs, lin->w_int8.data, lin->w_iscale.data, mm, N, K, lin->q_group, stream);
-        else rc = s2p_int8_gemv(ys, xs, lin->w_int8.data, (const float*)lin->w_iscale.data, mm, N, K, stream);
+        const s2p_status rc = (s2p_status)gemv_rows(&lr, xs, ys, mm, early, stream);
         if (rc != S2P_OK) return rc;
     }
     return S2P_OK;
@@ -313,7 +311,7 @@ s2p_status s2p_linear_forward(const s2p_linear* lin, const void* x_bf16, void* y
     if (!G.inited) return S2P_ERR_STATE;
     const int N = lin->out_features, K = lin->in_features;
     if (mode == S2P_GEMM_INT8 && lin->int8_ready) {
-        if (M <= S2P_INT8_GEMV_MAX_M) return s2p_linear_gemv_rows(lin, x_bf16, y_bf16, M, stream);
+        if (M <= S2P_INT8_GEMV_MAX_M) return s2p_linear_gemv_rows(lin, x_bf16, y_bf16, M, 0, stream);
         /* S2P_PREFILL_TC=1 (the reference's switch, src/sched/gemm.c:458-466, off by default there and here
          * because the summation order differs from cuBLAS): prompt slices of any length go to the tensor
          * cores straight from the quantised weights, no bf16 copy of the layer is written or read. */

@@ -12,7 +12,8 @@
 #define S2P_KV_PLANES_PER_LAYER (2 * S2P_SLOW_KV_HEADS)
 
 int s2p_env_is_one(const char* name);
-s2p_status s2p_linear_gemv_rows(const s2p_linear* lin, const void* x_bf16, void* y_bf16, int M, cudaStream_t stream);
+/* early: the kernel in front in the stream does not write the weights */
+s2p_status s2p_linear_gemv_rows(const s2p_linear* lin, const void* x_bf16, void* y_bf16, int M, int early, cudaStream_t stream);
 int s2p_linear_rows_on_tc(const s2p_linear* lin, int M);
 void s2p_linear_tc_disable(void);
 /* what a tensor-parallel model may do (session.c) */

@@ -168,7 +168,7 @@ static s2p_status lin_apply(s2p_model* m, const s2p_linear* lin, const void* wid
     }
     m->tick_kernels += !decode ? 2 : (m->mode == S2P_GEMM_INT8 && lin->int8_ready && s2p_linear_rows_on_tc(lin, rows))
                                          ? 1 : (rows + S2P_INT8_GEMV_MAX_M - 1) / S2P_INT8_GEMV_MAX_M;
-    if (decode && m->mode == S2P_GEMM_INT8 && lin->int8_ready) return s2p_linear_gemv_rows(lin, x, y, rows, m->stream);
+    if (decode && m->mode == S2P_GEMM_INT8 && lin->int8_ready) return s2p_linear_gemv_rows(lin, x, y, rows, 1, m->stream);
     return s2p_linear_forward(lin, x, y, rows, m->mode, m->stream);
 }
 
