@@ -35,7 +35,7 @@ namespace s2p {
 
 constexpr int ATTN_PREFILL_PRODUCERS = 128; /* threads that widen the tiles */
 
-template <bool KV8, int QT, int NW> struct AttnPrefillSmem {
+template <bool KV8, int QT, int NW, bool APART> struct AttnPrefillSmem {
     static constexpr int M = 2 * QT * NW;               /* queries of a CTA */
     alignas(16) float q[128][M];                        /* pre-scaled queries, dimension-major */
     alignas(16) float k[128][128];                      /* key tile, dimension-major */
@@ -46,7 +46,8 @@ template <bool KV8, int QT, int NW> struct AttnPrefillSmem {
      * flipped so that the two halves of a warp read different banks */
     alignas(16) float p[NW][2][QT][128];
     alignas(16) __half ksc[KV8 ? 4 : 1][128], vsc[KV8 ? 4 : 1][128]; /* group scales of the tile */
-    alignas(8) uint64_t kfull, kempty, vfull, vempty;
+    alignas(16) float corr[NW][2][QT], l[NW][2][QT];    /* APART, beside p: the factor of the sums so far, the weights' total */
+    alignas(8) uint64_t kfull, kempty, vfull, vempty, pfull[NW], pempty[NW]; /* the last two: APART */
 };
 
 /* 16 payload bytes, from an address that may be aligned to 4 bytes only */
@@ -55,63 +56,90 @@ __device__ __forceinline__ uint4 attn_prefill_load16(const unsigned char* src, i
     const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
-/* a key tile to f32, dimension-major: a thread per position, so the transposed stores are conflict-free */
+/* 16 bytes of a key, chunk c of position r, to f32: dimension-major, so with a thread per position the stores are conflict-free */
 template <bool KV8>
-__device__ __forceinline__ void attn_prefill_keys(float (*k)[128], const unsigned char* src, int r, int lim, int wide) {
-    constexpr int NCH = KV8 ? 8 : 16; /* 16-byte chunks of a cached vector */
-#pragma unroll 1
-    for (int c0 = 0; c0 < NCH; c0 += 2) {
-        uint4 x[2];
+__device__ __forceinline__ void attn_prefill_key(float (*k)[128], int c, int r, const uint4& x) {
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    float(*d)[128] = k + c * (KV8 ? 16 : 8);
 #pragma unroll
-        for (int u = 0; u < 2; u++)
-            x[u] = r < lim ? attn_prefill_load16(src + (size_t)r * (NCH * 16) + (c0 + u) * 16, wide) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-            float(*d)[128] = k + (c0 + u) * (KV8 ? 16 : 8);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (KV8) {
-                    const uint32_t b = s8x4_bias(w[j]);
-                    d[4 * j][r] = s8_biased_to_f32<0>(b);
-                    d[4 * j + 1][r] = s8_biased_to_f32<1>(b);
-                    d[4 * j + 2][r] = s8_biased_to_f32<2>(b);
-                    d[4 * j + 3][r] = s8_biased_to_f32<3>(b);
-                } else {
-                    d[2 * j][r] = bf_lo(w[j]);
-                    d[2 * j + 1][r] = bf_hi(w[j]);
-                }
-            }
-        }
-    }
-}
-/* a value tile to f32, rows in the slot order of AttnPrefillSmem::v */
-template <bool KV8>
-__device__ __forceinline__ void attn_prefill_values(float (*v)[128], const unsigned char* src, int pt, int lim, int wide) {
-    constexpr int NCH = KV8 ? 8 : 16;
-    const int c = pt % NCH;
-#pragma unroll 2
-    for (int r = pt / NCH; r < 128; r += ATTN_PREFILL_PRODUCERS / NCH) {
-        const uint4 x = r < lim ? attn_prefill_load16(src + (size_t)r * (NCH * 16) + c * 16, wide) : make_uint4(0, 0, 0, 0);
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-        float4* d = reinterpret_cast<float4*>(v[r]);
+    for (int j = 0; j < 4; j++) {
         if (KV8) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint32_t b = s8x4_bias(w[j]);
-                d[(j & 1) * 16 + c * 2 + (j >> 1)] = make_float4(s8_biased_to_f32<0>(b), s8_biased_to_f32<1>(b), s8_biased_to_f32<2>(b), s8_biased_to_f32<3>(b));
-            }
+            const uint32_t b = s8x4_bias(w[j]);
+            d[4 * j][r] = s8_biased_to_f32<0>(b);
+            d[4 * j + 1][r] = s8_biased_to_f32<1>(b);
+            d[4 * j + 2][r] = s8_biased_to_f32<2>(b);
+            d[4 * j + 3][r] = s8_biased_to_f32<3>(b);
         } else {
-            d[c] = make_float4(bf_lo(w[0]), bf_hi(w[0]), bf_lo(w[1]), bf_hi(w[1]));
-            d[16 + c] = make_float4(bf_lo(w[2]), bf_hi(w[2]), bf_lo(w[3]), bf_hi(w[3]));
+            d[2 * j][r] = bf_lo(w[j]);
+            d[2 * j + 1][r] = bf_hi(w[j]);
         }
     }
 }
-__device__ __forceinline__ void attn_prefill_scales(__half (*dst)[128], const __half* src, int r, int lim) {
-    const unsigned short* s = reinterpret_cast<const unsigned short*>(src) + (size_t)r * 4;
+/* 16 bytes of a value, chunk c of position r, to f32 in the slot order of AttnPrefillSmem::v */
+template <bool KV8>
+__device__ __forceinline__ void attn_prefill_value(float (*v)[128], int c, int r, const uint4& x) {
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    float4* d = reinterpret_cast<float4*>(v[r]);
+    if (KV8) {
 #pragma unroll
-    for (int g = 0; g < 4; g++) dst[g][r] = __ushort_as_half(r < lim ? s[g] : (unsigned short)0);
+        for (int j = 0; j < 4; j++) {
+            const uint32_t b = s8x4_bias(w[j]);
+            d[(j & 1) * 16 + c * 2 + (j >> 1)] = make_float4(s8_biased_to_f32<0>(b), s8_biased_to_f32<1>(b), s8_biased_to_f32<2>(b), s8_biased_to_f32<3>(b));
+        }
+    } else {
+        d[c] = make_float4(bf_lo(w[0]), bf_hi(w[0]), bf_lo(w[1]), bf_hi(w[1]));
+        d[16 + c] = make_float4(bf_lo(w[2]), bf_hi(w[2]), bf_lo(w[3]), bf_hi(w[3]));
+    }
 }
+/* What a producer thread brings of a key or value tile: a position's whole key, or one chunk of every PRODUCERS / NCH-th
+ * value.  AHEAD: all of it is asked for before the thread waits for the buffer to come free, so that the memory's latency passes
+ * meanwhile (a small block's consumers are done with a tile sooner than four round trips take: 8 rows, 10.1 -> 9.4 us per
+ * tile).  Otherwise two requests at a time, for the producers that have given their registers away. */
+template <bool KV8, bool AHEAD, bool KEYS> struct AttnPrefillFeed {
+    static constexpr int NCH = KV8 ? 8 : 16; /* 16-byte chunks of a cached vector */
+    uint4 x[AHEAD ? NCH : 1];
+    unsigned short sc[AHEAD ? 4 : 1];
+    const unsigned char* src;
+    const unsigned short* scales;
+    int pt, wide, lim;
+
+    __device__ __forceinline__ uint4 fetch(int i) const {
+        const int r = KEYS ? pt : pt / NCH + i * (ATTN_PREFILL_PRODUCERS / NCH), c = KEYS ? i : pt % NCH;
+        return r < lim ? attn_prefill_load16(src + (size_t)r * (NCH * 16) + c * 16, wide) : make_uint4(0, 0, 0, 0);
+    }
+    /* rows past `lim` become zero */
+    __device__ __forceinline__ void ask(const unsigned char* tile, const __half* tile_scales, int positions) {
+        src = tile; scales = reinterpret_cast<const unsigned short*>(tile_scales) + (size_t)pt * 4; lim = positions;
+        if (AHEAD) {
+#pragma unroll
+            for (int i = 0; i < NCH; i++) x[i] = fetch(i);
+            if (KV8)
+#pragma unroll
+                for (int g = 0; g < 4; g++) sc[g] = scale(g);
+        }
+    }
+    __device__ __forceinline__ unsigned short scale(int g) const { return pt < lim ? scales[g] : (unsigned short)0; }
+    __device__ __forceinline__ void put(float (*to)[128], __half (*to_scales)[128]) const {
+        auto one = [&](int i, const uint4& v) {
+            if (KEYS) attn_prefill_key<KV8>(to, i, pt, v);
+            else attn_prefill_value<KV8>(to, pt % NCH, pt / NCH + i * (ATTN_PREFILL_PRODUCERS / NCH), v);
+        };
+        if (AHEAD) {
+#pragma unroll
+            for (int i = 0; i < NCH; i++) one(i, x[i]);
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < NCH; i += 2) {
+                const uint4 a = fetch(i), b = fetch(i + 1);
+                one(i, a);
+                one(i + 1, b);
+            }
+        }
+        if (KV8)
+#pragma unroll
+            for (int g = 0; g < 4; g++) to_scales[g][pt] = __ushort_as_half(AHEAD ? sc[AHEAD ? g : 0] : scale(g));
+    }
+};
 __device__ __forceinline__ f32x2 half2_to_f32x2(uint32_t h) {
     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
     return pack2(f.x, f.y);
@@ -142,14 +170,18 @@ __device__ __forceinline__ void attn_prefill_dim(const float* krow, const float*
 /* NW consumer warps and four producer warps.  The producers widen key tile t + 1 while the consumers are in the value
  * phase of tile t, and value tile t + 1 under score phase t + 1; the four mbarriers let every consumer warp run at its own
  * pace inside that window, so one warp's soft-max overlaps another's fma.  SPLIT_REGS: 512 threads at 128 registers, of
- * which the producers give theirs up (12 x 32 x 160 + 4 x 32 x 32 = 65536 = what the block was launched with). */
-template <bool KV8, int QT, int NW>
-__global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_prefill(AttnArgs a, int rows, int wide, int* status) {
+ * which the producers give theirs up (12 x 32 x 160 + 4 x 32 x 32 = 65536 = what the block was launched with).
+ *
+ * APART: 2 NW consumer warps, of which warp w forms the weights of its queries (they need nothing from the value sums) and warp
+ * NW + w adds the values up, a tile behind.  A small block has one or two warps per scheduler, whose chains wait on themselves;
+ * apart, both products of neighbouring tiles run at once.  Per tile (INT8): 4 rows 7.0 -> 5.8 us, 8 rows 9.4 -> 9.0. */
+template <bool KV8, int QT, int NW, bool APART>
+__global__ void __launch_bounds__((APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_prefill(AttnArgs a, int rows, int wide, int* status) {
     extern __shared__ __align__(16) unsigned char attn_prefill_smem[];
-    typedef AttnPrefillSmem<KV8, QT, NW> Smem;
+    typedef AttnPrefillSmem<KV8, QT, NW, APART> Smem;
     Smem& sm = *reinterpret_cast<Smem*>(attn_prefill_smem);
-    constexpr bool SPLIT_REGS = NW == 12;
-    constexpr int M = Smem::M, RB = M / 4, NC = 32 * NW, VB = KV8 ? 128 : 256;
+    constexpr int M = Smem::M, RB = M / 4, NC = (APART ? 64 : 32) * NW, VB = KV8 ? 128 : 256;
+    constexpr bool SPLIT_REGS = !APART && NW == 12, AHEAD = NC + ATTN_PREFILL_PRODUCERS <= (KV8 ? 512 : 384) && !SPLIT_REGS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     /* the last rows of the slice look furthest back: their blocks start first, the short ones fill in behind them */
     const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * RB, kvh = blockIdx.y;
@@ -161,6 +193,7 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
         mbar_init(&sm.vfull, ATTN_PREFILL_PRODUCERS);
         mbar_init(&sm.kempty, NW);
         mbar_init(&sm.vempty, NW);
+        for (int w = 0; w < NW; w++) { mbar_init(&sm.pfull[w], 1); mbar_init(&sm.pempty[w], 1); }
         mbar_init_fence();
     }
     grid_wait();
@@ -188,25 +221,28 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
     }
     __syncthreads();
 
-    if (warp >= NW) { /* ---- producers ---- */
+    if (tid >= NC) { /* ---- producers ---- */
         if (SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         const size_t plane = (size_t)kvh * a.max_seq;
         const unsigned char* kc = kv_payload(a.kv, r0) + a.kv.k_off + plane * VB; /* one cache for all rows of the block */
         const unsigned char* vc = kv_payload(a.kv, r0) + a.kv.v_off + plane * VB;
         const __half* ks = KV8 ? reinterpret_cast<const __half*>(kv_scales(a.kv, r0) + a.kv.ks_off) + plane * 4 : nullptr;
         const __half* vs = KV8 ? reinterpret_cast<const __half*>(kv_scales(a.kv, r0) + a.kv.vs_off) + plane * 4 : nullptr;
-        const int pt = tid - NC;
+        AttnPrefillFeed<KV8, AHEAD, true> keys;
+        AttnPrefillFeed<KV8, AHEAD, false> values;
+        keys.pt = values.pt = tid - NC;
+        keys.wide = values.wide = wide;
         unsigned phase = 1; /* the buffers start empty: the first waits pass at once */
+        keys.ask(kc, ks, min(128, len_max));
         for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1) {
-            /* rows past the last position any query sees become zero */
-            const int lim = min(128, len_max - t0);
+            values.ask(vc + (size_t)t0 * VB, vs + (size_t)t0 * 4, min(128, len_max - t0));
             if (!mbar_wait_bounded(&sm.kempty, phase, status)) return;
-            attn_prefill_keys<KV8>(sm.k, kc + (size_t)t0 * VB, pt, lim, wide);
-            if (KV8) attn_prefill_scales(sm.ksc, ks + (size_t)t0 * 4, pt, lim);
+            keys.put(sm.k, sm.ksc);
             mbar_arrive(&sm.kfull);
+            const int t1 = t0 + 128;
+            if (t1 < len_max) keys.ask(kc + (size_t)t1 * VB, ks + (size_t)t1 * 4, min(128, len_max - t1));
             if (!mbar_wait_bounded(&sm.vempty, phase, status)) return;
-            attn_prefill_values<KV8>(sm.v, vc + (size_t)t0 * VB, pt, lim, wide);
-            if (KV8) attn_prefill_scales(sm.vsc, vs + (size_t)t0 * 4, pt, lim);
+            values.put(sm.v, sm.vsc);
             mbar_arrive(&sm.vfull);
         }
         return;
@@ -214,11 +250,13 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
     if (SPLIT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
 
     /* ---- consumers ---- */
+    const int w = APART && warp >= NW ? warp - NW : warp;
     const int tx = lane >> 1, qg = lane & 1; /* neighbouring lanes read the same key / value: 16-byte shared reads merge pairs */
-    const int q0 = (warp * 2 + qg) * QT;     /* this thread's queries q0 .. q0 + QT - 1; query = 4 * (row in block) + head */
-    float* const pw = &sm.p[warp][qg][0][0];
+    const int q0 = (w * 2 + qg) * QT;        /* this thread's queries q0 .. q0 + QT - 1; query = 4 * (row in block) + head */
+    float* const pw = &sm.p[w][qg][0][0];
     const int flip = qg << 4;
-    float m[QT], l[QT];
+    unsigned phase = 0;
+    float m[QT], l[QT], corr[QT];
     f32x2 acc[QT][4];
 #pragma unroll
     for (int i = 0; i < QT; i++) {
@@ -227,10 +265,8 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
 #pragma unroll
         for (int c = 0; c < 4; c++) acc[i][c] = 0ull;
     }
-    unsigned phase = 0;
-    for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1) {
-        const int lim_max = min(128, len_max - t0);
-        if (!mbar_wait_bounded(&sm.kfull, phase, status)) return;
+    auto weights = [&](int t0) -> bool {
+        if (!mbar_wait_bounded(&sm.kfull, phase, status)) return false;
         /* ---- scores of QT queries x positions {4 tx .. +3, 64 + 4 tx .. +3}, two positions per packed fma ---- */
         f32x2 d[QT][4];
 #pragma unroll
@@ -262,8 +298,10 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.kempty);
 
-        /* ---- soft-max of the tile, one query after another; the query's eight weights of this thread go to shared memory ---- */
-        float corr[QT];
+        /* soft-max of the tile, one query after another; its eight weights of this thread go to shared memory */
+        if (APART && !mbar_wait_bounded(&sm.pempty[w], phase ^ 1, status)) return false;
+
+        /* soft-max of the tile, one query after another; its eight weights of this thread go to shared memory */
 #pragma unroll
         for (int i = 0; i < QT; i++) {
             const int row = (q0 + i) >> 2;
@@ -304,6 +342,17 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
             } else {
                 corr[i] = 1.f;
             }
+            if (APART && tx == 0) { sm.corr[w][qg][i] = corr[i]; sm.l[w][qg][i] = l[i]; }
+        }
+        __syncwarp();
+        if (APART && lane == 0) mbar_arrive(&sm.pfull[w]);
+        return true;
+    };
+    auto values = [&](int t0) -> bool {
+        if (APART) {
+            if (!mbar_wait_bounded(&sm.pfull[w], phase, status)) return false;
+#pragma unroll
+            for (int i = 0; i < QT; i++) { corr[i] = sm.corr[w][qg][i]; l[i] = sm.l[w][qg][i]; }
         }
 #pragma unroll
         for (int i = 0; i < QT; i++) {
@@ -311,12 +360,11 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
 #pragma unroll
             for (int c = 0; c < 4; c++) acc[i][c] = fmul2(acc[i][c], cc);
         }
-        __syncwarp();
 
         /* ---- value sums of QT queries x dimensions 8 tx .. +7 (one scale group), two dimensions per packed fma.
          * Positions a query does not see have weight 0 and finite values: their fma leaves the sum as it is. ---- */
-        const int n4 = (lim_max + 3) & ~3;
-        if (!mbar_wait_bounded(&sm.vfull, phase, status)) return;
+        const int n4 = (min(128, len_max - t0) + 3) & ~3;
+        if (!mbar_wait_bounded(&sm.vfull, phase, status)) return false;
 #pragma unroll 1
         for (int j = 0; j < n4; j += 4) {
             f32x2 w01[QT], w23[QT];
@@ -349,7 +397,23 @@ __global__ void __launch_bounds__(32 * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_pr
             }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.vempty);
+        if (lane == 0) {
+            mbar_arrive(&sm.vempty);
+            if (APART) mbar_arrive(&sm.pempty[w]);
+        }
+        return true;
+    };
+    if (APART) {
+        if (warp < NW) {
+            for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1)
+                if (!weights(t0)) return;
+            return;
+        }
+        for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1)
+            if (!values(t0)) return;
+    } else {
+        for (int t0 = 0; t0 < len_max; t0 += 128, phase ^= 1)
+            if (!weights(t0) || !values(t0)) return;
     }
 #pragma unroll
     for (int i = 0; i < QT; i++) {

@@ -407,17 +407,17 @@ __global__ void __launch_bounds__(512) k_attn_single(AttnArgs a) {
 /* prompt slices: consecutive rows of one session go to the row-block kernel (attn_prefill.cuh) */
 static __device__ int g_attn_prefill_status; /* code of a bounded wait that gave up (pipe.cuh), 0 otherwise */
 
-template <bool KV8, int QT, int NW>
+template <bool KV8, int QT, int NW, bool APART>
 static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, cudaStream_t st) {
     static int* status[64] = {nullptr};
-    constexpr size_t smem = sizeof(AttnPrefillSmem<KV8, QT, NW>);
+    constexpr size_t smem = sizeof(AttnPrefillSmem<KV8, QT, NW, APART>);
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!status[dev]) {
-        e = cudaFuncSetAttribute(k_attn_prefill<KV8, QT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k_attn_prefill<KV8, QT, NW, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         int* p = nullptr;
         e = cudaGetSymbolAddress((void**)&p, g_attn_prefill_status);
@@ -428,29 +428,34 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, cudaStream_t
     if (a->kv8) all |= (uintptr_t)a->kv.sbase0 | a->kv.ks_off | a->kv.vs_off;
     constexpr int RB = QT * NW / 2;
     dim3 grid((unsigned)((rows + RB - 1) / RB), (unsigned)a->kv_heads);
-    return launch_after(k_attn_prefill<KV8, QT, NW>, grid, 32 * NW + ATTN_PREFILL_PRODUCERS, smem, st, *a, rows, (int)((all & 15) == 0), status[dev]);
+    return launch_after(k_attn_prefill<KV8, QT, NW, APART>, grid, (APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCERS, smem, st, *a, rows, (int)((all & 15) == 0), status[dev]);
 }
 
-/* A CTA fills an SM whatever its size, so a launch takes (waves of CTAs) x (time per 128-position tile): 7.5 us with blocks of
- * 4 rows, 10.1 with 8, 15.2 with 16, 20.0 with 24 (INT8 cache; bf16 within 10 %).  Large blocks are the cheapest per row (0.83 us
- * against 1.9), small ones fill the GPU when the slice is short.  The single-block kernel before this one: 9 us for blocks
- * of 4.  Measured (us, before -> now): 2048 rows after 6052 positions 12595 -> 5466, 512 after none 162 -> 112, 77 after
- * 1024 154 -> 95, 20 after 2000 157 -> 120. */
+/* A CTA fills an SM whatever its size, so a launch takes (waves of CTAs) x (time per 128-position tile).  Large blocks are the
+ * cheapest per row (0.80 us a tile with 24 rows, 2.3 with 2), small ones fill the GPU when the slice is short.  The times below
+ * are the measured ones for an INT8 cache; bf16 is within 10 %.  16 and 24 rows keep a scheduler busy with warps that do both
+ * products (15.3 and 19.3 us; products apart 16.1 and too many registers); up to 12 rows they are apart (8 rows 9.4 -> 9.0 us,
+ * 4 rows 7.0 -> 5.8, see attn_prefill.cuh).
+ * Measured (us; first kernel of one block size, four sizes of one kind, now): 2048 rows after 6052 positions 12590, 5430, 5396; 77
+ * after 1024 154, 93, 73; 50 after 1000 89, 68, 57; 20 after 2000 161, 120, 82. */
 template <bool KV8>
 static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, cudaStream_t st) {
-    static const int block_rows[4] = {24, 16, 8, 4}, tile_ns[4] = {20000, 15200, 10100, 7500};
+    static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {19300, 15300, 12600, 9000, 7300, 5800, 4700};
     int best = 0;
     long long best_cost = 0;
-    for (int v = 0; v < 4; v++) {
+    for (int v = 0; v < 7; v++) {
         const int ctas = (rows + block_rows[v] - 1) / block_rows[v] * a->kv_heads;
         const long long cost = (long long)((ctas + device_sm_count() - 1) / device_sm_count()) * tile_ns[v];
         if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
     switch (best) {
-    case 0: return launch_attn_prefill<KV8, 4, 12>(a, rows, st);
-    case 1: return launch_attn_prefill<KV8, 4, 8>(a, rows, st);
-    case 2: return launch_attn_prefill<KV8, 2, 8>(a, rows, st);
-    default: return launch_attn_prefill<KV8, 2, 4>(a, rows, st);
+    case 0: return launch_attn_prefill<KV8, 4, 12, false>(a, rows, st);
+    case 1: return launch_attn_prefill<KV8, 4, 8, false>(a, rows, st);
+    case 2: return launch_attn_prefill<KV8, 4, 6, true>(a, rows, st);
+    case 3: return launch_attn_prefill<KV8, 4, 4, true>(a, rows, st);
+    case 4: return launch_attn_prefill<KV8, 2, 6, true>(a, rows, st);
+    case 5: return launch_attn_prefill<KV8, 2, 4, true>(a, rows, st);
+    default: return launch_attn_prefill<KV8, 2, 2, true>(a, rows, st);
     }
 }
 

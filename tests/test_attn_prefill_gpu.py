@@ -11,9 +11,9 @@ QH, KVH, HD = 32, 8, 128
 
 @pytest.mark.parametrize("kv8", [0, 1])
 @pytest.mark.parametrize("shift", [0, 4])
-@pytest.mark.parametrize("pos0,rows", [(0, 2), (0, 129), (127, 2), (126, 5), (250, 73), (128, 128), (1000, 21), (0, 300), (40, 460), (3000, 450)])
+@pytest.mark.parametrize("pos0,rows", [(0, 2), (0, 129), (127, 2), (126, 5), (250, 73), (128, 128), (1000, 21), (0, 300), (40, 460), (3000, 450), (100, 50), (63, 150)])
 def test_rows_of_a_slice_equal_single_rows(testlib, kv8, shift, pos0, rows):
-    """All four block sizes (their choice depends on the slice's length), ragged last blocks, tiles cut by the diagonal,
+    """All block sizes (their choice depends on the slice's length), ragged last blocks, tiles cut by the diagonal,
     and caches that are aligned to 4 bytes only."""
     import torch
     testlib.attn_single.argtypes = [C.POINTER(AttnArgs), C.c_int, C.c_void_p]
