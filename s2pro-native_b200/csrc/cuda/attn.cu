@@ -49,7 +49,7 @@ static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, cudaStream_t s
 }
 constexpr int ATTN_TEAMS_KV8 = 4, ATTN_TEAMS_BF16 = 3; /* two CTAs per SM either way */
 static bool attn_team_serves(const AttnArgs& a, int rows) {
-    if (rows < 2 || a.out_ll || a.n_out_peers > 0 || (a.max_seq & 1)) return false;
+    if (a.out_ll || a.n_out_peers > 0 || (a.max_seq & 1)) return false;
     if ((a.kv.k_off | a.kv.v_off) & 15u) return false;
     if (a.kv8 && ((a.kv.ks_off | a.kv.vs_off) & 15u)) return false;
     if (!a.kv.bases && (a.kv.row_stride & 15u)) return false;

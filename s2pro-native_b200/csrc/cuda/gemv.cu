@@ -131,11 +131,30 @@ extern "C" cudaError_t gemv_setup_all(void) {
  * weight row per warp for INT8; mixed bf16 fma, one to four for INT4) and now, at 2 / 4 / 8 / 16 rows:
  *   INT8  52 / 84 / 148 / 258 -> 44 / 56 / 83 / 138      INT4  46 / 70 / 103 / 180 -> 46 / 58 / 85 / 144
  * 16 rows of 19456 x 2560 run at 13.5 T fma/s; the pipe's rate is 36 T. */
+/* A SwiGLU over stacked [gate | up] rows (SW): a warp's four rows are two of either half, so gate and up of an output meet in
+ * the warp; both round to bf16 first, as where a kernel of its own follows the linear. */
+template <bool SW> __device__ __forceinline__ int gemv_row_of(int n0, int r, int F) {
+    return SW ? min(n0 + (r & 1), F - 1) + (r >> 1) * F : min(n0 + r, F - 1);
+}
+__device__ __forceinline__ float gemv_swiglu(float a) {
+    const float g = bf16_round(a), up = bf16_round(__shfl_down_sync(S2P_FULL_MASK, a, 16));
+    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
+    return __fmul_rn(bf16_round(__fmul_rn(g, sig)), up);
+}
 template <int WK> struct BatchCodes;
 template <> struct BatchCodes<WK_INT8_CH> {
     static __device__ __forceinline__ f32x2 twice(uint32_t u, uint32_t sel, float minus) {
         const float f = __uint_as_float(__byte_perm(u, 0x4B000000u, sel));
         return fadd2(pack2(f, f), pack2(minus, minus));
+    }
+    /* codes k = 8 h + 0..7 of two rows as f32 pairs (row a, row b) */
+    static __device__ __forceinline__ f32x2 both(uint32_t a, uint32_t b, uint32_t sel, float minus) {
+        return fadd2(pack2(__uint_as_float(__byte_perm(a, 0x4B000000u, sel)), __uint_as_float(__byte_perm(b, 0x4B000000u, sel))), pack2(minus, minus));
+    }
+    static __device__ __forceinline__ void widen8(const uint4& a, const uint4& b, int h, f32x2 (&w)[8]) {
+        const uint32_t ua[2] = {s8x4_bias(h ? a.z : a.x), s8x4_bias(h ? a.w : a.y)}, ub[2] = {s8x4_bias(h ? b.z : b.x), s8x4_bias(h ? b.w : b.y)};
+#pragma unroll
+        for (int j = 0; j < 8; j++) w[j] = both(ua[j >> 2], ub[j >> 2], 0x7440u + (j & 3), -8388736.0f);
     }
     /* codes k = 8 h + 0..7 of a lane as f32 pairs of equals */
     static __device__ __forceinline__ void widen8(const uint4& a, int h, f32x2 (&w)[8]) {
@@ -146,6 +165,14 @@ template <> struct BatchCodes<WK_INT8_CH> {
 };
 template <> struct BatchCodes<WK_INT8_GRP> : BatchCodes<WK_INT8_CH> {};
 template <> struct BatchCodes<WK_INT4_PACK> {
+    static __device__ __forceinline__ void widen8(const uint2& a, const uint2& b, int h, f32x2 (&w)[8]) {
+        const uint32_t ua = h ? a.y : a.x, ub = h ? b.y : b.x;
+        const uint32_t ea = (ua & 0x0F0F0F0Fu) ^ 0x08080808u, oa = ((ua >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+        const uint32_t eb = (ub & 0x0F0F0F0Fu) ^ 0x08080808u, ob = ((ub >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            w[j] = BatchCodes<WK_INT8_CH>::both(j & 1 ? oa : ea, j & 1 ? ob : eb, 0x7440u + (j >> 1), -8388616.0f);
+    }
     static __device__ __forceinline__ void widen8(const uint2& a, int h, f32x2 (&w)[8]) {
         const uint32_t u = h ? a.y : a.x; /* two's complement nibble -> code + 8, even and odd k apart */
         const uint32_t e = (u & 0x0F0F0F0Fu) ^ 0x08080808u, o = ((u >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
@@ -154,7 +181,7 @@ template <> struct BatchCodes<WK_INT4_PACK> {
     }
 };
 
-template <int WK, int MM, int NS>
+template <int WK, int MM, int NS, bool SW>
 __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
                                                        const void* __restrict__ w, const void* __restrict__ scales,
                                                        int M, int N, int K, int gshift) {
@@ -164,19 +191,20 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
     constexpr int FM = NS == 1 ? MM : (MM + NS - 1) / NS; /* activation rows whose sums this warp keeps */
     __shared__ float part[NS == 1 ? 1 : 2 * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][m, then the scales][row][lane] */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n0 = (blockIdx.x * (4 / NS) + warp / NS) * R, ns = warp % NS;
-    if (n0 >= N) return; /* NS > 1: uniform over the CTA */
+    const int F = SW ? N >> 1 : N; /* outputs */
+    const int n0 = (blockIdx.x * (4 / NS) + warp / NS) * (SW ? R / 2 : R), ns = warp % NS;
+    if (n0 >= F) return; /* NS > 1: uniform over the CTA */
     const size_t row_bytes = (WK == WK_INT4_PACK) ? (size_t)(K >> 1) : (size_t)K;
     const int T = K >> 9, spr = K >> gshift;
     /* the grid's y dimension walks groups of MM activation rows */
     x += (size_t)blockIdx.y * MM * K + lane * 16;
-    y += (size_t)blockIdx.y * MM * N;
+    y += (size_t)blockIdx.y * MM * F;
     M = min(MM, M - (int)blockIdx.y * MM);
     const unsigned char* wrow[R];
     const __half* srow[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) { /* rows beyond N repeat row N - 1 and are not stored */
-        const int n = min(n0 + r, N - 1);
+    for (int r = 0; r < R; r++) { /* rows beyond the last repeat it and are not stored */
+        const int n = gemv_row_of<SW>(n0, r, F);
         wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
         srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
     }
@@ -284,43 +312,181 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
     }
     /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
     const int r = lane >> 3, n = n0 + r;
-    const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[min(n, N - 1)] : 1.f;
+    const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[gemv_row_of<SW>(n0, r, F)] : 1.f;
 #pragma unroll
     for (int m = 0; m < FM; m++) {
         const int mm = NS == 1 ? m : ns * FM + m;
         float a = warp_tree4<false>(acc[m][0], acc[m][1], acc[m][2], acc[m][3], lane);
         if (WK == WK_INT8_CH) a = __fmul_rn(a, rs);
-        if ((lane & 7) == 0 && mm < M && n < N) y[(size_t)mm * N + n] = f2bf(a);
+        if (SW) a = gemv_swiglu(a);
+        if ((lane & 7) == 0 && mm < M && n < F && r < (SW ? R / 2 : R)) y[(size_t)mm * F + n] = f2bf(a);
     }
 }
 
-template <int WK, int MM, int NS>
+template <int WK, int MM, int NS, bool SW>
 static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
     constexpr int rows = 4 * (4 / NS); /* weight rows of a CTA */
-    return launch_gemv(k_gemv_batch<WK, MM, NS>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, early, stream,
+    return launch_gemv(k_gemv_batch<WK, MM, NS, SW>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, early, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift);
 }
-template <int WK>
+template <int WK, bool SW>
 cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K,
                               int gshift, int early, cudaStream_t stream) {
     /* As few groups of activation rows as eight a group allow (each converts every code once), of even size.  Four warps share
      * four rows where one warp each would leave a scheduler with less than 2.5, which do not hide each other's latencies, provided
      * that three quarters of the rounds' turns have a tile (a CTA waits for its slowest warp: at K = 2560, five tiles
-     * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all. */
+     * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all.  (A SwiGLU's pairs of rows
+     * meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
     const int groups = (M + 7) / 8, mm = ((M + groups - 1) / groups + 1) & ~1;
     const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
     const int T = K >> 9, turns = (T + 3) / 4 * 4;
-    const bool shared = 2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns);
+    const bool shared = !SW && (2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
 #define S2P_GB(MM)                                                                                            \
     do {                                                                                                      \
-        if (shared) return run_gemv_batch<WK, MM, 4>(y, x, w, scales, M, N, K, gshift, early, stream);        \
-        return run_gemv_batch<WK, MM, 1>(y, x, w, scales, M, N, K, gshift, early, stream);                    \
+        if (shared) return run_gemv_batch<WK, MM, SW ? 1 : 4, SW>(y, x, w, scales, M, N, K, gshift, early, stream); \
+        return run_gemv_batch<WK, MM, 1, SW>(y, x, w, scales, M, N, K, gshift, early, stream);                \
     } while (0)
     if (mm == 2) S2P_GB(2);
     if (mm == 4) S2P_GB(4);
-    if (mm == 6) S2P_GB(6);
-    S2P_GB(8);
+    if constexpr (!SW) {
+        if (mm == 6) S2P_GB(6);
+        S2P_GB(8);
+    }
+    return cudaErrorInvalidValue;
 #undef S2P_GB
+}
+
+/* ---- one row ---------------------------------------------------------------
+ * The linear alone, as a caller's own layers and the frames outside the persistent tick use it.
+ *
+ * What bounds it: DRAM, at a few thousand warps whose weights are all under way at once.  A warp carries four rows as two
+ * packed chains (a register pair holds the same k of two rows), PD tiles at a time side by side, since every tile starts a chain of its
+ * own; the next PD tiles' weights are in registers meanwhile.  Where there are too few rows for that NS = 4 warps share
+ * four rows as in k_gemv_batch.
+ * Measured, us (before: a CTA per SM with the tiles' sums in shared memory): INT4 6144 x 2560 10.2 -> 6.4, 2560 x 4096 8.2 -> 4.6,
+ * 19456 x 2560 25.3 -> 13.5, 2560 x 9728 14.9 -> 9.7; INT8 8.5 -> 6.2, 6.8 -> 4.8, 18.9 -> 11.2, 10.7 -> 8.6. */
+template <int WK, int PD, int NS, bool SW>
+__global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+                                                     const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift) {
+    typedef typename LaneTile<WK>::type tile_t;
+    constexpr int R = 4;
+    __shared__ float part[NS == 1 ? 1 : 2 * PD * NS * 2 * R * 32]; /* [round parity][tile of the round][sums, then scales][row][lane] */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int F = SW ? N >> 1 : N; /* outputs */
+    const int n0 = (blockIdx.x * (4 / NS) + warp / NS) * (SW ? R / 2 : R), ns = warp % NS;
+    if (n0 >= F) return; /* NS > 1: uniform over the CTA */
+    const size_t row_bytes = (WK == WK_INT4_PACK) ? (size_t)(K >> 1) : (size_t)K;
+    const int T = K >> 9, spr = K >> gshift;
+    const unsigned char* wrow[R];
+    const __half* srow[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) { /* rows beyond the last repeat it and are not stored */
+        const int n = gemv_row_of<SW>(n0, r, F);
+        wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
+        srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
+    }
+    tile_t nxt[PD][R];
+    __half gnx[PD][R];
+    auto tile_of = [&](int rnd, int d) { return (rnd * NS + ns) * PD + d; };
+    auto fetch = [&](int rnd) {
+#pragma unroll
+        for (int d = 0; d < PD; d++) {
+            const int i = min(tile_of(rnd, d), T - 1);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                nxt[d][r] = __ldcs(reinterpret_cast<const tile_t*>(wrow[r] + (size_t)i * 32 * sizeof(tile_t)));
+                gnx[d][r] = WK != WK_INT8_CH ? srow[r][(i * 512 + lane * 16) >> gshift] : __half(0.f);
+            }
+        }
+    };
+    fetch(0);
+    grid_wait();
+    grid_release();
+    float acc[R] = {0.f, 0.f, 0.f, 0.f};
+    const int rounds = (T + NS * PD - 1) / (NS * PD);
+    for (int rnd = 0; rnd < rounds; rnd++) {
+        uint4 xv[PD][2];
+#pragma unroll
+        for (int d = 0; d < PD; d++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) xv[d][h] = *reinterpret_cast<const uint4*>(x + min(tile_of(rnd, d), T - 1) * 512 + lane * 16 + h * 8);
+        tile_t cur[PD][R];
+        float gs[PD][R];
+#pragma unroll
+        for (int d = 0; d < PD; d++)
+#pragma unroll
+            for (int r = 0; r < R; r++) { cur[d][r] = nxt[d][r]; gs[d][r] = __half2float(gnx[d][r]); }
+        if (rnd + 1 < rounds) fetch(rnd + 1);
+        f32x2 s[PD][R / 2];
+#pragma unroll
+        for (int d = 0; d < PD; d++) s[d][0] = s[d][1] = 0ull;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            f32x2 wf[PD][R / 2][8];
+#pragma unroll
+            for (int d = 0; d < PD; d++)
+#pragma unroll
+                for (int q = 0; q < R / 2; q++) BatchCodes<WK>::widen8(cur[d][2 * q], cur[d][2 * q + 1], h, wf[d][q]);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+#pragma unroll
+                for (int d = 0; d < PD; d++) {
+                    const uint4& v = xv[d][h];
+                    const uint32_t u = (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w;
+                    const float xf = j & 1 ? bf_hi(u) : bf_lo(u);
+                    const f32x2 xx = pack2(xf, xf);
+#pragma unroll
+                    for (int q = 0; q < R / 2; q++) ffma2(s[d][q], wf[d][q][j], xx);
+                }
+        }
+        auto fold = [&](int r, float v, float g) { acc[r] = WK == WK_INT8_CH ? acc[r] + v : __fmaf_rn(v, g, acc[r]); };
+#pragma unroll
+        for (int d = 0; d < PD; d++) {
+            if (tile_of(rnd, d) >= T) continue;
+            float v[R];
+            unpack2(s[d][0], v[0], v[1]);
+            unpack2(s[d][1], v[2], v[3]);
+            float* at = part + (((rnd & 1) * NS + ns) * PD + d) * (2 * R * 32) + lane;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (NS == 1) fold(r, v[r], gs[d][r]);
+                else { at[r * 32] = v[r]; at[(R + r) * 32] = gs[d][r]; }
+            }
+        }
+        if (NS > 1) { /* the round's tiles in ascending order; warp ns keeps row ns */
+            __syncthreads();
+            const int live = min(NS * PD, T - rnd * NS * PD);
+            const float* at = part + (rnd & 1) * NS * PD * (2 * R * 32) + ns * 32 + lane;
+            for (int t = 0; t < live; t++) fold(0, at[t * (2 * R * 32)], at[t * (2 * R * 32) + R * 32]);
+        }
+    }
+    if (NS == 1) {
+        /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
+        const int r = lane >> 3, n = n0 + r;
+        float a = warp_tree4<false>(acc[0], acc[1], acc[2], acc[3], lane);
+        if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[gemv_row_of<SW>(n0, r, F)]);
+        if (SW) a = gemv_swiglu(a);
+        if ((lane & 7) == 0 && n < F && r < (SW ? R / 2 : R)) y[n] = f2bf(a);
+    } else {
+        float a = warp_tree_sum(acc[0]);
+        if (n0 + ns < N && lane == 0) {
+            if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[n0 + ns]);
+            y[n0 + ns] = f2bf(a);
+        }
+    }
+}
+
+template <int WK, bool SW>
+static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const void* scales, int N, int K, int gshift, int early, cudaStream_t stream) {
+    /* Four warps share four rows where one each would give a scheduler less than 1.5, if most of their turns have a tile
+     * (2560 x 9728: 14.0 -> 9.7 us, 6144 x 2560 the other way round 6.4 -> 7.7).  From six warps per scheduler on a tile at a time
+     * and twice the warps resident hide more than two tiles side by side (19456 x 2560: 14.4 -> 13.5; 6144: 6.4 -> 6.7). */
+    const int warps = (N + 3) / 4, sched = 4 * device_sm_count();
+    const bool shared = !SW && 2 * warps < 3 * sched && K > 4 * 512, many = warps >= 6 * sched;
+    void (*kernel)(__nv_bfloat16*, const __nv_bfloat16*, const void*, const void*, int, int, int) =
+        shared ? k_gemv_row<WK, 2, SW ? 1 : 4, SW> : many ? k_gemv_row<WK, 1, 1, SW> : k_gemv_row<WK, 2, 1, SW>;
+    return launch_gemv(kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, early, stream,
+                       (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, N, K, gshift);
 }
 
 int gshift_of(int G) {
@@ -330,19 +496,16 @@ int gshift_of(int G) {
     return s;
 }
 
-template <int WK>
+template <int WK, bool SW = false>
 s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, const void* scales, int M, int N,
                       int K, int gshift, int early, cudaStream_t stream) {
     /* 16-byte loads of activations and weight tiles */
     if (((uintptr_t)x | (uintptr_t)w) & 15) return S2P_ERR_INVALID;
     cudaError_t ce;
     if (M == 1) {
-        GemvStage g = {};
-        g.w = w; g.scales = scales; g.N = N; g.K = K; g.gshift = gshift;
-        g.x = (const __nv_bfloat16*)x; g.y = (__nv_bfloat16*)y;
-        ce = launch_gemv_stage<WK, PRO_VEC, EPI_STORE>(g, early, stream);
+        ce = launch_gemv_row<WK, SW>(y, x, w, scales, N, K, gshift, early, stream);
     } else {
-        ce = launch_gemv_batch<WK>(y, x, w, scales, M, N, K, gshift, early, stream);
+        ce = launch_gemv_batch<WK, SW>(y, x, w, scales, M, N, K, gshift, early, stream);
     }
     if (ce != cudaSuccess) {
         fprintf(stderr, "[s2pro] %s launch (M=%d,N=%d,K=%d): %s\n", what, M, N, K, cudaGetErrorString(ce));
@@ -355,17 +518,20 @@ s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, c
 
 using namespace s2p;
 
-extern "C" int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t stream) {
+template <bool SW>
+static s2p_status gemv_rows_of(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t stream) {
     if (!lin || !lin->w || !lin->scales || !x || !y || M <= 0 || M > S2P_INT8_GEMV_MAX_M || lin->N <= 0 || lin->K <= 0 || lin->K % 512 ||
-        (lin->kind != WK_INT8_CH && lin->K % (1 << lin->gshift)))
+        (lin->kind != WK_INT8_CH && lin->K % (1 << lin->gshift)) || (SW && (lin->N % 2 || M > GEMV_SWIGLU_ROWS)))
         return S2P_ERR_INVALID;
     switch (lin->kind) {
-    case WK_INT8_CH: return gemv_entry<WK_INT8_CH>("int8 gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, 0, early, stream);
-    case WK_INT8_GRP: return gemv_entry<WK_INT8_GRP>("intq gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
-    case WK_INT4_PACK: return gemv_entry<WK_INT4_PACK>("int4p gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
+    case WK_INT8_CH: return gemv_entry<WK_INT8_CH, SW>("int8 gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, 0, early, stream);
+    case WK_INT8_GRP: return gemv_entry<WK_INT8_GRP, SW>("intq gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
+    case WK_INT4_PACK: return gemv_entry<WK_INT4_PACK, SW>("int4p gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
     }
     return S2P_ERR_INVALID;
 }
+extern "C" int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t stream) { return gemv_rows_of<false>(lin, x, y, M, early, stream); }
+extern "C" int gemv_rows_swiglu(const LinRef* lin, const void* x, void* h, int M, cudaStream_t stream) { return gemv_rows_of<true>(lin, x, h, M, 1, stream); }
 
 extern "C" s2p_status s2p_int8_gemv(void* y_bf16, const void* x_bf16, const void* w_i8, const float* scales, int M,
                                     int N, int K, cudaStream_t stream) {

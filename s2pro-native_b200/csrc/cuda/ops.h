@@ -136,6 +136,11 @@ cudaError_t tick_finish_keys(const unsigned long long* keys, int rows, int32_t* 
 cudaError_t gemv_setup_all(void); /* once per device, before any stream capture */
 /* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: see launch_gemv in gemv.cu */
 int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t st);
+/* h[M, N / 2] = silu(gate) * up for stacked [gate | up] rows, otherwise as gemv_rows with early.  Up to four rows the launch it
+ * saves counts (tick of 1 row 3.53 -> 3.43 ms, 3 rows 5.61 -> 5.55); the kernels of eight rows have no registers left for it (8 rows
+ * 8.39 -> 8.42, 16 rows 12.9 -> 13.2). */
+#define GEMV_SWIGLU_ROWS 4
+int gemv_rows_swiglu(const LinRef* lin, const void* x, void* h, int M, cudaStream_t st);
 
 /* batched decode linear on the tensor cores (skinny.cu): y[M, N] = x[M, K] · W^T, 1 <= M <= 256 */
 cudaError_t skinny_gemm_tc(const LinRef* lin, const void* x, int M, void* y, const void* resid, cudaStream_t st);

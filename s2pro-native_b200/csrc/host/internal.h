@@ -55,6 +55,7 @@ struct s2p_model {
     int n_slow;        /* backbone layers found in the checkpoint (<= S2P_SLOW_LAYERS) */
     int scratch_rows;  /* prefill row capacity */
     int fused_b1;      /* batch-1 fused stages enabled */
+    int persistent_b1; /* ... and wanted on one GPU too (s2p_model_load) */
     /* persistent batch-1 tick: stage program in device memory, sync words, grid size */
     int mega_ok, mega_ctas, mega_n_stages, mega_built;
     int mega_barriers;          /* grid barriers of one tick */

@@ -663,45 +663,39 @@ static s2p_status tick_general(s2p_model* m, s2p_session* const* act, int bd, in
     return S2P_OK;
 }
 
-/* batch-1 tick out of fused stages; `decode` = 0 when the row is freshly prefilled */
-static s2p_status tick_fused_b1(s2p_model* m, s2p_session* const* act, int decode) {
+/* batch-1 tick of a decoding row out of fused stages */
+static s2p_status tick_fused_b1(s2p_model* m) {
     cudaStream_t st = m->stream;
     tick_dev d;
     tick_views(m, &d);
     S2P_CUDA_TRY(cudaMemcpyAsync(m->d_up, m->h_up, m->up_bytes, cudaMemcpyHostToDevice, st));
     LinRef lr;
     VecRef xr;
-    if (decode) {
-        S2P_TRY(tick_begin_rows(m, &d, 1));
-        AttnArgs aa;
-        memset(&aa, 0, sizeof(aa));
-        aa.out = BF(m->sattn);
-        aa.q_heads = S2P_SLOW_Q_HEADS; aa.kv_heads = S2P_SLOW_KV_HEADS; aa.max_seq = m->ctx_len; aa.kv8 = m->kv8;
-        aa.pos_arr = d.pos; aa.kv.bases = d.kv_bases; aa.kv.sbases = d.kvs_bases;
-        aa.part = (float*)m->attn_part.data; aa.counters = m->attn_ctr;
-        aa.n_split_slots = m->n_split_slots; aa.workers = attn_workers_for(1); aa.head_dim = S2P_HEAD_DIM;
-        memset(&xr, 0, sizeof(xr));
-        xr.base = BF(m->sx);
-        for (int l = 0; l < m->n_slow; l++) {
-            const s2p_layer* L = &m->slow[l];
-            s2p_lin_ref(&L->wqkv, &lr);
-            S2P_LAUNCH(m, stage_norm_gemv(&lr, &xr, L->attn_norm.data, S2P_NORM_EPS, BF(m->sqkv), st));
-            slow_kv_offsets(m, l, &aa.kv);
-            S2P_LAUNCH(m, stage_attn_decode_prep(&aa, BF(m->sqkv), L->q_norm.data, L->k_norm.data, S2P_NORM_EPS,
-                                                S2P_ROPE_BASE, 1, st));
-            s2p_lin_ref(&L->wo, &lr);
-            S2P_LAUNCH(m, stage_gemv_resid(&lr, BF(m->sattn), &xr, BF(m->sx), st));
-            s2p_lin_ref(&L->gate_up, &lr);
-            S2P_LAUNCH(m, stage_norm_swiglu(&lr, &xr, L->ffn_norm.data, S2P_NORM_EPS, BF(m->sffn), st));
-            s2p_lin_ref(&L->w2, &lr);
-            S2P_LAUNCH(m, stage_gemv_resid(&lr, BF(m->sffn), &xr, BF(m->sx), st));
-        }
-        S2P_LAUNCH(m, rms_norm(m->sx.data, m->final_norm.data, m->shidden.data, 1, S2P_DIM, S2P_NORM_EPS, st));
-    } else {
-        S2P_CUDA_TRY(cudaMemcpyAsync(m->shidden.data, act[0]->pending_hidden, (size_t)S2P_DIM * 2,
-                                     cudaMemcpyDeviceToDevice, st));
-        S2P_CUDA_TRY(cudaMemsetAsync(m->fkeys, 0, 9 * sizeof(unsigned long long), st));
+    S2P_TRY(tick_begin_rows(m, &d, 1));
+    AttnArgs aa;
+    memset(&aa, 0, sizeof(aa));
+    aa.out = BF(m->sattn);
+    aa.q_heads = S2P_SLOW_Q_HEADS; aa.kv_heads = S2P_SLOW_KV_HEADS; aa.max_seq = m->ctx_len; aa.kv8 = m->kv8;
+    aa.pos_arr = d.pos; aa.kv.bases = d.kv_bases; aa.kv.sbases = d.kvs_bases;
+    aa.part = (float*)m->attn_part.data; aa.counters = m->attn_ctr;
+    aa.n_split_slots = m->n_split_slots; aa.workers = attn_workers_for(1); aa.head_dim = S2P_HEAD_DIM;
+    memset(&xr, 0, sizeof(xr));
+    xr.base = BF(m->sx);
+    for (int l = 0; l < m->n_slow; l++) {
+        const s2p_layer* L = &m->slow[l];
+        s2p_lin_ref(&L->wqkv, &lr);
+        S2P_LAUNCH(m, stage_norm_gemv(&lr, &xr, L->attn_norm.data, S2P_NORM_EPS, BF(m->sqkv), st));
+        slow_kv_offsets(m, l, &aa.kv);
+        S2P_LAUNCH(m, stage_attn_decode_prep(&aa, BF(m->sqkv), L->q_norm.data, L->k_norm.data, S2P_NORM_EPS,
+                                            S2P_ROPE_BASE, 1, st));
+        s2p_lin_ref(&L->wo, &lr);
+        S2P_LAUNCH(m, stage_gemv_resid(&lr, BF(m->sattn), &xr, BF(m->sx), st));
+        s2p_lin_ref(&L->gate_up, &lr);
+        S2P_LAUNCH(m, stage_norm_swiglu(&lr, &xr, L->ffn_norm.data, S2P_NORM_EPS, BF(m->sffn), st));
+        s2p_lin_ref(&L->w2, &lr);
+        S2P_LAUNCH(m, stage_gemv_resid(&lr, BF(m->sffn), &xr, BF(m->sx), st));
     }
+    S2P_LAUNCH(m, rms_norm(m->sx.data, m->final_norm.data, m->shidden.data, 1, S2P_DIM, S2P_NORM_EPS, st));
     S2P_TRY(head_and_sample(m, &d, 1, 0));
 
     /* fast-AR: the input of a pass is a row selected on the device — the slow hidden
@@ -1120,10 +1114,10 @@ s2p_status s2p_model_batch_next_frame(s2p_model* m, s2p_session** sess, int n, i
 
     /* the library GEMM of the BF16 mode is kept out of stream capture */
     const int graphs = !s2p_env_is_one("S2P_NO_GRAPHS") && dump_dir() == NULL && m->mode == S2P_GEMM_INT8;
-    const int fused = m->fused_b1 && nact == 1 && !m->head_full;
+    const int fused = m->fused_b1 && nact == 1 && bd == 1 && !m->head_full && (m->tp_world > 1 || m->persistent_b1);
     s2p_status rc = S2P_OK;
-    if (fused && bd == 1 && m->mega_ok && !m->mega_built && dump_dir() == NULL) S2P_TRY(mega_build(m));
-    const int mega = fused && bd == 1 && m->mega_ok && m->mega_built && dump_dir() == NULL;
+    if (fused && m->mega_ok && !m->mega_built && dump_dir() == NULL) S2P_TRY(mega_build(m));
+    const int mega = fused && m->mega_ok && m->mega_built && dump_dir() == NULL;
     const int steady = bd == nact && graphs && !mega; /* every row decoding: the launch sequence is frame-invariant */
     if (s2p_tp_guard_tick(m->tp_world, bd, mega) != S2P_OK) {
         fprintf(stderr, "[s2pro] tensor-parallel model: this tick (%d decoding rows%s) cannot run as the persistent kernel, and no "
@@ -1137,7 +1131,7 @@ s2p_status s2p_model_batch_next_frame(s2p_model* m, s2p_session** sess, int n, i
     } else if (steady) {
         if (!m->gready[bd]) {
             S2P_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            rc = fused ? tick_fused_b1(m, act, 1) : tick_general(m, act, bd, nact);
+            rc = fused ? tick_fused_b1(m) : tick_general(m, act, bd, nact);
             m->graph_kernels[bd] = m->tick_kernels;
             cudaGraph_t g = NULL;
             const cudaError_t ce = cudaStreamEndCapture(st, &g);
@@ -1162,7 +1156,7 @@ s2p_status s2p_model_batch_next_frame(s2p_model* m, s2p_session** sess, int n, i
         m->tick_kernels = m->graph_kernels[bd];
     } else {
         S2P_CUDA_TRY(cudaEventRecord(m->ev0, st));
-        rc = fused ? tick_fused_b1(m, act, bd == 1) : tick_general(m, act, bd, nact);
+        rc = fused ? tick_fused_b1(m) : tick_general(m, act, bd, nact);
         if (rc != S2P_OK) return rc;
     }
     S2P_CUDA_TRY(cudaEventRecord(m->ev1, st));
