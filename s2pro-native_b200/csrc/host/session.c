@@ -245,6 +245,11 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
         L->gate_up.out_features == 2 * S2P_FFN_DIM) {
         m->tick_kernels += 1; /* gate/up linear and SwiGLU in one launch */
         S2P_TRY(s2p_linear_tc_swiglu(&L->gate_up, norm, hff, rows, st));
+    } else if (c->decode && m->mode == S2P_GEMM_INT8 && L->gate_up.int8_ready && rows <= GEMV_SWIGLU_ROWS) {
+        LinRef lr;
+        s2p_lin_ref(&L->gate_up, &lr);
+        m->tick_kernels += 1;
+        S2P_TRY((s2p_status)gemv_rows_swiglu(&lr, norm, hff, rows, st));
     } else {
         S2P_TRY(lin_apply(m, &L->gate_up, L->wide[2], norm, gu, rows, c->decode));
         S2P_LAUNCH(m, silu_mul(gu, hff, rows, S2P_FFN_DIM, st));
