@@ -324,6 +324,8 @@ cudaError_t wide_norm(const void* src, const WidePart* part, const void* alt, vo
 cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WidePart* part, const void* alt, int32_t* codes_out, void* x, const void* w,
                             void* y_tiled, int kind, int rows, cudaStream_t st);
 cudaError_t qkv_post_part(const QkvPostArgs* a, const WidePart* part, int rows, cudaStream_t st);
+/* qkv_post_part and the attention of one position of all rows, at most FAST_ATTN_MAX positions in a bf16 cache (a->q is not written) */
+cudaError_t fast_attn(const QkvPostArgs* a, const WidePart* part, void* out, int head_dim, int rows, cudaStream_t st);
 /* x = src, y = norm(x) */
 cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st);
 /* x = table[code], y = norm(x); the codes are given, or the arg-max of each row of `logits`, which also goes to codes_out */

@@ -202,6 +202,24 @@ __global__ void __launch_bounds__(256) k_rope(__nv_bfloat16* __restrict__ x, int
  * heads instead of once per element, which is what bounded the thread-per-element form (512 rows: 29.9 -> 10.5 us, 2048: 107 -> 29).
  * grid (rows, (q_heads + 2 kv_heads) / 16), 512 threads. */
 constexpr int QKV_HEADS_PER_CTA = 16;
+/* norm (if there is a gain) and rotation of one head vector, elements 4 lane .. +3 of a warp */
+__device__ __forceinline__ void qkv_head_vector(float (&v)[4], bool gain, uint2 nw, float eps, const float2* cs, int lane) {
+    if (gain) {
+        float k = warp_tree4<false>(__fmaf_rn(v[0], v[0], 0.f), __fmaf_rn(v[1], v[1], 0.f), __fmaf_rn(v[2], v[2], 0.f), __fmaf_rn(v[3], v[3], 0.f), lane);
+        k += __shfl_xor_sync(S2P_FULL_MASK, k, 16); /* level 2 of the halving tree: the sums of elements j and j + 2 */
+        k += __shfl_xor_sync(S2P_FULL_MASK, k, 8);  /* level 1 */
+        const float inv = rsqrtf(__fdiv_rn(k, 128.0f) + eps);
+        const float w[4] = {bf_lo(nw.x), bf_hi(nw.x), bf_lo(nw.y), bf_hi(nw.y)};
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = bf16_round(__fmul_rn(__fmul_rn(v[j], inv), w[j]));
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+        const float2 f = cs[lane * 2 + (j >> 1)];
+        const float e = rope_elem(0, v[j], v[j + 1], f.x, f.y), o = rope_elem(1, v[j + 1], v[j], f.x, f.y);
+        v[j] = e; v[j + 1] = o;
+    }
+}
 __global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs a, WidePart part) {
     __shared__ float2 cs[64];
     const int r = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * QKV_HEADS_PER_CTA + (threadIdx.x >> 5);
@@ -219,23 +237,7 @@ __global__ void __launch_bounds__(32 * QKV_HEADS_PER_CTA) k_qkv_post(QkvPostArgs
     __syncthreads();
     if (!live) return;
     float v[4] = {bf_lo(x.x), bf_hi(x.x), bf_lo(x.y), bf_hi(x.y)};
-    if (rotated) {
-        if (gain) {
-            float k = warp_tree4<false>(__fmaf_rn(v[0], v[0], 0.f), __fmaf_rn(v[1], v[1], 0.f), __fmaf_rn(v[2], v[2], 0.f), __fmaf_rn(v[3], v[3], 0.f), lane);
-            k += __shfl_xor_sync(S2P_FULL_MASK, k, 16); /* level 2 of the halving tree: the sums of elements j and j + 2 */
-            k += __shfl_xor_sync(S2P_FULL_MASK, k, 8);  /* level 1 */
-            const float inv = rsqrtf(__fdiv_rn(k, 128.0f) + a.eps);
-            const float w[4] = {bf_lo(nw.x), bf_hi(nw.x), bf_lo(nw.y), bf_hi(nw.y)};
-#pragma unroll
-            for (int j = 0; j < 4; j++) v[j] = bf16_round(__fmul_rn(__fmul_rn(v[j], inv), w[j]));
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j += 2) {
-            const float2 f = cs[lane * 2 + (j >> 1)];
-            const float e = rope_elem(0, v[j], v[j + 1], f.x, f.y), o = rope_elem(1, v[j + 1], v[j], f.x, f.y);
-            v[j] = e; v[j + 1] = o;
-        }
-    }
+    if (rotated) qkv_head_vector(v, gain != nullptr, nw, a.eps, cs, lane);
     auto store_bf16 = [&](__nv_bfloat16* dst) {
         *reinterpret_cast<uint2*>(dst + lane * 4) = make_uint2((uint32_t)__bfloat16_as_ushort(f2bf(v[0])) | ((uint32_t)__bfloat16_as_ushort(f2bf(v[1])) << 16),
                                                                (uint32_t)__bfloat16_as_ushort(f2bf(v[2])) | ((uint32_t)__bfloat16_as_ushort(f2bf(v[3])) << 16));
@@ -274,6 +276,94 @@ cudaError_t qkv_post_part(const QkvPostArgs* a, const WidePart* part, int rows, 
     return launch_after(k_qkv_post, grid, 32 * QKV_HEADS_PER_CTA, 0, st, *a, part ? *part : WidePart());
 }
 cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st) { return qkv_post_part(a, nullptr, rows, st); }
+
+/* ---- the same and the attention over the few positions of the fast stack ------
+ * A frame makes 40 passes over a context of at most ten positions.  What bounds one is latency: qkv_post, a launch, then the
+ * single-row kernel, which stages both tiles and walks two 128-wide trees behind fourteen CTA barriers (2.5 + 5 us).  Here a CTA of six
+ * warps owns a (row, kv head): four query heads, the key and the value are rotated at once, the key and value go to the cache and to
+ * shared memory, and each query warp attends with a position per lane, the older positions' keys and values having been asked for
+ * before the wait for the kernel in front (passes further back wrote them).  Same chains, and the trees' other 112 or more
+ * values are zeros or -inf, so the bits are those of k_attn_single.  Bf16 caches, one position for all rows. */
+constexpr int FAST_ATTN_MAX = 16; /* positions */
+__global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part, __nv_bfloat16* __restrict__ out, int head_dim) {
+    __shared__ float2 cs[64];
+    __shared__ __align__(16) float sq[4][128];
+    __shared__ __align__(16) __nv_bfloat16 now[2][128]; /* this position's key and value */
+    const int r = blockIdx.x, kvh = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int QH = a.q_heads, KVH = a.kv_heads, heads = QH + 2 * KVH, pos = a.pos0;
+    const bool is_q = warp < 4;
+    const int h = is_q ? kvh * 4 + warp : warp == 4 ? QH + kvh : QH + KVH + kvh;
+    unsigned char* const base = kv_payload(a.kv, r);
+    __nv_bfloat16* const kc = reinterpret_cast<__nv_bfloat16*>(base + a.kv.k_off) + (size_t)kvh * a.max_seq * 128;
+    __nv_bfloat16* const vc = reinterpret_cast<__nv_bfloat16*>(base + a.kv.v_off) + (size_t)kvh * a.max_seq * 128;
+    uint4 k[16];
+    uint2 vv[FAST_ATTN_MAX], nw = make_uint2(0u, 0u);
+    if (is_q) {
+#pragma unroll
+        for (int c = 0; c < 16; c++) k[c] = lane < pos ? reinterpret_cast<const uint4*>(kc + lane * 128)[c] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int j = 0; j < FAST_ATTN_MAX; j++) vv[j] = j < pos ? reinterpret_cast<const uint2*>(vc + j * 128)[lane] : make_uint2(0u, 0u);
+    }
+    const __nv_bfloat16* gain = is_q ? a.q_norm : warp == 4 ? a.k_norm : nullptr;
+    if (gain) nw = *reinterpret_cast<const uint2*>(gain + lane * 4);
+    if (threadIdx.x < 64) rope_cs(threadIdx.x, pos, a.rope_base, cs[threadIdx.x].x, cs[threadIdx.x].y);
+    grid_wait();
+    grid_release();
+    const uint2 x = part.partial ? wide_part4_bf16(part, h * 128 + lane * 4, r) : *reinterpret_cast<const uint2*>(a.qkv + ((size_t)r * heads + h) * 128 + lane * 4);
+    __syncthreads();
+    float v[4] = {bf_lo(x.x), bf_hi(x.x), bf_lo(x.y), bf_hi(x.y)};
+    if (warp != 5) qkv_head_vector(v, gain != nullptr, nw, a.eps, cs, lane);
+    if (is_q) {
+        const float scale = rsqrtf((float)head_dim); /* run-time value on purpose, see AttnArgs */
+#pragma unroll
+        for (int j = 0; j < 4; j++) sq[warp][lane * 4 + j] = __fmul_rn(bf16_round(v[j]), scale);
+    } else {
+        const uint2 o = make_uint2((uint32_t)__bfloat16_as_ushort(f2bf(v[0])) | ((uint32_t)__bfloat16_as_ushort(f2bf(v[1])) << 16),
+                                   (uint32_t)__bfloat16_as_ushort(f2bf(v[2])) | ((uint32_t)__bfloat16_as_ushort(f2bf(v[3])) << 16));
+        reinterpret_cast<uint2*>(now[warp - 4])[lane] = o;
+        reinterpret_cast<uint2*>((warp == 4 ? kc : vc) + (size_t)pos * 128)[lane] = o;
+    }
+    __syncthreads();
+    if (!is_q) return;
+    if (lane == pos)
+#pragma unroll
+        for (int c = 0; c < 16; c++) k[c] = reinterpret_cast<const uint4*>(now[0])[c];
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+        const uint32_t w[4] = {k[c].x, k[c].y, k[c].z, k[c].w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            s = __fmaf_rn(sq[warp][c * 8 + 2 * j], bf_lo(w[j]), s);
+            s = __fmaf_rn(sq[warp][c * 8 + 2 * j + 1], bf_hi(w[j]), s);
+        }
+    }
+    if (lane > pos) s = -INFINITY;
+    const float m = warp_tree_max(s);
+    const float p = s == -INFINITY ? 0.f : expf(s - m);
+    const float l = warp_tree_sum(p);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint2 mine = reinterpret_cast<const uint2*>(now[1])[lane];
+#pragma unroll
+    for (int j = 0; j < FAST_ATTN_MAX; j++) {
+        if (j > pos) break;
+        const float pj = __shfl_sync(S2P_FULL_MASK, p, j);
+        const uint2 u = j == pos ? mine : vv[j];
+        acc[0] = __fmaf_rn(pj, bf_lo(u.x), acc[0]); acc[1] = __fmaf_rn(pj, bf_hi(u.x), acc[1]);
+        acc[2] = __fmaf_rn(pj, bf_lo(u.y), acc[2]); acc[3] = __fmaf_rn(pj, bf_hi(u.y), acc[3]);
+    }
+    uint2 o;
+    o.x = (uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[0], l))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[1], l))) << 16);
+    o.y = (uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[2], l))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[3], l))) << 16);
+    reinterpret_cast<uint2*>(out + ((size_t)r * QH + h) * 128)[lane] = o;
+}
+cudaError_t fast_attn(const QkvPostArgs* a, const WidePart* part, void* out, int head_dim, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    if (a->kv8 || a->pos_arr || a->pos_row_step || a->pos0 < 0 || a->pos0 >= FAST_ATTN_MAX || a->pos0 >= a->max_seq || a->q_heads != 4 * a->kv_heads || head_dim != 128 ||
+        (((uintptr_t)a->kv.base0 | a->kv.k_off | a->kv.v_off | a->kv.row_stride) & 15))
+        return cudaErrorInvalidValue;
+    return launch_after(k_fast_attn, dim3((unsigned)rows, (unsigned)a->kv_heads), 192, 0, st, *a, part ? *part : WidePart(), (__nv_bfloat16*)out, head_dim);
+}
 
 /* ---- plain KV append (contract s2pk_kv_append, kernels.cu:172-195) --------- */
 __global__ void __launch_bounds__(256) k_kv_append(const __nv_bfloat16* __restrict__ k,

@@ -213,6 +213,10 @@ static s2p_status layer_attention(s2p_model* m, const s2p_layer* L, const layer_
     qa.eps = S2P_NORM_EPS; qa.rope_base = S2P_ROPE_BASE;
     qa.q_heads = S2P_SLOW_Q_HEADS; qa.kv_heads = S2P_SLOW_KV_HEADS; qa.max_seq = c->max_seq; qa.kv8 = c->kv8;
     qa.pos0 = c->pos0; qa.pos_row_step = c->pos_row_step; qa.pos_arr = c->pos_arr; qa.kv = c->kv;
+    if (c->decode && !c->split_k) { /* the fast stack */
+        S2P_LAUNCH(m, fast_attn(&qa, part, attn, S2P_HEAD_DIM, rows, st));
+        return S2P_OK;
+    }
     S2P_LAUNCH(m, qkv_post_part(&qa, part, rows, st));
     AttnArgs aa;
     memset(&aa, 0, sizeof(aa));
