@@ -63,6 +63,7 @@ struct NormRowArgs {
     int part_logits;
     uint4* tiled;                /* the norm also as matrix units of the next linear (wide.cuh), for a batch padded to 1 << lg rows */
     int tiled_int4, lg;
+    int settled;                 /* the gains are a model's: the kernel in front does not write them */
 };
 constexpr int NORM_MAX_WIDTH = 4096; /* two vectors per thread */
 __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
@@ -71,14 +72,16 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
     __shared__ unsigned long long best[8];
     const int tid = threadIdx.x, r = blockIdx.x, nv = a.width >> 3;
     const int v0 = tid, v1 = tid + 256;
+    uint4 g0 = make_uint4(0, 0, 0, 0), g1 = g0;
+    auto gains = [&] {
+        if (v0 < nv) g0 = reinterpret_cast<const uint4*>(a.w)[v0];
+        if (v1 < nv) g1 = reinterpret_cast<const uint4*>(a.w)[v1];
+    };
+    if (a.w && a.settled) gains();
     if (a.tiled) grid_release(); /* a wide linear is next: see launch.cuh */
     grid_wait();
     if (!a.tiled) grid_release();
-    uint4 g0 = make_uint4(0, 0, 0, 0), g1 = g0;
-    if (a.w) {
-        if (v0 < nv) g0 = reinterpret_cast<const uint4*>(a.w)[v0];
-        if (v1 < nv) g1 = reinterpret_cast<const uint4*>(a.w)[v1];
-    }
+    if (a.w && !a.settled) gains();
     size_t row = (size_t)r;
     auto offer = [](unsigned long long& key, float l, int i) {
         if (l != l) return; /* a row of NaN gives index 0, as the reference's */
@@ -719,12 +722,14 @@ cudaError_t rms_norm(const void* x, const void* w, void* y, int rows, int width,
 cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     NormRowArgs a = {};
+    a.settled = 1;
     a.src = (const __nv_bfloat16*)x; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
     return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }
 static NormRowArgs wide_norm_args(void* x, const void* w, void* y, void* y_tiled, int kind, int rows) {
     NormRowArgs a = {};
+    a.settled = 1;
     a.x_out = (__nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y;
     a.tiled = (uint4*)y_tiled; a.tiled_int4 = kind == WK_INT4_PACK; a.lg = wide_lg(rows);
     a.width = S2P_DIM; a.table_rows = S2P_CB_SIZE; a.eps = S2P_NORM_EPS;
@@ -751,6 +756,7 @@ cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WideP
 cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     NormRowArgs a = {};
+    a.settled = 1;
     a.src = (const __nv_bfloat16*)src; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
     return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
@@ -758,6 +764,7 @@ cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows
 cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logits, int32_t* codes_out, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     NormRowArgs a = {};
+    a.settled = 1;
     a.src = (const __nv_bfloat16*)table; a.codes = codes; a.logits = (const __nv_bfloat16*)logits; a.codes_out = codes_out;
     a.x_out = (__nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y;
     a.width = S2P_DIM; a.table_rows = S2P_CB_SIZE; a.eps = S2P_NORM_EPS;
