@@ -130,14 +130,15 @@ extern "C" cudaError_t gemv_setup_all(void) {
  * Measured, us for one layer's four matrices (N x K 6144 x 2560, 2560 x 4096, 19456 x 2560, 2560 x 9728), before (scalar fma, one
  * weight row per warp for INT8; mixed bf16 fma, one to four for INT4) and now, at 2 / 4 / 8 / 16 rows:
  *   INT8  52 / 84 / 148 / 258 -> 44 / 56 / 83 / 138      INT4  46 / 70 / 103 / 180 -> 46 / 58 / 85 / 144
+ * An odd row's chain is scalar: padded to a pair it held the fma pipe for two (3 rows INT4 58 -> 53, 5 rows 74 -> 68, 9 rows 119 -> 108).
  * 16 rows of 19456 x 2560 run at 13.5 T fma/s; the pipe's rate is 36 T. */
-/* A SwiGLU over stacked [gate | up] rows (SW): a warp's four rows are two of either half, so gate and up of an output meet in
+/* A SwiGLU over stacked [gate | up] rows (SW): half of a warp's rows are of either half, so gate and up of an output meet in
  * the warp; both round to bf16 first, as where a kernel of its own follows the linear. */
-template <bool SW> __device__ __forceinline__ int gemv_row_of(int n0, int r, int F) {
-    return SW ? min(n0 + (r & 1), F - 1) + (r >> 1) * F : min(n0 + r, F - 1);
+template <bool SW, int R> __device__ __forceinline__ int gemv_row_of(int n0, int r, int F) {
+    return SW ? min(n0 + r % (R / 2), F - 1) + r / (R / 2) * F : min(n0 + r, F - 1);
 }
-__device__ __forceinline__ float gemv_swiglu(float a) {
-    const float g = bf16_round(a), up = bf16_round(__shfl_down_sync(S2P_FULL_MASK, a, 16));
+__device__ __forceinline__ float gemv_swiglu(float gate, float up_) {
+    const float g = bf16_round(gate), up = bf16_round(up_);
     const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
     return __fmul_rn(bf16_round(__fmul_rn(g, sig)), up);
 }
@@ -186,7 +187,8 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
                                                        const void* __restrict__ w, const void* __restrict__ scales,
                                                        int M, int N, int K, int gshift) {
     typedef typename LaneTile<WK>::type tile_t;
-    constexpr int R = 4, P = MM / 2; /* weight rows of a warp, pairs of activation rows */
+    constexpr int R = 4, P = MM / 2; /* weight rows of a warp, pairs of activation rows; an odd last one has scalar chains */
+    constexpr bool ODD = MM % 2 != 0;
     constexpr int PD = WK == WK_INT4_PACK && MM <= 4 ? 2 : 1; /* tiles of weights under way */
     constexpr int FM = NS == 1 ? MM : (MM + NS - 1) / NS; /* activation rows whose sums this warp keeps */
     __shared__ float part[NS == 1 ? 1 : 2 * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][m, then the scales][row][lane] */
@@ -204,7 +206,7 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
     const __half* srow[R];
 #pragma unroll
     for (int r = 0; r < R; r++) { /* rows beyond the last repeat it and are not stored */
-        const int n = gemv_row_of<SW>(n0, r, F);
+        const int n = gemv_row_of<SW, R>(n0, r, F);
         wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
         srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
     }
@@ -239,10 +241,13 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
         if (i + PD * NS < T) fetch(d, i + PD * NS);
         if (NS == 1 || i < T) {
             f32x2 s[R][P];
+            float so[R];
 #pragma unroll
-            for (int r = 0; r < R; r++)
+            for (int r = 0; r < R; r++) {
+                so[r] = 0.f;
 #pragma unroll
                 for (int p = 0; p < P; p++) s[r][p] = 0ull;
+            }
 #pragma unroll
             for (int h = 0; h < 2; h++) { /* eight k of the lane's sixteen */
                 uint4 xv[MM];
@@ -253,40 +258,41 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
                 for (int r = 0; r < R; r++) BatchCodes<WK>::widen8(cur[r], h, wf[r]);
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
+                    auto word = [&](const uint4& v) { return (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w; };
+                    auto value = [&](int m) { return j & 1 ? bf_hi(word(xv[m])) : bf_lo(word(xv[m])); };
                     f32x2 xx[P];
 #pragma unroll
-                    for (int p = 0; p < P; p++) {
-                        auto word = [&](const uint4& v) { return (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w; };
-                        const uint32_t x0 = word(xv[2 * p]), x1 = word(xv[2 * p + 1]);
-                        xx[p] = j & 1 ? pack2(bf_hi(x0), bf_hi(x1)) : pack2(bf_lo(x0), bf_lo(x1));
-                    }
+                    for (int p = 0; p < P; p++) xx[p] = pack2(value(2 * p), value(2 * p + 1));
 #pragma unroll
-                    for (int r = 0; r < R; r++)
+                    for (int r = 0; r < R; r++) {
 #pragma unroll
                         for (int p = 0; p < P; p++) ffma2(s[r][p], wf[r][j], xx[p]);
+                        if (ODD) {
+                            float w0, w1;
+                            unpack2(wf[r][j], w0, w1);
+                            so[r] = __fmaf_rn(w0, value(MM - 1), so[r]);
+                        }
+                    }
                 }
             }
+            auto sum_of = [&](int r, int m) {
+                if (ODD && m == MM - 1) return so[r];
+                float lo, hi;
+                unpack2(s[r][m >> 1], lo, hi);
+                return m & 1 ? hi : lo;
+            };
             if (NS == 1) {
 #pragma unroll
                 for (int r = 0; r < R; r++)
 #pragma unroll
-                    for (int p = 0; p < P; p++) {
-                        float s0, s1;
-                        unpack2(s[r][p], s0, s1);
-                        acc[2 * p][r] = WK == WK_INT8_CH ? acc[2 * p][r] + s0 : __fmaf_rn(s0, gs[r], acc[2 * p][r]);
-                        acc[2 * p + 1][r] = WK == WK_INT8_CH ? acc[2 * p + 1][r] + s1 : __fmaf_rn(s1, gs[r], acc[2 * p + 1][r]);
-                    }
+                    for (int m = 0; m < MM; m++)
+                        acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + sum_of(r, m) : __fmaf_rn(sum_of(r, m), gs[r], acc[m][r]);
             } else {
                 float* at = part + ((rnd & 1) * NS + ns) * ((MM + 1) * R * 32) + lane;
 #pragma unroll
                 for (int r = 0; r < R; r++) {
 #pragma unroll
-                    for (int p = 0; p < P; p++) {
-                        float s0, s1;
-                        unpack2(s[r][p], s0, s1);
-                        at[((2 * p) * R + r) * 32] = s0;
-                        at[((2 * p + 1) * R + r) * 32] = s1;
-                    }
+                    for (int m = 0; m < MM; m++) at[(m * R + r) * 32] = sum_of(r, m);
                     if (WK != WK_INT8_CH) at[(MM * R + r) * 32] = gs[r];
                 }
             }
@@ -312,13 +318,13 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
     }
     /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
     const int r = lane >> 3, n = n0 + r;
-    const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[gemv_row_of<SW>(n0, r, F)] : 1.f;
+    const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)] : 1.f;
 #pragma unroll
     for (int m = 0; m < FM; m++) {
         const int mm = NS == 1 ? m : ns * FM + m;
         float a = warp_tree4<false>(acc[m][0], acc[m][1], acc[m][2], acc[m][3], lane);
         if (WK == WK_INT8_CH) a = __fmul_rn(a, rs);
-        if (SW) a = gemv_swiglu(a);
+        if (SW) a = gemv_swiglu(a, __shfl_down_sync(S2P_FULL_MASK, a, 16));
         if ((lane & 7) == 0 && mm < M && n < F && r < (SW ? R / 2 : R)) y[(size_t)mm * F + n] = f2bf(a);
     }
 }
@@ -332,12 +338,12 @@ static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const v
 template <int WK, bool SW>
 cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K,
                               int gshift, int early, cudaStream_t stream) {
-    /* As few groups of activation rows as eight a group allow (each converts every code once), of even size.  Four warps share
+    /* As few groups of activation rows as eight a group allow (each converts every code once), of one size.  Four warps share
      * four rows where one warp each would leave a scheduler with less than 2.5, which do not hide each other's latencies, provided
      * that three quarters of the rounds' turns have a tile (a CTA waits for its slowest warp: at K = 2560, five tiles
      * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all.  (A SwiGLU's pairs of rows
      * meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
-    const int groups = (M + 7) / 8, mm = ((M + groups - 1) / groups + 1) & ~1;
+    const int groups = (M + 7) / 8, mm = (M + groups - 1) / groups;
     const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
     const int T = K >> 9, turns = (T + 3) / 4 * 4;
     const bool shared = !SW && (2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
@@ -347,9 +353,12 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
         return run_gemv_batch<WK, MM, 1, SW>(y, x, w, scales, M, N, K, gshift, early, stream);                \
     } while (0)
     if (mm == 2) S2P_GB(2);
+    if (mm == 3) S2P_GB(3);
     if (mm == 4) S2P_GB(4);
     if constexpr (!SW) {
+        if (mm == 5) S2P_GB(5);
         if (mm == 6) S2P_GB(6);
+        if (mm == 7) S2P_GB(7);
         S2P_GB(8);
     }
     return cudaErrorInvalidValue;
@@ -359,17 +368,17 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
 /* ---- one row ---------------------------------------------------------------
  * The linear alone, as a caller's own layers and the frames outside the persistent tick use it.
  *
- * What bounds it: DRAM, at a few thousand warps whose weights are all under way at once.  A warp carries four rows as two
+ * What bounds it: DRAM, at a few thousand warps whose weights are all under way at once.  A warp carries four rows (or six) as
  * packed chains (a register pair holds the same k of two rows), PD tiles at a time side by side, since every tile starts a chain of its
  * own; the next PD tiles' weights are in registers meanwhile.  Where there are too few rows for that NS = 4 warps share
  * four rows as in k_gemv_batch.
  * Measured, us (before: a CTA per SM with the tiles' sums in shared memory): INT4 6144 x 2560 10.2 -> 6.4, 2560 x 4096 8.2 -> 4.6,
- * 19456 x 2560 25.3 -> 13.5, 2560 x 9728 14.9 -> 9.7; INT8 8.5 -> 6.2, 6.8 -> 4.8, 18.9 -> 11.2, 10.7 -> 8.6. */
-template <int WK, int PD, int NS, bool SW>
-__global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+ * 19456 x 2560 25.3 -> 12.9, 2560 x 9728 14.9 -> 9.7; INT8 8.5 -> 6.2, 6.8 -> 4.8, 18.9 -> 11.2, 10.7 -> 8.6. */
+template <int WK, int R, int PD, int NS, bool SW>
+__global__ void __launch_bounds__(128, R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
                                                      const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift) {
     typedef typename LaneTile<WK>::type tile_t;
-    constexpr int R = 4;
+    constexpr int P = R / 2;
     __shared__ float part[NS == 1 ? 1 : 2 * PD * NS * 2 * R * 32]; /* [round parity][tile of the round][sums, then scales][row][lane] */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int F = SW ? N >> 1 : N; /* outputs */
@@ -381,7 +390,7 @@ __global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16
     const __half* srow[R];
 #pragma unroll
     for (int r = 0; r < R; r++) { /* rows beyond the last repeat it and are not stored */
-        const int n = gemv_row_of<SW>(n0, r, F);
+        const int n = gemv_row_of<SW, R>(n0, r, F);
         wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
         srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
     }
@@ -402,7 +411,9 @@ __global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16
     fetch(0);
     grid_wait();
     grid_release();
-    float acc[R] = {0.f, 0.f, 0.f, 0.f};
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) acc[r] = 0.f;
     const int rounds = (T + NS * PD - 1) / (NS * PD);
     for (int rnd = 0; rnd < rounds; rnd++) {
         uint4 xv[PD][2];
@@ -417,16 +428,18 @@ __global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16
 #pragma unroll
             for (int r = 0; r < R; r++) { cur[d][r] = nxt[d][r]; gs[d][r] = __half2float(gnx[d][r]); }
         if (rnd + 1 < rounds) fetch(rnd + 1);
-        f32x2 s[PD][R / 2];
+        f32x2 s[PD][P];
 #pragma unroll
-        for (int d = 0; d < PD; d++) s[d][0] = s[d][1] = 0ull;
+        for (int d = 0; d < PD; d++)
+#pragma unroll
+            for (int q = 0; q < P; q++) s[d][q] = 0ull;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            f32x2 wf[PD][R / 2][8];
+            f32x2 wf[PD][P][8];
 #pragma unroll
             for (int d = 0; d < PD; d++)
 #pragma unroll
-                for (int q = 0; q < R / 2; q++) BatchCodes<WK>::widen8(cur[d][2 * q], cur[d][2 * q + 1], h, wf[d][q]);
+                for (int q = 0; q < P; q++) BatchCodes<WK>::widen8(cur[d][2 * q], cur[d][2 * q + 1], h, wf[d][q]);
 #pragma unroll
             for (int j = 0; j < 8; j++)
 #pragma unroll
@@ -436,7 +449,7 @@ __global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16
                     const float xf = j & 1 ? bf_hi(u) : bf_lo(u);
                     const f32x2 xx = pack2(xf, xf);
 #pragma unroll
-                    for (int q = 0; q < R / 2; q++) ffma2(s[d][q], wf[d][q][j], xx);
+                    for (int q = 0; q < P; q++) ffma2(s[d][q], wf[d][q][j], xx);
                 }
         }
         auto fold = [&](int r, float v, float g) { acc[r] = WK == WK_INT8_CH ? acc[r] + v : __fmaf_rn(v, g, acc[r]); };
@@ -444,8 +457,8 @@ __global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16
         for (int d = 0; d < PD; d++) {
             if (tile_of(rnd, d) >= T) continue;
             float v[R];
-            unpack2(s[d][0], v[0], v[1]);
-            unpack2(s[d][1], v[2], v[3]);
+#pragma unroll
+            for (int q = 0; q < P; q++) unpack2(s[d][q], v[2 * q], v[2 * q + 1]);
             float* at = part + (((rnd & 1) * NS + ns) * PD + d) * (2 * R * 32) + lane;
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -460,12 +473,23 @@ __global__ void __launch_bounds__(128, PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16
             for (int t = 0; t < live; t++) fold(0, at[t * (2 * R * 32)], at[t * (2 * R * 32) + R * 32]);
         }
     }
-    if (NS == 1) {
+    if (R != 4) { /* every lane has every sum */
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            acc[r] = warp_tree_sum(acc[r]);
+            if (WK == WK_INT8_CH) acc[r] = __fmul_rn(acc[r], static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
+        }
+#pragma unroll
+        for (int r = 0; r < (SW ? P : R); r++) {
+            const float a = SW ? gemv_swiglu(acc[r], acc[r + (SW ? P : 0)]) : acc[r];
+            if (lane == r && n0 + r < F) y[n0 + r] = f2bf(a);
+        }
+    } else if (NS == 1) {
         /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
         const int r = lane >> 3, n = n0 + r;
         float a = warp_tree4<false>(acc[0], acc[1], acc[2], acc[3], lane);
-        if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[gemv_row_of<SW>(n0, r, F)]);
-        if (SW) a = gemv_swiglu(a);
+        if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
+        if (SW) a = gemv_swiglu(a, __shfl_down_sync(S2P_FULL_MASK, a, 16));
         if ((lane & 7) == 0 && n < F && r < (SW ? R / 2 : R)) y[n] = f2bf(a);
     } else {
         float a = warp_tree_sum(acc[0]);
@@ -480,11 +504,14 @@ template <int WK, bool SW>
 static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const void* scales, int N, int K, int gshift, int early, cudaStream_t stream) {
     /* Four warps share four rows where one each would give a scheduler less than 1.5, if most of their turns have a tile
      * (2560 x 9728: 14.0 -> 9.7 us, 6144 x 2560 the other way round 6.4 -> 7.7).  From six warps per scheduler on a tile at a time
-     * and twice the warps resident hide more than two tiles side by side (19456 x 2560: 14.4 -> 13.5; 6144: 6.4 -> 6.7). */
-    const int warps = (N + 3) / 4, sched = 4 * device_sm_count();
-    const bool shared = !SW && 2 * warps < 3 * sched && K > 4 * 512, many = warps >= 6 * sched;
+     * with twice the warps resident hides more than two tiles side by side; INT4, whose tiles are half the loads, also takes six rows a
+     * warp there, which keeps 19456 rows from a second wave (INT4 14.4 -> 13.5 -> 12.9 us, INT8 12.5 -> 11.2, 11.5 with six rows). */
+    const int sms = device_sm_count(), quads = (N + 3) / 4;
+    const bool shared = !SW && 2 * quads < 3 * 4 * sms && K > 4 * 512, many = quads >= 6 * 4 * sms;
+    constexpr int MANY = WK == WK_INT4_PACK ? 6 : 4;
     void (*kernel)(__nv_bfloat16*, const __nv_bfloat16*, const void*, const void*, int, int, int) =
-        shared ? k_gemv_row<WK, 2, SW ? 1 : 4, SW> : many ? k_gemv_row<WK, 1, 1, SW> : k_gemv_row<WK, 2, 1, SW>;
+        shared ? k_gemv_row<WK, 4, 2, SW ? 1 : 4, SW> : many ? k_gemv_row<WK, MANY, 1, 1, SW> : k_gemv_row<WK, 4, 2, 1, SW>;
+    const int per_warp = many ? MANY : 4, warps = (N + per_warp - 1) / per_warp;
     return launch_gemv(kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, early, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, N, K, gshift);
 }
