@@ -365,7 +365,7 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
 #undef S2P_GB
 }
 
-/* ---- one row ---------------------------------------------------------------
+/* ---- one row, or two of a matrix of few rows ---------------------------------
  * The linear alone, as a caller's own layers and the frames outside the persistent tick use it.
  *
  * What bounds it: DRAM, at a few thousand warps whose weights are all under way at once.  A warp carries four rows (or six) as
@@ -374,12 +374,12 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
  * four rows as in k_gemv_batch.
  * Measured, us (before: a CTA per SM with the tiles' sums in shared memory): INT4 6144 x 2560 10.2 -> 6.4, 2560 x 4096 8.2 -> 4.6,
  * 19456 x 2560 25.3 -> 12.9, 2560 x 9728 14.9 -> 9.7; INT8 8.5 -> 6.2, 6.8 -> 4.8, 18.9 -> 11.2, 10.7 -> 8.6. */
-template <int WK, int R, int PD, int NS, bool SW>
-__global__ void __launch_bounds__(128, R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+template <int WK, int MM, int R, int PD, int NS, bool SW>
+__global__ void __launch_bounds__(128, MM == 2 ? 4 : R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
                                                      const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift) {
     typedef typename LaneTile<WK>::type tile_t;
     constexpr int P = R / 2;
-    __shared__ float part[NS == 1 ? 1 : 2 * PD * NS * 2 * R * 32]; /* [round parity][tile of the round][sums, then scales][row][lane] */
+    __shared__ float part[NS == 1 ? 1 : 2 * PD * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][sums, then scales][row][lane] */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int F = SW ? N >> 1 : N; /* outputs */
     const int n0 = (blockIdx.x * (4 / NS) + warp / NS) * (SW ? R / 2 : R), ns = warp % NS;
@@ -411,16 +411,20 @@ __global__ void __launch_bounds__(128, R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(
     fetch(0);
     grid_wait();
     grid_release();
-    float acc[R];
+    float acc[MM][R];
 #pragma unroll
-    for (int r = 0; r < R; r++) acc[r] = 0.f;
+    for (int m = 0; m < MM; m++)
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[m][r] = 0.f;
     const int rounds = (T + NS * PD - 1) / (NS * PD);
     for (int rnd = 0; rnd < rounds; rnd++) {
-        uint4 xv[PD][2];
+        uint4 xv[PD][2][MM];
 #pragma unroll
         for (int d = 0; d < PD; d++)
 #pragma unroll
-            for (int h = 0; h < 2; h++) xv[d][h] = *reinterpret_cast<const uint4*>(x + min(tile_of(rnd, d), T - 1) * 512 + lane * 16 + h * 8);
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int m = 0; m < MM; m++) xv[d][h][m] = *reinterpret_cast<const uint4*>(x + (size_t)m * K + min(tile_of(rnd, d), T - 1) * 512 + lane * 16 + h * 8);
         tile_t cur[PD][R];
         float gs[PD][R];
 #pragma unroll
@@ -428,11 +432,13 @@ __global__ void __launch_bounds__(128, R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(
 #pragma unroll
             for (int r = 0; r < R; r++) { cur[d][r] = nxt[d][r]; gs[d][r] = __half2float(gnx[d][r]); }
         if (rnd + 1 < rounds) fetch(rnd + 1);
-        f32x2 s[PD][P];
+        f32x2 s[PD][MM][P];
 #pragma unroll
         for (int d = 0; d < PD; d++)
 #pragma unroll
-            for (int q = 0; q < P; q++) s[d][q] = 0ull;
+            for (int m = 0; m < MM; m++)
+#pragma unroll
+                for (int q = 0; q < P; q++) s[d][m][q] = 0ull;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             f32x2 wf[PD][P][8];
@@ -444,73 +450,91 @@ __global__ void __launch_bounds__(128, R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(
             for (int j = 0; j < 8; j++)
 #pragma unroll
                 for (int d = 0; d < PD; d++) {
-                    const uint4& v = xv[d][h];
-                    const uint32_t u = (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w;
-                    const float xf = j & 1 ? bf_hi(u) : bf_lo(u);
-                    const f32x2 xx = pack2(xf, xf);
 #pragma unroll
-                    for (int q = 0; q < P; q++) ffma2(s[d][q], wf[d][q][j], xx);
+                    for (int m = 0; m < MM; m++) {
+                        const uint4& v = xv[d][h][m];
+                        const uint32_t u = (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w;
+                        const float xf = j & 1 ? bf_hi(u) : bf_lo(u);
+                        const f32x2 xx = pack2(xf, xf);
+#pragma unroll
+                        for (int q = 0; q < P; q++) ffma2(s[d][m][q], wf[d][q][j], xx);
+                    }
                 }
         }
-        auto fold = [&](int r, float v, float g) { acc[r] = WK == WK_INT8_CH ? acc[r] + v : __fmaf_rn(v, g, acc[r]); };
+        auto fold = [&](int m, int r, float v, float g) { acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + v : __fmaf_rn(v, g, acc[m][r]); };
 #pragma unroll
         for (int d = 0; d < PD; d++) {
             if (tile_of(rnd, d) >= T) continue;
-            float v[R];
+            float* at = part + (((rnd & 1) * NS + ns) * PD + d) * ((MM + 1) * R * 32) + lane;
 #pragma unroll
-            for (int q = 0; q < P; q++) unpack2(s[d][q], v[2 * q], v[2 * q + 1]);
-            float* at = part + (((rnd & 1) * NS + ns) * PD + d) * (2 * R * 32) + lane;
+            for (int m = 0; m < MM; m++) {
+                float v[R];
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                if (NS == 1) fold(r, v[r], gs[d][r]);
-                else { at[r * 32] = v[r]; at[(R + r) * 32] = gs[d][r]; }
+                for (int q = 0; q < P; q++) unpack2(s[d][m][q], v[2 * q], v[2 * q + 1]);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    if (NS == 1) fold(m, r, v[r], gs[d][r]);
+                    else at[(m * R + r) * 32] = v[r];
+                }
             }
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (NS > 1) at[(MM * R + r) * 32] = gs[d][r];
         }
         if (NS > 1) { /* the round's tiles in ascending order; warp ns keeps row ns */
             __syncthreads();
             const int live = min(NS * PD, T - rnd * NS * PD);
-            const float* at = part + (rnd & 1) * NS * PD * (2 * R * 32) + ns * 32 + lane;
-            for (int t = 0; t < live; t++) fold(0, at[t * (2 * R * 32)], at[t * (2 * R * 32) + R * 32]);
+            const float* at = part + (rnd & 1) * NS * PD * ((MM + 1) * R * 32) + ns * 32 + lane;
+            for (int t = 0; t < live; t++, at += (MM + 1) * R * 32)
+#pragma unroll
+                for (int m = 0; m < MM; m++) fold(m, 0, at[m * R * 32], at[MM * R * 32]);
         }
     }
+#pragma unroll
+    for (int m = 0; m < MM; m++, y += F) {
     if (R != 4) { /* every lane has every sum */
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            acc[r] = warp_tree_sum(acc[r]);
-            if (WK == WK_INT8_CH) acc[r] = __fmul_rn(acc[r], static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
+            acc[m][r] = warp_tree_sum(acc[m][r]);
+            if (WK == WK_INT8_CH) acc[m][r] = __fmul_rn(acc[m][r], static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
         }
 #pragma unroll
         for (int r = 0; r < (SW ? P : R); r++) {
-            const float a = SW ? gemv_swiglu(acc[r], acc[r + (SW ? P : 0)]) : acc[r];
+            const float a = SW ? gemv_swiglu(acc[m][r], acc[m][r + (SW ? P : 0)]) : acc[m][r];
             if (lane == r && n0 + r < F) y[n0 + r] = f2bf(a);
         }
     } else if (NS == 1) {
         /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
         const int r = lane >> 3, n = n0 + r;
-        float a = warp_tree4<false>(acc[0], acc[1], acc[2], acc[3], lane);
+        float a = warp_tree4<false>(acc[m][0], acc[m][1], acc[m][2], acc[m][3], lane);
         if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
         if (SW) a = gemv_swiglu(a, __shfl_down_sync(S2P_FULL_MASK, a, 16));
         if ((lane & 7) == 0 && n < F && r < (SW ? R / 2 : R)) y[n] = f2bf(a);
     } else {
-        float a = warp_tree_sum(acc[0]);
+        float a = warp_tree_sum(acc[m][0]);
         if (n0 + ns < N && lane == 0) {
             if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[n0 + ns]);
             y[n0 + ns] = f2bf(a);
         }
     }
+    }
 }
 
+/* Four warps share four rows where one each would give a scheduler less than 1.5, if most of their turns have a tile
+ * (2560 x 9728: 14.0 -> 9.7 us, 6144 x 2560 the other way round 6.4 -> 7.7). */
+static bool gemv_row_shared(int N, int K) { return 2 * ((N + 3) / 4) < 3 * 4 * device_sm_count() && K > 4 * 512; }
 template <int WK, bool SW>
-static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const void* scales, int N, int K, int gshift, int early, cudaStream_t stream) {
-    /* Four warps share four rows where one each would give a scheduler less than 1.5, if most of their turns have a tile
-     * (2560 x 9728: 14.0 -> 9.7 us, 6144 x 2560 the other way round 6.4 -> 7.7).  From six warps per scheduler on a tile at a time
-     * with twice the warps resident hides more than two tiles side by side; INT4, whose tiles are half the loads, also takes six rows a
-     * warp there, which keeps 19456 rows from a second wave (INT4 14.4 -> 13.5 -> 12.9 us, INT8 12.5 -> 11.2, 11.5 with six rows). */
-    const int sms = device_sm_count(), quads = (N + 3) / 4;
-    const bool shared = !SW && 2 * quads < 3 * 4 * sms && K > 4 * 512, many = quads >= 6 * 4 * sms;
+static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
+    /* From six warps per scheduler on a tile at a time with twice the warps resident hides more than two tiles side by side; INT4,
+     * whose tiles are half the loads, also takes six rows a warp there, which keeps 19456 rows from a second wave (INT4 14.4 -> 13.5 ->
+     * 12.9 us, INT8 12.5 -> 11.2, 11.5 with six rows). */
+    const bool shared = !SW && gemv_row_shared(N, K), many = (N + 3) / 4 >= 6 * 4 * device_sm_count();
     constexpr int MANY = WK == WK_INT4_PACK ? 6 : 4;
     void (*kernel)(__nv_bfloat16*, const __nv_bfloat16*, const void*, const void*, int, int, int) =
-        shared ? k_gemv_row<WK, 4, 2, SW ? 1 : 4, SW> : many ? k_gemv_row<WK, MANY, 1, 1, SW> : k_gemv_row<WK, 4, 2, 1, SW>;
+        many ? k_gemv_row<WK, 1, MANY, 1, 1, SW> : k_gemv_row<WK, 1, 4, 2, 1, SW>;
+    if constexpr (!SW) {
+        if (shared) kernel = M == 2 ? k_gemv_row<WK, 2, 4, 2, 4, false> : k_gemv_row<WK, 1, 4, 2, 4, false>;
+    }
     const int per_warp = many ? MANY : 4, warps = (N + per_warp - 1) / per_warp;
     return launch_gemv(kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, early, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, N, K, gshift);
@@ -529,8 +553,8 @@ s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, c
     /* 16-byte loads of activations and weight tiles */
     if (((uintptr_t)x | (uintptr_t)w) & 15) return S2P_ERR_INVALID;
     cudaError_t ce;
-    if (M == 1) {
-        ce = launch_gemv_row<WK, SW>(y, x, w, scales, N, K, gshift, early, stream);
+    if (M == 1 || (M == 2 && !SW && gemv_row_shared(N, K))) { /* two rows where rows are few: 2560 x 4096 INT4 7.6 -> 5.9 us, x 9728 16.0 -> 13.1 */
+        ce = launch_gemv_row<WK, SW>(y, x, w, scales, M, N, K, gshift, early, stream);
     } else {
         ce = launch_gemv_batch<WK, SW>(y, x, w, scales, M, N, K, gshift, early, stream);
     }
