@@ -482,12 +482,7 @@ def run_ours(args, rank, world):
         raise SystemExit("--tp shards the batch-1 tick")
     who = 0 if tp else rank  # tensor-parallel ranks must issue identical calls: same prompt, same seed
     for attempt in range(8):  # a sampled EOS would end a session early: move to the next seed
-        replica = world > 1 and not tp and "S2P_NO_FUSED" not in os.environ
-        if replica:  # a rank's model expects to become tensor parallel; a replica runs the frame a single-GPU process would
-            os.environ["S2P_NO_FUSED"] = "1"
         eng = Engine(lib, capi, ckpt, ctx_len, max(args.batch, 1))
-        if replica:
-            del os.environ["S2P_NO_FUSED"]
         if tp:
             tp_attach(lib, capi, eng, rank, world)
         eng.record = []

@@ -308,9 +308,9 @@ s2p_status s2p_model_load(const char* model_dir, const s2p_model_opts* opts, s2p
     m->fused_b1 = (m->mode == S2P_GEMM_INT8) && !s2p_env_is_one("S2P_NO_FUSED");
     /* One decoding row on one GPU is served by the launches of the general tick: overlapped, in a graph, they take 3.25 / 2.99 / 3.80 ms
      * against the persistent kernel's 3.79 / 4.54 / 5.41 ms (INT4 / INT8 / INT4 after 8000 positions), which pays a grid-wide hand-over for
-     * each of 394 stages.  Tensor-parallel models need the persistent kernel; S2P_NO_MEGA=0 asks for it and S2P_NO_MEGA=1
-     * for the fused stages; S2P_TICK_TRACE=1, and a rank of a multi-process job, whose models may become tensor parallel, keep it. */
-    m->persistent_b1 = getenv("S2P_NO_MEGA") != NULL || s2p_env_is_one("S2P_TICK_TRACE") || (getenv("WORLD_SIZE") && atoi(getenv("WORLD_SIZE")) > 1);
+     * each of 394 stages.  S2P_NO_MEGA=0 asks for the persistent kernel, S2P_NO_MEGA=1 for the fused stages, and S2P_TICK_TRACE=1
+     * needs the former; a model that becomes tensor parallel runs it whatever this says (s2p_model_batch_next_frame). */
+    m->persistent_b1 = getenv("S2P_NO_MEGA") != NULL || s2p_env_is_one("S2P_TICK_TRACE");
 
     s2p_status rc;
     s2p_st* st = NULL;

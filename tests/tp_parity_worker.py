@@ -25,6 +25,7 @@ def main():
     prompt_len = int(sys.argv[4]) if len(sys.argv) > 4 else 64
     os.environ["S2P_INT8"] = "1"
     os.environ["S2P_QCACHE"] = "0"
+    os.environ["S2P_NO_MEGA"] = "0"  # the single-GPU run of the comparison on the persistent kernel too
     if mode == "int4":
         os.environ["S2P_INT4"] = "1"
         os.environ["S2P_INT4_ALL"] = "1"
