@@ -215,6 +215,8 @@ cudaError_t s2pk_rope(s2p_bf16* q, s2p_bf16* k, int rows, int q_heads, int kv_he
                       int pos, float rope_base, cudaStream_t st);
 cudaError_t s2pk_kv_append(const s2p_bf16* k, const s2p_bf16* v, s2p_bf16* k_cache, s2p_bf16* v_cache,
                            int rows, int kv_heads, int head_dim, int pos, int max_seq, cudaStream_t st);
+/* Several rows share a kernel whose waits are bounded.  The launch cannot know that one will give up: the next call on the
+ * device then launches nothing and returns cudaErrorLaunchTimeout, once; the rows of the calls before it are lost. */
 cudaError_t s2pk_attention(const s2p_bf16* q, const s2p_bf16* k_cache, const s2p_bf16* v_cache,
                            s2p_bf16* out, int rows, int q_heads, int kv_heads, int head_dim, int pos,
                            int max_seq, cudaStream_t st);

@@ -300,9 +300,9 @@ cudaError_t mega_launch(const MegaParams* p, int n_cta, cudaStream_t st);
 
 cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st);
 cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st);
-/* status of the prompt slices' attention (a bounded wait that gave up leaves a code), copied to pinned memory; and its reset */
-cudaError_t attn_prefill_status(int* host, cudaStream_t st);
-cudaError_t attn_prefill_reset(cudaStream_t st);
+/* the same, with the word that takes the code of a bounded wait that gave up; attn_single: the device's word for unwatched calls */
+cudaError_t attn_slice(const AttnArgs* a, int rows, int* status, cudaStream_t st);
+cudaError_t attn_prefill_set_wait_ns(unsigned long long ns); /* test hook: deadline of those waits */
 cudaError_t attn_decode(const AttnArgs* a, int rows, cudaStream_t st);
 
 cudaError_t rms_norm(const void* x, const void* w, void* y, int rows, int width, float eps, cudaStream_t st);

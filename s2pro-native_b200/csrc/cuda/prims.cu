@@ -8,6 +8,8 @@
  * namespace s2p serve the unfused decode tick and prefill (ops.h).
  */
 #include <math.h>
+#include <stdio.h>
+#include <string.h>
 #include "common.cuh"
 #include "launch.cuh"
 #include "gemv.cuh"
@@ -497,31 +499,43 @@ __global__ void __launch_bounds__(512) k_attn_single(AttnArgs a) {
     a.out[((size_t)row * QH + h) * 128 + t] = f2bf(__fdiv_rn(acc, l));
 }
 
-/* prompt slices: consecutive rows of one session go to the row-block kernel (attn_prefill.cuh) */
-static __device__ int g_attn_prefill_status; /* code of a bounded wait that gave up (pipe.cuh), 0 otherwise */
+/* ---- prompt slices: consecutive rows of one session go to the row-block kernel (attn_prefill.cuh) ----
+ * `status` takes the code of a bounded wait that gave up (pipe.cuh).  A model gives a word of its own on the device and reads it
+ * where a slice ends.  A call that no model watches has no such point: its word is pinned host memory, one per device,
+ * and the next such call reports the lost one. */
+static int* attn_unwatched_status() {
+    static int* const words = [] {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; /* the first call may be a captured one */
+        int* p = nullptr;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaHostAlloc((void**)&p, 64 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) memset(p, 0, 64 * sizeof(int));
+        else { p = nullptr; (void)cudaGetLastError(); }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return p;
+    }();
+    int dev = 0;
+    return words && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? words + dev : nullptr;
+}
 
 template <bool KV8, int QT, int NW, bool APART>
-static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, cudaStream_t st) {
-    static int* status[64] = {nullptr};
+static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, int* status, cudaStream_t st) {
+    static bool set_up[64] = {false};
     constexpr size_t smem = sizeof(AttnPrefillSmem<KV8, QT, NW, APART>);
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!status[dev]) {
+    if (!set_up[dev]) {
         e = cudaFuncSetAttribute(k_attn_prefill<KV8, QT, NW, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        int* p = nullptr;
-        e = cudaGetSymbolAddress((void**)&p, g_attn_prefill_status);
-        if (e != cudaSuccess) return e;
-        status[dev] = p;
+        set_up[dev] = true;
     }
     uintptr_t all = (uintptr_t)a->q | (uintptr_t)a->out | (uintptr_t)a->kv.base0 | a->kv.k_off | a->kv.v_off;
     if (a->kv8) all |= (uintptr_t)a->kv.sbase0 | a->kv.ks_off | a->kv.vs_off;
     constexpr int RB = QT * NW / 2;
     dim3 grid((unsigned)((rows + RB - 1) / RB), (unsigned)a->kv_heads);
-    return launch_after(k_attn_prefill<KV8, QT, NW, APART>, grid, (APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCERS, smem, st, *a, rows, (int)((all & 15) == 0), status[dev]);
+    return launch_after(k_attn_prefill<KV8, QT, NW, APART>, grid, (APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCERS, smem, st, *a, rows, (int)((all & 15) == 0), status);
 }
 
 /* A CTA fills an SM whatever its size, so a launch takes (waves of CTAs) x (time per 128-position tile).  Large blocks are the
@@ -532,7 +546,7 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, cudaStream_t
  * Measured (us; first kernel of one block size, four sizes of one kind, now): 2048 rows after 6052 positions 12590, 5430, 5396; 77
  * after 1024 154, 93, 73; 50 after 1000 89, 68, 57; 20 after 2000 161, 120, 82. */
 template <bool KV8>
-static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, cudaStream_t st) {
+static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, int* status, cudaStream_t st) {
     static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {19300, 15300, 12600, 9000, 7300, 5800, 4700};
     int best = 0;
     long long best_cost = 0;
@@ -542,34 +556,34 @@ static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, cudaStr
         if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
     switch (best) {
-    case 0: return launch_attn_prefill<KV8, 4, 12, false>(a, rows, st);
-    case 1: return launch_attn_prefill<KV8, 4, 8, false>(a, rows, st);
-    case 2: return launch_attn_prefill<KV8, 4, 6, true>(a, rows, st);
-    case 3: return launch_attn_prefill<KV8, 4, 4, true>(a, rows, st);
-    case 4: return launch_attn_prefill<KV8, 2, 6, true>(a, rows, st);
-    case 5: return launch_attn_prefill<KV8, 2, 4, true>(a, rows, st);
-    default: return launch_attn_prefill<KV8, 2, 2, true>(a, rows, st);
+    case 0: return launch_attn_prefill<KV8, 4, 12, false>(a, rows, status, st);
+    case 1: return launch_attn_prefill<KV8, 4, 8, false>(a, rows, status, st);
+    case 2: return launch_attn_prefill<KV8, 4, 6, true>(a, rows, status, st);
+    case 3: return launch_attn_prefill<KV8, 4, 4, true>(a, rows, status, st);
+    case 4: return launch_attn_prefill<KV8, 2, 6, true>(a, rows, status, st);
+    case 5: return launch_attn_prefill<KV8, 2, 4, true>(a, rows, status, st);
+    default: return launch_attn_prefill<KV8, 2, 2, true>(a, rows, status, st);
     }
 }
 
-/* copies the status word of the slices' attention to `host` (pinned) in stream order */
-cudaError_t attn_prefill_status(int* host, cudaStream_t st) {
-    return cudaMemcpyFromSymbolAsync(host, g_attn_prefill_status, sizeof(int), 0, cudaMemcpyDeviceToHost, st);
-}
-cudaError_t attn_prefill_reset(cudaStream_t st) {
-    static const int zero = 0;
-    return cudaMemcpyToSymbolAsync(g_attn_prefill_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, st);
-}
-
-cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st) {
+cudaError_t attn_slice(const AttnArgs* a, int rows, int* status, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     if (a->q_heads != a->kv_heads * 4 || a->head_dim != 128) return cudaErrorInvalidValue;
     if (rows >= 2 && !a->pos_arr && a->pos_row_step == 1 && !a->kv.bases && a->kv.row_stride == 0 &&
-        (!a->kv8 || (!a->kv.sbases && a->kv.srow_stride == 0)))
-        return a->kv8 ? launch_attn_prefill_rows<true>(a, rows, st) : launch_attn_prefill_rows<false>(a, rows, st);
+        (!a->kv8 || (!a->kv.sbases && a->kv.srow_stride == 0))) {
+        if (!status) return cudaErrorMemoryAllocation;
+        return a->kv8 ? launch_attn_prefill_rows<true>(a, rows, status, st) : launch_attn_prefill_rows<false>(a, rows, status, st);
+    }
     dim3 grid((unsigned)rows, (unsigned)a->kv_heads);
     return launch_after(a->kv8 ? k_attn_single<true> : k_attn_single<false>, grid, 512, 0, st, *a);
 }
+cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st) { return attn_slice(a, rows, attn_unwatched_status(), st); }
+/* 0, or once the code that an earlier unwatched call of this device left */
+static int attn_unwatched_lost() {
+    int* word = attn_unwatched_status();
+    return word && *reinterpret_cast<volatile int*>(word) ? __atomic_exchange_n(word, 0, __ATOMIC_ACQ_REL) : 0;
+}
+cudaError_t attn_prefill_set_wait_ns(unsigned long long ns) { return cudaMemcpyToSymbol(c_pipe_wait_ns, &ns, sizeof(ns)); }
 
 /* ---- SwiGLU (kernels.cu:1216-1229) ---------------------------------------- */
 __global__ void __launch_bounds__(256) k_silu_mul(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h,
@@ -866,6 +880,10 @@ extern "C" cudaError_t s2pk_attention(const s2p_bf16* q, const s2p_bf16* k_cache
                                       int max_seq, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     if (head_dim != 128) return cudaErrorInvalidValue;
+    if (const int code = attn_unwatched_lost()) {
+        fprintf(stderr, "[s2pro] s2pk_attention: an earlier call gave up on a bounded wait (code %d); its rows are lost\n", code);
+        return cudaErrorLaunchTimeout;
+    }
     AttnArgs a = {};
     a.q = (const __nv_bfloat16*)q; a.out = (__nv_bfloat16*)out;
     /* two independent planes: address both from the K plane's base */

@@ -108,8 +108,9 @@ struct s2p_model {
     void *d_up, *h_up;
     size_t out_bytes, off_sem, off_ocodes, off_eos;
     void *d_out, *h_out;
-    int* h_prefill_status;          /* pinned copy of the prompt attention's status word */
-    int* h_tc_status;               /* ... and of the batched tensor-core linears' */
+    int* d_prefill_status;          /* status word of the prompt attention, 0 unless a bounded wait gave up */
+    int* h_prefill_status;          /* ... its pinned copy */
+    int* h_tc_status;               /* pinned copy of the batched tensor-core linears' */
     /* one executable graph per steady batch size */
     cudaGraphExec_t gexec[S2P_MAX_BATCH + 1];
     unsigned char gready[S2P_MAX_BATCH + 1];

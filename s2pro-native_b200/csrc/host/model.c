@@ -187,6 +187,8 @@ static s2p_status alloc_workspace(s2p_model* m) {
     m->out_bytes = align_up(m->off_eos + (size_t)B, 16);
     S2P_CUDA_TRY(cudaMalloc(&m->d_out, m->out_bytes));
     S2P_CUDA_TRY(cudaMallocHost(&m->h_out, m->out_bytes));
+    S2P_CUDA_TRY(cudaMalloc((void**)&m->d_prefill_status, sizeof(int)));
+    S2P_CUDA_TRY(cudaMemsetAsync(m->d_prefill_status, 0, sizeof(int), m->stream));
     S2P_CUDA_TRY(cudaMallocHost((void**)&m->h_prefill_status, 2 * sizeof(int)));
     m->h_tc_status = m->h_prefill_status + 1;
     *m->h_tc_status = 0;
@@ -450,6 +452,7 @@ void s2p_model_free(s2p_model* m) {
     if (m->h_up) cudaFreeHost(m->h_up);
     if (m->d_out) cudaFree(m->d_out);
     if (m->h_out) cudaFreeHost(m->h_out);
+    if (m->d_prefill_status) cudaFree(m->d_prefill_status);
     if (m->h_prefill_status) cudaFreeHost(m->h_prefill_status);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);

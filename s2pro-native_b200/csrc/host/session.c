@@ -229,7 +229,7 @@ static s2p_status layer_attention(s2p_model* m, const s2p_layer* L, const layer_
         aa.n_split_slots = m->n_split_slots; aa.workers = attn_workers_for(rows);
         S2P_LAUNCH(m, attn_decode(&aa, rows, st));
     } else {
-        S2P_LAUNCH(m, attn_single(&aa, rows, st));
+        S2P_LAUNCH(m, attn_slice(&aa, rows, m->d_prefill_status, st));
     }
     return S2P_OK;
 }
@@ -395,11 +395,11 @@ s2p_status s2p_session_prefill(s2p_session* s, const int64_t* ids, const uint8_t
     S2P_LAUNCH(m, rms_norm(BF(m->sx) + (size_t)(n_ids - 1) * S2P_DIM, m->final_norm.data, s->pending_hidden, 1,
                           S2P_DIM, S2P_NORM_EPS, st));
     dump_bf16("backbone_final_norm", s->pending_hidden, S2P_DIM, st);
-    S2P_CUDA_TRY(attn_prefill_status(m->h_prefill_status, st));
+    S2P_CUDA_TRY(cudaMemcpyAsync(m->h_prefill_status, m->d_prefill_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     S2P_CUDA_TRY(cudaStreamSynchronize(st));
     if (*m->h_prefill_status != 0) {
         fprintf(stderr, "[s2pro] prompt attention gave up on a bounded wait (code %d); the slice is lost\n", *m->h_prefill_status);
-        S2P_CUDA_TRY(attn_prefill_reset(st));
+        S2P_CUDA_TRY(cudaMemsetAsync(m->d_prefill_status, 0, sizeof(int), st));
         return S2P_ERR_INTERNAL;
     }
     if (n_ids > S2P_INT8_GEMV_MAX_M && m->mode == S2P_GEMM_INT8 && s2p_env_is_one("S2P_PREFILL_TC")) {

@@ -129,3 +129,92 @@ def test_batched_tensor_core_linear_gives_up_cleanly_and_the_exact_kernel_takes_
     for s in sess:
         tl.s2p_session_destroy(s)
     tl.s2p_model_free(m)
+
+
+def _slice_waits(tl):
+    tl.attn_prefill_set_wait_ns.restype = C.c_int
+    tl.attn_prefill_set_wait_ns.argtypes = [C.c_ulonglong]
+    return tl
+
+
+def test_prompt_attention_of_a_caller_reports_a_wait_that_gave_up(testlib):
+    """s2pk_attention has no synchronisation of its own: with the deadline at 1 ns a call loses rows, the next one says so
+    without launching anything, and the one after that is whole again."""
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    tl = _slice_waits(testlib)
+    rows, pos, max_seq, width = 450, 3000, 3456, 32 * 128
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(rows, width, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(8, max_seq, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+
+    def attend():
+        out = torch.full_like(q, 7.0)
+        rc = tl.s2pk_attention(*[C.c_void_p(t.data_ptr()) for t in (q, k, v, out)], rows, 32, 8, 128, pos, max_seq, None)
+        torch.cuda.synchronize()
+        return rc, out
+
+    rc, want = attend()
+    assert rc == 0
+    try:
+        assert tl.attn_prefill_set_wait_ns(1) == 0
+        rc, _ = attend()
+    finally:
+        assert tl.attn_prefill_set_wait_ns(2_000_000_000) == 0
+    assert rc == 0
+    rc, out = attend()
+    assert rc == 702 and (out == 7).all()  # cudaErrorLaunchTimeout
+    rc, out = attend()
+    assert rc == 0 and torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
+def test_prompt_slice_whose_attention_gives_up_is_refused_and_can_be_repeated(testlib, capi):
+    """A model's slice answers S2P_ERR_INTERNAL and may be sent again; neither the model nor a caller of the primitive sees the
+    other's lost wait."""
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    tl = _slice_waits(_hooks(testlib))
+    synth = importlib.import_module("s2pro-native_b200.synth")
+    os.environ.update({"S2P_INT8": "1", "S2P_INT4": "1", "S2P_INT4_ALL": "1", "S2P_QCACHE": "0"})
+    ckpt = os.environ.get("S2P_TEST_CKPT_DIR", "/dev/shm") + "/s2p_synth_l2"
+    synth.write_checkpoint(ckpt, n_slow=2, seed=0, generator="auto")
+    opts, m = capi.ModelOpts(capi.GEMM_INT8, 2048, 2), C.c_void_p()
+    capi.check(tl.s2p_model_load(ckpt.encode(), C.byref(opts), C.byref(m)), "load")
+    ids = synth.random_prompt(1500, 5)
+    q = torch.zeros(64, 32 * 128, dtype=torch.bfloat16, device="cuda")
+    kv = torch.zeros(8, 64, 128, dtype=torch.bfloat16, device="cuda")
+
+    def primitive():
+        args = [C.c_void_p(t.data_ptr()) for t in (q, kv, kv, q)]
+        return tl.s2pk_attention(*args, 64, 32, 8, 128, 0, 64, None)
+
+    def opened():
+        cfg, s = tl.s2p_sampling_defaults(), C.c_void_p()
+        cfg.temperature = 0.0
+        capi.check(tl.s2p_session_create(m, C.byref(cfg), C.byref(s)), "session")
+        return s
+
+    def prefill(s):
+        return tl.s2p_session_prefill(s, ids.ctypes.data_as(C.c_void_p), None, len(ids), None, 0)
+
+    def frames(s):
+        codes, eos, out = (C.c_int32 * 10)(), C.c_int(0), []
+        for _ in range(3):
+            capi.check(tl.s2p_session_next_frame(s, codes, C.byref(eos)), "frame")
+            out.append(list(codes))
+        return out
+
+    one, two = opened(), opened()
+    assert prefill(one) == 0
+    want = frames(one)
+    try:
+        assert tl.attn_prefill_set_wait_ns(1) == 0
+        rc = prefill(two)
+    finally:
+        assert tl.attn_prefill_set_wait_ns(2_000_000_000) == 0
+    assert rc == S2P_ERR_INTERNAL
+    assert primitive() == 0
+    assert prefill(two) == 0 and frames(two) == want
+    for s in (one, two):
+        tl.s2p_session_destroy(s)
+    tl.s2p_model_free(m)
