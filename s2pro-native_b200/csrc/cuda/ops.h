@@ -16,6 +16,9 @@ typedef __nv_bfloat16 s2p_dev_bf16;
 typedef uint16_t s2p_dev_bf16;
 #endif
 
+/* cudaMalloc for the library's own buffers (host/core.c) */
+cudaError_t s2p_device_malloc(void** out, size_t bytes);
+
 /* Where the KV planes of row r live.  Payload base of row r is
  * (bases ? bases[r] : base0 + r * row_stride); the K plane [kv_heads, max_seq,
  * 128] starts k_off bytes in, the V plane v_off bytes in.  With an INT8 cache

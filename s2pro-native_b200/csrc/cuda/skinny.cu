@@ -563,9 +563,9 @@ extern "C" cudaError_t skinny_setup(int max_rows) {
     if (dev < 0 || dev >= 64 || max_rows < 1) return cudaErrorInvalidValue;
     if (g_partial[dev]) return cudaSuccess;
     const int rows = 256;
-    if ((e = cudaMalloc((void**)&g_partial[dev], (size_t)SK_SCRATCH_FLOATS_PER_ROW * rows * sizeof(float))) != cudaSuccess) return e;
+    if ((e = s2p_device_malloc((void**)&g_partial[dev], (size_t)SK_SCRATCH_FLOATS_PER_ROW * rows * sizeof(float))) != cudaSuccess) return e;
     if (!g_arrivals[dev]) {
-        if ((e = cudaMalloc((void**)&g_arrivals[dev], SK_MAX_SPLIT_TILES * sizeof(unsigned))) != cudaSuccess) return e;
+        if ((e = s2p_device_malloc((void**)&g_arrivals[dev], SK_MAX_SPLIT_TILES * sizeof(unsigned))) != cudaSuccess) return e;
         if ((e = cudaMemset(g_arrivals[dev], 0, SK_MAX_SPLIT_TILES * sizeof(unsigned))) != cudaSuccess) return e;
     }
     g_partial_rows[dev] = rows;
@@ -1143,7 +1143,7 @@ static cudaError_t xt_launch(const LinRef* lin, const void* x, int M, void* y, c
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
         if (g_xt[dev]) cudaFree(g_xt[dev]);
         g_xt[dev] = nullptr; g_xt_bytes[dev] = 0;
-        if ((e = cudaMalloc(&g_xt[dev], need)) != cudaSuccess) return e;
+        if ((e = s2p_device_malloc(&g_xt[dev], need)) != cudaSuccess) return e;
         g_xt_bytes[dev] = need;
     }
     /* split K where tiles x row blocks leave most SMs idle (short prompts, matrices of few rows) */

@@ -7,7 +7,7 @@
  * src/core/tensor.c:60-127).
  */
 #include <string.h>
-#include "s2p_b200_abi.h"
+#include "internal.h"
 
 /* ---- status --------------------------------------------------------------------------- */
 
@@ -64,13 +64,23 @@ static int shape_bytes(s2p_dtype dt, int ndim, const int64_t* shape, size_t* byt
     return 1;
 }
 
+/* Device memory for the library's own buffers.  A refusal does not stay behind as the "last error" that the next launch would return. */
+cudaError_t s2p_device_malloc(void** out, size_t bytes) {
+    const cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaSuccess) return e;
+    (void)cudaGetLastError();
+    *out = NULL;
+    return e;
+}
+
 static s2p_status tensor_alloc(s2p_tensor* t, s2p_dtype dt, int ndim, const int64_t* shape, int on_device) {
     size_t bytes = 0;
     if (!t || !shape_bytes(dt, ndim, shape, &bytes)) return S2P_ERR_INVALID;
     void* mem = NULL;
-    const cudaError_t e = on_device ? cudaMalloc(&mem, bytes) : cudaMallocHost(&mem, bytes);
+    const cudaError_t e = on_device ? s2p_device_malloc(&mem, bytes) : cudaMallocHost(&mem, bytes);
     memset(t, 0, sizeof(*t));
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();
         fprintf(stderr, "[s2pro] %s(%zu) failed: %s\n", on_device ? "cudaMalloc" : "cudaMallocHost", bytes, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? S2P_ERR_OOM : S2P_ERR_CUDA;
     }

@@ -335,7 +335,7 @@ s2p_status s2p_linear_forward(const s2p_linear* lin, const void* x_bf16, void* y
             if (G.deq) cudaFree(G.deq);
             G.deq = NULL;
             G.deq_bytes = 0;
-            if (rc == S2P_OK && cudaMalloc(&G.deq, need) != cudaSuccess) rc = S2P_ERR_OOM;
+            if (rc == S2P_OK && s2p_device_malloc(&G.deq, need) != cudaSuccess) rc = S2P_ERR_OOM;
             if (rc == S2P_OK) G.deq_bytes = need;
         }
         if (rc == S2P_OK) {

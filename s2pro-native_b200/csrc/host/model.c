@@ -147,7 +147,7 @@ static s2p_status alloc_workspace(s2p_model* m) {
     {
         const int64_t n[1] = {B * S2P_SLOW_Q_HEADS * (int64_t)m->n_split_slots * (S2P_HEAD_DIM + 2)};
         S2P_TRY(s2p_tensor_device_alloc(&m->attn_part, S2P_DT_F32, 1, n));
-        S2P_CUDA_TRY(cudaMalloc((void**)&m->attn_ctr, (size_t)B * S2P_SLOW_KV_HEADS * sizeof(unsigned int)));
+        S2P_CUDA_TRY(s2p_device_malloc((void**)&m->attn_ctr, (size_t)B * S2P_SLOW_KV_HEADS * sizeof(unsigned int)));
         S2P_CUDA_TRY(cudaMemset(m->attn_ctr, 0, (size_t)B * S2P_SLOW_KV_HEADS * sizeof(unsigned int)));
     }
     /* fast-AR */
@@ -162,9 +162,9 @@ static s2p_status alloc_workspace(s2p_model* m) {
     S2P_TRY(alloc2(&m->flogits, B, S2P_CB_SIZE, S2P_DT_BF16));
     S2P_TRY(alloc2(&m->fkv, (int64_t)S2P_FAST_LAYERS * B, 2 * FA_KVSZ, S2P_DT_BF16));
     S2P_CUDA_TRY(cudaMemset(m->fkv.data, 0, m->fkv.bytes));
-    S2P_CUDA_TRY(cudaMalloc((void**)&m->fstage, (size_t)9 * B * sizeof(int32_t)));
-    S2P_CUDA_TRY(cudaMalloc((void**)&m->fcodes, (size_t)B * sizeof(int32_t)));
-    S2P_CUDA_TRY(cudaMalloc((void**)&m->fkeys, (size_t)9 * B * sizeof(unsigned long long)));
+    S2P_CUDA_TRY(s2p_device_malloc((void**)&m->fstage, (size_t)9 * B * sizeof(int32_t)));
+    S2P_CUDA_TRY(s2p_device_malloc((void**)&m->fcodes, (size_t)B * sizeof(int32_t)));
+    S2P_CUDA_TRY(s2p_device_malloc((void**)&m->fkeys, (size_t)9 * B * sizeof(unsigned long long)));
     S2P_CUDA_TRY(cudaMemset(m->fkeys, 0, (size_t)9 * B * sizeof(unsigned long long)));
 
     /* per-tick upload block: pointer tables first (natural alignment), then ids, codes, pos, mask */
@@ -177,7 +177,7 @@ static s2p_status alloc_workspace(s2p_model* m) {
     m->off_pos = off;  off += (size_t)B * sizeof(int32_t);
     m->off_mask = off; off += (size_t)B;
     m->up_bytes = align_up(off, 16);
-    S2P_CUDA_TRY(cudaMalloc(&m->d_up, m->up_bytes));
+    S2P_CUDA_TRY(s2p_device_malloc(&m->d_up, m->up_bytes));
     S2P_CUDA_TRY(cudaMallocHost(&m->h_up, m->up_bytes));
     memset(m->h_up, 0, m->up_bytes);
     /* result block: i64 tok[B] | i32 sem[B] | i32 codes[10B] | u8 eos[B] */
@@ -185,9 +185,9 @@ static s2p_status alloc_workspace(s2p_model* m) {
     m->off_ocodes = m->off_sem + (size_t)B * sizeof(int32_t);
     m->off_eos = m->off_ocodes + (size_t)B * S2P_NUM_CODEBOOKS * sizeof(int32_t);
     m->out_bytes = align_up(m->off_eos + (size_t)B, 16);
-    S2P_CUDA_TRY(cudaMalloc(&m->d_out, m->out_bytes));
+    S2P_CUDA_TRY(s2p_device_malloc(&m->d_out, m->out_bytes));
     S2P_CUDA_TRY(cudaMallocHost(&m->h_out, m->out_bytes));
-    S2P_CUDA_TRY(cudaMalloc((void**)&m->d_prefill_status, sizeof(int)));
+    S2P_CUDA_TRY(s2p_device_malloc((void**)&m->d_prefill_status, sizeof(int)));
     S2P_CUDA_TRY(cudaMemsetAsync(m->d_prefill_status, 0, sizeof(int), m->stream));
     S2P_CUDA_TRY(cudaMallocHost((void**)&m->h_prefill_status, 2 * sizeof(int)));
     m->h_tc_status = m->h_prefill_status + 1;
@@ -321,7 +321,7 @@ s2p_status s2p_model_load(const char* model_dir, const s2p_model_opts* opts, s2p
     if (gemv_setup_all() != cudaSuccess) { rc = S2P_ERR_CUDA; goto fail; }
     if (m->max_sessions > 1 && skinny_setup(m->max_sessions) != cudaSuccess) { rc = S2P_ERR_OOM; goto fail; }
     if (m->fused_b1 && !s2p_env_is_one("S2P_NO_MEGA")) {
-        if (mega_setup(&m->mega_ctas) == cudaSuccess && cudaMalloc(&m->tp_arena, S2P_TP_ARENA_BYTES) == cudaSuccess &&
+        if (mega_setup(&m->mega_ctas) == cudaSuccess && s2p_device_malloc(&m->tp_arena, S2P_TP_ARENA_BYTES) == cudaSuccess &&
             cudaMemset(m->tp_arena, 0, S2P_TP_ARENA_BYTES) == cudaSuccess) {
             m->mega_ok = 1;
             m->tp_base[0] = m->tp_arena;

@@ -87,7 +87,7 @@ static size_t session_block(const s2p_model* m, size_t* scales, size_t* hidden, 
 
 static s2p_status block_take(s2p_model* m, size_t bytes, void** out) {
     if (m->n_pool > 0) { *out = m->pool[--m->n_pool]; return S2P_OK; }
-    const cudaError_t e = cudaMalloc(out, bytes);
+    const cudaError_t e = s2p_device_malloc(out, bytes);
     if (e == cudaSuccess) return S2P_OK;
     fprintf(stderr, "[s2pro] cudaMalloc(%zu) for a session failed: %s\n", bytes, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? S2P_ERR_OOM : S2P_ERR_CUDA;
@@ -993,13 +993,13 @@ static s2p_status mega_build(s2p_model* m) {
                         "using per-stage launches\n");
         return S2P_OK;
     }
-    cudaError_t e = cudaMalloc((void**)&m->d_mega_stages, (size_t)n * sizeof(MegaStage));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_mega_sync, 2 * sizeof(unsigned int));
+    cudaError_t e = s2p_device_malloc((void**)&m->d_mega_stages, (size_t)n * sizeof(MegaStage));
+    if (e == cudaSuccess) e = s2p_device_malloc((void**)&m->d_mega_sync, 2 * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&m->h_mega_status, sizeof(int));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m->d_mega_stages, prog, (size_t)n * sizeof(MegaStage), cudaMemcpyHostToDevice, m->stream);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_mega_cmds, (n_cmds ? n_cmds : 1) * sizeof(MegaCopyCmd));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_mega_cmd_start, ((size_t)n_cta + 1) * sizeof(int));
+    if (e == cudaSuccess) e = s2p_device_malloc((void**)&m->d_mega_cmds, (n_cmds ? n_cmds : 1) * sizeof(MegaCopyCmd));
+    if (e == cudaSuccess) e = s2p_device_malloc((void**)&m->d_mega_cmd_start, ((size_t)n_cta + 1) * sizeof(int));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m->d_mega_cmds, cmds, n_cmds * sizeof(MegaCopyCmd), cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess)
@@ -1007,7 +1007,7 @@ static s2p_status mega_build(s2p_model* m) {
                             m->stream);
     if (e == cudaSuccess && s2p_env_is_one("S2P_TICK_TRACE")) {
         const size_t tb = (size_t)n * (16 + 2 * (size_t)n_cta) * sizeof(unsigned long long);
-        e = cudaMalloc((void**)&m->d_mega_trace, tb);
+        e = s2p_device_malloc((void**)&m->d_mega_trace, tb);
         if (e == cudaSuccess) e = cudaMemsetAsync(m->d_mega_trace, 0, tb, m->stream);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);

@@ -1,0 +1,82 @@
+/* The library's handling of device memory against a driver that has little of it: session.c and core.c as they are, linked
+ * with the few runtime calls below instead of the CUDA runtime.  Prints nothing and returns 0, or the line that failed. */
+#include <stdlib.h>
+#include <string.h>
+#include "internal.h"
+
+static size_t total, used;
+static cudaError_t last;
+static struct { void* p; size_t bytes; } block[256];
+
+cudaError_t cudaMalloc(void** p, size_t bytes) {
+    if (used + bytes > total) return last = cudaErrorMemoryAllocation;
+    for (int i = 0; i < 256; i++)
+        if (!block[i].p) {
+            used += block[i].bytes = bytes;
+            *p = block[i].p = malloc(1);
+            return cudaSuccess;
+        }
+    abort();
+}
+cudaError_t cudaFree(void* p) {
+    for (int i = 0; p && i < 256; i++)
+        if (block[i].p == p) {
+            used -= block[i].bytes;
+            free(p);
+            block[i].p = NULL;
+            return cudaSuccess;
+        }
+    abort();
+}
+cudaError_t cudaGetLastError(void) { const cudaError_t e = last; last = cudaSuccess; return e; }
+const char* cudaGetErrorString(cudaError_t e) { (void)e; return "no memory"; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind k, cudaStream_t st) { (void)d; (void)s; (void)n; (void)k; (void)st; return cudaSuccess; }
+
+size_t s2p_kv_vec_bytes(const s2p_model* m) { return m->kv8 ? S2P_HEAD_DIM : S2P_HEAD_DIM * 2; }
+size_t s2p_kv_plane_bytes(const s2p_model* m) { return (size_t)m->ctx_len * s2p_kv_vec_bytes(m); }
+size_t s2p_kvs_plane_bytes(const s2p_model* m) { return m->kv8 ? (size_t)m->ctx_len * 8 : 0; }
+void s2p_sampler_init(s2p_sampler* sp, const s2p_sampling_cfg* cfg, uint64_t entropy) { (void)cfg; (void)entropy; memset(sp, 0, sizeof(*sp)); }
+
+static s2p_model* model(void) {
+    s2p_model* m = calloc(1, sizeof(*m));
+    m->n_slow = 2; m->ctx_len = 1024; m->kv8 = 1; m->max_sessions = 64;
+    return m;
+}
+static size_t session_bytes(void) { /* of one session of such a model */
+    s2p_model* m = model();
+    s2p_session* s;
+    total = (size_t)1 << 40;
+    if (s2p_session_create(m, NULL, &s) != S2P_OK) abort();
+    const size_t n = used;
+    s2p_session_destroy(s);
+    s2p_session_pool_clear(m);
+    free(m);
+    return n;
+}
+#define CHECK(x) do { if (!(x)) return __LINE__; } while (0)
+
+int main(void) {
+    const size_t one = session_bytes();
+    CHECK(used == 0);
+    s2p_model* a = model();
+    s2p_session* s[8];
+    s2p_tensor t;
+
+    /* a refused session leaves no error behind that a healthy session's next launch would return */
+    total = 2 * one;
+    CHECK(s2p_session_create(a, NULL, &s[0]) == S2P_OK && s2p_session_create(a, NULL, &s[1]) == S2P_OK);
+    CHECK(s2p_session_create(a, NULL, &s[2]) == S2P_ERR_OOM && a->n_sessions == 2);
+    CHECK(cudaGetLastError() == cudaSuccess);
+    const int64_t too_many[1] = {(int64_t)one};
+    CHECK(s2p_tensor_device_alloc(&t, S2P_DT_U8, 1, too_many) == S2P_ERR_OOM && !t.data);
+    CHECK(cudaGetLastError() == cudaSuccess);
+
+    s2p_session_destroy(s[0]);
+    s2p_session_destroy(s[1]);
+    s2p_session_pool_clear(a);
+    CHECK(used == 0);
+    free(a);
+    return 0;
+}
