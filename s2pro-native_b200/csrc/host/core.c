@@ -64,12 +64,14 @@ static int shape_bytes(s2p_dtype dt, int ndim, const int64_t* shape, size_t* byt
     return 1;
 }
 
-/* Device memory for the library's own buffers.  A refusal does not stay behind as the "last error" that the next launch would return. */
+/* Device memory for the library's own buffers.  Where the driver has none left, the blocks that models keep for their next
+ * sessions go back to it first.  A refusal does not stay behind as the "last error" that the next launch would return. */
 cudaError_t s2p_device_malloc(void** out, size_t bytes) {
-    const cudaError_t e = cudaMalloc(out, bytes);
+    cudaError_t e = cudaMalloc(out, bytes);
     if (e == cudaSuccess) return e;
+    if (e == cudaErrorMemoryAllocation && s2p_session_pools_release()) e = cudaMalloc(out, bytes);
     (void)cudaGetLastError();
-    *out = NULL;
+    if (e != cudaSuccess) *out = NULL;
     return e;
 }
 

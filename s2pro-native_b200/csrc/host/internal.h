@@ -77,7 +77,9 @@ struct s2p_model {
     cudaStream_t stream;
     /* device blocks of closed sessions, for the next ones (session.c) */
     void* pool[S2P_POOL_MAX];
-    int n_pool;
+    int n_pool, pool_listed;
+    s2p_model* pool_next; /* the next model that may keep blocks */
+    int device;
 
     /* weights */
     s2p_tensor embed, embed_i8, embed_scale;
@@ -138,6 +140,7 @@ struct s2p_session {
 };
 
 void s2p_session_pool_clear(s2p_model* m);
+int s2p_session_pools_release(void); /* all models' pools on the current device; returns the number of blocks freed */
 
 /* model.c helpers used by session.c */
 size_t s2p_kv_vec_bytes(const s2p_model* m);

@@ -307,6 +307,7 @@ s2p_status s2p_model_load(const char* model_dir, const s2p_model_opts* opts, s2p
         if (m->kv8) fprintf(stderr, "[s2pro] S2P_KV8: INT8 KV cache (g32 per head vector, f16 scales)\n");
     }
     m->tp_world = 1;
+    (void)cudaGetDevice(&m->device);
     m->fused_b1 = (m->mode == S2P_GEMM_INT8) && !s2p_env_is_one("S2P_NO_FUSED");
     /* One decoding row on one GPU is served by the launches of the general tick: overlapped, in a graph, they take 3.25 / 2.99 / 3.80 ms
      * against the persistent kernel's 3.79 / 4.54 / 5.41 ms (INT4 / INT8 / INT4 after 8000 positions), which pays a grid-wide hand-over for

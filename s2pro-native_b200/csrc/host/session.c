@@ -12,6 +12,7 @@
  * Either is captured once per batch size into a CUDA graph and replayed; all
  * per-frame variation travels through the pinned upload block.
  */
+#include <pthread.h>
 #include <stdlib.h>
 #include <string.h>
 #include <time.h>
@@ -67,11 +68,33 @@ static void dump_bf16(const char* name, const void* dev, int64_t n, cudaStream_t
  * sessions are kept for the next ones, because the driver's calls cost more than a short prompt: cudaMalloc + cudaFree of
  * the four former buffers took 1.5 ms per request at a 2048-token context and 90 ms (mostly the unmapping in cudaFree) at
  * 9216 tokens.  The pool belongs to the model and holds at most S2P_POOL_BYTES (or one block, if a block is larger): enough
- * for the turnover of a server, 1/64 of the GPU.  It is given back when the model is freed. */
+ * for the turnover of a server, 1/64 of the GPU.  It is given back when the model is freed, and when this library finds no memory
+ * for anything else on the GPU, for this model or another (s2p_device_malloc); so the pools of all models are under one lock. */
 #define S2P_POOL_BYTES ((size_t)2816 << 20)
+static pthread_mutex_t pool_mu = PTHREAD_MUTEX_INITIALIZER;
+static s2p_model* pool_models; /* those that have kept a block */
 
-void s2p_session_pool_clear(s2p_model* m) {
+static int pool_free(s2p_model* m) {
+    const int n = m->n_pool;
     while (m->n_pool > 0) cudaFree(m->pool[--m->n_pool]);
+    return n;
+}
+void s2p_session_pool_clear(s2p_model* m) {
+    pthread_mutex_lock(&pool_mu);
+    pool_free(m);
+    for (s2p_model** p = &pool_models; *p; p = &(*p)->pool_next)
+        if (*p == m) { *p = m->pool_next; break; }
+    m->pool_listed = 0;
+    pthread_mutex_unlock(&pool_mu);
+}
+int s2p_session_pools_release(void) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    pthread_mutex_lock(&pool_mu);
+    for (s2p_model* m = pool_models; m; m = m->pool_next)
+        if (m->device == dev) n += pool_free(m);
+    pthread_mutex_unlock(&pool_mu);
+    return n;
 }
 
 static size_t block_align(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -86,7 +109,10 @@ static size_t session_block(const s2p_model* m, size_t* scales, size_t* hidden, 
 }
 
 static s2p_status block_take(s2p_model* m, size_t bytes, void** out) {
-    if (m->n_pool > 0) { *out = m->pool[--m->n_pool]; return S2P_OK; }
+    pthread_mutex_lock(&pool_mu);
+    *out = m->n_pool > 0 ? m->pool[--m->n_pool] : NULL;
+    pthread_mutex_unlock(&pool_mu);
+    if (*out) return S2P_OK;
     const cudaError_t e = s2p_device_malloc(out, bytes);
     if (e == cudaSuccess) return S2P_OK;
     fprintf(stderr, "[s2pro] cudaMalloc(%zu) for a session failed: %s\n", bytes, cudaGetErrorString(e));
@@ -94,8 +120,16 @@ static s2p_status block_take(s2p_model* m, size_t bytes, void** out) {
 }
 
 static void block_give(s2p_model* m, void* block, size_t bytes) {
-    if (m->n_pool < S2P_POOL_MAX && (m->n_pool == 0 || (size_t)(m->n_pool + 1) * bytes <= S2P_POOL_BYTES)) m->pool[m->n_pool++] = block;
-    else cudaFree(block);
+    pthread_mutex_lock(&pool_mu);
+    const int keep = m->n_pool < S2P_POOL_MAX && (m->n_pool == 0 || (size_t)(m->n_pool + 1) * bytes <= S2P_POOL_BYTES);
+    if (keep) m->pool[m->n_pool++] = block;
+    if (keep && !m->pool_listed) {
+        m->pool_listed = 1;
+        m->pool_next = pool_models;
+        pool_models = m;
+    }
+    pthread_mutex_unlock(&pool_mu);
+    if (!keep) cudaFree(block);
 }
 
 s2p_status s2p_session_create(s2p_model* m, const s2p_sampling_cfg* cfg, s2p_session** out) {

@@ -39,13 +39,13 @@ size_t s2p_kv_plane_bytes(const s2p_model* m) { return (size_t)m->ctx_len * s2p_
 size_t s2p_kvs_plane_bytes(const s2p_model* m) { return m->kv8 ? (size_t)m->ctx_len * 8 : 0; }
 void s2p_sampler_init(s2p_sampler* sp, const s2p_sampling_cfg* cfg, uint64_t entropy) { (void)cfg; (void)entropy; memset(sp, 0, sizeof(*sp)); }
 
-static s2p_model* model(void) {
+static s2p_model* model(int device) {
     s2p_model* m = calloc(1, sizeof(*m));
-    m->n_slow = 2; m->ctx_len = 1024; m->kv8 = 1; m->max_sessions = 64;
+    m->n_slow = 2; m->ctx_len = 1024; m->kv8 = 1; m->max_sessions = 64; m->device = device;
     return m;
 }
 static size_t session_bytes(void) { /* of one session of such a model */
-    s2p_model* m = model();
+    s2p_model* m = model(0);
     s2p_session* s;
     total = (size_t)1 << 40;
     if (s2p_session_create(m, NULL, &s) != S2P_OK) abort();
@@ -60,7 +60,7 @@ static size_t session_bytes(void) { /* of one session of such a model */
 int main(void) {
     const size_t one = session_bytes();
     CHECK(used == 0);
-    s2p_model* a = model();
+    s2p_model *a = model(0), *b = model(0), *elsewhere = model(1);
     s2p_session* s[8];
     s2p_tensor t;
 
@@ -73,10 +73,38 @@ int main(void) {
     CHECK(s2p_tensor_device_alloc(&t, S2P_DT_U8, 1, too_many) == S2P_ERR_OOM && !t.data);
     CHECK(cudaGetLastError() == cudaSuccess);
 
+    /* closed sessions' blocks wait for the next session ... */
     s2p_session_destroy(s[0]);
     s2p_session_destroy(s[1]);
+    CHECK(used == 2 * one && a->n_pool == 2);
+    CHECK(s2p_session_create(a, NULL, &s[0]) == S2P_OK && used == 2 * one && a->n_pool == 1);
+    /* ... unless another buffer, or another model's session, needs the memory; a session's own block stays */
+    CHECK(s2p_tensor_device_alloc(&t, S2P_DT_U8, 1, too_many) == S2P_OK && a->n_pool == 0 && used == 2 * one);
+    CHECK(cudaGetLastError() == cudaSuccess);
+    s2p_tensor_free(&t);
+    CHECK(s2p_session_create(a, NULL, &s[1]) == S2P_OK);
+    s2p_session_destroy(s[1]);
+    CHECK(s2p_session_create(b, NULL, &s[1]) == S2P_OK && a->n_pool == 0 && used == 2 * one);
+
+    /* a pool on another GPU would not help */
+    total = 3 * one;
+    CHECK(s2p_session_create(elsewhere, NULL, &s[2]) == S2P_OK);
+    s2p_session_destroy(s[2]);
+    CHECK(s2p_session_create(b, NULL, &s[2]) == S2P_ERR_OOM && elsewhere->n_pool == 1);
+
+    /* freed models leave the list */
+    s2p_session_pool_clear(elsewhere);
+    free(elsewhere);
+    s2p_session_destroy(s[0]);
     s2p_session_pool_clear(a);
-    CHECK(used == 0);
     free(a);
+    CHECK(used == one);
+    total = 2 * one;
+    CHECK(s2p_session_create(b, NULL, &s[0]) == S2P_OK && s2p_session_create(b, NULL, &s[2]) == S2P_ERR_OOM);
+    s2p_session_destroy(s[0]);
+    s2p_session_destroy(s[1]);
+    s2p_session_pool_clear(b);
+    CHECK(used == 0);
+    free(b);
     return 0;
 }

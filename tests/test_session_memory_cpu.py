@@ -17,5 +17,5 @@ def run(tmp_path, name, sources):
     assert out.returncode == 0, f"{name}.c:{out.returncode} failed\n{out.stderr}"
 
 
-def test_refused_sessions(tmp_path):
+def test_sessions_and_pools(tmp_path):
     run(tmp_path, "session_memory", ["session.c", "core.c"])
