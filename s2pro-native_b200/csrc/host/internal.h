@@ -139,6 +139,7 @@ struct s2p_session {
     s2p_sampler sampler;
 };
 
+int s2p_model_give_back(s2p_model* m);
 void s2p_session_pool_clear(s2p_model* m);
 int s2p_session_pools_release(void); /* all models' pools on the current device; returns the number of blocks freed */
 

@@ -31,6 +31,8 @@ cudaError_t cudaFree(void* p) {
 cudaError_t cudaGetLastError(void) { const cudaError_t e = last; last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t e) { (void)e; return "no memory"; }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+static int graphs;
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t g) { (void)g; graphs--; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind k, cudaStream_t st) { (void)d; (void)s; (void)n; (void)k; (void)st; return cudaSuccess; }
 
@@ -103,6 +105,22 @@ int main(void) {
     CHECK(s2p_session_create(b, NULL, &s[0]) == S2P_OK && s2p_session_create(b, NULL, &s[2]) == S2P_ERR_OOM);
     s2p_session_destroy(s[0]);
     s2p_session_destroy(s[1]);
+    s2p_session_pool_clear(b);
+
+    /* resident copies of the weights give way to sessions: the bf16 ones, then the tiles and the graphs that read them */
+    total = 4 * one;
+    CHECK(cudaMalloc(&b->wide_weights, one) == cudaSuccess && cudaMalloc(&b->tc_weights, one / 2) == cudaSuccess && cudaMalloc(&b->xt_norm, one / 2) == cudaSuccess);
+    b->slow[1].wide[2] = b->wide_weights;
+    b->slow[1].tc[2] = b->fast[3].tc[0] = b->tc_fast_out = b->tc_weights;
+    b->xt_attn = b->xt_ffn = b->xt_norm;
+    b->gready[1] = b->gready[32] = 1;
+    graphs = 2;
+    CHECK(s2p_session_create(b, NULL, &s[0]) == S2P_OK && s2p_session_create(b, NULL, &s[1]) == S2P_OK && b->wide_weights);
+    CHECK(s2p_session_create(b, NULL, &s[2]) == S2P_OK && !b->wide_weights && !b->slow[1].wide[2] && b->tc_weights && graphs == 2);
+    CHECK(s2p_session_create(b, NULL, &s[3]) == S2P_OK && !b->tc_weights && !b->xt_norm && !b->xt_ffn && !b->xt_attn && !b->tc_fast_out);
+    CHECK(!b->slow[1].tc[2] && !b->fast[3].tc[0] && graphs == 0 && !b->gready[1] && !b->gready[32]);
+    CHECK(s2p_session_create(b, NULL, &s[4]) == S2P_ERR_OOM && cudaGetLastError() == cudaSuccess);
+    for (int i = 0; i < 4; i++) s2p_session_destroy(s[i]);
     s2p_session_pool_clear(b);
     CHECK(used == 0);
     free(b);
