@@ -259,8 +259,7 @@ __device__ __noinline__ bool gemv_stage_input(const MegaStage* sp) {
 }
 
 /* The streaming group's part of a GEMV stage after its input is staged; `q0`: chunks this CTA consumed before the stage.
- * Returns the stage's chunk count times two, plus one if no bounded wait gave up (uniform over
- * the group up to the end of the staging, per warp after it). */
+ * Returns the stage's chunk count times two, plus one if no bounded wait gave up (uniform over the warp). */
 template <int WK>
 __device__ __noinline__ int gemv_stream(const MegaStage* sp, unsigned q0, unsigned long long* trace) {
     typedef typename LaneTile<WK>::type tile_t;
@@ -289,9 +288,9 @@ __device__ __noinline__ int gemv_stream(const MegaStage* sp, unsigned q0, unsign
         const unsigned char* wsl = ring_slot(slot);
         float* part = part0 + b * part_floats;
         const long long c0 = trace ? clock64() : 0;
-        if (!mbar_wait_bounded(ring_full(slot), (q / MEGA_SLOTS) & 1u, status)) return 0;
+        if (!mbar_wait_warp(ring_full(slot), (q / MEGA_SLOTS) & 1u, status)) return 0;
         /* the buffer's previous chunk (q - MEGA_PARTS) must be folded */
-        if (q >= MEGA_PARTS && !mbar_wait_bounded(ring_pdone(b), ((q / MEGA_PARTS) - 1u) & 1u, status)) return 0;
+        if (q >= MEGA_PARTS && !mbar_wait_warp(ring_pdone(b), ((q / MEGA_PARTS) - 1u) & 1u, status)) return 0;
         const long long c1 = trace ? clock64() : 0;
         /* tile-major units; this warp's contiguous range, walked one tile segment at a time:
          * the activations of the tile stay in registers while up to four rows, whose chains
@@ -487,7 +486,7 @@ __device__ __noinline__ int gemv_fold(const MegaStage* gs, unsigned q0, unsigned
             }
         }
         const long long c0 = trace ? clock64() : 0;
-        if (!mbar_wait_bounded(ring_pfull(b), (q / MEGA_PARTS) & 1u, status)) return 0;
+        if (!mbar_wait_warp(ring_pfull(b), (q / MEGA_PARTS) & 1u, status)) return 0;
         const long long c1 = trace ? clock64() : 0;
         if (nch > 0) {
             float acc[MEGA_FOLD_CHAINS];
@@ -538,7 +537,7 @@ __device__ __noinline__ int gemv_fold(const MegaStage* gs, unsigned q0, unsigned
         for (int i = 0; i < g_tp.n; i++)
             atomicMax_system(reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(d.key) + g_tp.delta[i]), best);
     }
-    return 2 * ge.n_chunks + (ok ? 1 : 0);
+    return 2 * ge.n_chunks + (__all_sync(S2P_FULL_MASK, ok) ? 1 : 0); /* the issuer's verdict is its warp's */
 }
 
 /* ---- fast-AR attention stage: head RoPE, cache append and single-tile causal
@@ -715,8 +714,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
     unsigned char* const smem = g_smem;
     unsigned char* work = smem + (size_t)MEGA_SLOTS * P.lay.slot_bytes;
     unsigned char* tail = work + P.lay.x_bytes + MEGA_PARTS * P.lay.part_bytes + MEGA_RED_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
-    static_assert(MEGA_SLOTS + 2 * MEGA_PARTS + 1 <= 16, "the barrier words precede the staged command");
+    static_assert(MEGA_SLOTS + 2 * MEGA_PARTS <= 16, "the barrier words precede the staged command");
     /* cta / n_cta: position in the grid of all ranks (they equal blockIdx.x / gridDim.x on one GPU) */
     const int n_local = gridDim.x, tid = threadIdx.x;
     const int cta = P.tp_rank * n_local + blockIdx.x, n_cta = P.tp_world * n_local;
@@ -735,7 +733,6 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
             }
         g_tp.n = n;
     }
-    uint64_t* join = bars + MEGA_SLOTS + 2 * MEGA_PARTS; /* where the two groups meet before a stage that needs the whole CTA */
     if (tid == MEGA_ISSUER) {
         g_ring.status = P.status;
         g_ring.seq_base = P.seq_base;
@@ -750,7 +747,6 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
             mbar_init(ring_pfull(i), MEGA_STREAM_WARPS);
             mbar_init(ring_pdone(i), MEGA_FOLD_WARPS);
         }
-        mbar_init(join, GEMV_WARPS);
         mbar_init_fence();
         ring_load_next();
         ring_issue_upto(MEGA_SLOTS);
@@ -759,7 +755,6 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
     unsigned char* kinds = tail + 256 + 2 * sizeof(MegaStage);
 #define MEGA_KINDS() (g_smem + g_ring.tail_off + 256 + 2 * sizeof(MegaStage))
 #define MEGA_STBUF() reinterpret_cast<MegaStage*>(g_smem + g_ring.tail_off + 256)
-#define MEGA_JOIN() (reinterpret_cast<uint64_t*>(g_smem + g_ring.tail_off) + MEGA_SLOTS + 2 * MEGA_PARTS)
 #define MEGA_TR() ((P.trace && blockIdx.x == 0) ? P.trace + (size_t)si * 16 : nullptr)
     for (int i = tid; i < P.n_stages; i += MEGA_THREADS)
         kinds[i] = (unsigned char)(__ldg(&P.stages[i].type) | (__ldg(&P.stages[i].flags) << 4));
@@ -778,12 +773,12 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads(); /* barriers initialised, first descriptor and the kinds table in place */
 
-    /* `ok` turns false when a bounded wait of this thread gave up (the status word is set then, and
-     * every other wait gives up soon after).  A thread that sees it leaves the stage loop; nobody
-     * may be left behind at a barrier, so the verdict is made uniform where a barrier follows: over
-     * the streaming group at its barrier on entering a GEMV stage, over the CTA at the join
-     * (an mbarrier with a bounded wait). */
-    unsigned n_bar = 0, n_join = 0, consumed = 0; /* consumed: chunks of the ring this CTA is through (every thread counts) */
+    /* `ok` turns false when a bounded wait of this warp gave up (the status word is set then, and every other wait gives up
+     * soon after).  Nobody may be left behind at a barrier, and the hardware's barriers know no limit: so a warp whose wait gave
+     * up does no more work but goes on through the stages, taking part in the streaming group's barriers, up to the next join.
+     * There the CTA comes to one verdict and stays or leaves as a whole.  Between two joins every wait is bounded, so all of
+     * its warps do get there. */
+    unsigned n_bar = 0, consumed = 0; /* consumed: chunks of the ring this CTA is through (every thread counts) */
     bool ok = true;
     for (int si = 0; si < P.n_stages; si++) {
         const int stage_type = MEGA_KINDS()[si] & 15, no_barrier = (MEGA_KINDS()[si] >> 4) & MEGA_NO_BARRIER;
@@ -793,33 +788,34 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
                 /* the descriptor was staged while the previous stage ran; the group barrier inside
                  * gemv_stream (or the join below) publishes it to the group */
                 asm volatile("cp.async.wait_all;" ::: "memory");
-                if (!stream_sync_and(ok)) { ok = false; break; }
-                const MegaStage& s = MEGA_STBUF()[si & 1];
-                stage_prefetch(si + 1); /* the other buffer held stage si - 1, which the group has left */
-                if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[0] = clock64();
-                /* (the group barrier above: every streaming warp has left the previous stage's activation) */
-                int rc = 0;
-                bool staged;
-                switch (s.lin.kind) {
-                case WK_INT8_CH: staged = gemv_stage_input<WK_INT8_CH>(&s); break;
-                case WK_INT8_GRP: staged = gemv_stage_input<WK_INT8_GRP>(&s); break;
-                default: staged = gemv_stage_input<WK_INT4_PACK>(&s); break;
+                ok = stream_sync_and(ok);
+                if (ok) {
+                    const MegaStage& s = MEGA_STBUF()[si & 1];
+                    stage_prefetch(si + 1); /* the other buffer held stage si - 1, which the group has left */
+                    if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[0] = clock64();
+                    /* (the group barrier above: every streaming warp has left the previous stage's activation) */
+                    int rc = 0;
+                    bool staged;
+                    switch (s.lin.kind) {
+                    case WK_INT8_CH: staged = gemv_stage_input<WK_INT8_CH>(&s); break;
+                    case WK_INT8_GRP: staged = gemv_stage_input<WK_INT8_GRP>(&s); break;
+                    default: staged = gemv_stage_input<WK_INT4_PACK>(&s); break;
+                    }
+                    if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[1] = clock64();
+                    if (P.trace && threadIdx.x == 0) { /* every CTA: when its input was staged, on the GPU-wide timer */
+                        unsigned long long gt;
+                        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
+                        P.trace[(size_t)P.n_stages * (16 + (int)gridDim.x) + (size_t)si * (int)gridDim.x + blockIdx.x] = gt;
+                    }
+                    if (staged) switch (s.lin.kind) {
+                    case WK_INT8_CH: rc = gemv_stream<WK_INT8_CH>(&s, consumed, MEGA_TR()); break;
+                    case WK_INT8_GRP: rc = gemv_stream<WK_INT8_GRP>(&s, consumed, MEGA_TR()); break;
+                    default: rc = gemv_stream<WK_INT4_PACK>(&s, consumed, MEGA_TR()); break;
+                    }
+                    ok = rc & 1; consumed += (unsigned)(rc >> 1);
+                    if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[2] = clock64();
                 }
-                if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[1] = clock64();
-                if (P.trace && threadIdx.x == 0) { /* every CTA: when its input was staged, on the GPU-wide timer */
-                    unsigned long long gt;
-                    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
-                    P.trace[(size_t)P.n_stages * (16 + (int)gridDim.x) + (size_t)si * (int)gridDim.x + blockIdx.x] = gt;
-                }
-                if (staged) switch (s.lin.kind) {
-                case WK_INT8_CH: rc = gemv_stream<WK_INT8_CH>(&s, consumed, MEGA_TR()); break;
-                case WK_INT8_GRP: rc = gemv_stream<WK_INT8_GRP>(&s, consumed, MEGA_TR()); break;
-                default: rc = gemv_stream<WK_INT4_PACK>(&s, consumed, MEGA_TR()); break;
-                }
-                ok = rc & 1; consumed += (unsigned)(rc >> 1);
-                if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[2] = clock64();
-            } else {
-                if (!ok) break; /* the folding warps share no barrier: each leaves on its own */
+            } else if (ok) { /* the folding warps share no barrier */
                 const MegaStage* gs = P.stages + si;
                 int rc;
                 switch (__ldg(&gs->lin.kind)) {
@@ -837,17 +833,13 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
             }
             if (no_barrier) continue; /* the groups go on separately; the next stage's waits order them */
         }
-        /* A stage of the whole CTA (or a grid barrier) follows: the groups meet.  One arrival per
-         * warp; the wait is bounded like every other, so a group that gave up cannot strand the other. */
-        if (!ok) break; /* without arriving: the others' wait at the join runs out */
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive(MEGA_JOIN());
-        if (!mbar_wait_bounded(MEGA_JOIN(), n_join & 1u, P.status)) { ok = false; break; }
-        n_join++;
-        /* all sixteen warps arrived, so all of them are fine and take the CTA barriers below */
+        /* A stage of the whole CTA (or a grid barrier) follows: the groups meet, and agree on whether to go on.  (A join on an
+         * mbarrier whose wait may give up does not do: a warp that arrives and then gives up leaves, the others take its arrival
+         * for consent, and the next barrier of the streaming group waits for it for good.) */
+        if (threadIdx.x < MEGA_GROUP_THREADS) asm volatile("cp.async.wait_all;" ::: "memory");
+        ok = cta_sync_and(ok);
+        if (!ok) break;
         if (stage_type != MEGA_GEMV) {
-            if (threadIdx.x < MEGA_GROUP_THREADS) asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncthreads();
             if (MEGA_TR() && threadIdx.x == 0) MEGA_TR()[0] = clock64();
             if (stage_type == MEGA_ATTN_SLOW) cta_stage_attn_slow(MEGA_STBUF() + (si & 1), my_tag);
             else cta_stage_other(MEGA_STBUF() + (si & 1), stage_type, my_tag);
@@ -872,7 +864,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
     /* A wait gave up: the copies this CTA already started still land in its shared memory,
      * so it stays until they have (bounded), then leaves. */
     if (!ok && threadIdx.x == MEGA_ISSUER) {
-        for (unsigned q = consumed; q < g_ring.issued; q++) {
+        /* at most the last MEGA_SLOTS of them (a stage that gave up half way has not counted its chunks as consumed) */
+        for (unsigned q = max(consumed, g_ring.issued > MEGA_SLOTS ? g_ring.issued - MEGA_SLOTS : 0u); q < g_ring.issued; q++) {
             uint64_t* bar = ring_full(q % MEGA_SLOTS);
             const unsigned parity = (q / MEGA_SLOTS) & 1u;
             PipeDeadline dl; /* these copies do land (nothing but memory is waited for): a fixed, generous limit, whatever
@@ -885,7 +878,6 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_tick_mega(MegaParams P) {
 
 #undef MEGA_KINDS
 #undef MEGA_STBUF
-#undef MEGA_JOIN
 #undef MEGA_TR
 
 extern "C" void mega_layout(int x_bytes, MegaLayout* out) {

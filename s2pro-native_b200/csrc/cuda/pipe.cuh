@@ -89,6 +89,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
     return false;
 }
 
+/* The same by all lanes of a converged warp, with one verdict: what follows may synchronise the warp, and a lane that gave
+ * up alone would not come. */
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, unsigned parity, int* status) {
+    return __all_sync(S2P_FULL_MASK, mbar_wait_bounded(bar, parity, status));
+}
+
 /* ---- flagged words -------------------------------------------------------------
  * A value handed from one CTA (or GPU) to another without a barrier: a 32-bit word
  * carrying a bf16 payload in its low half and a 16-bit tag in its high half.  The

@@ -81,6 +81,40 @@ def test_persistent_tick_gives_up_cleanly_and_the_model_falls_back(testlib, capi
     tl.s2p_model_free(m)
 
 
+@pytest.mark.parametrize("limit_ns", [1, 300, 900, 1500, 4000, 10000, 40000])
+def test_persistent_tick_ends_wherever_its_waits_run_out(testlib, capi, limit_ns):
+    """Deadlines from one poll to several stages: the tick gives up at different places, some warps of a CTA while others of it
+    find what they wait for, and it always ends - with a frame or with S2P_ERR_INTERNAL - and the session goes on."""
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    tl = _hooks(testlib)
+    capi.bind(tl, capi.EXT_PROTOTYPES)
+    synth = importlib.import_module("s2pro-native_b200.synth")
+    os.environ.update({"S2P_INT8": "1", "S2P_INT4": "1", "S2P_INT4_ALL": "1", "S2P_QCACHE": "0", "S2P_NO_FUSED": "0", "S2P_NO_MEGA": "0"})
+    ckpt = os.environ.get("S2P_TEST_CKPT_DIR", "/dev/shm") + "/s2p_synth_l2"
+    synth.write_checkpoint(ckpt, n_slow=2, seed=0, generator="auto")
+    opts, m, s = capi.ModelOpts(capi.GEMM_INT8, 1024, 1), C.c_void_p(), C.c_void_p()
+    capi.check(tl.s2p_model_load(ckpt.encode(), C.byref(opts), C.byref(m)), "load")
+    cfg = tl.s2p_sampling_defaults(); cfg.temperature = 0.0
+    capi.check(tl.s2p_session_create(m, C.byref(cfg), C.byref(s)), "session")
+    ids = synth.random_prompt(24, 5)
+    capi.check(tl.s2p_session_prefill(s, ids.ctypes.data_as(C.c_void_p), None, len(ids), None, 0), "prefill")
+    codes = (C.c_int32 * 10)(); eos = C.c_int(0)
+    for _ in range(2):
+        capi.check(tl.s2p_session_next_frame(s, codes, C.byref(eos)), "frame")
+    try:
+        assert tl.mega_set_wait_ns(limit_ns) == 0
+        rc = tl.s2p_session_next_frame(s, codes, C.byref(eos))
+    finally:
+        assert tl.mega_set_wait_ns(2_000_000_000) == 0
+    assert rc in ((S2P_ERR_INTERNAL,) if limit_ns <= 300 else (0, S2P_ERR_INTERNAL)), rc
+    torch.cuda.synchronize()
+    for _ in range(2):
+        capi.check(tl.s2p_session_next_frame(s, codes, C.byref(eos)), "frame after it")
+    tl.s2p_session_destroy(s)
+    tl.s2p_model_free(m)
+
+
 def test_batched_tensor_core_linear_gives_up_cleanly_and_the_exact_kernel_takes_over(testlib, capi):
     """A lockstep batch of 17 sessions runs its linears on the tensor-core kernel; with that kernel's wait
     deadline at 100 ns its first wait runs out: the tick answers S2P_ERR_INTERNAL, TMEM is released, the
