@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(NT + 32, 1) k_skinny_tc(const void* __restrict
             if (x_issued < nk) issue_x();
             if (j_in == 0 && w_issued < nsup) issue_w();
             asm volatile("cp.async.commit_group;" ::: "memory");
-            if (it >= NST) ok = mbar_wait_bounded(done + s, done_parity, status); /* the MMAs that read this stage */
+            if (it >= NST) ok = mbar_wait_warp(done + s, done_parity, status); /* the MMAs that read this stage */
             if (!ok) break;
             const unsigned char* sup = wring + w_rslot;
             unsigned char* A = smem + s * G::A_BYTES;
@@ -371,19 +371,19 @@ __global__ void __launch_bounds__(NT + 32, 1) k_skinny_tc(const void* __restrict
                 if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
         }
     } else {
-        /* ---- the MMA warp (its lane 0 issues) */
-        /* instruction descriptor: D f32, A and B f16, both K-major, N = NB, M = 128 */
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
-        const uint64_t desc_a0 = sk_smem_desc(smem_u32(smem), SK_BM * 16, 128);
-        const uint64_t desc_b0 = sk_smem_desc(smem_u32(stage_b0), (uint32_t)NB * 16, 128);
-        int s = 0, issued = 0;
-        unsigned full_parity = 0;
-        for (int it = 0; it < nk; it++) {
-            ok = mbar_wait_bounded(full + s, full_parity, status);
-            if (ok && XT) ok = mbar_wait_bounded(bx + s, full_parity, status);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
+        /* ---- the MMA warp: one lane waits, issues and gives up; the others wait for it, so the warp has one verdict */
+        if (warp_elect()) {
+            /* instruction descriptor: D f32, A and B f16, both K-major, N = NB, M = 128 */
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
+            const uint64_t desc_a0 = sk_smem_desc(smem_u32(smem), SK_BM * 16, 128);
+            const uint64_t desc_b0 = sk_smem_desc(smem_u32(stage_b0), (uint32_t)NB * 16, 128);
+            int s = 0, issued = 0;
+            unsigned full_parity = 0;
+            for (int it = 0; it < nk; it++) {
+                ok = mbar_wait_bounded(full + s, full_parity, status);
+                if (ok && XT) ok = mbar_wait_bounded(bx + s, full_parity, status);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 /* the start-address field counts 16-byte units: stage s and K step kk are plain additions */
                 const uint64_t da0 = desc_a0 + (uint64_t)((s * G::A_BYTES) >> 4);
                 const uint64_t db0 = desc_b0 + (uint64_t)((s * NBLK * b_bytes) >> 4);
@@ -401,21 +401,21 @@ __global__ void __launch_bounds__(NT + 32, 1) k_skinny_tc(const void* __restrict
                 }
                 /* arrives on the barrier once every MMA issued so far has completed */
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(done + s)) : "memory");
+                issued = it + 1;
+                if (++s == NST) { s = 0; full_parity ^= 1u; }
             }
-            __syncwarp();
-            issued = it + 1;
-            if (++s == NST) { s = 0; full_parity ^= 1u; }
+            if (!ok && issued > 0) {
+                /* giving up with MMAs in flight: they complete by themselves (nothing but the tensor core is
+                 * waited for), and TMEM must not be freed under them.  Wait for the last commit with a fixed,
+                 * generous limit, whatever deadline the other waits have. */
+                uint64_t* bar = done + ((issued - 1) % NST);
+                const unsigned parity = (unsigned)((issued - 1) / NST) & 1u;
+                PipeDeadline dl;
+                for (unsigned i = 0; i < PIPE_MBAR_TRIES && !mbar_try_wait(bar, parity); i++)
+                    if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
+            }
         }
-        if (!ok && issued > 0) {
-            /* giving up with MMAs in flight: they complete by themselves (nothing but the tensor core is
-             * waited for), and TMEM must not be freed under them.  Wait for the last commit with a fixed,
-             * generous limit, whatever deadline the other waits have. */
-            uint64_t* bar = done + ((issued - 1) % NST);
-            const unsigned parity = (unsigned)((issued - 1) / NST) & 1u;
-            PipeDeadline dl;
-            for (unsigned i = 0; i < PIPE_MBAR_TRIES && !mbar_try_wait(bar, parity); i++)
-                if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
-        }
+        __syncwarp();
     }
     /* the last commit covers every MMA before it */
     if (ok) ok = mbar_wait_bounded(done + ((nk - 1) % NST), (unsigned)((nk - 1) / NST) & 1u, status);
@@ -934,17 +934,17 @@ __global__ void __launch_bounds__(WD_EPI + 64, 1) k_wide_tc(WideArgs a) {
                 }
         }
         __syncwarp();
-    } else if (warp == WD_EPI / 32 + 1) { /* ---- the MMA warp (its lane 0) */
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
-        const uint64_t desc_a0 = sk_smem_desc(smem_u32(smem), SK_BM * 16, 128);
-        const uint64_t desc_b0 = sk_smem_desc(smem_u32(stage_b0), (uint32_t)NB * 16, 128);
-        int s = 0, issued = 0;
-        unsigned parity = 0;
-        for (int it = 0; it < nk; it++) {
-            ok = mbar_wait_bounded(full + s, parity, status);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
+    } else if (warp == WD_EPI / 32 + 1) { /* ---- the MMA warp: one lane, as in k_skinny_tc */
+        if (warp_elect()) {
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
+            const uint64_t desc_a0 = sk_smem_desc(smem_u32(smem), SK_BM * 16, 128);
+            const uint64_t desc_b0 = sk_smem_desc(smem_u32(stage_b0), (uint32_t)NB * 16, 128);
+            int s = 0, issued = 0;
+            unsigned parity = 0;
+            for (int it = 0; it < nk; it++) {
+                ok = mbar_wait_bounded(full + s, parity, status);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da0 = desc_a0 + (uint64_t)((s * WD_A_BYTES) >> 4), db0 = desc_b0 + (uint64_t)((s * b_bytes) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < WD_KC / 16; kk++) {
@@ -955,16 +955,16 @@ __global__ void __launch_bounds__(WD_EPI + 64, 1) k_wide_tc(WideArgs a) {
                         ::"r"(tmem), "l"(da0 + (uint64_t)(kk * 2 * SK_BM)), "l"(db0 + (uint64_t)(kk * 2 * NB)), "r"(idesc), "r"(accumulate) : "memory");
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(done + s)) : "memory");
+                issued = it + 1;
+                if (++s == stages) { s = 0; parity ^= 1u; }
             }
-            __syncwarp();
-            issued = it + 1;
-            if (++s == stages) { s = 0; parity ^= 1u; }
+            if (!ok && issued > 0) { /* TMEM must not be freed under MMAs in flight: the last commit, with a limit of its own */
+                PipeDeadline dl;
+                for (unsigned i = 0; i < PIPE_MBAR_TRIES && !mbar_try_wait(done + (issued - 1) % stages, (unsigned)((issued - 1) / stages) & 1u); i++)
+                    if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
+            }
         }
-        if (!ok && issued > 0) { /* TMEM must not be freed under MMAs in flight: the last commit, with a limit of its own */
-            PipeDeadline dl;
-            for (unsigned i = 0; i < PIPE_MBAR_TRIES && !mbar_try_wait(done + (issued - 1) % stages, (unsigned)((issued - 1) / stages) & 1u); i++)
-                if ((i & 63u) == 63u && dl.expired(2000000000ull)) break;
-        }
+        __syncwarp();
     }
     /* the last commit covers every MMA before it */
     if (ok) ok = mbar_wait_bounded(done + (nk - 1) % stages, (unsigned)((nk - 1) / stages) & 1u, status);
