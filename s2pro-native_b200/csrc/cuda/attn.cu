@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(512) k_attn_decode(AttnArgs a, AttnPrep pz) {
 /* The kernel for lockstep batches on one GPU, no fused prologue: a team of two warps per split
  * (attn_team.cuh). */
 template <bool KV8, int NT>
-static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, cudaStream_t st) {
+static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, int early, cudaStream_t st) {
     static bool attr_set[64] = {false};
     constexpr size_t smem = sizeof(AttnTeamSmem<KV8, NT>);
     int dev = 0;
@@ -45,7 +45,7 @@ static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, cudaStream_t s
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    return launch_after(k_attn_decode_team<KV8, NT>, grid, NT * 64, smem, st, a);
+    return launch_early(early, k_attn_decode_team<KV8, NT>, grid, NT * 64, smem, st, a);
 }
 constexpr int ATTN_TEAMS_KV8 = 4, ATTN_TEAMS_BF16 = 3; /* two CTAs per SM either way */
 static bool attn_team_serves(const AttnArgs& a, int rows) {
@@ -59,12 +59,13 @@ static bool attn_team_serves(const AttnArgs& a, int rows) {
     return (size_t)a.n_split_slots * 32 + 16 <= tiles;
 }
 
-cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows, cudaStream_t st) {
+/* early: the kernel in front writes nothing of the cache but the last position, and no position table (launch.cuh) */
+cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows, int early, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     if (a.q_heads != a.kv_heads * 4 || !a.part || !a.counters || a.workers < 1) return cudaErrorInvalidValue;
     dim3 grid((unsigned)rows, (unsigned)a.kv_heads, (unsigned)a.workers);
     if (!prep && attn_team_serves(a, rows))
-        return a.kv8 ? launch_attn_team<true, ATTN_TEAMS_KV8>(a, grid, st) : launch_attn_team<false, ATTN_TEAMS_BF16>(a, grid, st);
+        return a.kv8 ? launch_attn_team<true, ATTN_TEAMS_KV8>(a, grid, early, st) : launch_attn_team<false, ATTN_TEAMS_BF16>(a, grid, early, st);
     AttnPrep pz = {};
     /* one score chain per thread (HPT 1): sharing a key's conversion between the heads of a position
      * (HPT 2 or 4) measured slower on a lockstep batch of 32, fewer warps being busy in the score phase */
@@ -80,7 +81,7 @@ cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows
 }
 
 extern "C" cudaError_t attn_decode(const AttnArgs* a, int rows, cudaStream_t st) {
-    return launch_attn_decode(*a, nullptr, rows, st);
+    return launch_attn_decode(*a, nullptr, rows, 1, st);
 }
 
 /* ---- allocation-free variant (include/s2p_b200_ext.h) --------------------------
@@ -145,7 +146,7 @@ extern "C" s2p_status s2p_b200_attention_decode_noalloc(const s2p_bf16* q, const
     a.counters = counters;
     a.n_split_slots = NOALLOC_SLOTS;
     a.workers = 16;
-    S2P_CUDA_TRY(launch_attn_decode(a, nullptr, 1, stream));
+    S2P_CUDA_TRY(launch_attn_decode(a, nullptr, 1, 0, stream)); /* the caller may have written any of the cache just before */
     return S2P_OK;
 }
 

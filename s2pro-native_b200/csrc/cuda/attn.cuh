@@ -18,6 +18,6 @@ struct AttnPrep {
     int* status;
 };
 
-cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows, cudaStream_t st);
+cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows, int early, cudaStream_t st);
 
 }  // namespace s2p

@@ -26,15 +26,6 @@ int device_sm_count() {
     return n;
 }
 
-/* Both kernels fetch their first weights before they wait for the kernel in front (launch.cuh).  `early` says that it is
- * not that kernel which writes them: so inside a tick, not where a caller may have queued a quantisation just before. */
-template <class... P, class... A>
-static cudaError_t launch_gemv(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, int early, cudaStream_t st, A... args) {
-    if (early) return launch_after(kernel, grid, threads, smem, st, args...);
-    kernel<<<grid, threads, smem, st>>>(args...);
-    return cudaGetLastError();
-}
-
 template <int WK, int PRO, int EPI>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) k_gemv_stage(GemvStage g) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -78,7 +69,7 @@ cudaError_t launch_gemv_stage(GemvStage g, int early, cudaStream_t stream) {
     const int rows_per_cta = (units + grid - 1) / grid;
     g.rows_per_pass = gemv_rows_per_pass(WK, rows_per_cta, g.K, g.gshift, EPI == EPI_SWIGLU, limit);
     const size_t smem = gemv_smem_bytes(WK, g.rows_per_pass * (EPI == EPI_SWIGLU ? 2 : 1), g.K, g.gshift);
-    return launch_gemv(k_gemv_stage<WK, PRO, EPI>, dim3((unsigned)grid), GEMV_THREADS, smem, early, stream, g);
+    return launch_early(early, k_gemv_stage<WK, PRO, EPI>, dim3((unsigned)grid), GEMV_THREADS, smem, stream, g);
 }
 
 /* instantiations used by the tick live here so that every kernel is compiled once */
@@ -332,7 +323,7 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
 template <int WK, int MM, int NS, bool SW>
 static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
     constexpr int rows = 4 * (4 / NS); /* weight rows of a CTA */
-    return launch_gemv(k_gemv_batch<WK, MM, NS, SW>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, early, stream,
+    return launch_early(early, k_gemv_batch<WK, MM, NS, SW>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift);
 }
 template <int WK, bool SW>
@@ -536,7 +527,7 @@ static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const 
         if (shared) kernel = M == 2 ? k_gemv_row<WK, 2, 4, 2, 4, false> : k_gemv_row<WK, 1, 4, 2, 4, false>;
     }
     const int per_warp = many ? MANY : 4, warps = (N + per_warp - 1) / per_warp;
-    return launch_gemv(kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, early, stream,
+    return launch_early(early, kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, N, K, gshift);
 }
 

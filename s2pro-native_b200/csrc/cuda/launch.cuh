@@ -35,3 +35,12 @@ static inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
+
+/* For kernels that read before grid_wait what the kernel in front does not write inside a tick (weights, settled cache), but
+ * what a caller of the public entry points may have written just before: early only inside a tick. */
+template <class... P, class... A>
+static inline cudaError_t launch_early(int early, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+    if (early) return launch_after(kernel, grid, threads, smem, st, args...);
+    kernel<<<grid, threads, smem, st>>>(static_cast<P>(args)...);
+    return cudaGetLastError();
+}

@@ -137,7 +137,7 @@ cudaError_t tick_begin(const TickBeginArgs* a, int rows, cudaStream_t st);
 cudaError_t tick_finish_keys(const unsigned long long* keys, int rows, int32_t* codes, cudaStream_t st);
 
 cudaError_t gemv_setup_all(void); /* once per device, before any stream capture */
-/* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: see launch_gemv in gemv.cu */
+/* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: see launch_early (launch.cuh) */
 int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t st);
 /* h[M, N / 2] = silu(gate) * up for stacked [gate | up] rows, otherwise as gemv_rows with early.  Up to four rows the launch it
  * saves counts (tick of 1 row 3.53 -> 3.43 ms, 3 rows 5.61 -> 5.55); the kernels of eight rows have no registers left for it (8 rows

@@ -70,7 +70,7 @@ extern "C" cudaError_t stage_attn_decode_prep(const AttnArgs* a, const __nv_bflo
                                               const __nv_bfloat16* q_norm, const __nv_bfloat16* k_norm, float eps,
                                               float rope_base, int rows, cudaStream_t st) {
     AttnPrep p = {qkv, q_norm, k_norm, eps, rope_base};
-    return launch_attn_decode(*a, &p, rows, st);
+    return launch_attn_decode(*a, &p, rows, 1, st);
 }
 
 /* ---- frame start (src/slowar/slowar.c:481-498; fastar.cu:104-127) ----------- */
