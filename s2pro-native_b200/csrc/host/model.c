@@ -390,7 +390,11 @@ s2p_status s2p_model_load(const char* model_dir, const s2p_model_opts* opts, s2p
         if (rc != S2P_OK) goto fail;
     }
     if ((rc = alloc_workspace(m)) != S2P_OK) goto fail;
-    if (m->mode == S2P_GEMM_INT8 && ((rc = widen_backbone(m)) != S2P_OK || (rc = tile_linears(m)) != S2P_OK)) goto fail;
+    {   /* resident copies of the weights, unless S2P_RESIDENT=0 asks for a small model instead of a fast one */
+        const char* e = getenv("S2P_RESIDENT");
+        const int wanted = m->mode == S2P_GEMM_INT8 && !(e && e[0] == '0' && e[1] == '\0');
+        if (wanted && ((rc = widen_backbone(m)) != S2P_OK || (rc = tile_linears(m)) != S2P_OK)) goto fail;
+    }
     if (cudaEventCreate(&m->ev0) != cudaSuccess || cudaEventCreate(&m->ev1) != cudaSuccess) { rc = S2P_ERR_CUDA; goto fail; }
     if (cudaStreamSynchronize(m->stream) != cudaSuccess) { rc = S2P_ERR_CUDA; goto fail; }
     s2p_st_close(st);

@@ -18,8 +18,9 @@ def test_frames_do_not_depend_on_the_copies(testlib, synth, capi, monkeypatch, i
     ckpt = ("/dev/shm" if os.path.isdir("/dev/shm") else "/tmp") + "/s2p_synth_l2"
     synth.write_checkpoint(ckpt, n_slow=2, seed=0, generator="auto")
     runs = []
-    for give_back in (0, 1):  # 1: the bf16 copies before the prompts, the tiles between two ticks
-        m = C.c_void_p()
+    for way in ("kept", "given back", "never made"):  # given back: the bf16 copies before the prompts, the tiles between two ticks
+        monkeypatch.setenv("S2P_RESIDENT", "0" if way == "never made" else "1")
+        m, give_back = C.c_void_p(), way == "given back"
         opts = capi.ModelOpts(capi.GEMM_INT8, 512, ROWS)
         capi.check(tl.s2p_model_load(ckpt.encode(), C.byref(opts), C.byref(m)), "load")
         if give_back:
@@ -38,11 +39,14 @@ def test_frames_do_not_depend_on_the_copies(testlib, synth, capi, monkeypatch, i
                 assert tl.s2p_model_give_back(m) == 1 and tl.s2p_model_give_back(m) == 0
             capi.check(tl.s2p_model_batch_next_frame(m, sessions, ROWS, codes, eos), "tick")
             frames.append((list(codes), list(eos)))
+        if way != "kept":
+            assert tl.s2p_model_give_back(m) == 0
         blob = torch.empty(int(tl.s2p_session_kv_bytes(m, 32)), dtype=torch.uint8, device="cuda")
         capi.check(tl.s2p_session_kv_save(sessions[7], 32, C.c_void_p(blob.data_ptr())), "save")
         for s in sessions:
             tl.s2p_session_destroy(s)
         tl.s2p_model_free(m)
         runs.append((frames, blob))
-    assert runs[0][0] == runs[1][0]
-    assert torch.equal(runs[0][1], runs[1][1])
+    for frames, blob in runs[1:]:
+        assert frames == runs[0][0]
+        assert torch.equal(blob, runs[0][1])
