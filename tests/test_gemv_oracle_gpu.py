@@ -1,0 +1,42 @@
+"""The exact-order linear against the CPU oracle, bit for bit: every batch size it serves, both weight formats and grouped INT8, tiles of
+K whole to a warp and shared by a CTA's warps, ragged rows."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+G = 32
+
+
+def p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("kind", ["int8", "int8_grouped", "int4"])
+@pytest.mark.parametrize("n,k,all_rows", [(37, 512, True), (1029, 4608, True), (6145, 1024, True), (19457, 512, False)])
+def test_every_batch_size_gives_the_oracles_bits(mine, oracle, kind, n, k, all_rows):
+    from oracle import oracle_api
+    rng = np.random.default_rng(n)
+    w = rng.integers(0, 256, size=(n, k // 2 if kind == "int4" else k), dtype=np.uint8)
+    s = rng.random((n, 1 if kind == "int8" else k // G), dtype=np.float32) * 0.01 + 0.001
+    s = s if kind == "int8" else s.astype(np.float16)
+    x = oracle_api.f32_to_bf16(rng.standard_normal((16, k), dtype=np.float32))
+    want = np.empty((16, n), np.uint16)
+    args = [oracle_api.ptr(a) for a in (want, x, w, s)] + [16, n, k]
+    if kind == "int8":
+        oracle.s2po_gemv_int8(*args)
+    else:
+        (oracle.s2po_gemv_g if kind == "int8_grouped" else oracle.s2po_gemv_p)(*args, G)
+    dw, ds, dx = (torch.from_numpy(a.view(np.int16) if a.dtype == np.uint16 else a).cuda() for a in (w, s, x))
+    for rows in range(1, 17) if all_rows else (1, 2):  # many rows of weights: what differs is the one-row kernel
+        y = torch.full((rows + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+        args = [p(y), p(dx), p(dw), p(ds), rows, n, k]
+        if kind == "int8":
+            assert mine.s2p_int8_gemv(*args, None) == 0
+        else:
+            assert (mine.s2p_intq_gemv if kind == "int8_grouped" else mine.s2p_int4p_gemv)(*args, G, None) == 0
+        got = y.view(torch.int16).cpu().numpy().view(np.uint16)
+        assert np.array_equal(got[:rows], want[:rows]), rows
+        assert (got[rows] == oracle_api.f32_to_bf16(np.float32([7.0]))[0]).all()
