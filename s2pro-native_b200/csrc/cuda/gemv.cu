@@ -334,7 +334,11 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
      * that three quarters of the rounds' turns have a tile (a CTA waits for its slowest warp: at K = 2560, five tiles
      * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all.  (A SwiGLU's pairs of rows
      * meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
-    const int groups = (M + 7) / 8, mm = (M + groups - 1) / groups;
+    const int groups = (M + 7) / 8;
+    /* Seven rows of packed INT4 take the kernel of eight: the seventh row's scalar chains spill there (86.8 us for a layer's four
+     * matrices, 85.4 padded).  Two groups of seven have two warps to a scheduler and are faster as they are (13 rows 142.4, padded
+     * 145.3), and so is INT8 (7 rows 79.2, padded 80.7). */
+    const int mm = WK == WK_INT4_PACK && M == 7 ? 8 : (M + groups - 1) / groups;
     const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
     const int T = K >> 9, turns = (T + 3) / 4 * 4;
     const bool shared = !SW && (2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
