@@ -57,7 +57,7 @@ cudaError_t gemv_stage_setup() {
 }
 
 template <int WK, int PRO, int EPI>
-cudaError_t launch_gemv_stage(GemvStage g, int early, cudaStream_t stream) {
+cudaError_t launch_gemv_stage(GemvStage g, cudaStream_t stream) {
     const size_t limit = GEMV_SMEM_LIMIT;
     {
         const cudaError_t e = gemv_stage_setup<WK, PRO, EPI>();
@@ -69,18 +69,15 @@ cudaError_t launch_gemv_stage(GemvStage g, int early, cudaStream_t stream) {
     const int rows_per_cta = (units + grid - 1) / grid;
     g.rows_per_pass = gemv_rows_per_pass(WK, rows_per_cta, g.K, g.gshift, EPI == EPI_SWIGLU, limit);
     const size_t smem = gemv_smem_bytes(WK, g.rows_per_pass * (EPI == EPI_SWIGLU ? 2 : 1), g.K, g.gshift);
-    return launch_early(early, k_gemv_stage<WK, PRO, EPI>, dim3((unsigned)grid), GEMV_THREADS, smem, stream, g);
+    return launch_after(k_gemv_stage<WK, PRO, EPI>, dim3((unsigned)grid), GEMV_THREADS, smem, stream, g);
 }
 
 /* instantiations used by the tick live here so that every kernel is compiled once */
-template cudaError_t launch_gemv_stage<WK_INT8_CH, PRO_VEC, EPI_STORE>(GemvStage, int, cudaStream_t);
-template cudaError_t launch_gemv_stage<WK_INT8_GRP, PRO_VEC, EPI_STORE>(GemvStage, int, cudaStream_t);
-template cudaError_t launch_gemv_stage<WK_INT4_PACK, PRO_VEC, EPI_STORE>(GemvStage, int, cudaStream_t);
 #define S2P_INST(WK)                                                                         \
-    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_STORE>(GemvStage, int, cudaStream_t); \
-    template cudaError_t launch_gemv_stage<WK, PRO_VEC, EPI_RESID>(GemvStage, int, cudaStream_t);  \
-    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_SWIGLU>(GemvStage, int, cudaStream_t);\
-    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_ARGMAX>(GemvStage, int, cudaStream_t);
+    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_STORE>(GemvStage, cudaStream_t); \
+    template cudaError_t launch_gemv_stage<WK, PRO_VEC, EPI_RESID>(GemvStage, cudaStream_t);  \
+    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_SWIGLU>(GemvStage, cudaStream_t);\
+    template cudaError_t launch_gemv_stage<WK, PRO_NORM, EPI_ARGMAX>(GemvStage, cudaStream_t);
 S2P_INST(WK_INT8_CH)
 S2P_INST(WK_INT8_GRP)
 S2P_INST(WK_INT4_PACK)
@@ -92,7 +89,6 @@ extern "C" cudaError_t gemv_setup_all(void) {
     cudaError_t e = cudaSuccess;
 #define S2P_SETUP(WK, PRO, EPI) if (e == cudaSuccess) e = gemv_stage_setup<WK, PRO, EPI>();
 #define S2P_SETUP_WK(WK)               \
-    S2P_SETUP(WK, PRO_VEC, EPI_STORE)  \
     S2P_SETUP(WK, PRO_NORM, EPI_STORE) \
     S2P_SETUP(WK, PRO_VEC, EPI_RESID)  \
     S2P_SETUP(WK, PRO_NORM, EPI_SWIGLU) \

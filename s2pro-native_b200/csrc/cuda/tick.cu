@@ -20,14 +20,14 @@
 namespace s2p {
 
 template <int WK, int PRO, int EPI>
-cudaError_t launch_gemv_stage(GemvStage g, int early, cudaStream_t stream); /* gemv.cu */
+cudaError_t launch_gemv_stage(GemvStage g, cudaStream_t stream); /* gemv.cu */
 
 template <int PRO, int EPI>
 static cudaError_t dispatch_kind(int kind, const GemvStage& g, cudaStream_t st) {
     switch (kind) {
-    case WK_INT8_CH: return launch_gemv_stage<WK_INT8_CH, PRO, EPI>(g, 1, st);
-    case WK_INT8_GRP: return launch_gemv_stage<WK_INT8_GRP, PRO, EPI>(g, 1, st);
-    case WK_INT4_PACK: return launch_gemv_stage<WK_INT4_PACK, PRO, EPI>(g, 1, st);
+    case WK_INT8_CH: return launch_gemv_stage<WK_INT8_CH, PRO, EPI>(g, st);
+    case WK_INT8_GRP: return launch_gemv_stage<WK_INT8_GRP, PRO, EPI>(g, st);
+    case WK_INT4_PACK: return launch_gemv_stage<WK_INT4_PACK, PRO, EPI>(g, st);
     }
     return cudaErrorInvalidValue;
 }
