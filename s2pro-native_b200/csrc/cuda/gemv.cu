@@ -516,17 +516,24 @@ __global__ void __launch_bounds__(128, MM == 2 ? 4 : R == 6 ? 6 : PD == 1 ? 8 : 
 static bool gemv_row_shared(int N, int K) { return 2 * ((N + 3) / 4) < 3 * 4 * device_sm_count() && K > 4 * 512; }
 template <int WK, bool SW>
 static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
-    /* From six warps per scheduler on a tile at a time with twice the warps resident hides more than two tiles side by side; INT4,
-     * whose tiles are half the loads, also takes six rows a warp there, which keeps 19456 rows from a second wave (INT4 14.4 -> 13.5 ->
-     * 12.9 us, INT8 12.5 -> 11.2, 11.5 with six rows). */
-    const bool shared = !SW && gemv_row_shared(N, K), many = (N + 3) / 4 >= 6 * 4 * device_sm_count();
-    constexpr int MANY = WK == WK_INT4_PACK ? 6 : 4;
+    /* From six warps per scheduler on a tile at a time with twice the warps resident hides more than two tiles side by side (19456
+     * rows INT8 12.5 -> 11.2 us).  There packed INT4, whose tiles are half the loads, takes six rows a warp where the warps of four do
+     * not fit the GPU at once (8 CTAs of 4 x 4 rows to an SM; of six 6 CTAs, so 144 rows instead of 128).  K = 2560, us with six /
+     * four rows: one wave of either 14208 rows 12.2 / 10.9, 18944 13.3 / 11.6; beyond it 21312 13.3 / 13.9, 24576 13.9 / 15.0,
+     * 28416 17.0 / 16.7, 38912 20.3 / 21.5, 155776 70.5 / 73.1.  (19456 rows: 13.4 / 13.1 in a chain of early launches, 12.9 / 13.5
+     * launched the ordinary way.) */
+    const int sms = device_sm_count();
+    const bool shared = !SW && gemv_row_shared(N, K), many = (N + 3) / 4 >= 6 * 4 * sms;
+    const bool six = WK == WK_INT4_PACK && N > 8 * 4 * 4 * sms;
     void (*kernel)(__nv_bfloat16*, const __nv_bfloat16*, const void*, const void*, int, int, int) =
-        many ? k_gemv_row<WK, 1, MANY, 1, 1, SW> : k_gemv_row<WK, 1, 4, 2, 1, SW>;
+        many ? k_gemv_row<WK, 1, 4, 1, 1, SW> : k_gemv_row<WK, 1, 4, 2, 1, SW>;
+    if constexpr (WK == WK_INT4_PACK) {
+        if (six) kernel = k_gemv_row<WK, 1, 6, 1, 1, SW>;
+    }
     if constexpr (!SW) {
         if (shared) kernel = M == 2 ? k_gemv_row<WK, 2, 4, 2, 4, false> : k_gemv_row<WK, 1, 4, 2, 4, false>;
     }
-    const int per_warp = many ? MANY : 4, warps = (N + per_warp - 1) / per_warp;
+    const int per_warp = six ? 6 : 4, warps = (N + per_warp - 1) / per_warp;
     return launch_early(early, kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, N, K, gshift);
 }

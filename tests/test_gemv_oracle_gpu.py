@@ -15,7 +15,7 @@ def p(t):
 
 
 @pytest.mark.parametrize("kind", ["int8", "int8_grouped", "int4"])
-@pytest.mark.parametrize("n,k,all_rows", [(37, 512, True), (1029, 4608, True), (6145, 1024, True), (19457, 512, False)])
+@pytest.mark.parametrize("n,k,all_rows", [(37, 512, True), (1029, 4608, True), (6145, 1024, True), (14209, 512, False), (19457, 512, False)])
 def test_every_batch_size_gives_the_oracles_bits(mine, oracle, kind, n, k, all_rows):
     from oracle import oracle_api
     rng = np.random.default_rng(n)
