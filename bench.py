@@ -287,7 +287,7 @@ def isolated_gemv_roofline(lib, torch, mode, peak_gbs):
         e0.record(); g.replay(); e1.record(); torch.cuda.synchronize()
         us = e0.elapsed_time(e1) * 1e3 / reps
         byts = per + (N * (K // G) * 2 if mode == "int4" else N * 4)
-        out.append({"kernel": f"k_gemv_stage[{name} {N}x{K} {mode}]", "us": round(us, 2), "bytes": byts,
+        out.append({"kernel": f"k_gemv_row[{name} {N}x{K} {mode}]", "us": round(us, 2), "bytes": byts,
                     "achieved_gbs": round(byts / us / 1e3, 1), "frac": round(byts / us / 1e3 / peak_gbs, 3)})
         del w, sc
     return out
@@ -545,7 +545,7 @@ def run_ours(args, rank, world):
                          "traffic": traffic, "traffic_source": NCU_TRAFFIC_SOURCE if traffic else None, "peak_source": peak_kind,
                          "kernel": "k_tick_mega (one launch = one frame)" if stats.last_tick_persistent else "whole tick (per-stage launches)",
                          "note": "algorithmic weight bytes per frame / device time of the tick, CUDA events on the model stream; "
-                                 "roofline_kernels lists the stand-alone GEMV stage kernels of the non-persistent path",
+                                 "roofline_kernels lists the one-row linears of a frame, launched alone",
                          "algorithmic_bytes_per_frame": int(algo), "modelled_bytes_with_kv": int(traffic_model)},
             "clocks": sampler.summary(),
         }
@@ -569,7 +569,7 @@ def run_ours(args, rank, world):
             line["roofline_kernels"] = isolated_gemv_roofline(lib, torch, args.mode, peak)
         if not args.no_prefill_block and args.batch == 1:
             line["prefill"] = prefill_block(lib, capi, synth, ckpt, args.prompt,
-                                            {"ms_dequant_cublas": "0", "ms_tensor_core": "1"})
+                                            {"ms_cublas": "0", "ms_tensor_core": "1"})  # resident bf16 weights; packed weights
         if not args.no_cpu_baseline:
             line["cpu_baseline"] = cpu_baseline(args.mode, layers=args.layers)
     return line
@@ -620,7 +620,7 @@ def run_reference(args, rank, world):
         step = (time.perf_counter() - t0) * 1e3 / args.steps
         eng.close()
         if not args.no_prefill_block and args.batch == 1:
-            base["prefill"] = prefill_block(ref, capi, synth, ckpt, args.prompt, {"ms_dequant_cublas": "0"})
+            base["prefill"] = prefill_block(ref, capi, synth, ckpt, args.prompt, {"ms_cublas": "0"})
         base.update({"value": round(step, 4), "ms_per_step": round(step, 4),
                      "config": config_block(args, seed_used, world, 1, 4096, False,
                                             "reference CUDA path rebuilt unchanged for sm_100a (oracle/_ref), same GPU, same API calls"),

@@ -18,9 +18,10 @@
  *
  * Measured (INT8 cache, 2048 rows after 6052 positions, 119 G fma): 12.6 ms with four rows per 512-thread CTA, keys converted
  * by every reader and trees over shared memory; 10.6 ms register-tiled 2 x 8; 6.5 ms 4 x 8; 5.7 ms with 12 warps instead of
- * 8; 5.5 ms = 21.7 T fma/s with the producers, 0.58 of the fp32 peak.  The score phase runs at nine tenths of the fma
- * rate; the value phase pays one multiplication per weight and group scale.  8 x 8 tiles measured the same per row with
- * worse waves; 2 queries x 16 dimensions per thread in the value phase slower (more shared reads).
+ * 8; 5.4 ms = 22 T fma/s with the producers, 0.6 of the fp32 peak.  Counters of that launch: fma pipe 77 % of its cycles
+ * busy (the value phase pays one multiplication per weight and group scale beside its fma), issue slots 59 %, the shared-memory
+ * data path 59 %.  77 rows after 1024 positions (104 CTAs, nine tiles in sequence): 50 %, 47 % and 50 %.  8 x 8 tiles measured
+ * the same per row with worse waves; 2 queries x 16 dimensions per thread in the value phase slower (more shared reads).
  */
 #pragma once
 #include <math.h>
@@ -300,7 +301,6 @@ __global__ void __launch_bounds__((APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCER
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.kempty);
 
-        /* soft-max of the tile, one query after another; its eight weights of this thread go to shared memory */
         if (APART && !mbar_wait_bounded(&sm.pempty[w], phase ^ 1, status)) return false;
 
         /* soft-max of the tile, one query after another; its eight weights of this thread go to shared memory */

@@ -2,11 +2,11 @@
  * s2p_int8_gemv, s2p_intq_gemv, s2p_int4p_gemv — the reference's
  * src/sched/int8_gemv.cu:964-986, :773-799, :836-902.
  *
- * M == 1 runs the batch-1 streaming stage of gemv.cuh.  2 <= M <= 16 runs the
- * exact-order small-batch kernel below: every row of x is an independent
- * product with the same summation order as M == 1 (the reference's batched
- * GEMV computes rows independently, int8_gemv.cu:77-91), codes are widened
- * once per tile and reused for all M rows.
+ * One row, and two of a matrix of few rows, run k_gemv_row; up to 16 rows run
+ * k_gemv_batch, where codes are widened once per tile for up to eight rows.  Every
+ * row of x is an independent product with one summation order (the reference's
+ * batched GEMV computes rows independently too, int8_gemv.cu:77-91).  The stage
+ * kernel of gemv.cuh (k_gemv_stage) serves the fused per-stage frame only.
  */
 #include <stdio.h>
 #include "gemv.cuh"
@@ -116,9 +116,11 @@ extern "C" cudaError_t gemv_setup_all(void) {
  * folds a quarter of the activation rows, tiles ascending.
  * Measured, us for one layer's four matrices (N x K 6144 x 2560, 2560 x 4096, 19456 x 2560, 2560 x 9728), before (scalar fma, one
  * weight row per warp for INT8; mixed bf16 fma, one to four for INT4) and now, at 2 / 4 / 8 / 16 rows:
- *   INT8  52 / 84 / 148 / 258 -> 44 / 56 / 83 / 138      INT4  46 / 70 / 103 / 180 -> 46 / 58 / 85 / 144
+ *   INT8  52 / 84 / 148 / 258 -> 44 / 56 / 81 / 135      INT4  46 / 70 / 103 / 180 -> 46 / 56 / 85 / 146
+ * (2 rows now share the one-row kernel where rows are few: 38 and 39).
  * An odd row's chain is scalar: padded to a pair it held the fma pipe for two (3 rows INT4 58 -> 53, 5 rows 74 -> 68, 9 rows 119 -> 108).
- * 16 rows of 19456 x 2560 run at 13.5 T fma/s; the pipe's rate is 36 T. */
+ * 16 rows of 19456 x 2560 INT4 run at 11.4 T fma/s; the pipe's rate is 36 T.  Counters there: issue slots 59 %, fma pipe 51 %, integer
+ * pipe 44 % busy, 11 of 64 warps resident (168 registers), 5 % of DRAM. */
 /* A SwiGLU over stacked [gate | up] rows (SW): half of a warp's rows are of either half, so gate and up of an output meet in
  * the warp; both round to bf16 first, as where a kernel of its own follows the linear. */
 template <bool SW, int R> __device__ __forceinline__ int gemv_row_of(int n0, int r, int F) {
@@ -357,9 +359,10 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
 }
 
 /* ---- one row, or two of a matrix of few rows ---------------------------------
- * The linear alone, as a caller's own layers and the frames outside the persistent tick use it.
+ * The linear alone, as callers' own layers and one-row frames of a model on one GPU use it.
  *
- * What bounds it: DRAM, at a few thousand warps whose weights are all under way at once.  A warp carries four rows (or six) as
+ * What bounds it: instruction issue inside a wave of CTAs too short to be steady (19456 x 2560 INT4: issue slots 63 %, integer pipe
+ * 57 %, fma pipe 43 % busy over the launch, DRAM 22 %).  So a few thousand warps have their weights under way at once.  A warp carries four rows (or six) as
  * packed chains (a register pair holds the same k of two rows), PD tiles at a time side by side, since every tile starts a chain of its
  * own; the next PD tiles' weights are in registers meanwhile.  Where there are too few rows for that NS = 4 warps share
  * four rows as in k_gemv_batch.

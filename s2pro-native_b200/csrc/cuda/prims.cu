@@ -542,7 +542,8 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, int* status,
  * cheapest per row (0.80 us a tile with 24 rows, 2.3 with 2), small ones fill the GPU when the slice is short.  The times below
  * are the measured ones for an INT8 cache; bf16 is within 10 %.  16 and 24 rows keep a scheduler busy with warps that do both
  * products (15.3 and 19.3 us; products apart 16.1 and too many registers); up to 12 rows they are apart (8 rows 9.4 -> 9.0 us,
- * 4 rows 7.0 -> 5.8, see attn_prefill.cuh).
+ * 4 rows 7.0 -> 5.8, see attn_prefill.cuh).  The estimate takes all CTAs to see equally many tiles, which holds for a slice behind
+ * a long context; at position 0 the first block of a slice sees one tile and the last all of them, and what decides is the longest.
  * Measured (us; first kernel of one block size, four sizes of one kind, now): 2048 rows after 6052 positions 12590, 5430, 5396; 77
  * after 1024 154, 93, 73; 50 after 1000 89, 68, 57; 20 after 2000 161, 120, 82. */
 template <bool KV8>
