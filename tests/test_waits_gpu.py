@@ -172,8 +172,9 @@ def _slice_waits(tl):
 
 
 def test_prompt_attention_of_a_caller_reports_a_wait_that_gave_up(testlib):
-    """s2pk_attention has no synchronisation of its own: with the deadline at 1 ns a call loses rows, the next one says so
-    without launching anything, and the one after that is whole again."""
+    """s2pk_attention has no synchronisation of its own: with the deadline at 1 ns a call loses rows (nearly always: a wait that the
+    hardware suspends may also be satisfied before its first look at the clock), the next one says so without launching
+    anything, and the one after that is whole again."""
     if not torch.cuda.is_available():
         pytest.fail("CUDA device required for -m gpu tests")
     tl = _slice_waits(testlib)
@@ -192,12 +193,13 @@ def test_prompt_attention_of_a_caller_reports_a_wait_that_gave_up(testlib):
     assert rc == 0
     try:
         assert tl.attn_prefill_set_wait_ns(1) == 0
-        rc, _ = attend()
+        for _ in range(100):
+            rc, out = attend()
+            if rc != 0:
+                break
     finally:
         assert tl.attn_prefill_set_wait_ns(2_000_000_000) == 0
-    assert rc == 0
-    rc, out = attend()
-    assert rc == 702 and (out == 7).all()  # cudaErrorLaunchTimeout
+    assert rc == 702 and (out == 7).all()  # cudaErrorLaunchTimeout, for the call before
     rc, out = attend()
     assert rc == 0 and torch.equal(out.view(torch.int16), want.view(torch.int16))
 
@@ -243,7 +245,12 @@ def test_prompt_slice_whose_attention_gives_up_is_refused_and_can_be_repeated(te
     want = frames(one)
     try:
         assert tl.attn_prefill_set_wait_ns(1) == 0
-        rc = prefill(two)
+        for _ in range(50):
+            rc = prefill(two)
+            if rc != 0:
+                break
+            tl.s2p_session_destroy(two)
+            two = opened()
     finally:
         assert tl.attn_prefill_set_wait_ns(2_000_000_000) == 0
     assert rc == S2P_ERR_INTERNAL
