@@ -5,18 +5,18 @@
  * src/fastar/fastar.cu:726-788) is about 400 dependent stages, each a few
  * microseconds of work for the whole GPU.  Launched separately, every stage
  * pays a launch, a cold start of its weight stream and a tail; here the CTAs
- * (one per SM, 512 threads) stay resident and walk a stage list, meeting at a
- * grid barrier between stages.
+ * (one per SM, 512 threads) stay resident and walk a stage list, handing a stage's
+ * outputs over as flagged words; twelve grid barriers a frame remain.
  *
  * Weights reach the SM through a ring of shared-memory slots filled by 1-D TMA
  * bulk copies (cp.async.bulk + mbarrier transaction counts).  Each CTA owns a
  * fixed row block of every matrix, cut into chunks of whole rows that fit a
  * slot; one thread issues the copies from a per-CTA command list the host built
  * at load time, three chunks ahead of the one being consumed.  The list runs
- * across stage boundaries, so while the CTA waits at a grid barrier (or does
+ * across stage boundaries, so while the CTA waits for its input (or does
  * attention) the ring already holds the next GEMV stage's first chunks: weight
  * addresses never depend on activations.
- * The bytes in flight per SM are bounded by the ring (4 x 32 KB), not by
+ * The bytes in flight per SM are bounded by the ring (4 x 41 KB), not by
  * registers, which is what keeps HBM busy at 16 warps per SM.
  *
  * Arithmetic is that of the per-stage kernels (gemv.cuh, attn_body.cuh,
