@@ -22,6 +22,21 @@
 #define S2P_CTA_SYNC() __syncthreads()
 #endif
 
+/* One byte permutation, or one three-input logic operation with its truth table (a = 0xF0, b = 0xCC, c = 0xAA), as the one instruction
+ * it is.  Written with __byte_perm or with & and ^, the compiler takes a conversion's masks and constants apart and puts them
+ * together again as two or three instructions. */
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+template <int TABLE> __device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(r) : "r"(a), "r"(b), "r"(c), "n"(TABLE));
+    return r;
+}
+constexpr int LOP_AND_XOR = (0xF0 & 0xCC) ^ 0xAA; /* (a & b) ^ c */
+
 __device__ __forceinline__ float bf_bits_to_f32(uint32_t hi16) { return __uint_as_float(hi16 << 16); }
 /* the two bf16 of a 32-bit word (lower address first) */
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
@@ -31,7 +46,7 @@ __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 
  * both steps are exact, so the value equals (float)(int8_t)b. */
 __device__ __forceinline__ uint32_t s8x4_bias(uint32_t w) { return w ^ 0x80808080u; }
 template <int I> __device__ __forceinline__ float s8_biased_to_f32(uint32_t biased_word) {
-    return __fsub_rn(__uint_as_float(__byte_perm(biased_word, 0x4B000000u, 0x7440 + I)), 8388736.0f);
+    return __fsub_rn(__uint_as_float(prmt(biased_word, 0x4B000000u, 0x7440 + I)), 8388736.0f);
 }
 /* one sign-extended byte: added to the bit pattern of 2^23 + 2^22, whose mantissa absorbs either sign */
 __device__ __forceinline__ float s8_to_f32(int v) { return __fsub_rn(__int_as_float(0x4B400000 + v), 12582912.0f); }
@@ -126,6 +141,6 @@ __device__ __forceinline__ float tree256_sum(float v, float* red) {
  * by 8) to exact f32: the byte is planted in the mantissa of 2^23 and the bias
  * is removed by one exact subtraction. */
 __device__ __forceinline__ float biased_byte_to_f32(uint32_t word, int byte_idx, float magic_minus) {
-    const uint32_t bits = __byte_perm(word, 0x4B000000u, 0x7540u | (uint32_t)byte_idx);
+    const uint32_t bits = prmt(word, 0x4B000000u, 0x7540u | (uint32_t)byte_idx);
     return __uint_as_float(bits) - magic_minus;
 }

@@ -2,7 +2,7 @@
  * s2p_int8_gemv, s2p_intq_gemv, s2p_int4p_gemv — the reference's
  * src/sched/int8_gemv.cu:964-986, :773-799, :836-902.
  *
- * One row, and two of a matrix of few rows, run k_gemv_row; up to 16 rows run
+ * One and two rows, and up to four of a matrix of few rows, run k_gemv_row; up to 16 rows run
  * k_gemv_batch, where codes are widened once per tile for up to eight rows.  Every
  * row of x is an independent product with one summation order (the reference's
  * batched GEMV computes rows independently too, int8_gemv.cu:77-91).  The stage
@@ -83,6 +83,8 @@ S2P_INST(WK_INT8_GRP)
 S2P_INST(WK_INT4_PACK)
 #undef S2P_INST
 
+template <int WK> cudaError_t gemv_row_setup_kind();
+
 /* Attribute set-up for every instantiation, to be called once before any stream
  * capture (function attributes are not stream operations). */
 extern "C" cudaError_t gemv_setup_all(void) {
@@ -98,6 +100,9 @@ extern "C" cudaError_t gemv_setup_all(void) {
     S2P_SETUP_WK(WK_INT4_PACK)
 #undef S2P_SETUP_WK
 #undef S2P_SETUP
+    if (e == cudaSuccess) e = gemv_row_setup_kind<WK_INT8_CH>();
+    if (e == cudaSuccess) e = gemv_row_setup_kind<WK_INT8_GRP>();
+    if (e == cudaSuccess) e = gemv_row_setup_kind<WK_INT4_PACK>();
     return e;
 }
 
@@ -358,187 +363,337 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
 #undef S2P_GB
 }
 
-/* ---- one row, or two of a matrix of few rows ---------------------------------
- * The linear alone, as callers' own layers and one-row frames of a model on one GPU use it.
- *
- * What bounds it: instruction issue inside a wave of CTAs too short to be steady (19456 x 2560 INT4: issue slots 63 %, integer pipe
- * 57 %, fma pipe 43 % busy over the launch, DRAM 22 %).  So a few thousand warps have their weights under way at once.  A warp carries four rows (or six) as
- * packed chains (a register pair holds the same k of two rows), PD tiles at a time side by side, since every tile starts a chain of its
- * own; the next PD tiles' weights are in registers meanwhile.  Where there are too few rows for that NS = 4 warps share
- * four rows as in k_gemv_batch.
- * Measured, us (before: a CTA per SM with the tiles' sums in shared memory): INT4 6144 x 2560 10.2 -> 6.4, 2560 x 4096 8.2 -> 4.6,
- * 19456 x 2560 25.3 -> 12.9, 2560 x 9728 14.9 -> 9.7; INT8 8.5 -> 6.2, 6.8 -> 4.8, 18.9 -> 11.2, 10.7 -> 8.6. */
-template <int WK, int MM, int R, int PD, int NS, bool SW>
-__global__ void __launch_bounds__(128, MM == 2 ? 4 : R == 6 ? 6 : PD == 1 ? 8 : 4) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
-                                                     const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift) {
-    typedef typename LaneTile<WK>::type tile_t;
-    constexpr int P = R / 2;
-    __shared__ float part[NS == 1 ? 1 : 2 * PD * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][sums, then scales][row][lane] */
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int F = SW ? N >> 1 : N; /* outputs */
-    const int n0 = (blockIdx.x * (4 / NS) + warp / NS) * (SW ? R / 2 : R), ns = warp % NS;
-    if (n0 >= F) return; /* NS > 1: uniform over the CTA */
-    const size_t row_bytes = (WK == WK_INT4_PACK) ? (size_t)(K >> 1) : (size_t)K;
-    const int T = K >> 9, spr = K >> gshift;
-    const unsigned char* wrow[R];
-    const __half* srow[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) { /* rows beyond the last repeat it and are not stored */
-        const int n = gemv_row_of<SW, R>(n0, r, F);
-        wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
-        srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
+/* Codes of a lane as operands of the mixed fma (fma.rn.f32.bf16: bf16 x bf16 + f32, one rounding, the same bits as fmaf on the widened
+ * values).  STEP codes are converted together; get(w, j) is the j-th of them.  An activation needs no conversion at all: the fma
+ * takes either half of a register. */
+__device__ __forceinline__ unsigned short half_of(uint32_t v, bool high) {
+    unsigned short lo, hi;
+    asm("mov.b32 {%0, %1}, %2;" : "=h"(lo), "=h"(hi) : "r"(v));
+    return high ? hi : lo;
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) { /* two f32 adds, each rounded to bf16 */
+    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
+}
+template <int WK> struct Codes;
+template <> struct Codes<WK_INT8_CH> {
+    static constexpr int STEP = 2, WORDS = 2;
+    /* two bytes planted in the mantissa of 2^23, one packed subtraction: an f32 whose upper half is the code as bf16 */
+    static __device__ __forceinline__ void widen(const uint4& a, int k, uint32_t (&w)[WORDS]) {
+        const uint32_t u = s8x4_bias(k < 4 ? a.x : k < 8 ? a.y : k < 12 ? a.z : a.w);
+        float lo, hi;
+        unpack2(fadd2(pack2(__uint_as_float(prmt(u, 0x4B000000u, 0x7440u + (k & 3))), __uint_as_float(prmt(u, 0x4B000000u, 0x7441u + (k & 3)))),
+                      pack2(-8388736.0f, -8388736.0f)), lo, hi);
+        w[0] = __float_as_uint(lo); w[1] = __float_as_uint(hi);
     }
-    tile_t nxt[PD][R];
-    __half gnx[PD][R];
-    auto tile_of = [&](int rnd, int d) { return (rnd * NS + ns) * PD + d; };
-    auto fetch = [&](int rnd) {
+    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j], true); }
+};
+template <> struct Codes<WK_INT8_GRP> : Codes<WK_INT8_CH> {};
+template <> struct Codes<WK_INT4_PACK> {
+    static constexpr int STEP = 8, WORDS = 4;
+    /* nibbles j and j + 4 as bf16 128 + 8 + code, one packed subtraction of 136 */
+    static __device__ __forceinline__ void widen(const uint2& a, int k, uint32_t (&w)[WORDS]) {
+        const uint32_t u = k < 8 ? a.x : a.y;
 #pragma unroll
-        for (int d = 0; d < PD; d++) {
-            const int i = min(tile_of(rnd, d), T - 1);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                nxt[d][r] = __ldcs(reinterpret_cast<const tile_t*>(wrow[r] + (size_t)i * 32 * sizeof(tile_t)));
-                gnx[d][r] = WK != WK_INT8_CH ? srow[r][(i * 512 + lane * 16) >> gshift] : __half(0.f);
-            }
+        for (int j = 0; j < 4; j++) {
+            const uint32_t v = lop3<LOP_AND_XOR>(u >> (4 * j), 0x000F000Fu, 0x43084308u);
+            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(w[j]) : "r"(v), "r"(0x43084308u));
         }
-    };
-    fetch(0);
-    grid_wait();
-    grid_release();
-    float acc[MM][R];
+    }
+    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j & 3], j >= 4); }
+};
+/* the first step of a chain, which starts at zero */
+__device__ __forceinline__ float fma_bf16_first(unsigned short w, unsigned short x) {
+    float s;
+    asm("fma.rn.f32.bf16 %0, %1, %2, 0f00000000;" : "=f"(s) : "h"(w), "h"(x));
+    return s;
+}
+/* sixteen steps of the chains of R weight rows against MM activation rows: s[m][r] */
+template <int WK, int MM, int R, class X>
+__device__ __forceinline__ void lane_chains(const typename LaneTile<WK>::type (&t)[R], X x_word, float (&s)[MM][R]) {
+    typedef Codes<WK> C;
 #pragma unroll
-    for (int m = 0; m < MM; m++)
+    for (int k = 0; k < 16; k += C::STEP) {
+        uint32_t w[R][C::WORDS];
 #pragma unroll
-        for (int r = 0; r < R; r++) acc[m][r] = 0.f;
-    const int rounds = (T + NS * PD - 1) / (NS * PD);
-    for (int rnd = 0; rnd < rounds; rnd++) {
-        uint4 xv[PD][2][MM];
+        for (int r = 0; r < R; r++) C::widen(t[r], k, w[r]);
 #pragma unroll
-        for (int d = 0; d < PD; d++)
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-#pragma unroll
-                for (int m = 0; m < MM; m++) xv[d][h][m] = *reinterpret_cast<const uint4*>(x + (size_t)m * K + min(tile_of(rnd, d), T - 1) * 512 + lane * 16 + h * 8);
-        tile_t cur[PD][R];
-        float gs[PD][R];
-#pragma unroll
-        for (int d = 0; d < PD; d++)
-#pragma unroll
-            for (int r = 0; r < R; r++) { cur[d][r] = nxt[d][r]; gs[d][r] = __half2float(gnx[d][r]); }
-        if (rnd + 1 < rounds) fetch(rnd + 1);
-        f32x2 s[PD][MM][P];
-#pragma unroll
-        for (int d = 0; d < PD; d++)
-#pragma unroll
-            for (int m = 0; m < MM; m++)
-#pragma unroll
-                for (int q = 0; q < P; q++) s[d][m][q] = 0ull;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            f32x2 wf[PD][P][8];
-#pragma unroll
-            for (int d = 0; d < PD; d++)
-#pragma unroll
-                for (int q = 0; q < P; q++) BatchCodes<WK>::widen8(cur[d][2 * q], cur[d][2 * q + 1], h, wf[d][q]);
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-#pragma unroll
-                for (int d = 0; d < PD; d++) {
-#pragma unroll
-                    for (int m = 0; m < MM; m++) {
-                        const uint4& v = xv[d][h][m];
-                        const uint32_t u = (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w;
-                        const float xf = j & 1 ? bf_hi(u) : bf_lo(u);
-                        const f32x2 xx = pack2(xf, xf);
-#pragma unroll
-                        for (int q = 0; q < P; q++) ffma2(s[d][m][q], wf[d][q][j], xx);
-                    }
-                }
-        }
-        auto fold = [&](int m, int r, float v, float g) { acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + v : __fmaf_rn(v, g, acc[m][r]); };
-#pragma unroll
-        for (int d = 0; d < PD; d++) {
-            if (tile_of(rnd, d) >= T) continue;
-            float* at = part + (((rnd & 1) * NS + ns) * PD + d) * ((MM + 1) * R * 32) + lane;
+        for (int j = 0; j < C::STEP; j++)
 #pragma unroll
             for (int m = 0; m < MM; m++) {
-                float v[R];
+                const unsigned short xv = half_of(x_word(m, (k + j) >> 1), j & 1);
 #pragma unroll
-                for (int q = 0; q < P; q++) unpack2(s[d][m][q], v[2 * q], v[2 * q + 1]);
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    if (NS == 1) fold(m, r, v[r], gs[d][r]);
-                    else at[(m * R + r) * 32] = v[r];
-                }
+                for (int r = 0; r < R; r++) s[m][r] = k + j == 0 ? fma_bf16_first(C::get(w[r], j), xv) : fma_bf16(C::get(w[r], j), xv, s[m][r]);
             }
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                if (NS > 1) at[(MM * R + r) * 32] = gs[d][r];
-        }
-        if (NS > 1) { /* the round's tiles in ascending order; warp ns keeps row ns */
-            __syncthreads();
-            const int live = min(NS * PD, T - rnd * NS * PD);
-            const float* at = part + (rnd & 1) * NS * PD * ((MM + 1) * R * 32) + ns * 32 + lane;
-            for (int t = 0; t < live; t++, at += (MM + 1) * R * 32)
-#pragma unroll
-                for (int m = 0; m < MM; m++) fold(m, 0, at[m * R * 32], at[MM * R * 32]);
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < MM; m++, y += F) {
-    if (R != 4) { /* every lane has every sum */
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            acc[m][r] = warp_tree_sum(acc[m][r]);
-            if (WK == WK_INT8_CH) acc[m][r] = __fmul_rn(acc[m][r], static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
-        }
-#pragma unroll
-        for (int r = 0; r < (SW ? P : R); r++) {
-            const float a = SW ? gemv_swiglu(acc[m][r], acc[m][r + (SW ? P : 0)]) : acc[m][r];
-            if (lane == r && n0 + r < F) y[n0 + r] = f2bf(a);
-        }
-    } else if (NS == 1) {
-        /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
-        const int r = lane >> 3, n = n0 + r;
-        float a = warp_tree4<false>(acc[m][0], acc[m][1], acc[m][2], acc[m][3], lane);
-        if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)]);
-        if (SW) a = gemv_swiglu(a, __shfl_down_sync(S2P_FULL_MASK, a, 16));
-        if ((lane & 7) == 0 && n < F && r < (SW ? R / 2 : R)) y[n] = f2bf(a);
-    } else {
-        float a = warp_tree_sum(acc[m][0]);
-        if (n0 + ns < N && lane == 0) {
-            if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[n0 + ns]);
-            y[n0 + ns] = f2bf(a);
-        }
-    }
     }
 }
 
-/* Four warps share four rows where one each would give a scheduler less than 1.5, if most of their turns have a tile
- * (2560 x 9728: 14.0 -> 9.7 us, 6144 x 2560 the other way round 6.4 -> 7.7). */
-static bool gemv_row_shared(int N, int K) { return 2 * ((N + 3) / 4) < 3 * 4 * device_sm_count() && K > 4 * 512; }
+/* ---- one and two rows; up to four of a matrix of few rows --------------------------
+ * The linear alone, as callers' own layers and small ticks of a model on one GPU use it.
+ *
+ * A CTA per SM owns a contiguous block of rows.  Its work is cut into units of four rows x one K tile, tile-major, and a warp takes a
+ * contiguous run of units: its activations stay in registers, its weights have no order to wait for (all units are independent chains),
+ * so D units of them are under way, the first before the kernel in front has ended.  Lane sums go to shared memory, [tile][unit][row][lane];
+ * after one CTA barrier a warp folds four rows, tiles ascending, with scales that came to shared memory meanwhile.  So a matrix of 2560
+ * rows occupies every warp whatever its K, and no warp of a large one has more than its share.
+ *
+ * What bounds it: about 3 us of fixed cost per launch (the wait, the first activations, barrier, fold), then the issue of conversions and
+ * chains: 3.3 cycles per weight and scheduler for INT4, 4.1 for INT8 in a loop of nothing else, which is 4.5 us for 19456 x 2560 INT4
+ * (its bytes take 4.3).  The mixed fma runs at the rate of fmaf and reads either half of its registers, so an activation costs nothing and
+ * an INT4 pair one logic operation, one shift and one subtraction; packed f32 chains needed a conversion of either side.
+ * Measured, us, launches of one matrix back to back in a graph, before (k packed over two rows of weights, warps of four rows, four warps to
+ * a row's tiles where rows are few) and now:
+ *             6144 x 2560    2560 x 4096    19456 x 2560   2560 x 9728
+ *   INT4 1    7.6 -> 4.4     3.8 -> 3.9     13.1 -> 9.5    9.0 -> 6.2
+ *   INT4 2    7.5 -> 6.1     5.0 -> 5.1     15.6 -> 13.5   12.3 -> 8.2
+ *   INT8 1    6.6 -> 5.3     4.1 -> 4.7     10.1 -> 11.1   8.8 -> 7.1
+ *   INT8 2    8.2 -> 7.1     5.8 -> 6.1     13.8 -> 14.8   12.5 -> 9.1
+ *   INT4 3                   7.3 -> 5.9                    16.8 -> 10.0        (INT8 8.2 -> 6.3, 15.8 -> 10.2)
+ *   INT4 4                   7.1 -> 6.9                    16.8 -> 14.9        (INT8 8.8 -> 7.3, 16.7 -> 11.7)
+ * At 64 registers, two CTAs to an SM, the frame took 3.67 ms instead of 2.68; 24 warps of 80 registers and other depths were within 1 %.
+ *
+ * NORM: the residual add and the norm in front of the linear, taken by every CTA while its first weights are on their way, instead of a
+ * launch of k_norm_row: frame of one row 2.67 -> 2.52 ms INT4, 2.97 -> 2.79 INT8. */
+template <int WK, int MM> struct RowPlan {
+    static constexpr int WARPS = 16, R = 4;
+    static constexpr int D = WK == WK_INT4_PACK ? 4 : MM <= 2 ? 3 : 2; /* units of weights under way in a warp */
+    static constexpr bool XN = MM <= 2;                                  /* the next tile's activations too */
+    static constexpr size_t LIMIT = 200 * 1024;
+    static constexpr int NORM_K = 8 * WARPS * 32; /* longest activation whose norm the kernel takes itself: a vector of eight per thread */
+    static size_t norm_smem(int K) { return (size_t)MM * (K * 2 + 257 * sizeof(float)); }
+    static size_t smem(int outputs, int K, int gshift, bool sw) {
+        const int rows_a = sw ? 2 : 4, units = (outputs + rows_a - 1) / rows_a, T = K / 512;
+        return (size_t)MM * units * R * T * 32 * sizeof(float) + (WK == WK_INT8_CH ? 0 : ((size_t)units * R * (K >> gshift) * 2 + 15) & ~(size_t)15);
+    }
+    /* CTAs: one per SM, or as many per SM as keep the sums in shared memory; 0 where four rows do not fit, or offsets would not fit 32 bits */
+    static int grid(int F, int K, int gshift, bool sw, int sms) {
+        if (smem(1, K, gshift, sw) > LIMIT || (size_t)F * (sw ? 2 : 1) * K > 0xF0000000ull) return 0;
+        int g = sms;
+        while (smem((F + g - 1) / g, K, gshift, sw) > LIMIT) g += sms;
+        return g < F ? g : F;
+    }
+};
+template <int WK, int MM, bool SW, bool NORM>
+__global__ void __launch_bounds__(RowPlan<WK, MM>::WARPS * 32, 1) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x, NormIn nm,
+                                                                            const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift) {
+    typedef typename LaneTile<WK>::type tile_t;
+    constexpr int R = 4, RA = SW ? 2 : 4, W = RowPlan<WK, MM>::WARPS, D = RowPlan<WK, MM>::D; /* RA: rows of a unit that follow one another */
+    constexpr bool XN = RowPlan<WK, MM>::XN;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int T = K >> 9, spr = K >> gshift;
+    const unsigned row_bytes = WK == WK_INT4_PACK ? (unsigned)(K >> 1) : (unsigned)K;
+    const int F = SW ? N >> 1 : N; /* outputs */
+    const int o0 = (int)((long long)F * blockIdx.x / gridDim.x), outs = (int)((long long)F * (blockIdx.x + 1) / gridDim.x) - o0;
+    const int per_tile = (outs + RA - 1) / RA, units = per_tile * T;
+    float* sums = reinterpret_cast<float*>(smem);                          /* [m][tile][unit of the tile][row][lane] */
+    __half* ssc = reinterpret_cast<__half*>(sums + (size_t)MM * units * R * 32); /* [row (SW: gates, then ups)][spr] */
+    if (WK != WK_INT8_CH) {
+#pragma unroll
+        for (int part = 0; part < R / RA; part++) {
+            const __half* src = static_cast<const __half*>(scales) + (size_t)(o0 + part * F) * spr;
+            __half* dst = ssc + part * per_tile * RA * spr;
+            const int n = outs * spr;
+            if ((((uintptr_t)src | (uintptr_t)dst | (unsigned)(n * 2)) & 15) == 0) {
+                for (int c = threadIdx.x * 8; c < n; c += W * 32 * 8)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + c)), "l"(src + c) : "memory");
+            } else {
+                for (int c = threadIdx.x; c < n; c += W * 32) dst[c] = src[c];
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int u0 = (int)((long long)units * warp / W);
+    const int n_units = (int)((long long)units * (warp + 1) / W) - u0;
+    int t = u0 / per_tile, ru = u0 - t * per_tile;
+    /* 32-bit offsets from the block's first row */
+    const unsigned char* wb = static_cast<const unsigned char*>(w) + (size_t)o0 * row_bytes;
+    constexpr unsigned TILE = 32 * sizeof(tile_t);
+    unsigned at_row[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) at_row[r] = (r % RA) * row_bytes + (r / RA) * F * row_bytes;
+    int lu = ru, left = n_units; /* where the loads are */
+    unsigned at_tile = t * TILE + lane * (unsigned)sizeof(tile_t), at = at_tile + ru * RA * row_bytes;
+    tile_t q[D][R];
+    auto load = [&](int d) {
+        if (left <= 0) return;
+        left--;
+        if ((lu + 1) * RA <= outs) {
+#pragma unroll
+            for (int r = 0; r < R; r++) q[d][r] = __ldcs(reinterpret_cast<const tile_t*>(wb + (at + at_row[r])));
+        } else { /* rows beyond the last repeat it and are not stored */
+            const int last = outs - 1 - lu * RA;
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                q[d][r] = __ldcs(reinterpret_cast<const tile_t*>(wb + (at + min(r % RA, last) * row_bytes + (r / RA) * F * row_bytes)));
+        }
+        at += RA * row_bytes;
+        if (++lu == per_tile) { lu = 0; at = at_tile += TILE; }
+    };
+#pragma unroll
+    for (int d = 0; d < D; d++) load(d);
+    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem + nm.at); /* NORM: the normalised rows */
+    uint4 gain = make_uint4(0, 0, 0, 0);
+    const int v = threadIdx.x, nv = K >> 3;
+    if (NORM && v < nv) gain = reinterpret_cast<const uint4*>(nm.gain)[v];
+    grid_wait();
+    grid_release();
+    if (NORM) { /* k_norm_row's pairs and roundings (prims.cu), in every CTA; the first one keeps the sum */
+        static_assert(!NORM || MM <= 2, "256 threads a row");
+        float* red = reinterpret_cast<float*>(xs + MM * K);
+        uint4 q[MM];
+#pragma unroll
+        for (int m = 0; m < MM; m++) {
+            if (v >= nv) continue;
+            q[m] = reinterpret_cast<const uint4*>(nm.src + (size_t)m * K)[v];
+            const uint4 a = reinterpret_cast<const uint4*>(nm.add + (size_t)m * K)[v];
+            q[m] = make_uint4(add_bf16x2(q[m].x, a.x), add_bf16x2(q[m].y, a.y), add_bf16x2(q[m].z, a.z), add_bf16x2(q[m].w, a.w));
+            reinterpret_cast<uint4*>(xs + (size_t)m * K)[v] = q[m];
+            if (blockIdx.x == 0) reinterpret_cast<uint4*>(nm.x_out + (size_t)m * K)[v] = q[m];
+        }
+        __syncthreads();
+        const int mine = threadIdx.x >> 8, i0 = threadIdx.x & 255;
+        float* r = red + mine * 257;
+        if (mine < MM) {
+            float ss = 0.f;
+            for (int i = i0; i < K; i += 256) {
+                const float e = bf2f(xs[(size_t)mine * K + i]);
+                ss = __fmaf_rn(e, e, ss);
+            }
+            r[i0] = ss;
+        }
+        __syncthreads();
+        if (mine < MM && i0 < 32) { /* tree256_sum: the pairs of the levels 128, 64 and 32, then shuffles */
+            const float a0 = r[i0] + r[i0 + 128], a1 = r[i0 + 32] + r[i0 + 160], a2 = r[i0 + 64] + r[i0 + 192], a3 = r[i0 + 96] + r[i0 + 224];
+            const float tot = warp_tree_sum((a0 + a2) + (a1 + a3));
+            if (i0 == 0) r[256] = tot;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < MM; m++)
+            if (v < nv) reinterpret_cast<uint4*>(xs + (size_t)m * K)[v] = norm_vec8(q[m], gain, rsqrtf(__fdiv_rn(red[m * 257 + 256], (float)K) + nm.eps));
+        __syncthreads();
+    }
+    uint4 xv[MM][2], xn[MM][2];
+    const __nv_bfloat16* xp = (NORM ? xs : x) + (size_t)min(t, T - 1) * 512 + lane * 16;
+    auto load_x = [&](uint4 (&v)[MM][2]) {
+#pragma unroll
+        for (int m = 0; m < MM; m++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) v[m][h] = *reinterpret_cast<const uint4*>(xp + (size_t)m * K + h * 8);
+    };
+    load_x(xv);
+    if (XN) {
+        if (t + 1 < T) xp += 512;
+        load_x(xn);
+    }
+    float* sp = sums + u0 * (R * 32) + lane;
+    const int plane = units * R * 32;
+#pragma unroll 1
+    for (int n = n_units; n > 0; n -= D)
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            if (d && d >= n) break;
+            float s[MM][R];
+            lane_chains<WK, MM, R>(q[d], [&](int m, int i2) {
+                const uint4& v = xv[m][i2 >> 2];
+                return (i2 & 3) == 0 ? v.x : (i2 & 3) == 1 ? v.y : (i2 & 3) == 2 ? v.z : v.w;
+            }, s);
+            load(d);
+#pragma unroll
+            for (int m = 0; m < MM; m++)
+#pragma unroll
+                for (int r = 0; r < R; r++) sp[m * plane + r * 32] = s[m][r];
+            sp += R * 32;
+            if (++ru == per_tile) {
+                ru = 0; t++;
+                if (XN) {
+#pragma unroll
+                    for (int m = 0; m < MM; m++) { xv[m][0] = xn[m][0]; xv[m][1] = xn[m][1]; }
+                }
+                if (t + (XN ? 1 : 0) < T) {
+                    xp += 512;
+                    if (XN) load_x(xn); else load_x(xv);
+                }
+            }
+        }
+    if (WK != WK_INT8_CH) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int g = warp; g < per_tile * MM; g += W) {
+        const int m = MM == 1 ? 0 : g / per_tile, u = MM == 1 ? g : g - m * per_tile;
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = 0.f;
+        const float* at = sums + (size_t)(m * units + u) * (R * 32) + lane;
+        const __half* sc = ssc + u * RA * spr + ((lane * 16) >> gshift);
+#pragma unroll 2
+        for (int i = 0; i < T; i++, at += per_tile * (R * 32), sc += 512 >> gshift)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const float v = at[r * 32];
+                acc[r] = WK == WK_INT8_CH ? acc[r] + v : __fmaf_rn(v, __half2float(sc[(r % RA) * spr + r / RA * per_tile * RA * spr]), acc[r]);
+            }
+        /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
+        const int r = lane >> 3, o = u * RA + r % RA;
+        float a = warp_tree4<false>(acc[0], acc[1], acc[2], acc[3], lane);
+        if (WK == WK_INT8_CH) a = __fmul_rn(a, static_cast<const float*>(scales)[o0 + min(o, outs - 1) + r / RA * F]);
+        if (SW) a = gemv_swiglu(a, __shfl_down_sync(S2P_FULL_MASK, a, 16));
+        if ((lane & 7) == 0 && r < RA && o < outs) y[(size_t)m * F + o0 + o] = f2bf(a);
+    }
+}
+template <int WK, int MM, bool SW, bool NORM>
+static cudaError_t gemv_row_setup() {
+    static int done_mask = 0; /* bit per device ordinal */
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (done_mask & (1 << (dev & 31))) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(k_gemv_row<WK, MM, SW, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(RowPlan<WK, MM>::LIMIT + (NORM ? RowPlan<WK, MM>::norm_smem(RowPlan<WK, MM>::NORM_K) : 0)));
+    if (e == cudaSuccess) done_mask |= 1 << (dev & 31);
+    return e;
+}
+template <int WK> cudaError_t gemv_row_setup_kind() {
+    const cudaError_t e[] = {gemv_row_setup<WK, 1, false, false>(), gemv_row_setup<WK, 2, false, false>(), gemv_row_setup<WK, 3, false, false>(),
+                             gemv_row_setup<WK, 4, false, false>(), gemv_row_setup<WK, 1, true, false>(), gemv_row_setup<WK, 2, true, false>(),
+                             gemv_row_setup<WK, 3, true, false>(), gemv_row_setup<WK, 4, true, false>(), gemv_row_setup<WK, 1, false, true>(),
+                             gemv_row_setup<WK, 2, false, true>(), gemv_row_setup<WK, 1, true, true>(), gemv_row_setup<WK, 2, true, true>()};
+    for (cudaError_t c : e)
+        if (c != cudaSuccess) return c;
+    return cudaSuccess;
+}
+template <int WK, int MM, bool SW, bool NORM = false>
+static cudaError_t run_gemv_row(int grid, void* y, const void* x, const NormIn* norm, const void* w, const void* scales, int N, int K, int gshift, int early, cudaStream_t stream) {
+    typedef RowPlan<WK, MM> Plan;
+    const cudaError_t e = gemv_row_setup<WK, MM, SW, NORM>();
+    if (e != cudaSuccess) return e;
+    const int F = SW ? N >> 1 : N;
+    size_t smem = Plan::smem((F + grid - 1) / grid, K, gshift, SW);
+    NormIn nm = {};
+    if (NORM) {
+        nm = *norm;
+        nm.at = (unsigned)smem;
+        smem += Plan::norm_smem(K);
+    }
+    return launch_early(early, k_gemv_row<WK, MM, SW, NORM>, dim3((unsigned)grid), Plan::WARPS * 32, smem, stream,
+                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, nm, w, scales, N, K, gshift);
+}
+/* The CTAs of k_gemv_row for M rows, 0 where k_gemv_batch takes them.  Three and four rows only where the batch kernel would leave a
+ * scheduler fewer than two warps: 3 / 4 rows INT4 of 2560 x 9728 10.0 / 14.9 us (batch 15.3 / 16.5), but 7.4 / 8.4 (6.6 / 7.2) of 6144 x 2560
+ * and 19.6 / 23.2 (16.9 / 18.4) of 19456 x 2560, whose sums need two CTAs to an SM. */
+template <int WK, bool SW> static int gemv_row_grid(int M, int N, int K, int gshift) {
+    const int F = SW ? N >> 1 : N, sms = device_sm_count();
+    if (M > 4 || (M > 2 && (N + 3) / 4 >= 2 * 4 * sms)) return 0;
+    return M == 1 ? RowPlan<WK, 1>::grid(F, K, gshift, SW, sms) : M == 2 ? RowPlan<WK, 2>::grid(F, K, gshift, SW, sms)
+         : M == 3 ? RowPlan<WK, 3>::grid(F, K, gshift, SW, sms) : RowPlan<WK, 4>::grid(F, K, gshift, SW, sms);
+}
 template <int WK, bool SW>
-static cudaError_t launch_gemv_row(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
-    /* From six warps per scheduler on a tile at a time with twice the warps resident hides more than two tiles side by side (19456
-     * rows INT8 12.5 -> 11.2 us).  There packed INT4, whose tiles are half the loads, takes six rows a warp where the warps of four do
-     * not fit the GPU at once (8 CTAs of 4 x 4 rows to an SM; of six 6 CTAs, so 144 rows instead of 128).  K = 2560, us with six /
-     * four rows: one wave of either 14208 rows 12.2 / 10.9, 18944 13.3 / 11.6; beyond it 21312 13.3 / 13.9, 24576 13.9 / 15.0,
-     * 28416 17.0 / 16.7, 38912 20.3 / 21.5, 155776 70.5 / 73.1.  (19456 rows: 13.4 / 13.1 in a chain of early launches, 12.9 / 13.5
-     * launched the ordinary way.) */
-    const int sms = device_sm_count();
-    const bool shared = !SW && gemv_row_shared(N, K), many = (N + 3) / 4 >= 6 * 4 * sms;
-    const bool six = WK == WK_INT4_PACK && N > 8 * 4 * 4 * sms;
-    void (*kernel)(__nv_bfloat16*, const __nv_bfloat16*, const void*, const void*, int, int, int) =
-        many ? k_gemv_row<WK, 1, 4, 1, 1, SW> : k_gemv_row<WK, 1, 4, 2, 1, SW>;
-    if constexpr (WK == WK_INT4_PACK) {
-        if (six) kernel = k_gemv_row<WK, 1, 6, 1, 1, SW>;
+static cudaError_t launch_gemv_row(int grid, void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
+    switch (M) {
+    case 1: return run_gemv_row<WK, 1, SW>(grid, y, x, nullptr, w, scales, N, K, gshift, early, stream);
+    case 2: return run_gemv_row<WK, 2, SW>(grid, y, x, nullptr, w, scales, N, K, gshift, early, stream);
+    case 3: return run_gemv_row<WK, 3, SW>(grid, y, x, nullptr, w, scales, N, K, gshift, early, stream);
+    case 4: return run_gemv_row<WK, 4, SW>(grid, y, x, nullptr, w, scales, N, K, gshift, early, stream);
     }
-    if constexpr (!SW) {
-        if (shared) kernel = M == 2 ? k_gemv_row<WK, 2, 4, 2, 4, false> : k_gemv_row<WK, 1, 4, 2, 4, false>;
-    }
-    const int per_warp = six ? 6 : 4, warps = (N + per_warp - 1) / per_warp;
-    return launch_early(early, kernel, dim3((unsigned)(shared ? warps : (warps + 3) / 4)), 128, 0, stream,
-                       (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, N, K, gshift);
+    return cudaErrorInvalidValue;
 }
 
 int gshift_of(int G) {
@@ -548,14 +703,23 @@ int gshift_of(int G) {
     return s;
 }
 
+/* the same with the add and the norm in front of it in the kernel, one or two rows */
+template <int WK, bool SW> static cudaError_t launch_gemv_row_norm(const LinRef* lin, const NormIn* norm, void* y, int M, cudaStream_t stream) {
+    const int grid = gemv_row_grid<WK, SW>(M, lin->N, lin->K, lin->gshift);
+    if (!grid || M > 2 || lin->K > RowPlan<WK, 1>::NORM_K) return cudaErrorInvalidValue;
+    return M == 1 ? run_gemv_row<WK, 1, SW, true>(grid, y, nullptr, norm, lin->w, lin->scales, lin->N, lin->K, lin->gshift, 1, stream)
+                  : run_gemv_row<WK, 2, SW, true>(grid, y, nullptr, norm, lin->w, lin->scales, lin->N, lin->K, lin->gshift, 1, stream);
+}
+
 template <int WK, bool SW = false>
 s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, const void* scales, int M, int N,
                       int K, int gshift, int early, cudaStream_t stream) {
     /* 16-byte loads of activations and weight tiles */
     if (((uintptr_t)x | (uintptr_t)w) & 15) return S2P_ERR_INVALID;
     cudaError_t ce;
-    if (M == 1 || (M == 2 && !SW && gemv_row_shared(N, K))) { /* two rows where rows are few: 2560 x 4096 INT4 7.6 -> 5.9 us, x 9728 16.0 -> 13.1 */
-        ce = launch_gemv_row<WK, SW>(y, x, w, scales, M, N, K, gshift, early, stream);
+    const int grid = gemv_row_grid<WK, SW>(M, N, K, gshift);
+    if (grid) {
+        ce = launch_gemv_row<WK, SW>(grid, y, x, w, scales, M, N, K, gshift, early, stream);
     } else {
         ce = launch_gemv_batch<WK, SW>(y, x, w, scales, M, N, K, gshift, early, stream);
     }
@@ -581,6 +745,23 @@ static s2p_status gemv_rows_of(const LinRef* lin, const void* x, void* y, int M,
     case WK_INT4_PACK: return gemv_entry<WK_INT4_PACK, SW>("int4p gemv", y, x, lin->w, lin->scales, M, lin->N, lin->K, lin->gshift, early, stream);
     }
     return S2P_ERR_INVALID;
+}
+extern "C" int gemv_norm_serves(const LinRef* lin, int swiglu, int M) {
+    if (!lin || M < 1 || M > 2 || lin->K % 512 || lin->K > RowPlan<WK_INT8_CH, 1>::NORM_K) return 0;
+    switch (lin->kind) {
+    case WK_INT8_CH: return (swiglu ? gemv_row_grid<WK_INT8_CH, true>(M, lin->N, lin->K, 0) : gemv_row_grid<WK_INT8_CH, false>(M, lin->N, lin->K, 0)) != 0;
+    case WK_INT8_GRP: return (swiglu ? gemv_row_grid<WK_INT8_GRP, true>(M, lin->N, lin->K, lin->gshift) : gemv_row_grid<WK_INT8_GRP, false>(M, lin->N, lin->K, lin->gshift)) != 0;
+    case WK_INT4_PACK: return (swiglu ? gemv_row_grid<WK_INT4_PACK, true>(M, lin->N, lin->K, lin->gshift) : gemv_row_grid<WK_INT4_PACK, false>(M, lin->N, lin->K, lin->gshift)) != 0;
+    }
+    return 0;
+}
+extern "C" cudaError_t gemv_rows_norm(const LinRef* lin, const NormIn* norm, void* y, int swiglu, int M, cudaStream_t stream) {
+    if (!gemv_norm_serves(lin, swiglu, M) || !norm || norm->src == norm->x_out) return cudaErrorInvalidValue;
+    switch (lin->kind) {
+    case WK_INT8_CH: return swiglu ? launch_gemv_row_norm<WK_INT8_CH, true>(lin, norm, y, M, stream) : launch_gemv_row_norm<WK_INT8_CH, false>(lin, norm, y, M, stream);
+    case WK_INT8_GRP: return swiglu ? launch_gemv_row_norm<WK_INT8_GRP, true>(lin, norm, y, M, stream) : launch_gemv_row_norm<WK_INT8_GRP, false>(lin, norm, y, M, stream);
+    default: return swiglu ? launch_gemv_row_norm<WK_INT4_PACK, true>(lin, norm, y, M, stream) : launch_gemv_row_norm<WK_INT4_PACK, false>(lin, norm, y, M, stream);
+    }
 }
 extern "C" int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t stream) { return gemv_rows_of<false>(lin, x, y, M, early, stream); }
 extern "C" int gemv_rows_swiglu(const LinRef* lin, const void* x, void* h, int M, cudaStream_t stream) { return gemv_rows_of<true>(lin, x, h, M, 1, stream); }

@@ -144,6 +144,16 @@ int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaS
  * 8.39 -> 8.42, 16 rows 12.9 -> 13.2). */
 #define GEMV_SWIGLU_ROWS 4
 int gemv_rows_swiglu(const LinRef* lin, const void* x, void* h, int M, cudaStream_t st);
+/* The linear of norm(src + add) for one or two rows, the sum and the norm taken by the kernel itself (a launch less, in a chain where
+ * each costs two microseconds).  The sum goes to x_out, which no CTA may still be reading: not src.  `swiglu`: as gemv_rows_swiglu. */
+typedef struct {
+    const s2p_dev_bf16 *src, *add, *gain; /* [M, K], [M, K], [K]; the gains are a model's: read before the kernel in front has ended */
+    s2p_dev_bf16* x_out;                  /* [M, K] */
+    float eps;
+    unsigned at;                          /* (filled by the launcher) */
+} NormIn;
+int gemv_norm_serves(const LinRef* lin, int swiglu, int M);
+cudaError_t gemv_rows_norm(const LinRef* lin, const NormIn* norm, void* y, int swiglu, int M, cudaStream_t st);
 
 /* batched decode linear on the tensor cores (skinny.cu): y[M, N] = x[M, K] · W^T, 1 <= M <= 256 */
 cudaError_t skinny_gemm_tc(const LinRef* lin, const void* x, int M, void* y, const void* resid, cudaStream_t st);
@@ -319,6 +329,8 @@ cudaError_t scale_div(void* x, int64_t n, float divisor, cudaStream_t st);
 cudaError_t scale_rows_masked(void* x, const uint8_t* mask, int rows, int dim, float scale, cudaStream_t st);
 /* rows of the model width, all 16-byte aligned: x += add, then y = norm(x) with gain w (w NULL: no norm) */
 cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st);
+/* the same with the sum in another place than src */
+cudaError_t add_norm_to(const void* src, const void* add, void* x, const void* w, void* y, int rows, cudaStream_t st);
 /* The same around wide_gemm.  `part` with `alt` is its output: the partials, or alt where it wrote that.
  * x = src (+ the output, if part is given); or, with a table, its row `codes[r]`, or the one that the arg-max of the output
  * selects (to codes_out).  y = norm(x) with gain w (NULL: none), as bf16 and / or as the units of a linear of kind `kind`. */

@@ -734,11 +734,12 @@ cudaError_t rms_norm(const void* x, const void* w, void* y, int rows, int width,
     k_rms_norm<<<rows, 256, 0, st>>>(a.src, a.w, a.y, width, eps);
     return cudaGetLastError();
 }
-cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st) {
+cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st) { return add_norm_to(x, add, x, w, y, rows, st); }
+cudaError_t add_norm_to(const void* src, const void* add, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     NormRowArgs a = {};
     a.settled = 1;
-    a.src = (const __nv_bfloat16*)x; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
+    a.src = (const __nv_bfloat16*)src; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
     return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
 }

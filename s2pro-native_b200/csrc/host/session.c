@@ -329,6 +329,56 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
     return S2P_OK;
 }
 
+/* One or two decoding rows: the adds and norms between the linears are the linears' own.  The residual stream alternates between two
+ * buffers, because every CTA of a linear forms the sum that one of them writes. */
+typedef struct {
+    s2p_dev_bf16 *x, *other; /* the stream, and where its next sum goes */
+    int pending;             /* a projection is still to be added to it */
+} residual;
+
+static int layers_fold_norms(const s2p_model* m, const s2p_layer* layers, int n, int rows) {
+    if (m->mode != S2P_GEMM_INT8) return 0;
+    for (int l = 0; l < n; l++) {
+        const s2p_layer* L = &layers[l];
+        LinRef qkv, gu;
+        if (!L->wqkv.int8_ready || !L->gate_up.int8_ready || L->gate_up.out_features != 2 * S2P_FFN_DIM || s2p_linear_rows_on_tc(&L->wqkv, rows)) return 0;
+        s2p_lin_ref(&L->wqkv, &qkv);
+        s2p_lin_ref(&L->gate_up, &gu);
+        if (!gemv_norm_serves(&qkv, 0, rows) || !gemv_norm_serves(&gu, 1, rows)) return 0;
+    }
+    return 1;
+}
+
+static s2p_status linear_of_norm(s2p_model* m, const s2p_linear* lin, residual* r, const void* proj, const void* gain, void* y, int swiglu, int rows) {
+    LinRef lr;
+    s2p_lin_ref(lin, &lr);
+    NormIn in;
+    memset(&in, 0, sizeof(in));
+    in.src = r->x; in.add = (const s2p_dev_bf16*)proj; in.gain = (const s2p_dev_bf16*)gain; in.x_out = r->other; in.eps = S2P_NORM_EPS;
+    S2P_LAUNCH(m, gemv_rows_norm(&lr, &in, y, swiglu, rows, m->stream));
+    s2p_dev_bf16* t = r->x;
+    r->x = r->other; r->other = t;
+    return S2P_OK;
+}
+
+/* On entry either a projection is pending in proj or `norm` holds the norm of the stream with the layer's first gain; on exit a
+ * projection is pending. */
+static s2p_status layer_few_rows(s2p_model* m, const s2p_layer* L, const layer_ctx* c, residual* r, s2p_dev_bf16* norm, s2p_dev_bf16* qkv,
+                                 s2p_dev_bf16* q, s2p_dev_bf16* attn, s2p_dev_bf16* proj, s2p_dev_bf16* hff) {
+    if (r->pending) S2P_TRY(linear_of_norm(m, &L->wqkv, r, proj, L->attn_norm.data, qkv, 0, c->rows));
+    else S2P_TRY(lin_apply(m, &L->wqkv, NULL, norm, qkv, c->rows, 1));
+    S2P_TRY(layer_attention(m, L, c, qkv, NULL, q, attn));
+    S2P_TRY(lin_apply(m, &L->wo, NULL, attn, proj, c->rows, 1));
+    S2P_TRY(linear_of_norm(m, &L->gate_up, r, proj, L->ffn_norm.data, hff, 1, c->rows));
+    r->pending = 1;
+    return lin_apply(m, &L->w2, NULL, hff, proj, c->rows, 1);
+}
+/* the last sum, into the stream's first buffer, and its norm (gain NULL: none) */
+static s2p_status residual_close(s2p_model* m, residual* r, s2p_dev_bf16* x, const void* proj, const void* gain, void* out, int rows) {
+    S2P_LAUNCH(m, add_norm_to(r->x, proj, x, gain, out, rows, m->stream));
+    return S2P_OK;
+}
+
 /* A decode layer of a batch on the tensor cores with resident f16 tiles: the activations between the linears travel as matrix
  * units, and outputs whose K range was split are added by the kernel that consumes them.  On entry m->xt_norm holds the norm of x
  * with the layer's first gain; on exit, unless next is NULL, the norm with the gain `next`, as units of a linear of kind
@@ -664,10 +714,17 @@ static s2p_status fast_frame_general(s2p_model* m, const tick_dev* d, int nact, 
     layer_ctx c;
     memset(&c, 0, sizeof(c));
     c.rows = nact; c.max_seq = S2P_FAST_SEQ; c.kv8 = 0; c.pos_row_step = 0; c.decode = 1; c.split_k = 0;
+    const int fold = layers_fold_norms(m, m->fast, S2P_FAST_LAYERS, nact);
     S2P_LAUNCH(m, copy_norm(m->shidden.data, m->fx.data, m->fast[0].attn_norm.data, m->ft.data, nact, st));
     for (int cb = 0; cb < S2P_NUM_CODEBOOKS; cb++) {
         c.pos0 = cb;
-        for (int l = 0; l < S2P_FAST_LAYERS; l++) {
+        residual r = {BF(m->fx), BF(m->fgu), 0};
+        for (int l = 0; fold && l < S2P_FAST_LAYERS; l++) {
+            fast_kv_ref(m, l, &c.kv);
+            S2P_TRY(layer_few_rows(m, &m->fast[l], &c, &r, BF(m->ft), BF(m->fqkv), BF(m->fq), BF(m->fattn), BF(m->fproj), BF(m->fhff)));
+        }
+        if (fold) S2P_TRY(residual_close(m, &r, BF(m->fx), m->fproj.data, cb ? m->fast_norm.data : NULL, m->ft.data, nact));
+        for (int l = 0; !fold && l < S2P_FAST_LAYERS; l++) {
             fast_kv_ref(m, l, &c.kv);
             S2P_TRY(layer_general(m, &m->fast[l], &c, BF(m->fx), BF(m->ft), BF(m->fqkv), BF(m->fq), BF(m->fattn),
                                   BF(m->fproj), BF(m->fgu), BF(m->fhff),
@@ -714,7 +771,14 @@ static s2p_status tick_general(s2p_model* m, s2p_session* const* act, int bd, in
         s2p_lin_ref(&m->slow[0].wqkv, &lr);
         if (wide) S2P_LAUNCH(m, wide_norm(m->sx.data, NULL, NULL, NULL, m->slow[0].attn_norm.data, NULL, m->xt_norm, lr.kind, bd, st));
         else S2P_LAUNCH(m, rms_norm(m->sx.data, m->slow[0].attn_norm.data, m->snorm.data, bd, S2P_DIM, S2P_NORM_EPS, st));
-        for (int l = 0; l < m->n_slow; l++) {
+        const int fold = !wide && layers_fold_norms(m, m->slow, m->n_slow, bd);
+        residual res = {BF(m->sx), BF(m->sgu), 0};
+        for (int l = 0; fold && l < m->n_slow; l++) {
+            slow_kv_offsets(m, l, &c.kv);
+            S2P_TRY(layer_few_rows(m, &m->slow[l], &c, &res, BF(m->snorm), BF(m->sqkv), BF(m->sq), BF(m->sattn), BF(m->sproj), BF(m->sffn)));
+        }
+        if (fold) S2P_TRY(residual_close(m, &res, BF(m->sx), m->sproj.data, m->final_norm.data, m->shidden.data, bd));
+        for (int l = 0; !fold && l < m->n_slow; l++) {
             const int last = l + 1 == m->n_slow;
             const void* next = last ? m->final_norm.data : m->slow[l + 1].attn_norm.data;
             slow_kv_offsets(m, l, &c.kv);
