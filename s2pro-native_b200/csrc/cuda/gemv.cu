@@ -110,22 +110,19 @@ extern "C" cudaError_t gemv_setup_all(void) {
  * Lane l owns k = 512 i + 16 l .. +15 of every tile i, as for M == 1; a warp carries four weight rows and MM activation
  * rows, 4 x MM independent chains.
  *
- * What bounds it: fp32 fma and what surrounds one.  Two activation rows share a register pair, so a chain step is packed
- * (fma.rn.f32x2: two independent roundings, the same bits as fmaf on either half); an activation becomes f32 with one
- * instruction, a code (a byte planted in the mantissa of 2^23 twice and one packed subtraction, exact) once per MM activation rows.
- * The chains of a k advance side by side, because each waits for its own previous step.  Weights go from DRAM to registers a tile
- * ahead; the activations of a tile are shared by the SM's warps through L1.
+ * What bounds it: issue.  A chain step is one mixed fma (bf16 x bf16 + f32: the bits of fmaf), which costs 1.33 cycles of a scheduler because
+ * its three operands come through two register ports; an activation needs no conversion, a code one per MM activation rows.  The
+ * chains of a k advance side by side, because each waits for its own previous step, those of one activation one after another, so that its
+ * register is read once for four of them.  Weights go from DRAM to registers a tile ahead; the activations of a tile are shared by the
+ * SM's warps through L1.
  *
  * A matrix of few rows does not fill the GPU with warps of four rows, and a lone warp per scheduler waits on its own
  * latencies.  There NS = 4 warps share four rows and take tiles in turn; the tiles' chain results meet in shared memory and each warp
  * folds a quarter of the activation rows, tiles ascending.
- * Measured, us for one layer's four matrices (N x K 6144 x 2560, 2560 x 4096, 19456 x 2560, 2560 x 9728), before (scalar fma, one
- * weight row per warp for INT8; mixed bf16 fma, one to four for INT4) and now, at 2 / 4 / 8 / 16 rows:
- *   INT8  52 / 84 / 148 / 258 -> 44 / 56 / 81 / 135      INT4  46 / 70 / 103 / 180 -> 46 / 56 / 85 / 146
- * (2 rows now share the one-row kernel where rows are few: 38 and 39).
- * An odd row's chain is scalar: padded to a pair it held the fma pipe for two (3 rows INT4 58 -> 53, 5 rows 74 -> 68, 9 rows 119 -> 108).
- * 16 rows of 19456 x 2560 INT4 run at 11.4 T fma/s; the pipe's rate is 36 T.  Counters there: issue slots 59 %, fma pipe 51 %, integer
- * pipe 44 % busy, 11 of 64 warps resident (168 registers), 5 % of DRAM. */
+ * Measured, ticks of the full model, ms, before (two activation rows to a packed fma, each widened to f32; 168 registers) and now: 3 rows INT4
+ * 4.25 -> 4.06, 8 rows INT4 8.12 -> 6.55, 16 rows INT8 12.80 -> 10.81.  CTAs to an SM: of the shared form 5 (8 rows 7.23 with 4); of the other 4,
+ * where up to four rows are slower by 1 % than with 3.  16 rows of 19456 x 2560 INT4 take 50 us, 16 T fma/s of the 30 that a loop of mixed fma
+ * alone reaches. */
 /* A SwiGLU over stacked [gate | up] rows (SW): half of a warp's rows are of either half, so gate and up of an output meet in
  * the warp; both round to bf16 first, as where a kernel of its own follows the linear. */
 template <bool SW, int R> __device__ __forceinline__ int gemv_row_of(int n0, int r, int F) {
@@ -136,53 +133,92 @@ __device__ __forceinline__ float gemv_swiglu(float gate, float up_) {
     const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
     return __fmul_rn(bf16_round(__fmul_rn(g, sig)), up);
 }
-template <int WK> struct BatchCodes;
-template <> struct BatchCodes<WK_INT8_CH> {
-    static __device__ __forceinline__ f32x2 twice(uint32_t u, uint32_t sel, float minus) {
-        const float f = __uint_as_float(__byte_perm(u, 0x4B000000u, sel));
-        return fadd2(pack2(f, f), pack2(minus, minus));
+/* Codes of a lane as operands of the mixed fma (fma.rn.f32.bf16: bf16 x bf16 + f32, one rounding, the same bits as fmaf on the widened
+ * values).  STEP codes are converted together; get(w, j) is the j-th of them.  An activation needs no conversion at all: the fma
+ * takes either half of a register. */
+__device__ __forceinline__ unsigned short half_of(uint32_t v, bool high) {
+    unsigned short lo, hi;
+    asm("mov.b32 {%0, %1}, %2;" : "=h"(lo), "=h"(hi) : "r"(v));
+    return high ? hi : lo;
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) { /* two f32 adds, each rounded to bf16 */
+    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
+}
+template <int WK> struct Codes;
+template <> struct Codes<WK_INT8_CH> {
+    static constexpr int STEP = 2, WORDS = 2;
+    /* two bytes planted in the mantissa of 2^23, one packed subtraction: an f32 whose upper half is the code as bf16 */
+    static __device__ __forceinline__ void widen(const uint4& a, int k, uint32_t (&w)[WORDS]) {
+        const uint32_t u = s8x4_bias(k < 4 ? a.x : k < 8 ? a.y : k < 12 ? a.z : a.w);
+        float lo, hi;
+        unpack2(fadd2(pack2(__uint_as_float(prmt(u, 0x4B000000u, 0x7440u + (k & 3))), __uint_as_float(prmt(u, 0x4B000000u, 0x7441u + (k & 3)))),
+                      pack2(-8388736.0f, -8388736.0f)), lo, hi);
+        w[0] = __float_as_uint(lo); w[1] = __float_as_uint(hi);
     }
-    /* codes k = 8 h + 0..7 of two rows as f32 pairs (row a, row b) */
-    static __device__ __forceinline__ f32x2 both(uint32_t a, uint32_t b, uint32_t sel, float minus) {
-        return fadd2(pack2(__uint_as_float(__byte_perm(a, 0x4B000000u, sel)), __uint_as_float(__byte_perm(b, 0x4B000000u, sel))), pack2(minus, minus));
-    }
-    static __device__ __forceinline__ void widen8(const uint4& a, const uint4& b, int h, f32x2 (&w)[8]) {
-        const uint32_t ua[2] = {s8x4_bias(h ? a.z : a.x), s8x4_bias(h ? a.w : a.y)}, ub[2] = {s8x4_bias(h ? b.z : b.x), s8x4_bias(h ? b.w : b.y)};
-#pragma unroll
-        for (int j = 0; j < 8; j++) w[j] = both(ua[j >> 2], ub[j >> 2], 0x7440u + (j & 3), -8388736.0f);
-    }
-    /* codes k = 8 h + 0..7 of a lane as f32 pairs of equals */
-    static __device__ __forceinline__ void widen8(const uint4& a, int h, f32x2 (&w)[8]) {
-        const uint32_t u[2] = {s8x4_bias(h ? a.z : a.x), s8x4_bias(h ? a.w : a.y)};
-#pragma unroll
-        for (int j = 0; j < 8; j++) w[j] = twice(u[j >> 2], 0x7440u + (j & 3), -8388736.0f);
-    }
+    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j], true); }
 };
-template <> struct BatchCodes<WK_INT8_GRP> : BatchCodes<WK_INT8_CH> {};
-template <> struct BatchCodes<WK_INT4_PACK> {
-    static __device__ __forceinline__ void widen8(const uint2& a, const uint2& b, int h, f32x2 (&w)[8]) {
-        const uint32_t ua = h ? a.y : a.x, ub = h ? b.y : b.x;
-        const uint32_t ea = (ua & 0x0F0F0F0Fu) ^ 0x08080808u, oa = ((ua >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
-        const uint32_t eb = (ub & 0x0F0F0F0Fu) ^ 0x08080808u, ob = ((ub >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+template <> struct Codes<WK_INT8_GRP> : Codes<WK_INT8_CH> {};
+/* INT8 where registers count: two codes to a register.  0x43bb with the byte's sign in the exponent's last bit: 128 + low seven bits
+ * less 128 or 256 */
+struct CodesInt8Packed {
+    static constexpr int STEP = 4, WORDS = 2;
+    static __device__ __forceinline__ void widen(const uint4& a, int k, uint32_t (&w)[WORDS]) {
+        const uint32_t u = k < 4 ? a.x : k < 8 ? a.y : k < 12 ? a.z : a.w;
 #pragma unroll
-        for (int j = 0; j < 8; j++)
-            w[j] = BatchCodes<WK_INT8_CH>::both(j & 1 ? oa : ea, j & 1 ? ob : eb, 0x7440u + (j >> 1), -8388616.0f);
+        for (int j = 0; j < 2; j++) {
+            const uint32_t t = prmt(u, 0x43434343u, j ? 0x4342u : 0x4140u);
+            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(w[j]) : "r"(lop3<0xC0>(t, 0x437F437Fu, 0u)), "r"(lop3<0xC0>(t, 0x43804380u, 0u)));
+        }
     }
-    static __device__ __forceinline__ void widen8(const uint2& a, int h, f32x2 (&w)[8]) {
-        const uint32_t u = h ? a.y : a.x; /* two's complement nibble -> code + 8, even and odd k apart */
-        const uint32_t e = (u & 0x0F0F0F0Fu) ^ 0x08080808u, o = ((u >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
-#pragma unroll
-        for (int j = 0; j < 8; j++) w[j] = BatchCodes<WK_INT8_CH>::twice(j & 1 ? o : e, 0x7440u + (j >> 1), -8388616.0f);
-    }
+    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j >> 1], j & 1); }
 };
+template <> struct Codes<WK_INT4_PACK> {
+    static constexpr int STEP = 8, WORDS = 4;
+    /* nibbles j and j + 4 as bf16 128 + 8 + code, one packed subtraction of 136 */
+    static __device__ __forceinline__ void widen(const uint2& a, int k, uint32_t (&w)[WORDS]) {
+        const uint32_t u = k < 8 ? a.x : a.y;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t v = lop3<LOP_AND_XOR>(u >> (4 * j), 0x000F000Fu, 0x43084308u);
+            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(w[j]) : "r"(v), "r"(0x43084308u));
+        }
+    }
+    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j & 3], j >= 4); }
+};
+/* the first step of a chain, which starts at zero */
+__device__ __forceinline__ float fma_bf16_first(unsigned short w, unsigned short x) {
+    float s;
+    asm("fma.rn.f32.bf16 %0, %1, %2, 0f00000000;" : "=f"(s) : "h"(w), "h"(x));
+    return s;
+}
+/* sixteen steps of the chains of R weight rows against MM activation rows: s[m][r] */
+template <int WK> struct BatchCodes : Codes<WK> {};
+template <> struct BatchCodes<WK_INT8_CH> : CodesInt8Packed {};
+template <> struct BatchCodes<WK_INT8_GRP> : CodesInt8Packed {};
+template <class C, int MM, int R, class T, class X>
+__device__ __forceinline__ void lane_chains(const T (&t)[R], X x_word, float (&s)[MM][R]) {
+#pragma unroll
+    for (int k = 0; k < 16; k += C::STEP) {
+        uint32_t w[R][C::WORDS];
+#pragma unroll
+        for (int r = 0; r < R; r++) C::widen(t[r], k, w[r]);
+#pragma unroll
+        for (int j = 0; j < C::STEP; j++)
+#pragma unroll
+            for (int m = 0; m < MM; m++) {
+                const unsigned short xv = half_of(x_word(m, (k + j) >> 1), j & 1);
+#pragma unroll
+                for (int r = 0; r < R; r++) s[m][r] = k + j == 0 ? fma_bf16_first(C::get(w[r], j), xv) : fma_bf16(C::get(w[r], j), xv, s[m][r]);
+            }
+    }
+}
 
 template <int WK, int MM, int NS, bool SW>
-__global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
                                                        const void* __restrict__ w, const void* __restrict__ scales,
                                                        int M, int N, int K, int gshift) {
     typedef typename LaneTile<WK>::type tile_t;
-    constexpr int R = 4, P = MM / 2; /* weight rows of a warp, pairs of activation rows; an odd last one has scalar chains */
-    constexpr bool ODD = MM % 2 != 0;
+    constexpr int R = 4; /* weight rows of a warp */
     constexpr int PD = WK == WK_INT4_PACK && MM <= 4 ? 2 : 1; /* tiles of weights under way */
     constexpr int FM = NS == 1 ? MM : (MM + NS - 1) / NS; /* activation rows whose sums this warp keeps */
     __shared__ float part[NS == 1 ? 1 : 2 * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][m, then the scales][row][lane] */
@@ -222,6 +258,12 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
     for (int d = 0; d < PD; d++) fetch(d, min(d * NS + ns, T - 1));
     grid_wait();
     grid_release();
+    unsigned x_row[MM];
+#pragma unroll
+    for (int m = 0; m < MM; m++) {
+        x_row[m] = (unsigned)min(m, M - 1) * (unsigned)K;
+        if (MM > 4) asm("" : "+r"(x_row[m])); /* stays in a register: left to the compiler, it is recomputed for every load (tick of 8 rows 6.70 -> 6.55 ms) */
+    }
     const int rounds = (T + NS - 1) / NS;
     for (int rnd0 = 0; rnd0 < rounds; rnd0 += PD)
 #pragma unroll
@@ -234,59 +276,26 @@ __global__ void __launch_bounds__(128, 3) k_gemv_batch(__nv_bfloat16* __restrict
         for (int r = 0; r < R; r++) { cur[r] = nxt[d][r]; gs[r] = __half2float(gnx[d][r]); }
         if (i + PD * NS < T) fetch(d, i + PD * NS);
         if (NS == 1 || i < T) {
-            f32x2 s[R][P];
-            float so[R];
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                so[r] = 0.f;
-#pragma unroll
-                for (int p = 0; p < P; p++) s[r][p] = 0ull;
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) { /* eight k of the lane's sixteen */
-                uint4 xv[MM];
-#pragma unroll
-                for (int m = 0; m < MM; m++) xv[m] = *reinterpret_cast<const uint4*>(x + (size_t)min(m, M - 1) * K + i * 512 + h * 8);
-                f32x2 wf[R][8];
-#pragma unroll
-                for (int r = 0; r < R; r++) BatchCodes<WK>::widen8(cur[r], h, wf[r]);
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    auto word = [&](const uint4& v) { return (j >> 1) == 0 ? v.x : (j >> 1) == 1 ? v.y : (j >> 1) == 2 ? v.z : v.w; };
-                    auto value = [&](int m) { return j & 1 ? bf_hi(word(xv[m])) : bf_lo(word(xv[m])); };
-                    f32x2 xx[P];
-#pragma unroll
-                    for (int p = 0; p < P; p++) xx[p] = pack2(value(2 * p), value(2 * p + 1));
-#pragma unroll
-                    for (int r = 0; r < R; r++) {
-#pragma unroll
-                        for (int p = 0; p < P; p++) ffma2(s[r][p], wf[r][j], xx[p]);
-                        if (ODD) {
-                            float w0, w1;
-                            unpack2(wf[r][j], w0, w1);
-                            so[r] = __fmaf_rn(w0, value(MM - 1), so[r]);
-                        }
-                    }
-                }
-            }
-            auto sum_of = [&](int r, int m) {
-                if (ODD && m == MM - 1) return so[r];
-                float lo, hi;
-                unpack2(s[r][m >> 1], lo, hi);
-                return m & 1 ? hi : lo;
-            };
+            float s[MM][R];
+            uint4 xv[MM];
+            const __nv_bfloat16* xt = x + i * 512;
+            lane_chains<BatchCodes<WK>, MM, R>(cur, [&](int m, int i2) {
+                if ((i2 & 3) == 0) xv[m] = *reinterpret_cast<const uint4*>(xt + x_row[m] + i2 * 2);
+                const uint4& v = xv[m];
+                return (i2 & 3) == 0 ? v.x : (i2 & 3) == 1 ? v.y : (i2 & 3) == 2 ? v.z : v.w;
+            }, s);
             if (NS == 1) {
 #pragma unroll
                 for (int r = 0; r < R; r++)
 #pragma unroll
                     for (int m = 0; m < MM; m++)
-                        acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + sum_of(r, m) : __fmaf_rn(sum_of(r, m), gs[r], acc[m][r]);
+                        acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + s[m][r] : __fmaf_rn(s[m][r], gs[r], acc[m][r]);
             } else {
                 float* at = part + ((rnd & 1) * NS + ns) * ((MM + 1) * R * 32) + lane;
 #pragma unroll
                 for (int r = 0; r < R; r++) {
 #pragma unroll
-                    for (int m = 0; m < MM; m++) at[(m * R + r) * 32] = sum_of(r, m);
+                    for (int m = 0; m < MM; m++) at[(m * R + r) * 32] = s[m][r];
                     if (WK != WK_INT8_CH) at[(MM * R + r) * 32] = gs[r];
                 }
             }
@@ -338,10 +347,7 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
      * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all.  (A SwiGLU's pairs of rows
      * meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
     const int groups = (M + 7) / 8;
-    /* Seven rows of packed INT4 take the kernel of eight: the seventh row's scalar chains spill there (86.8 us for a layer's four
-     * matrices, 85.4 padded).  Two groups of seven have two warps to a scheduler and are faster as they are (13 rows 142.4, padded
-     * 145.3), and so is INT8 (7 rows 79.2, padded 80.7). */
-    const int mm = WK == WK_INT4_PACK && M == 7 ? 8 : (M + groups - 1) / groups;
+    const int mm = (M + groups - 1) / groups;
     const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
     const int T = K >> 9, turns = (T + 3) / 4 * 4;
     const bool shared = !SW && (2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
@@ -361,70 +367,6 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
     }
     return cudaErrorInvalidValue;
 #undef S2P_GB
-}
-
-/* Codes of a lane as operands of the mixed fma (fma.rn.f32.bf16: bf16 x bf16 + f32, one rounding, the same bits as fmaf on the widened
- * values).  STEP codes are converted together; get(w, j) is the j-th of them.  An activation needs no conversion at all: the fma
- * takes either half of a register. */
-__device__ __forceinline__ unsigned short half_of(uint32_t v, bool high) {
-    unsigned short lo, hi;
-    asm("mov.b32 {%0, %1}, %2;" : "=h"(lo), "=h"(hi) : "r"(v));
-    return high ? hi : lo;
-}
-__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) { /* two f32 adds, each rounded to bf16 */
-    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
-}
-template <int WK> struct Codes;
-template <> struct Codes<WK_INT8_CH> {
-    static constexpr int STEP = 2, WORDS = 2;
-    /* two bytes planted in the mantissa of 2^23, one packed subtraction: an f32 whose upper half is the code as bf16 */
-    static __device__ __forceinline__ void widen(const uint4& a, int k, uint32_t (&w)[WORDS]) {
-        const uint32_t u = s8x4_bias(k < 4 ? a.x : k < 8 ? a.y : k < 12 ? a.z : a.w);
-        float lo, hi;
-        unpack2(fadd2(pack2(__uint_as_float(prmt(u, 0x4B000000u, 0x7440u + (k & 3))), __uint_as_float(prmt(u, 0x4B000000u, 0x7441u + (k & 3)))),
-                      pack2(-8388736.0f, -8388736.0f)), lo, hi);
-        w[0] = __float_as_uint(lo); w[1] = __float_as_uint(hi);
-    }
-    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j], true); }
-};
-template <> struct Codes<WK_INT8_GRP> : Codes<WK_INT8_CH> {};
-template <> struct Codes<WK_INT4_PACK> {
-    static constexpr int STEP = 8, WORDS = 4;
-    /* nibbles j and j + 4 as bf16 128 + 8 + code, one packed subtraction of 136 */
-    static __device__ __forceinline__ void widen(const uint2& a, int k, uint32_t (&w)[WORDS]) {
-        const uint32_t u = k < 8 ? a.x : a.y;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t v = lop3<LOP_AND_XOR>(u >> (4 * j), 0x000F000Fu, 0x43084308u);
-            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(w[j]) : "r"(v), "r"(0x43084308u));
-        }
-    }
-    static __device__ __forceinline__ unsigned short get(const uint32_t (&w)[WORDS], int j) { return half_of(w[j & 3], j >= 4); }
-};
-/* the first step of a chain, which starts at zero */
-__device__ __forceinline__ float fma_bf16_first(unsigned short w, unsigned short x) {
-    float s;
-    asm("fma.rn.f32.bf16 %0, %1, %2, 0f00000000;" : "=f"(s) : "h"(w), "h"(x));
-    return s;
-}
-/* sixteen steps of the chains of R weight rows against MM activation rows: s[m][r] */
-template <int WK, int MM, int R, class X>
-__device__ __forceinline__ void lane_chains(const typename LaneTile<WK>::type (&t)[R], X x_word, float (&s)[MM][R]) {
-    typedef Codes<WK> C;
-#pragma unroll
-    for (int k = 0; k < 16; k += C::STEP) {
-        uint32_t w[R][C::WORDS];
-#pragma unroll
-        for (int r = 0; r < R; r++) C::widen(t[r], k, w[r]);
-#pragma unroll
-        for (int j = 0; j < C::STEP; j++)
-#pragma unroll
-            for (int m = 0; m < MM; m++) {
-                const unsigned short xv = half_of(x_word(m, (k + j) >> 1), j & 1);
-#pragma unroll
-                for (int r = 0; r < R; r++) s[m][r] = k + j == 0 ? fma_bf16_first(C::get(w[r], j), xv) : fma_bf16(C::get(w[r], j), xv, s[m][r]);
-            }
-    }
 }
 
 /* ---- one and two rows; up to four of a matrix of few rows --------------------------
@@ -594,7 +536,7 @@ __global__ void __launch_bounds__(RowPlan<WK, MM>::WARPS * 32, 1) k_gemv_row(__n
         for (int d = 0; d < D; d++) {
             if (d && d >= n) break;
             float s[MM][R];
-            lane_chains<WK, MM, R>(q[d], [&](int m, int i2) {
+            lane_chains<Codes<WK>, MM, R>(q[d], [&](int m, int i2) {
                 const uint4& v = xv[m][i2 >> 2];
                 return (i2 & 3) == 0 ? v.x : (i2 & 3) == 1 ? v.y : (i2 & 3) == 2 ? v.z : v.w;
             }, s);
