@@ -47,7 +47,10 @@ static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, int early, cud
     }
     return launch_early(early, k_attn_decode_team<KV8, NT>, grid, NT * 64, smem, st, a);
 }
-constexpr int ATTN_TEAMS_KV8 = 4, ATTN_TEAMS_BF16 = 3; /* two CTAs per SM either way */
+/* Teams to a CTA.  INT8 cache: three, and three CTAs to an SM (18 warps of 96 registers) from three rows on; four, and two CTAs, for one and two
+ * rows, whose few CTAs are better the larger.  us at 1 x 8000 / 3 x 700 / 8 x 1024 / 64 x 3000 / 32 x 8192 / 128 x 1024 rows x positions: four
+ * 22.5 / 10.7 / 20.4 / 175 / 244 / 127, three 27.0 / 10.1 / 17.6 / 169 / 229 / 124.  Bf16 cache: three, and two CTAs. */
+constexpr int ATTN_TEAMS_FEW = 4, ATTN_TEAMS_KV8 = 3, ATTN_TEAMS_BF16 = 3;
 static bool attn_team_serves(const AttnArgs& a, int rows) {
     if (a.out_ll || a.n_out_peers > 0 || (a.max_seq & 1)) return false;
     if ((a.kv.k_off | a.kv.v_off) & 15u) return false;
@@ -65,7 +68,8 @@ cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows
     if (a.q_heads != a.kv_heads * 4 || !a.part || !a.counters || a.workers < 1) return cudaErrorInvalidValue;
     dim3 grid((unsigned)rows, (unsigned)a.kv_heads, (unsigned)a.workers);
     if (!prep && attn_team_serves(a, rows))
-        return a.kv8 ? launch_attn_team<true, ATTN_TEAMS_KV8>(a, grid, early, st) : launch_attn_team<false, ATTN_TEAMS_BF16>(a, grid, early, st);
+        return !a.kv8 ? launch_attn_team<false, ATTN_TEAMS_BF16>(a, grid, early, st)
+             : rows <= 2 ? launch_attn_team<true, ATTN_TEAMS_FEW>(a, grid, early, st) : launch_attn_team<true, ATTN_TEAMS_KV8>(a, grid, early, st);
     AttnPrep pz = {};
     /* one score chain per thread (HPT 1): sharing a key's conversion between the heads of a position
      * (HPT 2 or 4) measured slower on a lockstep batch of 32, fewer warps being busy in the score phase */

@@ -163,7 +163,7 @@ __device__ __forceinline__ void team_copy_scales(__half* dst, const __half* src,
 }
 
 template <bool KV8, int NT>
-__global__ void __launch_bounds__(NT * 64) k_attn_decode_team(AttnArgs a) {
+__global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode_team(AttnArgs a) {
     extern __shared__ __align__(16) unsigned char attn_team_smem[];
     AttnTeamSmem<KV8, NT>& sm = *reinterpret_cast<AttnTeamSmem<KV8, NT>*>(attn_team_smem);
     constexpr int VB = AttnSplitTile<KV8>::VB;
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(NT * 64) k_attn_decode_team(AttnArgs a) {
      * decide here how many of the `workers` per (row, kv head) take part: enough teams for about
      * ATTN_SPLITS_PER_TEAM splits each, so that the copies of one split overlap the arithmetic of
      * another, but never so few CTAs that SMs stay empty.  The others go straight to the arrival counter. */
-    const int fill = (2 * 148 + (int)(gridDim.x * gridDim.y) - 1) / (int)(gridDim.x * gridDim.y);
-    const int eff = min(workers, max(max(n_active / (NT * ATTN_SPLITS_PER_TEAM), fill), 1));
+    const int fill = ((KV8 && NT == 3 ? 3 : 2) * 148 + (int)(gridDim.x * gridDim.y) - 1) / (int)(gridDim.x * gridDim.y);
+    const int eff = min(workers, max(max(NT == 3 ? (n_active + NT * ATTN_SPLITS_PER_TEAM - 1) / (NT * ATTN_SPLITS_PER_TEAM) : n_active / (NT * ATTN_SPLITS_PER_TEAM), fill), 1));
     const int first = wk < eff ? wk + eff * team : n_active, step = eff * NT;
 
     auto fetch_k = [&](int spl) {
