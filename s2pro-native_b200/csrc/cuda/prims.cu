@@ -68,22 +68,74 @@ struct NormRowArgs {
     int settled;                 /* the gains are a model's: the kernel in front does not write them */
 };
 constexpr int NORM_MAX_WIDTH = 4096; /* two vectors per thread */
+__device__ __forceinline__ uint32_t add_bf16_pair(uint32_t a, uint32_t b) {
+    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
+}
+/* sum of squares over a row in shared memory: 256 strided chains, then the halving tree.  All threads of the CTA call it. */
+__device__ __forceinline__ float norm_inv(const __nv_bfloat16* xs, int width, float eps, float* red) {
+    float ss = 0.f;
+    if (threadIdx.x < 256)
+        for (int i = threadIdx.x; i < width; i += 256) {
+            const float v = bf2f(xs[i]);
+            ss = __fmaf_rn(v, v, ss);
+        }
+    return rsqrtf(__fdiv_rn(tree256_sum(ss, red), (float)width) + eps);
+}
+/* prompt slices and callers' rows: norm of src (+ add), 256 threads */
 __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
     __shared__ __align__(16) __nv_bfloat16 xs[NORM_MAX_WIDTH];
     __shared__ float red[257];
-    __shared__ unsigned long long best[8];
-    const int tid = threadIdx.x, r = blockIdx.x, nv = a.width >> 3;
-    const int v0 = tid, v1 = tid + 256;
+    const int r = blockIdx.x, nv = a.width >> 3;
+    const int v0 = threadIdx.x, v1 = threadIdx.x + 256;
     uint4 g0 = make_uint4(0, 0, 0, 0), g1 = g0;
     auto gains = [&] {
         if (v0 < nv) g0 = reinterpret_cast<const uint4*>(a.w)[v0];
         if (v1 < nv) g1 = reinterpret_cast<const uint4*>(a.w)[v1];
     };
     if (a.w && a.settled) gains();
+    grid_wait();
+    grid_release();
+    if (a.w && !a.settled) gains();
+    const uint4* src = reinterpret_cast<const uint4*>(a.src + (size_t)r * a.width);
+    const uint4* add = a.add ? reinterpret_cast<const uint4*>(a.add + (size_t)r * a.width) : nullptr;
+    uint4* xo = a.x_out ? reinterpret_cast<uint4*>(a.x_out + (size_t)r * a.width) : nullptr;
+    auto load = [&](int v) {
+        uint4 q = src[v];
+        if (add) {
+            const uint4 p = add[v];
+            q = make_uint4(add_bf16_pair(q.x, p.x), add_bf16_pair(q.y, p.y), add_bf16_pair(q.z, p.z), add_bf16_pair(q.w, p.w));
+        }
+        if (xo) xo[v] = q;
+        reinterpret_cast<uint4*>(xs)[v] = q;
+        return q;
+    };
+    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+    if (v0 < nv) x0 = load(v0);
+    if (v1 < nv) x1 = load(v1);
+    if (!a.w) return;
+    __syncthreads();
+    const float inv = norm_inv(xs, a.width, a.eps, red);
+    uint4* y = reinterpret_cast<uint4*>(a.y + (size_t)r * a.width);
+    if (v0 < nv) y[v0] = norm_vec8(x0, g0, inv);
+    if (v1 < nv) y[v1] = norm_vec8(x1, g1, inv);
+}
+
+/* The same for the rows of a tick, of the model's width, with everything that may precede it.  A thread owns four columns, so that all of a
+ * row's loads are one round trip, the pieces of a split sum among them: what bounds it is latency, a chain of a launch, an L2 round
+ * trip, the tree and another.  With eight columns to each of 256 threads the pieces came in up to eight round trips (10.3 us a launch in the
+ * tick of 32 rows, 12.0 in that of 128). */
+constexpr int TICK_NORM_THREADS = S2P_DIM / 4;
+__global__ void __launch_bounds__(TICK_NORM_THREADS) k_norm_tick(NormRowArgs a) {
+    __shared__ __align__(16) __nv_bfloat16 xs[S2P_DIM];
+    __shared__ float red[257];
+    __shared__ unsigned long long best[TICK_NORM_THREADS / 32];
+    const int tid = threadIdx.x, r = blockIdx.x;
+    uint2 g = make_uint2(0, 0);
+    if (a.w && a.settled) g = reinterpret_cast<const uint2*>(a.w)[tid];
     if (a.tiled) grid_release(); /* a wide linear is next: see launch.cuh */
     grid_wait();
     if (!a.tiled) grid_release();
-    if (a.w && !a.settled) gains();
+    if (a.w && !a.settled) g = reinterpret_cast<const uint2*>(a.w)[tid];
     size_t row = (size_t)r;
     auto offer = [](unsigned long long& key, float l, int i) {
         if (l != l) return; /* a row of NaN gives index 0, as the reference's */
@@ -96,12 +148,12 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
     if (a.logits || a.part_logits) { /* larger value first, then lower index (kernels.cu:1326-1357); -0 counts as +0 */
         unsigned long long key = 0ull;
         if (a.part_logits)
-            for (int i = tid * 4; i < a.table_rows; i += 1024) {
+            for (int i = tid * 4; i < a.table_rows; i += TICK_NORM_THREADS * 4) {
                 const float4 l = wide_part4(a.part, i, r);
                 offer(key, bf16_round(l.x), i); offer(key, bf16_round(l.y), i + 1); offer(key, bf16_round(l.z), i + 2); offer(key, bf16_round(l.w), i + 3);
             }
         else
-            for (int i = tid; i < a.table_rows; i += 256) offer(key, bf2f(a.logits[(size_t)r * a.table_rows + i]), i);
+            for (int i = tid; i < a.table_rows; i += TICK_NORM_THREADS) offer(key, bf2f(a.logits[(size_t)r * a.table_rows + i]), i);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
             const unsigned long long o = __shfl_xor_sync(S2P_FULL_MASK, key, off);
@@ -110,54 +162,31 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
         if ((tid & 31) == 0) best[tid >> 5] = key;
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 8; k++) key = best[k] > key ? best[k] : key; /* every thread ends with the row's key */
+        for (int k = 0; k < TICK_NORM_THREADS / 32; k++) key = best[k] > key ? best[k] : key; /* every thread ends with the row's key */
         row = key ? 0xFFFFFFFFu - (uint32_t)key : 0u;
         if (tid == 0) a.codes_out[r] = (int32_t)row;
     } else if (a.codes) {
         row = (size_t)max(0, min(a.table_rows - 1, a.codes[r]));
     }
-    const uint4* src = reinterpret_cast<const uint4*>(a.src + row * a.width);
-    const uint4* add = a.add ? reinterpret_cast<const uint4*>(a.add + (size_t)r * a.width) : nullptr;
-    uint4* xo = a.x_out ? reinterpret_cast<uint4*>(a.x_out + (size_t)r * a.width) : nullptr;
-    const bool part_add = a.part.partial != nullptr && !a.part_logits;
-    auto load = [&](int v) {
-        uint4 q = src[v];
-        if (add || part_add) {
-            uint4 p;
-            if (part_add) {
-                const uint2 lo = wide_part4_bf16(a.part, v * 8, r), hi = wide_part4_bf16(a.part, v * 8 + 4, r);
-                p = make_uint4(lo.x, lo.y, hi.x, hi.y);
-            } else p = add[v];
-            uint32_t* qw = &q.x;
-            const uint32_t pw[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                qw[c] = (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(qw[c]), bf_lo(pw[c])))) |
-                        ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(qw[c]), bf_hi(pw[c])))) << 16);
-        }
-        if (xo) xo[v] = q;
-        reinterpret_cast<uint4*>(xs)[v] = q;
-        return q;
-    };
-    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
-    if (v0 < nv) x0 = load(v0);
-    if (v1 < nv) x1 = load(v1);
-    if (!a.w) return;
-    __syncthreads();
-    float ss = 0.f;
-    for (int i = tid; i < a.width; i += 256) {
-        const float v = bf2f(xs[i]);
-        ss = __fmaf_rn(v, v, ss);
+    uint2 x = reinterpret_cast<const uint2*>(a.src + row * S2P_DIM)[tid];
+    if (a.part.partial && !a.part_logits) {
+        const uint2 p = wide_part4_bf16(a.part, tid * 4, r);
+        x = make_uint2(add_bf16_pair(x.x, p.x), add_bf16_pair(x.y, p.y));
+    } else if (a.add) {
+        const uint2 p = reinterpret_cast<const uint2*>(a.add + (size_t)r * S2P_DIM)[tid];
+        x = make_uint2(add_bf16_pair(x.x, p.x), add_bf16_pair(x.y, p.y));
     }
-    const float tot = tree256_sum(ss, red);
-    const float inv = rsqrtf(__fdiv_rn(tot, (float)a.width) + a.eps);
-    uint4* y = a.y ? reinterpret_cast<uint4*>(a.y + (size_t)r * a.width) : nullptr;
-    auto put = [&](int v, const uint4& q) {
-        if (y) y[v] = q;
-        if (a.tiled) a.tiled[((size_t)v << a.lg) + r] = wide_unit(q, a.tiled_int4);
-    };
-    if (v0 < nv) put(v0, norm_vec8(x0, g0, inv));
-    if (v1 < nv) put(v1, norm_vec8(x1, g1, inv));
+    if (a.x_out) reinterpret_cast<uint2*>(a.x_out + (size_t)r * S2P_DIM)[tid] = x;
+    if (!a.w) return;
+    reinterpret_cast<uint2*>(xs)[tid] = x;
+    __syncthreads();
+    const float inv = norm_inv(xs, S2P_DIM, a.eps, red);
+    const uint4 n = norm_vec8(make_uint4(x.x, x.y, 0u, 0u), make_uint4(g.x, g.y, 0u, 0u), inv);
+    if (a.y) reinterpret_cast<uint2*>(a.y + (size_t)r * S2P_DIM)[tid] = make_uint2(n.x, n.y);
+    if (a.tiled) {
+        const uint32_t z = __shfl_down_sync(S2P_FULL_MASK, n.x, 1), w = __shfl_down_sync(S2P_FULL_MASK, n.y, 1);
+        if (!(tid & 1)) a.tiled[((size_t)(tid >> 1) << a.lg) + r] = wide_unit(make_uint4(n.x, n.y, z, w), a.tiled_int4);
+    }
 }
 
 /* ---- per-head RMSNorm, 128 partials (kernels.cu:81-101), in place ---------- */
@@ -734,6 +763,13 @@ cudaError_t rms_norm(const void* x, const void* w, void* y, int rows, int width,
     k_rms_norm<<<rows, 256, 0, st>>>(a.src, a.w, a.y, width, eps);
     return cudaGetLastError();
 }
+/* ticks have at most 256 rows, and so many CTAs of k_norm_tick fit the GPU at once; a prompt slice's rows are more */
+constexpr int TICK_NORM_ROWS = 256;
+static cudaError_t launch_norm(const NormRowArgs& a, int rows, cudaStream_t st) {
+    const bool plain = !a.codes && !a.logits && !a.part.partial && !a.tiled && (a.y || !a.w);
+    if (plain && rows > TICK_NORM_ROWS) return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    return launch_after(k_norm_tick, dim3((unsigned)rows), TICK_NORM_THREADS, 0, st, a);
+}
 cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st) { return add_norm_to(x, add, x, w, y, rows, st); }
 cudaError_t add_norm_to(const void* src, const void* add, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
@@ -741,7 +777,7 @@ cudaError_t add_norm_to(const void* src, const void* add, void* x, const void* w
     a.settled = 1;
     a.src = (const __nv_bfloat16*)src; a.add = (const __nv_bfloat16*)add; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
-    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    return launch_norm(a, rows, st);
 }
 static NormRowArgs wide_norm_args(void* x, const void* w, void* y, void* y_tiled, int kind, int rows) {
     NormRowArgs a = {};
@@ -758,7 +794,7 @@ cudaError_t wide_norm(const void* src, const WidePart* part, const void* alt, vo
     a.src = (const __nv_bfloat16*)src;
     if (part && part->partial) a.part = *part;
     else if (part) a.add = (const __nv_bfloat16*)alt;
-    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    return launch_norm(a, rows, st);
 }
 cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WidePart* part, const void* alt, int32_t* codes_out, void* x, const void* w,
                             void* y_tiled, int kind, int rows, cudaStream_t st) {
@@ -767,7 +803,7 @@ cudaError_t wide_embed_norm(const void* table, const int32_t* codes, const WideP
     a.src = (const __nv_bfloat16*)table; a.codes = codes; a.codes_out = codes_out;
     if (part && part->partial) { a.part = *part; a.part_logits = 1; }
     else if (part) a.logits = (const __nv_bfloat16*)alt;
-    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    return launch_norm(a, rows, st);
 }
 cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
@@ -775,7 +811,7 @@ cudaError_t copy_norm(const void* src, void* x, const void* w, void* y, int rows
     a.settled = 1;
     a.src = (const __nv_bfloat16*)src; a.x_out = (__nv_bfloat16*)x;
     a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y; a.width = S2P_DIM; a.eps = S2P_NORM_EPS;
-    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    return launch_norm(a, rows, st);
 }
 cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logits, int32_t* codes_out, void* x, const void* w, void* y, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
@@ -784,7 +820,7 @@ cudaError_t embed_norm(const void* table, const int32_t* codes, const void* logi
     a.src = (const __nv_bfloat16*)table; a.codes = codes; a.logits = (const __nv_bfloat16*)logits; a.codes_out = codes_out;
     a.x_out = (__nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.y = (__nv_bfloat16*)y;
     a.width = S2P_DIM; a.table_rows = S2P_CB_SIZE; a.eps = S2P_NORM_EPS;
-    return launch_after(k_norm_row, dim3((unsigned)rows), 256, 0, st, a);
+    return launch_norm(a, rows, st);
 }
 cudaError_t silu_mul(const void* gu, void* h, int rows, int ffn, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;

@@ -10,13 +10,13 @@ namespace s2p {
 __device__ __forceinline__ float4 wide_part4(const WidePart& p, int n, int m) {
     const float* at = p.partial + ((size_t)(n >> 7) * p.pieces * p.M + m) * 128 + (n & 127);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int q0 = 0; q0 < p.pieces; q0 += 4) {
-        float4 v[4];
+    for (int q0 = 0; q0 < p.pieces; q0 += 8) { /* a matrix of 2560 rows comes in seven: one round trip */
+        float4 v[8];
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < 8; q++)
             v[q] = q0 + q < p.pieces ? __ldcg(reinterpret_cast<const float4*>(at + (size_t)(q0 + q) * p.M * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < 8; q++)
             if (q0 + q < p.pieces) { s.x += v[q].x; s.y += v[q].y; s.z += v[q].z; s.w += v[q].w; }
     }
     if (p.scales) {
