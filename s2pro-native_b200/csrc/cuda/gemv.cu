@@ -566,14 +566,15 @@ __global__ void __launch_bounds__(RowPlan<WK, MM>::WARPS * 32, 1) k_gemv_row(__n
 #pragma unroll
         for (int r = 0; r < R; r++) acc[r] = 0.f;
         const float* at = sums + (size_t)(m * units + u) * (R * 32) + lane;
-        const __half* sc = ssc + u * RA * spr + ((lane * 16) >> gshift);
 #pragma unroll 2
-        for (int i = 0; i < T; i++, at += per_tile * (R * 32), sc += 512 >> gshift)
+        for (int i = 0; i < T; i++, at += per_tile * (R * 32)) {
+            const __half* sc = ssc + u * RA * spr + ((i * 512 + lane * 16) >> gshift); /* a group may be longer than a tile */
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 const float v = at[r * 32];
                 acc[r] = WK == WK_INT8_CH ? acc[r] + v : __fmaf_rn(v, __half2float(sc[(r % RA) * spr + r / RA * per_tile * RA * spr]), acc[r]);
             }
+        }
         /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
         const int r = lane >> 3, o = u * RA + r % RA;
         float a = warp_tree4<false>(acc[0], acc[1], acc[2], acc[3], lane);

@@ -41,9 +41,9 @@ def test_rows_equal_the_batch_kernels(mine, kind, n, k):
 
 
 @pytest.mark.parametrize("kind", [1, 2])
-@pytest.mark.parametrize("g,off", [(16, 0), (64, 2), (512, 0), (32, 2), (32, 14)])  # group sizes; scales that 16-byte copies cannot take
+@pytest.mark.parametrize("g,off", [(16, 0), (64, 2), (512, 0), (1024, 0), (2048, 6), (32, 2), (32, 14)])  # scales that 16-byte copies cannot take
 def test_groups_and_unaligned_scales(mine, kind, g, off):
-    n, k = 1031, 1536
+    n, k = 1031, 6144 if g > 512 else 1536  # groups shorter and longer than a tile
     w, s, gen = weights(kind, n, k, g, g + off, pad=8)
     x = torch.randn(5, k, device="cuda", generator=gen).bfloat16()
     want, got = (torch.empty((5, n), dtype=torch.bfloat16, device="cuda") for _ in range(2))
