@@ -176,17 +176,20 @@ __device__ __forceinline__ void attn_prefill_dim(const float* krow, const float*
  *
  * APART: 2 NW consumer warps, of which warp w forms the weights of its queries (they need nothing from the value sums) and warp
  * NW + w adds the values up, a tile behind.  A small block has one or two warps per scheduler, whose chains wait on themselves;
- * apart, both products of neighbouring tiles run at once.  Per tile (INT8): 4 rows 7.0 -> 5.8 us, 8 rows 9.4 -> 9.0. */
+ * apart, both products of neighbouring tiles run at once.  Per tile (INT8): 4 rows 7.0 -> 5.8 us; 8 rows 9.4 -> 9.0, and 8.7 with twice as many
+ * warps of half the queries, which load the schedulers evenly. */
 template <bool KV8, int QT, int NW, bool APART>
 __global__ void __launch_bounds__((APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCERS, 1) k_attn_prefill(AttnArgs a, int rows, int wide, int* status) {
     extern __shared__ __align__(16) unsigned char attn_prefill_smem[];
     typedef AttnPrefillSmem<KV8, QT, NW, APART> Smem;
     Smem& sm = *reinterpret_cast<Smem*>(attn_prefill_smem);
     constexpr int M = Smem::M, RB = Smem::RB, NC = (APART ? 64 : 32) * NW, VB = KV8 ? 128 : 256;
+    constexpr int DIMS = APART ? 8 : 4, FOURS = APART ? 2 : 1; /* unrolling; small blocks have the registers (2 % faster), 16 and 24 rows are slower with more */
     constexpr bool SPLIT_REGS = !APART && NW == 12, AHEAD = NC + ATTN_PREFILL_PRODUCERS <= (KV8 ? 512 : 384) && !SPLIT_REGS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    /* the last rows of the slice look furthest back: their blocks start first, the short ones fill in behind them */
-    const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * RB, kvh = blockIdx.y;
+    /* the last rows of the slice look furthest back: their blocks start first, of all heads (x varies fastest), the short ones fill in behind
+     * them (one head after another, 512 rows of a new prompt took 109 us instead of 76, 2048 912 instead of 806) */
+    const int r0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * RB, kvh = blockIdx.x;
     const int rb = min(RB, rows - r0);
     const int len0 = a.pos0 + r0 + 1;   /* positions row r0 attends over; row r0 + i: len0 + i */
     const int len_max = len0 + rb - 1;
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__((APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCER
                 for (int i = 0; i < QT; i++)
 #pragma unroll
                     for (int c = 0; c < 4; c++) pp[i][c] = 0ull;
-#pragma unroll 4
+#pragma unroll DIMS
                 for (int e = gi * 32; e < gi * 32 + 32; e++) attn_prefill_dim<QT>(sm.k[e], sm.q[e] + q0, tx, pp);
                 const uint2 ha = *reinterpret_cast<const uint2*>(&sm.ksc[gi][tx * 4]), hb = *reinterpret_cast<const uint2*>(&sm.ksc[gi][64 + tx * 4]);
 #pragma unroll
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__((APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCER
                 }
             }
         } else {
-#pragma unroll 4
+#pragma unroll DIMS
             for (int e = 0; e < 128; e++) attn_prefill_dim<QT>(sm.k[e], sm.q[e] + q0, tx, d);
         }
         __syncwarp();
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__((APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCER
         static_assert(QT == 2 || QT == 4, "a thread's queries are heads of one row");
         const int all_see = min(128, KV8 ? len0 - t0 : max(len0 - t0, 0)) & ~3; /* < 0: behind the first row's last tile */
         if (!mbar_wait_bounded(&sm.vfull, phase, status)) return false;
-#pragma unroll 1
+#pragma unroll FOURS
         for (int j = 0; j < all_see; j += 4) {
             f32x2 w01[QT], w23[QT];
 #pragma unroll

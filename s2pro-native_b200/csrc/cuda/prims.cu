@@ -563,33 +563,44 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, int* status,
     uintptr_t all = (uintptr_t)a->q | (uintptr_t)a->out | (uintptr_t)a->kv.base0 | a->kv.k_off | a->kv.v_off;
     if (a->kv8) all |= (uintptr_t)a->kv.sbase0 | a->kv.ks_off | a->kv.vs_off;
     constexpr int RB = QT * NW / 2;
-    dim3 grid((unsigned)((rows + RB - 1) / RB), (unsigned)a->kv_heads);
+    dim3 grid((unsigned)a->kv_heads, (unsigned)((rows + RB - 1) / RB));
     return launch_after(k_attn_prefill<KV8, QT, NW, APART>, grid, (APART ? 64 : 32) * NW + ATTN_PREFILL_PRODUCERS, smem, st, *a, rows, (int)((all & 15) == 0), status);
 }
 
-/* A CTA fills an SM whatever its size, so a launch takes (waves of CTAs) x (time per 128-position tile).  Large blocks are the
- * cheapest per row (0.80 us a tile with 24 rows, 2.3 with 2), small ones fill the GPU when the slice is short.  The times below
- * are the measured ones for an INT8 cache; bf16 is within 10 %.  16 and 24 rows keep a scheduler busy with warps that do both
- * products (15.3 and 19.3 us; products apart 16.1 and too many registers); up to 12 rows they are apart (8 rows 9.4 -> 9.0 us,
- * 4 rows 7.0 -> 5.8, see attn_prefill.cuh).  The estimate takes all CTAs to see equally many tiles, which holds for a slice behind
- * a long context; at position 0 the first block of a slice sees one tile and the last all of them, and what decides is the longest.
- * Measured (us; first kernel of one block size, four sizes of one kind, now): 2048 rows after 6052 positions 12590, 5430, 5396; 77
- * after 1024 154, 93, 73; 50 after 1000 89, 68, 57; 20 after 2000 161, 120, 82. */
+/* A CTA fills an SM whatever its size.  Large blocks are the cheapest per row (0.80 us a 128-position tile with 24 rows, 2.3 with 2), small ones
+ * fill the GPU when the slice is short: the block size with the smallest estimate is taken, a start for each wave and so many tiles in sequence.  How
+ * many: blocks of a slice see unequally many tiles and start longest first, so the schedule is about as long as the longest of
+ * the longest block, the tiles over the SMs, and, where an SM gets k blocks, k times the shortest that can be a k-th one.
+ * The times are measured ones for an INT8 cache (one block to an SM, 1 and 17 tiles); bf16 is within 10 %.  16 and 24 rows keep a scheduler busy
+ * with warps that do both products; up to 12 rows they are apart.  Sizes between these were no faster: 5 rows as 6, 18 and 20
+ * slower than 24, 10 and 14 than 12 and 16 (their warps load the schedulers unevenly).
+ * Measured, us, before (waves of CTAs, all taken to see equally many tiles) and now: 512 rows at 0 109 -> 76, 430 78 -> 62, 1000 287 -> 216, 2048 912 ->
+ * 806; behind a context, 77 after 1024 71 -> 70, 140 after 1000 90 -> 84, 2048 after 6052 5394 -> 5364. */
+static int attn_prefill_block(int rows, int pos0, int kv_heads, int sms, int block_rows) {
+    const int nb = (rows + block_rows - 1) / block_rows;
+    auto tiles = [&](int b) { return (pos0 + min(rows, (b + 1) * block_rows) + 127) / 128; };
+    long long total = 0;
+    for (int b = 0; b < nb; b++) total += tiles(b);
+    long long longest = (total * kv_heads + sms - 1) / sms;
+    for (int k = 1; (k - 1) * sms < nb * kv_heads; k++) longest = max(longest, (long long)k * tiles(nb - 1 - (k - 1) * sms / kv_heads));
+    return (int)min(longest, 1000000ll);
+}
 template <bool KV8>
 static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, int* status, cudaStream_t st) {
-    static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {19300, 15300, 12600, 9000, 7300, 5800, 4700};
+    static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {19200, 14700, 12100, 8700, 7200, 5650, 4700},
+                     start_ns[7] = {2000, 2200, 6000, 3200, 5100, 4200, 4000};
     int best = 0;
     long long best_cost = 0;
     for (int v = 0; v < 7; v++) {
-        const int ctas = (rows + block_rows[v] - 1) / block_rows[v] * a->kv_heads;
-        const long long cost = (long long)((ctas + device_sm_count() - 1) / device_sm_count()) * tile_ns[v];
+        const int ctas = (rows + block_rows[v] - 1) / block_rows[v] * a->kv_heads, sms = device_sm_count();
+        const long long cost = (long long)attn_prefill_block(rows, a->pos0, a->kv_heads, sms, block_rows[v]) * tile_ns[v] + (ctas + sms - 1) / sms * start_ns[v];
         if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
     switch (best) {
     case 0: return launch_attn_prefill<KV8, 4, 12, false>(a, rows, status, st);
     case 1: return launch_attn_prefill<KV8, 4, 8, false>(a, rows, status, st);
     case 2: return launch_attn_prefill<KV8, 4, 6, true>(a, rows, status, st);
-    case 3: return launch_attn_prefill<KV8, 4, 4, true>(a, rows, status, st);
+    case 3: return launch_attn_prefill<KV8, 2, 8, true>(a, rows, status, st);
     case 4: return launch_attn_prefill<KV8, 2, 6, true>(a, rows, status, st);
     case 5: return launch_attn_prefill<KV8, 2, 4, true>(a, rows, status, st);
     default: return launch_attn_prefill<KV8, 2, 2, true>(a, rows, status, st);
