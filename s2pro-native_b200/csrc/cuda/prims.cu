@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(TICK_NORM_THREADS) k_norm_tick(NormRowArgs a) 
     }
     uint2 x = reinterpret_cast<const uint2*>(a.src + row * S2P_DIM)[tid];
     if (a.part.partial && !a.part_logits) {
-        const uint2 p = wide_part4_bf16(a.part, tid * 4, r);
+        const uint2 p = wide_part4_bf16<8>(a.part, tid * 4, r);
         x = make_uint2(add_bf16_pair(x.x, p.x), add_bf16_pair(x.y, p.y));
     } else if (a.add) {
         const uint2 p = reinterpret_cast<const uint2*>(a.add + (size_t)r * S2P_DIM)[tid];

@@ -6,17 +6,19 @@
 
 namespace s2p {
 
-/* outputs n .. n + 3 (n a multiple of 4) of batch row m, before the rounding to bf16 */
+/* outputs n .. n + 3 (n a multiple of 4) of batch row m, before the rounding to bf16; AHEAD pieces are asked for at once (a matrix of 2560 rows
+ * comes in seven, one of 6144 in three) */
+template <int AHEAD = 4>
 __device__ __forceinline__ float4 wide_part4(const WidePart& p, int n, int m) {
     const float* at = p.partial + ((size_t)(n >> 7) * p.pieces * p.M + m) * 128 + (n & 127);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int q0 = 0; q0 < p.pieces; q0 += 8) { /* a matrix of 2560 rows comes in seven: one round trip */
-        float4 v[8];
+    for (int q0 = 0; q0 < p.pieces; q0 += AHEAD) {
+        float4 v[AHEAD];
 #pragma unroll
-        for (int q = 0; q < 8; q++)
+        for (int q = 0; q < AHEAD; q++)
             v[q] = q0 + q < p.pieces ? __ldcg(reinterpret_cast<const float4*>(at + (size_t)(q0 + q) * p.M * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int q = 0; q < 8; q++)
+        for (int q = 0; q < AHEAD; q++)
             if (q0 + q < p.pieces) { s.x += v[q].x; s.y += v[q].y; s.z += v[q].z; s.w += v[q].w; }
     }
     if (p.scales) {
@@ -25,8 +27,9 @@ __device__ __forceinline__ float4 wide_part4(const WidePart& p, int n, int m) {
     }
     return s;
 }
+template <int AHEAD = 4>
 __device__ __forceinline__ uint2 wide_part4_bf16(const WidePart& p, int n, int m) {
-    const float4 s = wide_part4(p, n, m);
+    const float4 s = wide_part4<AHEAD>(p, n, m);
     return make_uint2((uint32_t)__bfloat16_as_ushort(f2bf(s.x)) | ((uint32_t)__bfloat16_as_ushort(f2bf(s.y)) << 16),
                       (uint32_t)__bfloat16_as_ushort(f2bf(s.z)) | ((uint32_t)__bfloat16_as_ushort(f2bf(s.w)) << 16));
 }
