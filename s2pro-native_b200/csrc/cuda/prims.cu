@@ -316,13 +316,20 @@ cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st) { return q
  * single-row kernel, which stages both tiles and walks two 128-wide trees behind fourteen CTA barriers (2.5 + 5 us).  Here a CTA of six
  * warps owns a (row, kv head): four query heads, the key and the value are rotated at once, the key and value go to the cache and to
  * shared memory, and each query warp attends with a position per lane, the older positions' keys and values having been asked for
- * before the wait for the kernel in front (passes further back wrote them).  Same chains, and the trees' other 112 or more
+ * before the wait for the kernel in front (passes further back wrote them).  In a warp's registers those leave two CTAs to an SM, so batches
+ * that need more of them copy the older positions to shared memory (STAGED; 128 rows: tick 11.17 -> 10.93 ms; where all CTAs are
+ * resident anyway its later reads cost 1 to 2 %: frame of one row 2.50 -> 2.54, 8 rows 6.36 -> 6.44).  Same chains, and the trees' other 112 or more
  * values are zeros or -inf, so the bits are those of k_attn_single.  Bf16 caches, one position for all rows. */
 constexpr int FAST_ATTN_MAX = 16; /* positions */
+__device__ __forceinline__ void fast_attn_copy16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+template <bool STAGED>
 __global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part, __nv_bfloat16* __restrict__ out, int head_dim) {
     __shared__ float2 cs[64];
     __shared__ __align__(16) float sq[4][128];
     __shared__ __align__(16) __nv_bfloat16 now[2][128]; /* this position's key and value */
+    __shared__ __align__(16) __nv_bfloat16 ks[STAGED ? FAST_ATTN_MAX : 1][136], vs[STAGED ? FAST_ATTN_MAX : 1][128]; /* the older ones; keys 16 bytes apart */
     const int r = blockIdx.x, kvh = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int QH = a.q_heads, KVH = a.kv_heads, heads = QH + 2 * KVH, pos = a.pos0;
     const bool is_q = warp < 4;
@@ -332,7 +339,13 @@ __global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part,
     __nv_bfloat16* const vc = reinterpret_cast<__nv_bfloat16*>(base + a.kv.v_off) + (size_t)kvh * a.max_seq * 128;
     uint4 k[16];
     uint2 vv[FAST_ATTN_MAX], nw = make_uint2(0u, 0u);
-    if (is_q) {
+    if (STAGED) {
+        for (int c = threadIdx.x; c < pos * 16; c += 192) {
+            fast_attn_copy16(&ks[c >> 4][(c & 15) * 8], kc + c * 8);
+            fast_attn_copy16(&vs[c >> 4][(c & 15) * 8], vc + c * 8);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    } else if (is_q) {
 #pragma unroll
         for (int c = 0; c < 16; c++) k[c] = lane < pos ? reinterpret_cast<const uint4*>(kc + lane * 128)[c] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
@@ -357,15 +370,18 @@ __global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part,
         reinterpret_cast<uint2*>(now[warp - 4])[lane] = o;
         reinterpret_cast<uint2*>((warp == 4 ? kc : vc) + (size_t)pos * 128)[lane] = o;
     }
+    if (STAGED) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     if (!is_q) return;
-    if (lane == pos)
+    if (!STAGED && lane == pos)
 #pragma unroll
         for (int c = 0; c < 16; c++) k[c] = reinterpret_cast<const uint4*>(now[0])[c];
+    const uint4* kl = reinterpret_cast<const uint4*>(lane < pos ? ks[STAGED ? lane : 0] : now[0]);
     float s = 0.f;
 #pragma unroll
     for (int c = 0; c < 16; c++) {
-        const uint32_t w[4] = {k[c].x, k[c].y, k[c].z, k[c].w};
+        const uint4 kk = STAGED ? kl[c] : k[c];
+        const uint32_t w[4] = {kk.x, kk.y, kk.z, kk.w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             s = __fmaf_rn(sq[warp][c * 8 + 2 * j], bf_lo(w[j]), s);
@@ -382,7 +398,7 @@ __global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part,
     for (int j = 0; j < FAST_ATTN_MAX; j++) {
         if (j > pos) break;
         const float pj = __shfl_sync(S2P_FULL_MASK, p, j);
-        const uint2 u = j == pos ? mine : vv[j];
+        const uint2 u = j == pos ? mine : STAGED ? reinterpret_cast<const uint2*>(vs[STAGED ? j : 0])[lane] : vv[j];
         acc[0] = __fmaf_rn(pj, bf_lo(u.x), acc[0]); acc[1] = __fmaf_rn(pj, bf_hi(u.x), acc[1]);
         acc[2] = __fmaf_rn(pj, bf_lo(u.y), acc[2]); acc[3] = __fmaf_rn(pj, bf_hi(u.y), acc[3]);
     }
@@ -396,7 +412,8 @@ cudaError_t fast_attn(const QkvPostArgs* a, const WidePart* part, void* out, int
     if (a->kv8 || a->pos_arr || a->pos_row_step || a->pos0 < 0 || a->pos0 >= FAST_ATTN_MAX || a->pos0 >= a->max_seq || a->q_heads != 4 * a->kv_heads || head_dim != 128 ||
         (((uintptr_t)a->kv.base0 | a->kv.k_off | a->kv.v_off | a->kv.row_stride) & 15))
         return cudaErrorInvalidValue;
-    return launch_after(k_fast_attn, dim3((unsigned)rows, (unsigned)a->kv_heads), 192, 0, st, *a, part ? *part : WidePart(), (__nv_bfloat16*)out, head_dim);
+    const bool staged = rows * a->kv_heads > 2 * device_sm_count();
+    return launch_after(staged ? k_fast_attn<true> : k_fast_attn<false>, dim3((unsigned)rows, (unsigned)a->kv_heads), 192, 0, st, *a, part ? *part : WidePart(), (__nv_bfloat16*)out, head_dim);
 }
 
 /* ---- plain KV append (contract s2pk_kv_append, kernels.cu:172-195) --------- */
