@@ -16,8 +16,7 @@ constexpr int SMP_TOPK = 30;
 
 template <int NT> struct SamplerSmem {
     float cand[SMP_N_CAND];
-    float wtop_v[(NT / 32) * SMP_TOPK];  /* every warp's own top-30 */
-    int wtop_i[(NT / 32) * SMP_TOPK];
+    int wtop[(NT / 32) * SMP_TOPK];      /* every warp's own top-30, best first */
     float tv[SMP_TOPK];
     int ti[SMP_TOPK];
     float sh_temp, sh_topp;
@@ -36,7 +35,19 @@ static __device__ __forceinline__ uint64_t xoshiro_next(uint64_t* s) {
     return result;
 }
 
-__device__ __forceinline__ bool better(float v, int i, float bv, int bi) { return v > bv || (v == bv && i < bi); }
+/* (value descending, index ascending) as integers: larger key first, then lower index.  -0 counts as +0, NaN is never chosen (key 0). */
+__device__ __forceinline__ uint32_t sampler_key(float v) {
+    if (v != v) return 0u;
+    uint32_t u = __float_as_uint(v);
+    if (u == 0x80000000u) u = 0u;
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+/* the best of a warp's (key, index) pairs; index SMP_N_CAND where nothing is left */
+__device__ __forceinline__ int sampler_best(uint32_t key, int idx) {
+    const uint32_t top = __reduce_max_sync(S2P_FULL_MASK, key);
+    const int i = (int)__reduce_min_sync(S2P_FULL_MASK, key == top ? (unsigned)idx : (unsigned)SMP_N_CAND);
+    return top ? i : SMP_N_CAND;
+}
 
 /* logits: 4096 semantic logits of the row; eos_logit: its EOS logit; sp: its state;
  * outputs are the row's own slots. */
@@ -62,6 +73,17 @@ __device__ void sampler_cta(const __nv_bfloat16* lrow, const __nv_bfloat16* eos_
 
     const bool greedy = sp->temperature == 0.0f;
     const int capped = count0 < (uint64_t)window ? (int)count0 : window;
+    float pen = 0.f;
+    int pen_at = -1; /* the history's tokens side by side: all read the original values, equal tokens write equal ones */
+    if (tid < capped) {
+        const int64_t tok = hist[tid];
+        if (tok >= S2P_TOK_SEMANTIC_START && tok <= S2P_TOK_SEMANTIC_END) pen_at = (int)(tok - S2P_TOK_SEMANTIC_START);
+        else if (tok == S2P_TOK_EOS) pen_at = SMP_N_SEM;
+        if (pen_at >= 0) {
+            const float v = cand[pen_at], rep_penalty = sp->rep_penalty;
+            pen = v < 0.f ? __fmul_rn(v, rep_penalty) : __fdiv_rn(v, rep_penalty);
+        }
+    }
     if (tid == 0) {
         bool ras = false;
         if (!greedy && capped >= 4) {
@@ -75,144 +97,114 @@ __device__ void sampler_cta(const __nv_bfloat16* lrow, const __nv_bfloat16* eos_
         }
         sh_temp = ras ? 1.0f : sp->temperature;
         sh_topp = ras ? 0.9f : sp->top_p;
-        if (capped > 0) {
-            int ridx[64];
-            float rval[64];
-            int rn = 0;
-            const float rep_penalty = sp->rep_penalty;
-            for (int j = 0; j < capped; j++) {
-                const int64_t tok = hist[j];
-                int ci;
-                if (tok >= S2P_TOK_SEMANTIC_START && tok <= S2P_TOK_SEMANTIC_END) ci = (int)(tok - S2P_TOK_SEMANTIC_START);
-                else if (tok == S2P_TOK_EOS) ci = SMP_N_SEM;
-                else continue;
-                const float v = cand[ci];
-                ridx[rn] = ci;
-                rval[rn] = v < 0.f ? __fmul_rn(v, rep_penalty) : __fdiv_rn(v, rep_penalty);
-                rn++;
-            }
-            for (int j = 0; j < rn; j++) cand[ridx[j]] = rval[j];
-        }
     }
     S2P_CTA_SYNC();
+    if (pen_at >= 0) cand[pen_at] = pen;
+    S2P_CTA_SYNC();
 
-    /* top-30 in two warp-level passes without block-wide rounds: every warp selects the 30 best of
-     * its own candidates (i = tid + NT j, held in registers) with shuffles only; warp 0 then selects
-     * the 30 best of the warps' winners.  (value desc, index asc) is a total order, so the result
-     * is the block-wide top-30 in order. */
+    /* top-30 in two warp-level passes without block-wide rounds: every warp selects the 30 best of its own candidates
+     * (i = tid + NT j, keys in registers), two integer reductions a choice, after which only the owner looks through its
+     * candidates again; warp 0 then merges the warps' sorted lists, a list per lane.  (value desc, index asc) is a total order, so the
+     * result is the block-wide top-30 in order. */
     const int lane = tid & 31, warp = tid >> 5;
     constexpr int NW = SMP_THREADS / 32;
-    float* wtv = sm.wtop_v;
-    int* wti = sm.wtop_i;
+    int* wt = sm.wtop;
     {
-        float mine[SMP_PER_THREAD];
+        uint32_t mine[SMP_PER_THREAD], key = 0u;
+        int idx = SMP_N_CAND;
+        auto look = [&] {
+            key = 0u; idx = SMP_N_CAND;
+#pragma unroll
+            for (int j = 0; j < SMP_PER_THREAD; j++)
+                if (mine[j] > key) { key = mine[j]; idx = tid + j * SMP_THREADS; }
+        };
 #pragma unroll
         for (int j = 0; j < SMP_PER_THREAD; j++) {
             const int i = tid + j * SMP_THREADS;
-            mine[j] = i < SMP_N_CAND ? cand[i] : -INFINITY;
+            mine[j] = i < SMP_N_CAND ? sampler_key(cand[i]) : 0u;
         }
+        look();
         for (int k = 0; k < SMP_TOPK; k++) {
-            float bv = -INFINITY;
-            int bi = SMP_N_CAND;
-#pragma unroll
-            for (int j = 0; j < SMP_PER_THREAD; j++) {
-                const int i = tid + j * SMP_THREADS;
-                if (i < SMP_N_CAND && better(mine[j], i, bv, bi)) { bv = mine[j]; bi = i; }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ov = __shfl_xor_sync(S2P_FULL_MASK, bv, off);
-                const int oi = __shfl_xor_sync(S2P_FULL_MASK, bi, off);
-                if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-            }
-            if (lane == 0) { wtv[warp * SMP_TOPK + k] = bv; wti[warp * SMP_TOPK + k] = bi; }
-            if (bi < SMP_N_CAND && (bi % SMP_THREADS) == tid) { /* the owner retires the winner */
+            const int best = sampler_best(key, idx);
+            if (lane == 0) wt[warp * SMP_TOPK + k] = best;
+            if (best < SMP_N_CAND && best == idx) { /* the owner retires the winner */
 #pragma unroll
                 for (int j = 0; j < SMP_PER_THREAD; j++)
-                    if (tid + j * SMP_THREADS == bi) mine[j] = -INFINITY;
+                    if (tid + j * SMP_THREADS == best) mine[j] = 0u;
+                look();
             }
         }
     }
     S2P_CTA_SYNC();
     if (warp == 0) {
-        constexpr int PER2 = (NW * SMP_TOPK + 31) / 32;
-        float v2[PER2];
-        int i2[PER2];
-#pragma unroll
-        for (int j = 0; j < PER2; j++) {
-            const int e = lane + 32 * j;
-            v2[j] = e < NW * SMP_TOPK ? wtv[e] : -INFINITY;
-            i2[j] = e < NW * SMP_TOPK ? wti[e] : SMP_N_CAND;
-        }
+    {
+        int at = 0;
+        int idx = lane < NW ? wt[lane * SMP_TOPK] : SMP_N_CAND;
+        uint32_t key = idx < SMP_N_CAND ? sampler_key(cand[idx]) : 0u;
         for (int k = 0; k < SMP_TOPK; k++) {
-            float bv = -INFINITY;
-            int bi = SMP_N_CAND;
-#pragma unroll
-            for (int j = 0; j < PER2; j++)
-                if (i2[j] < SMP_N_CAND && better(v2[j], i2[j], bv, bi)) { bv = v2[j]; bi = i2[j]; }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ov = __shfl_xor_sync(S2P_FULL_MASK, bv, off);
-                const int oi = __shfl_xor_sync(S2P_FULL_MASK, bi, off);
-                if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+            const int best = sampler_best(key, idx);
+            if (lane == 0) { tv[k] = best < SMP_N_CAND ? cand[best] : -INFINITY; ti[k] = best; }
+            if (best < SMP_N_CAND && best == idx) {
+                at++;
+                idx = at < SMP_TOPK ? wt[lane * SMP_TOPK + at] : SMP_N_CAND;
+                key = idx < SMP_N_CAND ? sampler_key(cand[idx]) : 0u;
             }
-            if (lane == 0) { tv[k] = bv; ti[k] = bi; }
-#pragma unroll
-            for (int j = 0; j < PER2; j++)
-                if (i2[j] == bi) i2[j] = SMP_N_CAND; /* retired: an index never matches again */
         }
     }
-    S2P_CTA_SYNC();
-    if (tid == 0) {
+    __syncwarp();
     int choice = 0;
     if (!greedy) {
-        float e[SMP_TOPK], sum = 0.f;
-        const float m = tv[0];
+        /* a rank per lane; the sums are the reference's, rank after rank */
+        const bool rank = lane < SMP_TOPK;
+        const float v = tv[rank ? lane : 0], m = tv[0];
+        auto sum_of = [](float x) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < SMP_TOPK; j++) s = __fadd_rn(s, __shfl_sync(S2P_FULL_MASK, x, j));
+            return s;
+        };
+        const float e = expf(v - m);
+        const float share = __fdiv_rn(e, sum_of(e));
+        float cum = 0.f, upto = 0.f;
+#pragma unroll
         for (int j = 0; j < SMP_TOPK; j++) {
-            e[j] = expf(tv[j] - m);
-            sum = __fadd_rn(sum, e[j]);
+            cum = __fadd_rn(cum, __shfl_sync(S2P_FULL_MASK, share, j));
+            if (j == lane) upto = cum;
         }
-        bool masked[SMP_TOPK];
-        float cum = 0.f;
-        for (int j = 0; j < SMP_TOPK; j++) {
-            cum = __fadd_rn(cum, __fdiv_rn(e[j], sum));
-            masked[j] = (j > 0 && cum > sh_topp);
-        }
+        const bool masked = lane > 0 && upto > sh_topp;
         const float t = sh_temp < 1e-5f ? 1e-5f : sh_temp;
-        float p2[SMP_TOPK], s2 = 0.f;
-        const float m2 = __fdiv_rn(tv[0], t);
-        for (int j = 0; j < SMP_TOPK; j++) {
-            p2[j] = masked[j] ? 0.f : expf(__fsub_rn(__fdiv_rn(tv[j], t), m2));
-            s2 = __fadd_rn(s2, p2[j]);
-        }
-        for (int j = 0; j < SMP_TOPK; j++) p2[j] = __fdiv_rn(p2[j], s2);
+        const float m2 = __fdiv_rn(m, t);
+        float p2 = masked ? 0.f : expf(__fsub_rn(__fdiv_rn(v, t), m2));
+        p2 = __fdiv_rn(p2, sum_of(p2));
 
         if (sp->seeded) {
             const uint64_t step_seed = ((uint64_t)sp->seed31 * 19349663ULL) ^ (count0 * 73856093ULL);
-            float best = -INFINITY;
-            for (int j = 0; j < SMP_TOPK; j++) {
-                const uint64_t hashed = (step_seed * 8589934591ULL) ^ ((uint64_t)j * 479001599ULL);
-                float u = __fdiv_rn((float)(uint32_t)(hashed & 0xFFFFFFULL), 16777216.0f);
-                if (u < 1e-10f) u = 1e-10f;
-                const float g = -logf(-logf(u));
-                const float pert = __fadd_rn(logf(__fadd_rn(p2[j], 1e-10f)), g);
-                if (pert > best) { best = pert; choice = j; }
-            }
+            const uint64_t hashed = (step_seed * 8589934591ULL) ^ ((uint64_t)lane * 479001599ULL);
+            float u = __fdiv_rn((float)(uint32_t)(hashed & 0xFFFFFFULL), 16777216.0f);
+            if (u < 1e-10f) u = 1e-10f;
+            const float g = -logf(-logf(u));
+            const float pert = __fadd_rn(logf(__fadd_rn(p2, 1e-10f)), g);
+            /* the first largest; what does not exceed -inf is never chosen, and rank 0 stands where nothing is */
+            const uint32_t key = rank && pert > -INFINITY ? sampler_key(pert) : 0u;
+            const uint32_t top = __reduce_max_sync(S2P_FULL_MASK, key);
+            choice = top ? __ffs(__ballot_sync(S2P_FULL_MASK, key == top)) - 1 : 0;
         } else {
-            const double r = (double)(xoshiro_next(sp->rng) >> 11) * 0x1.0p-53;
+            double r = 0.0;
+            if (lane == 0) r = (double)(xoshiro_next(sp->rng) >> 11) * 0x1.0p-53;
             double cum2 = 0.0;
             int lastnz = 0;
             choice = -1;
-            for (int j = 0; j < SMP_TOPK; j++) {
-                if (p2[j] <= 0.f) continue;
+            for (int j = 0; j < SMP_TOPK; j++) { /* lane 0's result counts */
+                const float p = __shfl_sync(S2P_FULL_MASK, p2, j);
+                if (p <= 0.f) continue;
                 lastnz = j;
-                cum2 += (double)p2[j];
-                if (r < cum2) { choice = j; break; }
+                cum2 += (double)p;
+                if (choice < 0 && r < cum2) choice = j;
             }
             if (choice < 0) choice = lastnz;
         }
     }
-
+    if (tid == 0) {
     const int ci = ti[choice];
     if (ci == SMP_N_SEM) { /* EOS: semantic code forced to 0, sampler state untouched */
         *out_tok = S2P_TOK_EOS;
@@ -231,6 +223,7 @@ __device__ void sampler_cta(const __nv_bfloat16* lrow, const __nv_bfloat16* eos_
         sp->count = count0 + 1;
     }
     } /* tid == 0 */
+    } /* warp == 0 */
     S2P_CTA_SYNC();
     /* history update, the shift done by the threads side by side from the staged window */
     if (sm.fin_mode == 1) {
