@@ -819,6 +819,14 @@ struct WideArgs {
     float* partial;         /* [split tile][piece][M][128] */
 };
 
+/* columns gi .. gi + 7 of the SwiGLU's result, batch row m */
+__device__ __forceinline__ void wide_put_unit(const WideArgs& a, int gi, int m, const uint4& q) {
+    if (a.tiled) { a.tiled[((size_t)(gi >> 3) << a.lgNB) + m] = wide_unit(q, a.tiled_int4); return; }
+    const uint32_t o[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        if (gi + j < a.ffn) a.y[(size_t)m * a.ffn + gi + j] = __ushort_as_bfloat16((unsigned short)(o[j >> 1] >> (16 * (j & 1))));
+}
 /* SwiGLU results of rows r8 .. r8 + 7 of a tile's gate half, batch row m; g(r), u(r): the two products */
 template <class G, class U>
 __device__ __forceinline__ void wide_put_swiglu(const WideArgs& a, int tile, int r8, int m, G g, U u) {
@@ -829,39 +837,47 @@ __device__ __forceinline__ void wide_put_swiglu(const WideArgs& a, int tile, int
         const uint32_t v = __bfloat16_as_ushort(sk_swiglu(bf16_round(g(r8 + j)), bf16_round(u(r8 + j))));
         o[j >> 1] |= v << (16 * (j & 1));
     }
-    const uint4 q = make_uint4(o[0], o[1], o[2], o[3]);
-    if (a.tiled) { a.tiled[((size_t)(gi >> 3) << a.lgNB) + m] = wide_unit(q, a.tiled_int4); return; }
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-        if (gi + j < a.ffn) a.y[(size_t)m * a.ffn + gi + j] = __ushort_as_bfloat16((unsigned short)(o[j >> 1] >> (16 * (j & 1))));
+    wide_put_unit(a, gi, m, make_uint4(o[0], o[1], o[2], o[3]));
 }
 
-/* the split tiles of a SwiGLU pair, once their pieces are there; CTA = (split tile, batch row), a group of 8 rows per thread */
+/* the split tiles of a SwiGLU pair, once their pieces are there; CTA = (split tile, two batch rows), four gate rows and their up rows per
+ * thread.  What bounds it is latency, so all pieces of both are asked for at once (one after another 5.2 us a launch at 128 rows, so 3.1). */
+constexpr int WD_SURPLUS_ROWS = 2;
 template <int WK>
-__global__ void __launch_bounds__(32) k_wide_surplus(WideArgs a) {
+__global__ void __launch_bounds__(16 * WD_SURPLUS_ROWS) k_wide_surplus(WideArgs a) {
     grid_release(); /* a wide linear is next: see launch.cuh */
     grid_wait();
-    const int stile = blockIdx.x, m = blockIdx.y * 4 + (threadIdx.x >> 3), r8 = (threadIdx.x & 7) * 8;
+    const int stile = blockIdx.x, m = blockIdx.y * WD_SURPLUS_ROWS + (threadIdx.x >> 4), r4 = (threadIdx.x & 15) * 4;
     const int tile = (a.ffn + 63) / 64 - a.n_split_tiles + stile;
-    if (m >= a.M || tile * 64 + r8 >= a.ffn) return;
-    const float* at = a.partial + ((size_t)stile * a.KS * a.M + m) * SK_BM;
-    float g[8], u[8];
+    const bool live = m < a.M;
+    const float* at = a.partial + ((size_t)stile * a.KS * a.M + (live ? m : 0)) * SK_BM + r4;
+    float4 pg[SK_MAX_SPLIT], pu[SK_MAX_SPLIT];
 #pragma unroll
-    for (int j = 0; j < 8; j++) { g[j] = 0.f; u[j] = 0.f; }
-    for (int q = 0; q < a.KS; q++) {
-        const float4* pg = reinterpret_cast<const float4*>(at + (size_t)q * a.M * SK_BM + r8);
-        const float4 g0 = __ldcg(pg), g1 = __ldcg(pg + 1), u0 = __ldcg(pg + 16), u1 = __ldcg(pg + 17);
-        g[0] += g0.x; g[1] += g0.y; g[2] += g0.z; g[3] += g0.w; g[4] += g1.x; g[5] += g1.y; g[6] += g1.z; g[7] += g1.w;
-        u[0] += u0.x; u[1] += u0.y; u[2] += u0.z; u[3] += u0.w; u[4] += u1.x; u[5] += u1.y; u[6] += u1.z; u[7] += u1.w;
-    }
-    if (WK == WK_INT8_CH)
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int gi = min(tile * 64 + r8 + j, a.ffn - 1);
-            g[j] = __fmul_rn(g[j], static_cast<const float*>(a.scales)[gi]);
-            u[j] = __fmul_rn(u[j], static_cast<const float*>(a.scales)[a.ffn + gi]);
+    for (int q = 0; q < SK_MAX_SPLIT; q++)
+        if (q < a.KS) {
+            pg[q] = __ldcg(reinterpret_cast<const float4*>(at + (size_t)q * a.M * SK_BM));
+            pu[q] = __ldcg(reinterpret_cast<const float4*>(at + (size_t)q * a.M * SK_BM + 64));
         }
-    wide_put_swiglu(a, tile, r8, m, [&](int r) { return g[r & 7]; }, [&](int r) { return u[r & 7]; });
+    float g[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < SK_MAX_SPLIT; q++)
+        if (q < a.KS) {
+            g[0] += pg[q].x; g[1] += pg[q].y; g[2] += pg[q].z; g[3] += pg[q].w;
+            u[0] += pu[q].x; u[1] += pu[q].y; u[2] += pu[q].z; u[3] += pu[q].w;
+        }
+    const int gi = tile * 64 + r4;
+    uint32_t o[2] = {0u, 0u};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (WK == WK_INT8_CH) {
+            const int gr = min(gi + j, a.ffn - 1);
+            g[j] = __fmul_rn(g[j], static_cast<const float*>(a.scales)[gr]);
+            u[j] = __fmul_rn(u[j], static_cast<const float*>(a.scales)[a.ffn + gr]);
+        }
+        o[j >> 1] |= (uint32_t)__bfloat16_as_ushort(sk_swiglu(bf16_round(g[j]), bf16_round(u[j]))) << (16 * (j & 1));
+    }
+    const uint32_t p = __shfl_down_sync(S2P_FULL_MASK, o[0], 1), q = __shfl_down_sync(S2P_FULL_MASK, o[1], 1);
+    if (live && !(threadIdx.x & 1) && gi < a.ffn) wide_put_unit(a, gi, m, make_uint4(o[0], o[1], p, q));
 }
 
 template <int WK>
@@ -1047,7 +1063,7 @@ static cudaError_t wide_launch(const WideArgs& a, int grid, cudaStream_t st) {
     }
     err = launch_after(k_wide_tc<WK>, dim3((unsigned)grid), WD_EPI + 64, (size_t)a.stages * (WD_A_BYTES + (WD_KC * 2 << a.lgNB)) + 256, st, a);
     if (err == cudaSuccess && a.ffn && a.n_split_tiles)
-        err = launch_after(k_wide_surplus<WK>, dim3((unsigned)a.n_split_tiles, (unsigned)((a.M + 3) / 4)), 32, 0, st, a);
+        err = launch_after(k_wide_surplus<WK>, dim3((unsigned)a.n_split_tiles, (unsigned)((a.M + WD_SURPLUS_ROWS - 1) / WD_SURPLUS_ROWS)), 16 * WD_SURPLUS_ROWS, 0, st, a);
     return err;
 }
 
