@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(512) k_attn_decode(AttnArgs a, AttnPrep pz) {
 /* The kernel for lockstep batches on one GPU, no fused prologue: a team of two warps per split
  * (attn_team.cuh). */
 template <bool KV8, int NT>
-static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, int early, cudaStream_t st) {
+static cudaError_t launch_attn_team(const AttnArgs& a, const TiledOut& tiled, dim3 grid, int early, cudaStream_t st) {
     static bool attr_set[64] = {false};
     constexpr size_t smem = sizeof(AttnTeamSmem<KV8, NT>);
     int dev = 0;
@@ -45,7 +45,7 @@ static cudaError_t launch_attn_team(const AttnArgs& a, dim3 grid, int early, cud
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    return launch_early(early, k_attn_decode_team<KV8, NT>, grid, NT * 64, smem, st, a);
+    return launch_early(early, k_attn_decode_team<KV8, NT>, grid, NT * 64, smem, st, a, tiled);
 }
 /* Teams to a CTA.  INT8 cache: three, and three CTAs to an SM (18 warps of 96 registers) from three rows on; four, and two CTAs, for one and two
  * rows, whose few CTAs are better the larger.  us at 1 x 8000 / 3 x 700 / 8 x 1024 / 64 x 3000 / 32 x 8192 / 128 x 1024 rows x positions: four
@@ -62,14 +62,18 @@ static bool attn_team_serves(const AttnArgs& a, int rows) {
     return (size_t)a.n_split_slots * 32 + 16 <= tiles;
 }
 
+static cudaError_t launch_attn_teams(const AttnArgs& a, const TiledOut& tiled, int rows, int early, cudaStream_t st) {
+    dim3 grid((unsigned)rows, (unsigned)a.kv_heads, (unsigned)a.workers);
+    return !a.kv8 ? launch_attn_team<false, ATTN_TEAMS_BF16>(a, tiled, grid, early, st)
+         : rows <= 2 ? launch_attn_team<true, ATTN_TEAMS_FEW>(a, tiled, grid, early, st) : launch_attn_team<true, ATTN_TEAMS_KV8>(a, tiled, grid, early, st);
+}
+
 /* early: the kernel in front writes nothing of the cache but the last position, and no position table (launch.cuh) */
 cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows, int early, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     if (a.q_heads != a.kv_heads * 4 || !a.part || !a.counters || a.workers < 1) return cudaErrorInvalidValue;
     dim3 grid((unsigned)rows, (unsigned)a.kv_heads, (unsigned)a.workers);
-    if (!prep && attn_team_serves(a, rows))
-        return !a.kv8 ? launch_attn_team<false, ATTN_TEAMS_BF16>(a, grid, early, st)
-             : rows <= 2 ? launch_attn_team<true, ATTN_TEAMS_FEW>(a, grid, early, st) : launch_attn_team<true, ATTN_TEAMS_KV8>(a, grid, early, st);
+    if (!prep && attn_team_serves(a, rows)) return launch_attn_teams(a, TiledOut(), rows, early, st);
     AttnPrep pz = {};
     /* one score chain per thread (HPT 1): sharing a key's conversion between the heads of a position
      * (HPT 2 or 4) measured slower on a lockstep batch of 32, fewer warps being busy in the score phase */
@@ -84,6 +88,12 @@ cudaError_t launch_attn_decode(const AttnArgs& a, const AttnPrep* prep, int rows
     return cudaGetLastError();
 }
 
+extern "C" int attn_decode_tiled_serves(const AttnArgs* a, int rows) { return attn_team_serves(*a, rows); }
+extern "C" cudaError_t attn_decode_tiled(const AttnArgs* a, const TiledOut* tiled, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    if (a->q_heads != a->kv_heads * 4 || !a->part || !a->counters || a->workers < 1 || !attn_team_serves(*a, rows)) return cudaErrorInvalidValue;
+    return launch_attn_teams(*a, *tiled, rows, 1, st);
+}
 extern "C" cudaError_t attn_decode(const AttnArgs* a, int rows, cudaStream_t st) {
     return launch_attn_decode(*a, nullptr, rows, 1, st);
 }

@@ -41,6 +41,7 @@
 #include "ops.h"
 #include "launch.cuh"
 #include "packed.cuh"
+#include "wide.cuh"
 
 namespace s2p {
 
@@ -71,7 +72,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
  * and its exp-sum, so that each weight's expf is evaluated once instead of once per dimension; it
  * needs 8 floats per split and 4 more. */
 template <int THREADS>
-__device__ __forceinline__ void attn_merge_partials(const AttnArgs& a, int row, int kvh, int n_active, float* scratch) {
+__device__ __forceinline__ void attn_merge_partials(const AttnArgs& a, const TiledOut& tiled, int row, int kvh, int n_active, float* scratch) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int QH = a.q_heads;
     __threadfence();
@@ -117,7 +118,17 @@ __device__ __forceinline__ void attn_merge_partials(const AttnArgs& a, int row, 
             }
         }
 #pragma unroll
-        for (int g = 0; g < HP; g++) a.out[((size_t)row * QH + kvh * 4 + g0 + g) * 128 + dd] = f2bf(__fdiv_rn(acc[g], l[g]));
+        for (int g = 0; g < HP; g++) {
+            const __nv_bfloat16 o = f2bf(__fdiv_rn(acc[g], l[g]));
+            if (!tiled.out) {
+                a.out[((size_t)row * QH + kvh * 4 + g0 + g) * 128 + dd] = o;
+                continue;
+            }
+            /* a unit is eight dimensions: eight neighbouring lanes (whole warps get here, or none of their lanes) */
+            const uint32_t mine = __bfloat16_as_ushort(o), two = mine | __shfl_down_sync(S2P_FULL_MASK, mine, 1) << 16;
+            const uint4 u = make_uint4(two, __shfl_down_sync(S2P_FULL_MASK, two, 2), __shfl_down_sync(S2P_FULL_MASK, two, 4), __shfl_down_sync(S2P_FULL_MASK, two, 6));
+            if (!(dd & 7)) static_cast<uint4*>(tiled.out)[((size_t)((kvh * 4 + g0 + g) * 16 + (dd >> 3)) << tiled.lg) + row] = wide_unit(u, tiled.int4);
+        }
     }
 }
 
@@ -163,7 +174,7 @@ __device__ __forceinline__ void team_copy_scales(__half* dst, const __half* src,
 }
 
 template <bool KV8, int NT>
-__global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode_team(AttnArgs a) {
+__global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode_team(AttnArgs a, TiledOut tiled) {
     extern __shared__ __align__(16) unsigned char attn_team_smem[];
     AttnTeamSmem<KV8, NT>& sm = *reinterpret_cast<AttnTeamSmem<KV8, NT>*>(attn_team_smem);
     constexpr int VB = AttnSplitTile<KV8>::VB;
@@ -375,7 +386,7 @@ __global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode
     if (tid == 0) sm.s_last = (atomicAdd(ctr, 1u) == (unsigned)(workers - 1));
     __syncthreads();
     if (sm.s_last) {
-        attn_merge_partials<NT * 64>(a, row, kvh, n_active, reinterpret_cast<float*>(attn_team_smem));
+        attn_merge_partials<NT * 64>(a, tiled, row, kvh, n_active, reinterpret_cast<float*>(attn_team_smem));
         if (tid == 0) *ctr = 0u;
     }
 }

@@ -331,6 +331,13 @@ cudaError_t scale_rows_masked(void* x, const uint8_t* mask, int rows, int dim, f
 cudaError_t add_norm(void* x, const void* add, const void* w, void* y, int rows, cudaStream_t st);
 /* the same with the sum in another place than src */
 cudaError_t add_norm_to(const void* src, const void* add, void* x, const void* w, void* y, int rows, cudaStream_t st);
+/* Activations of a batch as the f16 units of a wide linear (wide.cuh), of kind `kind`, for a batch padded to 1 << lg rows */
+typedef struct { void* out; int lg, kind, int4; } TiledOut;
+/* fast_attn and attn_decode with the result in units instead of bf16 (`out` of the one, a->out of the other, are not written) */
+cudaError_t fast_attn_tiled(const QkvPostArgs* a, const WidePart* part, const TiledOut* tiled, int head_dim, int rows, cudaStream_t st);
+int attn_decode_tiled_serves(const AttnArgs* a, int rows);
+cudaError_t attn_decode_tiled(const AttnArgs* a, const TiledOut* tiled, int rows, cudaStream_t st);
+TiledOut wide_units(int kind, void* xt, int rows); /* units of a linear of kind `kind` at xt */
 /* The same around wide_gemm.  `part` with `alt` is its output: the partials, or alt where it wrote that.
  * x = src (+ the output, if part is given); or, with a table, its row `codes[r]`, or the one that the arg-max of the output
  * selects (to codes_out).  y = norm(x) with gain w (NULL: none), as bf16 and / or as the units of a linear of kind `kind`. */

@@ -325,7 +325,7 @@ __device__ __forceinline__ void fast_attn_copy16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 template <bool STAGED>
-__global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part, __nv_bfloat16* __restrict__ out, int head_dim) {
+__global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part, __nv_bfloat16* __restrict__ out, TiledOut tiled, int head_dim) {
     __shared__ float2 cs[64];
     __shared__ __align__(16) float sq[4][128];
     __shared__ __align__(16) __nv_bfloat16 now[2][128]; /* this position's key and value */
@@ -405,15 +405,31 @@ __global__ void __launch_bounds__(192) k_fast_attn(QkvPostArgs a, WidePart part,
     uint2 o;
     o.x = (uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[0], l))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[1], l))) << 16);
     o.y = (uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[2], l))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fdiv_rn(acc[3], l))) << 16);
-    reinterpret_cast<uint2*>(out + ((size_t)r * QH + h) * 128)[lane] = o;
+    if (!tiled.out) {
+        reinterpret_cast<uint2*>(out + ((size_t)r * QH + h) * 128)[lane] = o;
+        return;
+    }
+    const uint32_t o2 = __shfl_down_sync(S2P_FULL_MASK, o.x, 1), o3 = __shfl_down_sync(S2P_FULL_MASK, o.y, 1);
+    if (!(lane & 1)) static_cast<uint4*>(tiled.out)[((size_t)(h * 16 + (lane >> 1)) << tiled.lg) + r] = wide_unit(make_uint4(o.x, o.y, o2, o3), tiled.int4);
 }
-cudaError_t fast_attn(const QkvPostArgs* a, const WidePart* part, void* out, int head_dim, int rows, cudaStream_t st) {
+static cudaError_t launch_fast_attn(const QkvPostArgs* a, const WidePart* part, void* out, const TiledOut& tiled, int head_dim, int rows, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     if (a->kv8 || a->pos_arr || a->pos_row_step || a->pos0 < 0 || a->pos0 >= FAST_ATTN_MAX || a->pos0 >= a->max_seq || a->q_heads != 4 * a->kv_heads || head_dim != 128 ||
         (((uintptr_t)a->kv.base0 | a->kv.k_off | a->kv.v_off | a->kv.row_stride) & 15))
         return cudaErrorInvalidValue;
     const bool staged = rows * a->kv_heads > 2 * device_sm_count();
-    return launch_after(staged ? k_fast_attn<true> : k_fast_attn<false>, dim3((unsigned)rows, (unsigned)a->kv_heads), 192, 0, st, *a, part ? *part : WidePart(), (__nv_bfloat16*)out, head_dim);
+    return launch_after(staged ? k_fast_attn<true> : k_fast_attn<false>, dim3((unsigned)rows, (unsigned)a->kv_heads), 192, 0, st, *a, part ? *part : WidePart(), (__nv_bfloat16*)out, tiled, head_dim);
+}
+cudaError_t fast_attn(const QkvPostArgs* a, const WidePart* part, void* out, int head_dim, int rows, cudaStream_t st) {
+    return launch_fast_attn(a, part, out, TiledOut(), head_dim, rows, st);
+}
+cudaError_t fast_attn_tiled(const QkvPostArgs* a, const WidePart* part, const TiledOut* tiled, int head_dim, int rows, cudaStream_t st) {
+    return launch_fast_attn(a, part, nullptr, *tiled, head_dim, rows, st);
+}
+TiledOut wide_units(int kind, void* xt, int rows) {
+    TiledOut t;
+    t.out = xt; t.lg = wide_lg(rows); t.kind = kind; t.int4 = kind == WK_INT4_PACK;
+    return t;
 }
 
 /* ---- plain KV append (contract s2pk_kv_append, kernels.cu:172-195) --------- */

@@ -268,9 +268,10 @@ static int attn_workers_for(int rows) {
     return w < 1 ? 1 : (w > 16 ? 16 : w);
 }
 
-/* head norms, RoPE, cache append and attention of one layer; the projection is qkv, or left in partials */
+/* head norms, RoPE, cache append and attention of one layer; the projection is qkv, or left in partials.  `tiled`: the result as units of the
+ * next linear; where the attention kernel cannot write them its bf16 result is packed. */
 static s2p_status layer_attention(s2p_model* m, const s2p_layer* L, const layer_ctx* c, s2p_dev_bf16* qkv, const WidePart* part, s2p_dev_bf16* q,
-                                  s2p_dev_bf16* attn) {
+                                  s2p_dev_bf16* attn, const TiledOut* tiled) {
     cudaStream_t st = m->stream;
     const int rows = c->rows;
     QkvPostArgs qa;
@@ -281,7 +282,8 @@ static s2p_status layer_attention(s2p_model* m, const s2p_layer* L, const layer_
     qa.q_heads = S2P_SLOW_Q_HEADS; qa.kv_heads = S2P_SLOW_KV_HEADS; qa.max_seq = c->max_seq; qa.kv8 = c->kv8;
     qa.pos0 = c->pos0; qa.pos_row_step = c->pos_row_step; qa.pos_arr = c->pos_arr; qa.kv = c->kv;
     if (c->decode && !c->split_k) { /* the fast stack */
-        S2P_LAUNCH(m, fast_attn(&qa, part, attn, S2P_HEAD_DIM, rows, st));
+        if (tiled) S2P_LAUNCH(m, fast_attn_tiled(&qa, part, tiled, S2P_HEAD_DIM, rows, st));
+        else S2P_LAUNCH(m, fast_attn(&qa, part, attn, S2P_HEAD_DIM, rows, st));
         return S2P_OK;
     }
     S2P_LAUNCH(m, qkv_post_part(&qa, part, rows, st));
@@ -294,7 +296,12 @@ static s2p_status layer_attention(s2p_model* m, const s2p_layer* L, const layer_
     if (c->split_k) {
         aa.part = (float*)m->attn_part.data; aa.counters = m->attn_ctr;
         aa.n_split_slots = m->n_split_slots; aa.workers = attn_workers_for(rows);
-        S2P_LAUNCH(m, attn_decode(&aa, rows, st));
+        if (tiled && attn_decode_tiled_serves(&aa, rows)) {
+            S2P_LAUNCH(m, attn_decode_tiled(&aa, tiled, rows, st));
+        } else {
+            S2P_LAUNCH(m, attn_decode(&aa, rows, st));
+            if (tiled) S2P_LAUNCH(m, wide_pack(tiled->kind, attn, rows, S2P_Q_WIDTH, tiled->out, st));
+        }
     } else {
         S2P_LAUNCH(m, attn_slice(&aa, rows, m->d_prefill_status, st));
     }
@@ -310,7 +317,7 @@ static s2p_status layer_general(s2p_model* m, const s2p_layer* L, const layer_ct
     cudaStream_t st = m->stream;
     const int rows = c->rows;
     S2P_TRY(lin_apply(m, &L->wqkv, L->wide[0], norm, qkv, rows, c->decode));
-    S2P_TRY(layer_attention(m, L, c, qkv, NULL, q, attn));
+    S2P_TRY(layer_attention(m, L, c, qkv, NULL, q, attn, NULL));
     S2P_TRY(lin_add_norm(m, &L->wo, L->wide[1], attn, x, proj, L->ffn_norm.data, norm, rows, c->decode));
     if (c->decode && m->mode == S2P_GEMM_INT8 && L->gate_up.int8_ready && s2p_linear_rows_on_tc(&L->gate_up, rows) &&
         L->gate_up.out_features == 2 * S2P_FFN_DIM) {
@@ -367,7 +374,7 @@ static s2p_status layer_few_rows(s2p_model* m, const s2p_layer* L, const layer_c
                                  s2p_dev_bf16* q, s2p_dev_bf16* attn, s2p_dev_bf16* proj, s2p_dev_bf16* hff) {
     if (r->pending) S2P_TRY(linear_of_norm(m, &L->wqkv, r, proj, L->attn_norm.data, qkv, 0, c->rows));
     else S2P_TRY(lin_apply(m, &L->wqkv, NULL, norm, qkv, c->rows, 1));
-    S2P_TRY(layer_attention(m, L, c, qkv, NULL, q, attn));
+    S2P_TRY(layer_attention(m, L, c, qkv, NULL, q, attn, NULL));
     S2P_TRY(lin_apply(m, &L->wo, NULL, attn, proj, c->rows, 1));
     S2P_TRY(linear_of_norm(m, &L->gate_up, r, proj, L->ffn_norm.data, hff, 1, c->rows));
     r->pending = 1;
@@ -391,8 +398,8 @@ static s2p_status layer_wide(s2p_model* m, const s2p_layer* L, const layer_ctx* 
     s2p_lin_ref(&L->wqkv, &wqkv); s2p_lin_ref(&L->wo, &wo); s2p_lin_ref(&L->gate_up, &gate_up); s2p_lin_ref(&L->w2, &w2);
     WidePart part;
     S2P_LAUNCH(m, wide_gemm(&wqkv, L->tc[0], m->xt_norm, rows, 0, qkv, NULL, 0, &part, st));
-    S2P_TRY(layer_attention(m, L, c, qkv, part.partial ? &part : NULL, q, attn));
-    S2P_LAUNCH(m, wide_pack(wo.kind, attn, rows, S2P_Q_WIDTH, m->xt_attn, st));
+    const TiledOut units = wide_units(wo.kind, m->xt_attn, rows);
+    S2P_TRY(layer_attention(m, L, c, qkv, part.partial ? &part : NULL, q, attn, &units));
     S2P_LAUNCH(m, wide_gemm(&wo, L->tc[1], m->xt_attn, rows, 0, proj, NULL, 0, &part, st));
     S2P_LAUNCH(m, wide_norm(x, &part, proj, x, L->ffn_norm.data, NULL, m->xt_norm, gate_up.kind, rows, st));
     m->tick_kernels += 1; /* the tiles of the pair whose K range is split are a launch of their own */
