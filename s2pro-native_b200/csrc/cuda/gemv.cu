@@ -130,7 +130,7 @@ template <bool SW, int R> __device__ __forceinline__ int gemv_row_of(int n0, int
 }
 __device__ __forceinline__ float gemv_swiglu(float gate, float up_) {
     const float g = bf16_round(gate), up = bf16_round(up_);
-    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
+    const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-g))); /* correctly rounded, as the division */
     return __fmul_rn(bf16_round(__fmul_rn(g, sig)), up);
 }
 /* Codes of a lane as operands of the mixed fma (fma.rn.f32.bf16: bf16 x bf16 + f32, one rounding, the same bits as fmaf on the widened
