@@ -75,7 +75,6 @@ template <int THREADS>
 __device__ __forceinline__ void attn_merge_partials(const AttnArgs& a, const TiledOut& tiled, int row, int kvh, int n_active, float* scratch) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int QH = a.q_heads;
-    __threadfence();
     float* wm = scratch;              /* [4][n_active] */
     float* wl = wm + 4 * n_active;    /* [4][n_active] */
     float* hmax = wl + 4 * n_active;  /* [4] */
@@ -380,10 +379,13 @@ __global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode
     cp_async_wait<0>();
 
     /* the last CTA of this (row, kv head) to finish merges the partials in ascending split order */
-    __threadfence();
     __syncthreads();
     unsigned int* ctr = a.counters + (size_t)row * KVH + kvh;
-    if (tid == 0) sm.s_last = (atomicAdd(ctr, 1u) == (unsigned)(workers - 1));
+    if (tid == 0) { /* releases what the barrier has ordered before it, and acquires what the others released */
+        unsigned before;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(ctr) : "memory");
+        sm.s_last = before == (unsigned)(workers - 1);
+    }
     __syncthreads();
     if (sm.s_last) {
         attn_merge_partials<NT * 64>(a, tiled, row, kvh, n_active, reinterpret_cast<float*>(attn_team_smem));
