@@ -140,8 +140,8 @@ cudaError_t gemv_setup_all(void); /* once per device, before any stream capture 
 /* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: see launch_early (launch.cuh) */
 int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t st);
 /* h[M, N / 2] = silu(gate) * up for stacked [gate | up] rows, otherwise as gemv_rows with early.  Up to four rows the launch it
- * saves counts (tick of 1 row 3.53 -> 3.43 ms, 3 rows 5.61 -> 5.55); the kernels of eight rows have no registers left for it (8 rows
- * 8.39 -> 8.42, 16 rows 12.9 -> 13.2). */
+ * saves counts (tick of 1 row 3.53 -> 3.43 ms, 3 rows 5.61 -> 5.55, in the kernels of that time); in the kernels of more rows its epilogue costs
+ * more than that (8 rows 6.54 -> 6.58, 16 rows 10.79 -> 10.90). */
 #define GEMV_SWIGLU_ROWS 4
 int gemv_rows_swiglu(const LinRef* lin, const void* x, void* h, int M, cudaStream_t st);
 /* The linear of norm(src + add) for one or two rows, the sum and the norm taken by the kernel itself (a launch less, in a chain where
