@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+/* The same for two pointers whose loads the compiler may take for constant over the kernel (const __restrict__) and else move in front. */
+template <class P> __device__ __forceinline__ void grid_wait_for(P& a, P& b) { asm volatile("griddepcontrol.wait;" : "+l"(a), "+l"(b)::"memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>

@@ -116,3 +116,24 @@ def test_norm_in_the_linear_equals_the_two_kernels(testlib, kind, rows, n, swigl
     assert torch.equal(x.view(torch.int16), x_want.view(torch.int16)) and torch.equal(got.view(torch.int16), want.view(torch.int16))
     nm.x_out = src.data_ptr()  # every CTA reads src: it cannot be written
     assert testlib.gemv_rows_norm(C.byref(lin), C.byref(nm), p(got), swiglu, rows, None) != 0
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_weights_written_by_the_kernel_in_front(mine, kind):
+    """A linear starts while the kernel in front of it finishes: weights that this one writes are waited for all the same."""
+    n, k, gen = 4864, 1024, torch.Generator(device="cuda").manual_seed(kind)
+    per_row = k // 4 if kind == 2 else k // 2  # bf16 values whose bytes are a row of weights
+    gu = torch.randn((n, 2 * per_row), device="cuda", generator=gen).bfloat16()
+    x = torch.randn((9, k), device="cuda", generator=gen).bfloat16()
+    _, s, _ = weights(kind, n, k, 32, 5)
+    w, got, want = torch.empty((n, per_row), dtype=torch.bfloat16, device="cuda"), *(torch.empty((9, n), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    assert mine.s2pk_silu_mul(p(gu), p(w), n, per_row, None) == 0
+    torch.cuda.synchronize()
+    for rows in (1, 2, 3, 8, 9):
+        assert gemv(mine, kind, want, x, w, s, rows, n, k, 32) == 0
+        for _ in range(20):
+            w.view(torch.int16).fill_(0x1111)
+            torch.cuda.synchronize()
+            assert mine.s2pk_silu_mul(p(gu), p(w), n, per_row, None) == 0 and gemv(mine, kind, got, x, w, s, rows, n, k, 32) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(got[:rows].view(torch.int16), want[:rows].view(torch.int16)), rows
