@@ -52,9 +52,9 @@ template <bool KV8, int QT, int NW, bool APART> struct AttnPrefillSmem {
     alignas(8) uint64_t kfull, kempty, vfull, vempty, pfull[NW], pempty[NW]; /* the last two: APART */
 };
 
-/* 16 payload bytes, from an address that may be aligned to 4 bytes only */
+/* 16 payload bytes, from an address that may be aligned to 4 bytes only; an ordinary load, because the kernel in front writes the slice's own */
 __device__ __forceinline__ uint4 attn_prefill_load16(const unsigned char* src, int wide) {
-    if (wide) return __ldg(reinterpret_cast<const uint4*>(src));
+    if (wide) return *reinterpret_cast<const uint4*>(src);
     const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
     return make_uint4(w[0], w[1], w[2], w[3]);
 }

@@ -214,7 +214,7 @@ __device__ __forceinline__ void lane_chains(const T (&t)[R], X x_word, float (&s
 }
 
 template <int WK, int MM, int NS, bool SW>
-__global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* x,
                                                        const void* __restrict__ w, const void* __restrict__ scales,
                                                        int M, int N, int K, int gshift, int settled) {
     typedef typename LaneTile<WK>::type tile_t;
@@ -419,7 +419,7 @@ template <int WK, int MM> struct RowPlan {
     }
 };
 template <int WK, int MM, bool SW, bool NORM>
-__global__ void __launch_bounds__(RowPlan<WK, MM>::WARPS * 32, 1) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x, NormIn nm,
+__global__ void __launch_bounds__(RowPlan<WK, MM>::WARPS * 32, 1) k_gemv_row(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* x, NormIn nm,
                                                                             const void* __restrict__ w, const void* __restrict__ scales, int N, int K, int gshift, int settled) {
     typedef typename LaneTile<WK>::type tile_t;
     constexpr int R = 4, RA = SW ? 2 : 4, W = RowPlan<WK, MM>::WARPS, D = RowPlan<WK, MM>::D; /* RA: rows of a unit that follow one another */

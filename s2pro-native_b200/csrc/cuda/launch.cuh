@@ -19,7 +19,10 @@
 #include <cuda_runtime.h>
 
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-/* The same for two pointers whose loads the compiler may take for constant over the kernel (const __restrict__) and else move in front. */
+/* A load through const __restrict__ (or __ldg) counts as constant over the whole kernel, and the kernel begins before the one in front of it has
+ * ended: the compiler may move such a load in front of the wait, and take it from a cache that nobody keeps coherent.  So what an
+ * earlier kernel may have written is read behind the wait, through a pointer that is not restricted; or through one that comes out of the wait, where what
+ * it points at is settled in some calls and not in others: */
 template <class P> __device__ __forceinline__ void grid_wait_for(P& a, P& b) { asm volatile("griddepcontrol.wait;" : "+l"(a), "+l"(b)::"memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(256) k_silu_mul(const __nv_bfloat16* __restric
 
 /* the same, eight columns per thread (ffn a multiple of 8, 16-byte aligned rows): two 16-byte loads, one
  * 16-byte store, one division per eight elements instead of one 64-bit division per element */
-__global__ void __launch_bounds__(256) k_silu_mul8(const uint4* __restrict__ gu, uint4* __restrict__ h, unsigned n_units,
+__global__ void __launch_bounds__(256) k_silu_mul8(const uint4* gu, uint4* __restrict__ h, unsigned n_units,
                                                    unsigned f8) {
     grid_wait();
     grid_release();

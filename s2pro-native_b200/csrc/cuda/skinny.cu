@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(256) k_wide_convert(const void* __restrict__ w
 
 /* activations [M, K] bf16 -> f16 units [k / 8][NB rows], rows beyond M zero; a thread per unit, 8 units of 4 rows per warp */
 template <int WK>
-__global__ void __launch_bounds__(256) k_wide_pack(const __nv_bfloat16* __restrict__ x, int M, int K, int lgNB, uint4* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_wide_pack(const __nv_bfloat16* x, int M, int K, int lgNB, uint4* __restrict__ out) {
     grid_release(); /* a wide linear is next: see launch.cuh */
     grid_wait();
     const int u = blockIdx.x * 256 + threadIdx.x, lane = u & 31, g = u >> 5;
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(256) k_wide_pack(const __nv_bfloat16* __restri
     const int slab = g / rg, row = (g - slab * rg) * 4 + (lane >> 3), k8 = slab * 8 + (lane & 7);
     if (slab >= (K >> 6)) return;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (row < M) v = __ldg(reinterpret_cast<const uint4*>(x + (size_t)row * K) + k8);
+    if (row < M) v = reinterpret_cast<const uint4*>(x + (size_t)row * K)[k8];
     out[((size_t)k8 << lgNB) + row] = sk_x_unit<WK>(v);
 }
 

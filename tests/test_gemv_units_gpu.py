@@ -137,3 +137,29 @@ def test_weights_written_by_the_kernel_in_front(mine, kind):
             assert mine.s2pk_silu_mul(p(gu), p(w), n, per_row, None) == 0 and gemv(mine, kind, got, x, w, s, rows, n, k, 32) == 0
             torch.cuda.synchronize()
             assert torch.equal(got[:rows].view(torch.int16), want[:rows].view(torch.int16)), rows
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_activations_written_by_the_kernel_in_front(mine, kind):
+    """The same for the activations, which every caller's chain writes just before: SwiGLU, linear, SwiGLU, each reading the one in front."""
+    n, k, gen = 4864, 9728, torch.Generator(device="cuda").manual_seed(7 + kind)
+    w, s, _ = weights(kind, n, k, 32, 9)
+    gu = torch.randn((9, 2 * k), device="cuda", generator=gen).bfloat16()
+    bufs = [torch.empty((9, c), dtype=torch.bfloat16, device="cuda") for c in (k, n, n // 2)]  # x, y, h
+    for rows in (1, 2, 3, 8, 9):
+        def chain(wait):
+            x, y, h = bufs
+            assert mine.s2pk_silu_mul(p(gu), p(x), rows, k, None) == 0
+            wait()
+            assert gemv(mine, kind, y, x, w, s, rows, n, k, 32) == 0
+            wait()
+            assert mine.s2pk_silu_mul(p(y), p(h), rows, n // 2, None) == 0
+            torch.cuda.synchronize()
+        chain(torch.cuda.synchronize)
+        want = [b[:rows].clone() for b in bufs]
+        for _ in range(20):
+            for b in bufs:
+                b.view(torch.int16).fill_(0x4111)
+            torch.cuda.synchronize()
+            chain(lambda: None)
+            assert all(torch.equal(b[:rows].view(torch.int16), v.view(torch.int16)) for b, v in zip(bufs, want)), rows
