@@ -2,13 +2,14 @@
  * s2p_int8_gemv, s2p_intq_gemv, s2p_int4p_gemv — the reference's
  * src/sched/int8_gemv.cu:964-986, :773-799, :836-902.
  *
- * One and two rows, and up to four of a matrix of few rows, run k_gemv_row; up to 16 rows run
- * k_gemv_batch, where codes are widened once per tile for up to eight rows.  Every
+ * Up to 16 rows run k_gemv_batch, where codes are widened once per tile for up to eight rows, or up to four
+ * k_gemv_row where that is faster (gemv_row_grid), which also takes the norm in front.  Every
  * row of x is an independent product with one summation order (the reference's
  * batched GEMV computes rows independently too, int8_gemv.cu:77-91).  The stage
  * kernel of gemv.cuh (k_gemv_stage) serves the fused per-stage frame only.
  */
 #include <stdio.h>
+#include <type_traits>
 #include "gemv.cuh"
 #include "ops.h"
 #include "packed.cuh"
@@ -106,8 +107,8 @@ extern "C" cudaError_t gemv_setup_all(void) {
     return e;
 }
 
-/* ---- exact-order small batch (2 <= M <= 16) -------------------------------
- * Lane l owns k = 512 i + 16 l .. +15 of every tile i, as for M == 1; a warp carries four weight rows and MM activation
+/* ---- exact-order small batch (1 <= M <= 16) -------------------------------
+ * Lane l owns k = 512 i + 16 l .. +15 of every tile i; a warp carries four weight rows and MM activation
  * rows, 4 x MM independent chains.
  *
  * What bounds it: issue.  A chain step is one mixed fma (bf16 x bf16 + f32: the bits of fmaf), which costs 1.33 cycles of a scheduler because
@@ -118,10 +119,12 @@ extern "C" cudaError_t gemv_setup_all(void) {
  *
  * A matrix of few rows does not fill the GPU with warps of four rows, and a lone warp per scheduler waits on its own
  * latencies.  There NS = 4 warps share four rows and take tiles in turn; the tiles' chain results meet in shared memory and each warp
- * folds a quarter of the activation rows, tiles ascending.
+ * folds one of the weight rows for all activation rows, tiles ascending.  (Where a warp folded four weight rows for a share of the activation rows,
+ * three of the four had nothing to do for one row and less than their share for five to seven: 2560 x 4096 INT8, us, 1 / 5 / 8 rows 5.6 / 7.9 / 8.6, so
+ * 4.6 / 7.0 / 8.5.)
  * Measured, ticks of the full model, ms, before (two activation rows to a packed fma, each widened to f32; 168 registers) and now: 3 rows INT4
  * 4.25 -> 4.06, 8 rows INT4 8.12 -> 6.55, 16 rows INT8 12.80 -> 10.81.  CTAs to an SM: of the shared form 5 (8 rows 7.23 with 4); of the other 4,
- * where up to four rows are slower by 1 % than with 3.  16 rows of 19456 x 2560 INT4 take 50 us, 16 T fma/s of the 30 that a loop of mixed fma
+ * where up to four rows are slower by 1 % than with 3.  16 rows of 19456 x 2560 INT4 take 50 us, 16 T fma/s of the 28 that a loop of mixed fma
  * alone reaches. */
 /* A SwiGLU over stacked [gate | up] rows (SW): half of a warp's rows are of either half, so gate and up of an output meet in
  * the warp; both round to bf16 first, as where a kernel of its own follows the linear. */
@@ -213,14 +216,24 @@ __device__ __forceinline__ void lane_chains(const T (&t)[R], X x_word, float (&s
     }
 }
 
+/* Tiles of weights under way in a warp, CTAs to an SM.  One and two rows have registers for more of either; which hides more was measured for
+ * each, us.  Alone: INT8 6144 x 2560 and 19456 x 2560, one row 6.0 and 11.3 (6 CTAs, a tile: 5.5 and 11.8; 8: 5.9 and 12.8), grouped INT8 6.1 and 12.3 (two
+ * tiles 6.7 and 11.6), two rows 6.7 and 14.0 (5: 7.4 and 13.3; 8: 7.3 and 15.1); packed INT4 155776 x 2560, one row 53 (6 CTAs 61, two tiles 70).
+ * Shared: 2560 x 4096 in a tick, one row INT8 3.5, INT4 2.6 (6 CTAs, a tile 4.3, 3.0; 4 CTAs 3.4, 4.1); two rows 4.6 (4 CTAs, two tiles 6.1; 7: 4.9). */
+template <int WK, int MM, int NS> struct BatchPlan {
+    static constexpr int CTAS = NS > 1 ? (MM == 2 ? 6 : 5) : MM == 1 ? (WK == WK_INT4_PACK ? 8 : WK == WK_INT8_CH ? 5 : 6) : MM == 2 ? 6 : MM <= 4 ? 3 : 4;
+    static constexpr int PD = (MM == 1 && (NS > 1 || WK == WK_INT8_CH)) || (NS == 1 && MM > 2 && MM <= 4 && WK == WK_INT4_PACK) ? 2 : 1;
+};
 template <int WK, int MM, int NS, bool SW>
-__global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* x,
+__global__ void __launch_bounds__(128, (BatchPlan<WK, MM, NS>::CTAS)) k_gemv_batch(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* x,
                                                        const void* __restrict__ w, const void* __restrict__ scales,
                                                        int M, int N, int K, int gshift, int settled) {
     typedef typename LaneTile<WK>::type tile_t;
     constexpr int R = 4; /* weight rows of a warp */
-    constexpr int PD = WK == WK_INT4_PACK && MM <= 4 ? 2 : 1; /* tiles of weights under way */
-    constexpr int FM = NS == 1 ? MM : (MM + NS - 1) / NS; /* activation rows whose sums this warp keeps */
+    constexpr int PD = BatchPlan<WK, MM, NS>::PD;
+    constexpr int KEPT = NS == 1 ? R : 1; /* weight rows whose sums this warp keeps: all four, or the one of its number */
+    static_assert(NS == 1 || NS == R, "a weight row each");
+    typedef typename std::conditional<(MM <= 2), Codes<WK>, BatchCodes<WK>>::type C; /* few chains to a code leave registers for the cheaper conversion */
     __shared__ float part[NS == 1 ? 1 : 2 * NS * (MM + 1) * R * 32]; /* [round parity][tile of the round][m, then the scales][row][lane] */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int F = SW ? N >> 1 : N; /* outputs */
@@ -241,17 +254,18 @@ __global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batc
         wrow[r] = static_cast<const unsigned char*>(w) + (size_t)n * row_bytes + (size_t)lane * sizeof(tile_t);
         srow[r] = static_cast<const __half*>(scales) + (size_t)n * spr;
     }
-    float acc[FM][R];
+    float acc[MM][KEPT];
 #pragma unroll
-    for (int m = 0; m < FM; m++)
+    for (int m = 0; m < MM; m++)
 #pragma unroll
-        for (int r = 0; r < R; r++) acc[m][r] = 0.f;
+        for (int r = 0; r < KEPT; r++) acc[m][r] = 0.f;
     tile_t nxt[PD][R];
     __half gnx[PD][R];
     auto fetch = [&](int d, int i) {
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            nxt[d][r] = *reinterpret_cast<const tile_t*>(wrow[r] + (size_t)i * 32 * sizeof(tile_t));
+            const tile_t* at = reinterpret_cast<const tile_t*>(wrow[r] + (size_t)i * 32 * sizeof(tile_t));
+            nxt[d][r] = MM <= 2 ? __ldcs(at) : *at;
             gnx[d][r] = WK != WK_INT8_CH ? srow[r][(i * 512 + lane * 16) >> gshift] : __half(0.f);
         }
     };
@@ -280,14 +294,14 @@ __global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batc
             float s[MM][R];
             uint4 xv[MM];
             const __nv_bfloat16* xt = x + i * 512;
-            lane_chains<BatchCodes<WK>, MM, R>(cur, [&](int m, int i2) {
+            lane_chains<C, MM, R>(cur, [&](int m, int i2) {
                 if ((i2 & 3) == 0) xv[m] = *reinterpret_cast<const uint4*>(xt + x_row[m] + i2 * 2);
                 const uint4& v = xv[m];
                 return (i2 & 3) == 0 ? v.x : (i2 & 3) == 1 ? v.y : (i2 & 3) == 2 ? v.z : v.w;
             }, s);
             if (NS == 1) {
 #pragma unroll
-                for (int r = 0; r < R; r++)
+                for (int r = 0; r < KEPT; r++)
 #pragma unroll
                     for (int m = 0; m < MM; m++)
                         acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + s[m][r] : __fmaf_rn(s[m][r], gs[r], acc[m][r]);
@@ -301,35 +315,41 @@ __global__ void __launch_bounds__(128, NS > 1 ? 5 : MM <= 4 ? 3 : 4) k_gemv_batc
                 }
             }
         }
-        if (NS > 1) { /* the round's tiles in ascending order, for this warp's activation rows */
+        if (NS > 1) { /* the round's tiles in ascending order, for this warp's weight row */
             __syncthreads();
             const int live = min(NS, T - rnd * NS);
-            for (int t = 0; t < live; t++) {
-                const float* at = part + ((rnd & 1) * NS + t) * ((MM + 1) * R * 32) + lane;
+            const float* at = part + (rnd & 1) * NS * ((MM + 1) * R * 32) + ns * 32 + lane;
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const float g = WK != WK_INT8_CH ? at[(MM * R + r) * 32] : 1.f;
+            for (int t = 0; t < NS; t++, at += (MM + 1) * R * 32) {
+                if (t >= live) break;
+                const float g = WK != WK_INT8_CH ? at[MM * R * 32] : 1.f;
 #pragma unroll
-                    for (int m = 0; m < FM; m++) {
-                        const int mm = ns * FM + m;
-                        if (FM * NS > MM && mm >= MM) continue;
-                        const float v = at[(mm * R + r) * 32];
-                        acc[m][r] = WK == WK_INT8_CH ? acc[m][r] + v : __fmaf_rn(v, g, acc[m][r]);
-                    }
-                }
+                for (int m = 0; m < MM; m++) acc[m][0] = WK == WK_INT8_CH ? acc[m][0] + at[m * R * 32] : __fmaf_rn(at[m * R * 32], g, acc[m][0]);
             }
         }
+    }
+    if (NS > 1) { /* the lane trees of four activation rows packed into one: lane 8 j ends with the sum of row m + j */
+        const int n = n0 + ns;
+        const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[min(n, N - 1)] : 1.f;
+        auto of = [&](int m) { return m < MM ? acc[m < MM ? m : 0][0] : 0.f; };
+#pragma unroll
+        for (int m = 0; m < MM; m += 4) {
+            float a = MM == 1 ? warp_tree_sum(of(m)) : warp_tree4<false>(of(m), of(m + 1), of(m + 2), of(m + 3), lane);
+            if (WK == WK_INT8_CH) a = __fmul_rn(a, rs);
+            const int mm = m + (lane >> 3);
+            if ((lane & 7) == 0 && mm < M && n < N) y[(size_t)mm * N + n] = f2bf(a);
+        }
+        return;
     }
     /* the four rows' lane trees packed into one: lane 8 r ends with row r's sum */
     const int r = lane >> 3, n = n0 + r;
     const float rs = WK == WK_INT8_CH ? static_cast<const float*>(scales)[gemv_row_of<SW, R>(n0, r, F)] : 1.f;
 #pragma unroll
-    for (int m = 0; m < FM; m++) {
-        const int mm = NS == 1 ? m : ns * FM + m;
-        float a = warp_tree4<false>(acc[m][0], acc[m][1], acc[m][2], acc[m][3], lane);
+    for (int m = 0; m < MM; m++) {
+        float a = warp_tree4<false>(acc[m][0], acc[m][KEPT > 1 ? 1 : 0], acc[m][KEPT > 1 ? 2 : 0], acc[m][KEPT > 1 ? 3 : 0], lane);
         if (WK == WK_INT8_CH) a = __fmul_rn(a, rs);
         if (SW) a = gemv_swiglu(a, __shfl_down_sync(S2P_FULL_MASK, a, 16));
-        if ((lane & 7) == 0 && mm < M && n < F && r < (SW ? R / 2 : R)) y[(size_t)mm * F + n] = f2bf(a);
+        if ((lane & 7) == 0 && m < M && n < F && r < (SW ? R / 2 : R)) y[(size_t)m * F + n] = f2bf(a);
     }
 }
 
@@ -342,24 +362,26 @@ static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const v
     return launch_after(k_gemv_batch<WK, MM, NS, SW>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift, early);
 }
+/* Four warps share four rows where the CTAs of the shared form all fit the GPU at once, up to 2960 rows of weights, 3552 for two rows
+ * (3552 x 2560 INT8, us, shared and not, one row 5.4 and 4.6, two 4.4 and 5.7, three 6.8 and 5.2); also where one warp each would leave a scheduler with
+ * less than 2.5, which do not hide each other's latencies, provided that three quarters of the rounds' turns have a tile (a CTA waits for its slowest
+ * warp).  (A SwiGLU's pairs of rows meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
+static bool gemv_batch_fits_shared(int M, int N) { return (long long)((N + 3) / 4) * ((M + 7) / 8) <= (M == 2 ? 6ll : 5ll) * device_sm_count(); }
 template <int WK, bool SW>
 cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K,
                               int gshift, int early, cudaStream_t stream) {
-    /* As few groups of activation rows as eight a group allow (each converts every code once), of one size.  Four warps share
-     * four rows where one warp each would leave a scheduler with less than 2.5, which do not hide each other's latencies, provided
-     * that three quarters of the rounds' turns have a tile (a CTA waits for its slowest warp: at K = 2560, five tiles
-     * in eight turns, sharing loses), or where less than every second scheduler would get a warp at all.  (A SwiGLU's pairs of rows
-     * meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
+    /* as few groups of activation rows as eight a group allow (each converts every code once), of one size */
     const int groups = (M + 7) / 8;
     const int mm = (M + groups - 1) / groups;
     const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
     const int T = K >> 9, turns = (T + 3) / 4 * 4;
-    const bool shared = !SW && (2 * warps < sched || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
+    const bool shared = !SW && (gemv_batch_fits_shared(M, N) || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
 #define S2P_GB(MM)                                                                                            \
     do {                                                                                                      \
         if (shared) return run_gemv_batch<WK, MM, SW ? 1 : 4, SW>(y, x, w, scales, M, N, K, gshift, early, stream); \
         return run_gemv_batch<WK, MM, 1, SW>(y, x, w, scales, M, N, K, gshift, early, stream);                \
     } while (0)
+    if (mm == 1) S2P_GB(1);
     if (mm == 2) S2P_GB(2);
     if (mm == 3) S2P_GB(3);
     if (mm == 4) S2P_GB(4);
@@ -373,8 +395,8 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
 #undef S2P_GB
 }
 
-/* ---- one and two rows; up to four of a matrix of few rows --------------------------
- * The linear alone, as callers' own layers and small ticks of a model on one GPU use it.
+/* ---- one and two rows; up to four of a matrix of middling size ---------------------
+ * The linear alone or with the add and norm in front of it, as small ticks of a model on one GPU and callers' own layers use it.
  *
  * A CTA per SM owns a contiguous block of rows.  Its work is cut into units of four rows x one K tile, tile-major, and a warp takes a
  * contiguous run of units: its activations stay in registers, its weights have no order to wait for (all units are independent chains),
@@ -386,15 +408,19 @@ cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void*
  * chains: 3.3 cycles per weight and scheduler for INT4, 4.1 for INT8 in a loop of nothing else, which is 4.5 us for 19456 x 2560 INT4
  * (its bytes take 4.3).  The mixed fma runs at the rate of fmaf and reads either half of its registers, so an activation costs nothing and
  * an INT4 pair one logic operation, one shift and one subtraction; packed f32 chains needed a conversion of either side.
- * Measured, us, launches of one matrix back to back in a graph, before (k packed over two rows of weights, warps of four rows, four warps to
- * a row's tiles where rows are few) and now:
- *             6144 x 2560    2560 x 4096    19456 x 2560   2560 x 9728
- *   INT4 1    7.6 -> 4.4     3.8 -> 3.9     13.1 -> 9.5    9.0 -> 6.2
- *   INT4 2    7.5 -> 6.1     5.0 -> 5.1     15.6 -> 13.5   12.3 -> 8.2
- *   INT8 1    6.6 -> 5.3     4.1 -> 4.7     10.1 -> 11.1   8.8 -> 7.1
- *   INT8 2    8.2 -> 7.1     5.8 -> 6.1     13.8 -> 14.8   12.5 -> 9.1
- *   INT4 3                   7.3 -> 5.9                    16.8 -> 10.0        (INT8 8.2 -> 6.3, 15.8 -> 10.2)
- *   INT4 4                   7.1 -> 6.9                    16.8 -> 14.9        (INT8 8.8 -> 7.3, 16.7 -> 11.7)
+ * Measured, us, launches of one matrix back to back in a graph (more of its copies than L2 holds), before (k packed over two rows of weights, warps of
+ * four rows, four warps to a row's tiles where rows are few) and now; * is k_gemv_batch's now, see gemv_batch_faster:
+ *                   6144 x 2560    2560 x 4096     19456 x 2560     2560 x 9728
+ *   tick    INT4 1   7.4 -> 4.0     3.4 -> 2.6 *   13.1 -> 9.3      8.7 -> 5.4 *
+ *           INT4 2   7.3 -> 5.8     4.8 -> 4.6 *   15.5 -> 13.4    11.9 -> 8.0
+ *           INT8 1   6.4 -> 5.0     3.8 -> 3.5 *   10.4 -> 11.5     8.7 -> 7.0
+ *           INT8 2   8.1 -> 6.8     5.5 -> 4.7 *   14.1 -> 15.1    12.5 -> 9.0
+ *   caller  INT4 1   6.2 -> 5.0     4.8 -> 3.5 *   12.8 -> 10.6     9.9 -> 6.4 *
+ *           INT4 2   6.9 -> 6.2 *   6.0 -> 5.3 *   15.7 -> 12.9 *  13.2 -> 9.0
+ *           INT8 1   6.2 -> 6.0 *   4.8 -> 4.7 *   11.4 -> 11.5 *   8.7 -> 8.3
+ *           INT8 2   7.1 -> 6.7 *   6.5 -> 5.3 *   14.7 -> 13.9 *  12.2 -> 10.2
+ * (In a tick the two wide matrices carry the norm, which the launch that it saves pays for; 19456 x 2560 INT8 alone is the one entry that lost.
+ * 155776 x 2560, a caller's one row: INT8 61.7 -> 63.2, INT4 72 -> 53.)
  * At 64 registers, two CTAs to an SM, the frame took 3.67 ms instead of 2.68; 24 warps of 80 registers and other depths were within 1 %.
  *
  * NORM: the residual add and the norm in front of the linear, taken by every CTA while its first weights are on their way, instead of a
@@ -410,12 +436,11 @@ template <int WK, int MM> struct RowPlan {
         const int rows_a = sw ? 2 : 4, units = (outputs + rows_a - 1) / rows_a, T = K / 512;
         return (size_t)MM * units * R * T * 32 * sizeof(float) + (WK == WK_INT8_CH ? 0 : ((size_t)units * R * (K >> gshift) * 2 + 15) & ~(size_t)15);
     }
-    /* CTAs: one per SM, or as many per SM as keep the sums in shared memory; 0 where four rows do not fit, or offsets would not fit 32 bits */
+    /* CTAs, one per SM; 0 where the sums do not fit its shared memory (in several turns 155776 x 2560 took 68 us for one row of INT4 and
+     * 106 for two, k_gemv_batch 53 and 77), or offsets would not fit 32 bits */
     static int grid(int F, int K, int gshift, bool sw, int sms) {
-        if (smem(1, K, gshift, sw) > LIMIT || (size_t)F * (sw ? 2 : 1) * K > 0xF0000000ull) return 0;
-        int g = sms;
-        while (smem((F + g - 1) / g, K, gshift, sw) > LIMIT) g += sms;
-        return g < F ? g : F;
+        const int g = sms < F ? sms : F;
+        return smem((F + g - 1) / g, K, gshift, sw) > LIMIT || (size_t)F * (sw ? 2 : 1) * K > 0xF0000000ull ? 0 : g;
     }
 };
 template <int WK, int MM, bool SW, bool NORM>
@@ -624,14 +649,31 @@ static cudaError_t run_gemv_row(int grid, void* y, const void* x, const NormIn* 
     return launch_after(k_gemv_row<WK, MM, SW, NORM>, dim3((unsigned)grid), Plan::WARPS * 32, smem, stream,
                         (__nv_bfloat16*)y, (const __nv_bfloat16*)x, nm, w, scales, N, K, gshift, early);
 }
-/* The CTAs of k_gemv_row for M rows, 0 where k_gemv_batch takes them.  Three and four rows only where the batch kernel would leave a
- * scheduler fewer than two warps: 3 / 4 rows INT4 of 2560 x 9728 10.0 / 14.9 us (batch 15.3 / 16.5), but 7.4 / 8.4 (6.6 / 7.2) of 6144 x 2560
- * and 19.6 / 23.2 (16.9 / 18.4) of 19456 x 2560, whose sums need two CTAs to an SM. */
+/* the CTAs of k_gemv_row for M rows, 0 where it cannot take them */
 template <int WK, bool SW> static int gemv_row_grid(int M, int N, int K, int gshift) {
     const int F = SW ? N >> 1 : N, sms = device_sm_count();
-    if (M > 4 || (M > 2 && (N + 3) / 4 >= 2 * 4 * sms)) return 0;
-    return M == 1 ? RowPlan<WK, 1>::grid(F, K, gshift, SW, sms) : M == 2 ? RowPlan<WK, 2>::grid(F, K, gshift, SW, sms)
-         : M == 3 ? RowPlan<WK, 3>::grid(F, K, gshift, SW, sms) : RowPlan<WK, 4>::grid(F, K, gshift, SW, sms);
+    switch (M) {
+    case 1: return RowPlan<WK, 1>::grid(F, K, gshift, SW, sms);
+    case 2: return RowPlan<WK, 2>::grid(F, K, gshift, SW, sms);
+    case 3: return RowPlan<WK, 3>::grid(F, K, gshift, SW, sms);
+    case 4: return RowPlan<WK, 4>::grid(F, K, gshift, SW, sms);
+    }
+    return 0;
+}
+/* Whether k_gemv_batch is the faster of the two for a linear without the norm.  Both sides in us, k_gemv_row first; callers' calls, a tick's in brackets:
+ *  - few rows of weights, shared by a CTA's warps: 2560 x 4096, one row INT8 5.6 / 4.7 (4.4 / 3.5), grouped 5.6 / 4.8 (4.4 / 3.5), INT4 4.5 / 3.5 (3.7 / 2.6),
+ *    two 6.9 / 5.3, 6.8 / 5.5, 5.7 / 5.3, four INT4 7.6 / 5.5.  But each further round of a CTA's tiles costs two barriers, which few chains do not make
+ *    up for: one row INT8 x 6144 6.4 / 5.9 (5.2 / 5.3), x 9728 8.3 / 8.1 (7.0 / 7.5); two rows x 9728 INT4 9.0 / 10.2, four INT8 13.1 / 13.6.  One, three and four
+ *    rows of INT4 and four of grouped INT8 keep the gain at any length (x 9728 7.0 / 6.4, 10.8 / 9.4, 15.4 / 11.3; 16.7 / 13.7);
+ *  - from two warps of four rows to a scheduler, three and four rows (4097 x 2560, three rows INT4 5.9 / 6.3 (5.1 / 5.8); 6144 x 2560 7.4 / 6.5).  One and two rows only
+ *    outside a tick: a caller's weights are not asked for before the wait, and more, smaller CTAs have more of them under way then (6144 x 2560 INT8 two
+ *    rows 8.1 / 6.7 (7.0 / 6.4), 19456 x 2560 one row 13.1 / 11.5 (11.5 / 11.0), two 16.7 / 13.9 (15.3 / 13.7)).  One row of packed INT4 has too few
+ *    instructions for that to matter (5.0 / 5.3, 10.6 / 10.5). */
+template <int WK, bool SW> static bool gemv_batch_faster(int M, int N, int K, int early) {
+    if (M > 4) return true;
+    if (!SW && gemv_batch_fits_shared(M, N)) return K <= 12 * 512 || (WK == WK_INT4_PACK ? M != 2 : WK == WK_INT8_GRP && M == 4);
+    const bool many = (N + 3) / 4 >= 2 * 4 * device_sm_count();
+    return many && (M > 2 || (!early && (M == 2 || WK != WK_INT4_PACK)));
 }
 template <int WK, bool SW>
 static cudaError_t launch_gemv_row(int grid, void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
@@ -665,7 +707,7 @@ s2p_status gemv_entry(const char* what, void* y, const void* x, const void* w, c
     /* 16-byte loads of activations and weight tiles */
     if (((uintptr_t)x | (uintptr_t)w) & 15) return S2P_ERR_INVALID;
     cudaError_t ce;
-    const int grid = gemv_row_grid<WK, SW>(M, N, K, gshift);
+    const int grid = gemv_batch_faster<WK, SW>(M, N, K, early) ? 0 : gemv_row_grid<WK, SW>(M, N, K, gshift);
     if (grid) {
         ce = launch_gemv_row<WK, SW>(grid, y, x, w, scales, M, N, K, gshift, early, stream);
     } else {

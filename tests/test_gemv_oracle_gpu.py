@@ -14,23 +14,22 @@ def p(t):
     return C.c_void_p(t.data_ptr())
 
 
-@pytest.mark.parametrize("kind", ["int8", "int8_grouped", "int4"])
-@pytest.mark.parametrize("n,k,all_rows", [(37, 512, True), (1029, 4608, True), (6145, 1024, True), (14209, 512, False), (19457, 512, False)])
-def test_every_batch_size_gives_the_oracles_bits(mine, oracle, kind, n, k, all_rows):
+def against_the_oracle(mine, oracle, kind, n, k, batches):
     from oracle import oracle_api
+    most = max(batches)
     rng = np.random.default_rng(n)
     w = rng.integers(0, 256, size=(n, k // 2 if kind == "int4" else k), dtype=np.uint8)
     s = rng.random((n, 1 if kind == "int8" else k // G), dtype=np.float32) * 0.01 + 0.001
     s = s if kind == "int8" else s.astype(np.float16)
-    x = oracle_api.f32_to_bf16(rng.standard_normal((16, k), dtype=np.float32))
-    want = np.empty((16, n), np.uint16)
-    args = [oracle_api.ptr(a) for a in (want, x, w, s)] + [16, n, k]
+    x = oracle_api.f32_to_bf16(rng.standard_normal((most, k), dtype=np.float32))
+    want = np.empty((most, n), np.uint16)
+    args = [oracle_api.ptr(a) for a in (want, x, w, s)] + [most, n, k]
     if kind == "int8":
         oracle.s2po_gemv_int8(*args)
     else:
         (oracle.s2po_gemv_g if kind == "int8_grouped" else oracle.s2po_gemv_p)(*args, G)
     dw, ds, dx = (torch.from_numpy(a.view(np.int16) if a.dtype == np.uint16 else a).cuda() for a in (w, s, x))
-    for rows in range(1, 17) if all_rows else (1, 2):  # many rows of weights: what differs is the one-row kernel
+    for rows in batches:
         y = torch.full((rows + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
         args = [p(y), p(dx), p(dw), p(ds), rows, n, k]
         if kind == "int8":
@@ -40,3 +39,16 @@ def test_every_batch_size_gives_the_oracles_bits(mine, oracle, kind, n, k, all_r
         got = y.view(torch.int16).cpu().numpy().view(np.uint16)
         assert np.array_equal(got[:rows], want[:rows]), rows
         assert (got[rows] == oracle_api.f32_to_bf16(np.float32([7.0]))[0]).all()
+
+
+@pytest.mark.parametrize("kind", ["int8", "int8_grouped", "int4"])
+@pytest.mark.parametrize("n,k,all_rows", [(37, 512, True), (1029, 4608, True), (6145, 1024, True), (14209, 512, False), (19457, 512, False)])
+def test_every_batch_size_gives_the_oracles_bits(mine, oracle, kind, n, k, all_rows):
+    against_the_oracle(mine, oracle, kind, n, k, range(1, 17) if all_rows else (1, 2))  # many rows of weights: what differs is the one-row kernel
+
+
+# either side of where a CTA's warps stop sharing rows (148 SMs x 5 or 6 CTAs x 4 rows; 12 tiles of K) and of two warps to a scheduler
+@pytest.mark.parametrize("kind", ["int8", "int8_grouped", "int4"])
+@pytest.mark.parametrize("n,k", [(2960, 512), (2961, 1024), (3552, 512), (3553, 1024), (1029, 6144), (1029, 6656), (4732, 512), (4733, 1024)])
+def test_both_sides_of_a_rule_give_the_oracles_bits(mine, oracle, kind, n, k):
+    against_the_oracle(mine, oracle, kind, n, k, (1, 2, 3, 4, 5, 9))
