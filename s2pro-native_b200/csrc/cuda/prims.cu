@@ -764,17 +764,29 @@ __global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* __restrict_
 
 /* ---- VQ glue (fastar.cu:104-127; kernels.cu:1399-1421) --------------------- */
 /* a row per CTA, eight columns per thread, the vectors of all codebooks under way at once (one column and codebook after another 25 rows
- * took 52 us; a request with such a clip 6.94 -> 6.89 ms) */
+ * took 52 us; a request with such a clip 6.94 -> 6.89 ms).  WIDE: rows and table are 16-byte aligned, as a model's are; else an element at a time. */
 constexpr int VQ_THREADS = S2P_DIM / 8;
-__global__ void __launch_bounds__(VQ_THREADS) k_vq_embed_add(const uint4* __restrict__ table, const int32_t* __restrict__ codes, int T, uint4* __restrict__ rows) {
-    const int t = blockIdx.x, v = threadIdx.x;
+template <bool WIDE> __device__ __forceinline__ uint4 vq_load8(const __nv_bfloat16* at) {
+    if constexpr (WIDE) return *reinterpret_cast<const uint4*>(at);
+    else {
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) w[j] = (uint32_t)__bfloat16_as_ushort(at[2 * j]) | ((uint32_t)__bfloat16_as_ushort(at[2 * j + 1]) << 16);
+        return make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+template <bool WIDE>
+__global__ void __launch_bounds__(VQ_THREADS) k_vq_embed_add(const __nv_bfloat16* __restrict__ table, const int32_t* __restrict__ codes, int T,
+                                                             __nv_bfloat16* __restrict__ rows) {
+    const int t = blockIdx.x, v = threadIdx.x * 8;
     uint4 e[S2P_NUM_CODEBOOKS];
 #pragma unroll
     for (int cb = 0; cb < S2P_NUM_CODEBOOKS; cb++) {
         const int c = max(0, min(S2P_CB_SIZE - 1, codes[(size_t)cb * T + t]));
-        e[cb] = table[((size_t)cb * S2P_CB_SIZE + c) * VQ_THREADS + v];
+        e[cb] = vq_load8<WIDE>(table + ((size_t)cb * S2P_CB_SIZE + c) * S2P_DIM + v);
     }
-    uint4 x = rows[(size_t)t * VQ_THREADS + v];
+    __nv_bfloat16* const at = rows + (size_t)t * S2P_DIM + v;
+    uint4 x = vq_load8<WIDE>(at);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int cb = 0; cb < S2P_NUM_CODEBOOKS; cb++) {
@@ -786,7 +798,10 @@ __global__ void __launch_bounds__(VQ_THREADS) k_vq_embed_add(const uint4* __rest
 #pragma unroll
     for (int j = 0; j < 4; j++)
         xw[j] = add_bf16_pair(xw[j], (uint32_t)__bfloat16_as_ushort(f2bf(acc[2 * j])) | ((uint32_t)__bfloat16_as_ushort(f2bf(acc[2 * j + 1])) << 16));
-    rows[(size_t)t * VQ_THREADS + v] = x;
+    if (WIDE) *reinterpret_cast<uint4*>(at) = x;
+    else
+#pragma unroll
+        for (int j = 0; j < 8; j++) at[j] = __ushort_as_bfloat16((unsigned short)(xw[j >> 1] >> (16 * (j & 1))));
 }
 __global__ void __launch_bounds__(256) k_scale_div(__nv_bfloat16* __restrict__ x, int64_t n, float div) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -904,8 +919,8 @@ cudaError_t embed_rows_i8(const void* table, const float* scales, const int64_t*
 }
 cudaError_t vq_embed_add(const void* table, const int32_t* codes_dev, int T, void* rows, cudaStream_t st) {
     if (T <= 0) return cudaSuccess;
-    if (((uintptr_t)table | (uintptr_t)rows) & 15) return cudaErrorInvalidValue; /* model memory, 16-byte aligned */
-    k_vq_embed_add<<<T, VQ_THREADS, 0, st>>>((const uint4*)table, codes_dev, T, (uint4*)rows);
+    const bool wide = (((uintptr_t)table | (uintptr_t)rows) & 15) == 0;
+    (wide ? k_vq_embed_add<true> : k_vq_embed_add<false>)<<<T, VQ_THREADS, 0, st>>>((const __nv_bfloat16*)table, codes_dev, T, (__nv_bfloat16*)rows);
     return cudaGetLastError();
 }
 cudaError_t scale_div(void* x, int64_t n, float divisor, cudaStream_t st) {

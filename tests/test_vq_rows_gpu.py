@@ -8,12 +8,14 @@ torch = pytest.importorskip("torch")
 D, CB, N = 2560, 4096, 10
 
 
-@pytest.mark.parametrize("rows", [1, 25, 430])
-def test_rows(testlib, rows):
+@pytest.mark.parametrize("rows,table_off,rows_off", [(1, 0, 0), (25, 0, 0), (430, 0, 0), (3, 1, 0), (3, 0, 1), (3, 4, 2)])  # elements past an aligned address
+def test_rows(testlib, rows, table_off, rows_off):
     g = torch.Generator(device="cuda").manual_seed(rows)
-    table = (torch.randn(N * CB, D, device="cuda", generator=g) * 0.02).bfloat16()
+    at = lambda t, off: torch.cat([t.new_zeros(off), t.flatten()])[off:].view(t.shape)  # noqa: E731
+    table = at((torch.randn(N * CB, D, device="cuda", generator=g) * 0.02).bfloat16(), table_off)
     codes = torch.randint(-3, CB + 3, (N, rows), dtype=torch.int32, device="cuda", generator=g)  # clamped to the table
-    x = torch.randn(rows + 1, D, device="cuda", generator=g).bfloat16()
+    x = at(torch.randn(rows + 1, D, device="cuda", generator=g).bfloat16(), rows_off)
+    assert table.data_ptr() % 16 == 2 * table_off and x.data_ptr() % 16 == 2 * rows_off
     want = x.clone()
     acc = torch.zeros(rows, D, device="cuda")
     for c in range(N):
