@@ -26,7 +26,8 @@
  * single-buffered: the next split's keys are copied (cp.async, 16 bytes per request) while the
  * values of this one are summed, the next values while the next scores are formed.  Key rows are
  * staged with a 16-byte pad per row, which makes the per-lane 16-byte reads of 32 different rows
- * conflict-free.  Two CTAs of four teams fit an SM (16 warps); the kernel is bound by instruction
+ * conflict-free.  Three CTAs of three teams fit an SM with an INT8 cache (18 warps), two of four (16 warps) or, with
+ * a bf16 cache, of three (12 warps); the kernel is bound by instruction
  * issue on dependent chains, not by HBM, so warps per SM and instructions per split are what count
  * (one warp per split with twice the tiles per warp measured 6 % slower on INT8, 24 % on bf16).
  *
@@ -196,9 +197,18 @@ __global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode
     /* The grid is fixed per batch size (one captured graph serves every context length), so the CTAs
      * decide here how many of the `workers` per (row, kv head) take part: enough teams for about
      * ATTN_SPLITS_PER_TEAM splits each, so that the copies of one split overlap the arithmetic of
-     * another, but never so few CTAs that SMs stay empty.  The others go straight to the arrival counter. */
-    const int fill = ((KV8 && NT == 3 ? 3 : 2) * 148 + (int)(gridDim.x * gridDim.y) - 1) / (int)(gridDim.x * gridDim.y);
-    const int eff = min(workers, max(max(NT == 3 ? (n_active + NT * ATTN_SPLITS_PER_TEAM - 1) / (NT * ATTN_SPLITS_PER_TEAM) : n_active / (NT * ATTN_SPLITS_PER_TEAM), fill), 1));
+     * another, but never so few CTAs that SMs stay empty.  The others go straight to the arrival counter.
+     * Of the two counts around that share an INT8 cache's three CTAs to an SM take the higher: us, lower / higher, 8 x 8000 rows x positions 84 / 75,
+     * 16 x 6000 112 / 98, 64 x 1000 73 / 65, 64 x 3000 166 / 169, 128 x 1024 116 / 123.  With two CTAs to an SM it is the one whose CTAs take less
+     * time in all, a CTA the rounds of its busiest team and two more for its start and its partials: bf16 8 x 8000 97 / 93, 16 x 6000 120 / 114, 32 x 2000 72 / 77,
+     * 64 x 3000 183 / 191, 96 x 1000 100 / 116, 128 x 1024 134 / 147. */
+    constexpr bool THREES = KV8 && NT == 3;
+    constexpr int SHARE = NT * ATTN_SPLITS_PER_TEAM;
+    const int pairs = (int)(gridDim.x * gridDim.y), fill = ((THREES ? 3 : 2) * 148 + pairs - 1) / pairs;
+    auto time_of = [&](int e) { return e * ((n_active + e * NT - 1) / (e * NT) + 2); };
+    int share = (n_active + (THREES ? SHARE - 1 : 0)) / SHARE;
+    if (!THREES && share >= fill && share < workers && time_of(share + 1) < time_of(share)) share++;
+    const int eff = min(workers, max(share, fill));
     const int first = wk < eff ? wk + eff * team : n_active, step = eff * NT;
 
     auto fetch_k = [&](int spl) {
