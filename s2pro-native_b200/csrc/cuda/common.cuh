@@ -54,6 +54,17 @@ __device__ __forceinline__ float bf2f(__nv_bfloat16 v) { return __bfloat162float
 __device__ __forceinline__ __nv_bfloat16 f2bf(float v) { return __float2bfloat16(v); } /* RNE */
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
+/* two f32 adds of bf16 pairs, each rounded to bf16 */
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
+}
+/* silu(g) * u of bf16 values, before its own rounding (src/slowar/kernels.cu:1216-1229): silu is rounded to bf16 first.  The reciprocal is
+ * correctly rounded, so it has the bits of the division. */
+__device__ __forceinline__ float swiglu_f32(float g, float u) {
+    const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-g)));
+    return __fmul_rn(bf16_round(__fmul_rn(g, sig)), u);
+}
+
 /* Warp-level tree over lane values, off = 16,8,4,2,1; result in every lane. */
 __device__ __forceinline__ float warp_tree_sum(float v) {
 #pragma unroll
@@ -113,9 +124,15 @@ __device__ __forceinline__ float block_tree(float v, float* red) {
     return out;
 }
 
-/* The 256-value halving sum tree with two barriers instead of six: warp 0 forms the
- * pairs of the levels 128, 64 and 32 itself (lane t holds the values t + 32 j),
- * then the shuffle levels.  Same pairs as block_tree<256, false>, same result.
+/* The 256-value halving sum tree of red[0..255] in one warp: lane t forms the pairs of the levels 128, 64 and 32 itself (it
+ * holds the values t + 32 j), then the shuffle levels. */
+__device__ __forceinline__ float tree256_of(const float* red, int t) {
+    const float a0 = red[t] + red[t + 128], a1 = red[t + 32] + red[t + 160];
+    const float a2 = red[t + 64] + red[t + 192], a3 = red[t + 96] + red[t + 224];
+    return warp_tree_sum((a0 + a2) + (a1 + a3));
+}
+/* The 256-value halving sum tree with two barriers instead of six, the tree itself in warp 0.
+ * Same pairs as block_tree<256, false>, same result.
  * Thread t < 256 contributes v; `red` needs 256 floats and must not be written
  * again before the caller's next barrier.  All threads of the group must call it; `sync` is a
  * barrier over that group (the whole CTA in the two-argument form). */
@@ -125,9 +142,7 @@ __device__ __forceinline__ float tree256_sum(float v, float* red, SyncFn sync) {
     if (t < 256) red[t] = v;
     sync();
     if (t < 32) {
-        const float a0 = red[t] + red[t + 128], a1 = red[t + 32] + red[t + 160];
-        const float a2 = red[t + 64] + red[t + 192], a3 = red[t + 96] + red[t + 224];
-        const float r = warp_tree_sum((a0 + a2) + (a1 + a3));
+        const float r = tree256_of(red, t);
         if (t == 0) red[256] = r;
     }
     sync();

@@ -132,9 +132,7 @@ template <bool SW, int R> __device__ __forceinline__ int gemv_row_of(int n0, int
     return SW ? min(n0 + r % (R / 2), F - 1) + r / (R / 2) * F : min(n0 + r, F - 1);
 }
 __device__ __forceinline__ float gemv_swiglu(float gate, float up_) {
-    const float g = bf16_round(gate), up = bf16_round(up_);
-    const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-g))); /* correctly rounded, as the division */
-    return __fmul_rn(bf16_round(__fmul_rn(g, sig)), up);
+    return swiglu_f32(bf16_round(gate), bf16_round(up_));
 }
 /* Codes of a lane as operands of the mixed fma (fma.rn.f32.bf16: bf16 x bf16 + f32, one rounding, the same bits as fmaf on the widened
  * values).  STEP codes are converted together; get(w, j) is the j-th of them.  An activation needs no conversion at all: the fma
@@ -143,9 +141,6 @@ __device__ __forceinline__ unsigned short half_of(uint32_t v, bool high) {
     unsigned short lo, hi;
     asm("mov.b32 {%0, %1}, %2;" : "=h"(lo), "=h"(hi) : "r"(v));
     return high ? hi : lo;
-}
-__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) { /* two f32 adds, each rounded to bf16 */
-    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
 }
 template <int WK> struct Codes;
 template <> struct Codes<WK_INT8_CH> {
@@ -534,9 +529,8 @@ __global__ void __launch_bounds__(RowPlan<WK, MM>::WARPS * 32, 1) k_gemv_row(__n
             r[i0] = ss;
         }
         __syncthreads();
-        if (mine < MM && i0 < 32) { /* tree256_sum: the pairs of the levels 128, 64 and 32, then shuffles */
-            const float a0 = r[i0] + r[i0 + 128], a1 = r[i0 + 32] + r[i0 + 160], a2 = r[i0 + 64] + r[i0 + 192], a3 = r[i0 + 96] + r[i0 + 224];
-            const float tot = warp_tree_sum((a0 + a2) + (a1 + a3));
+        if (mine < MM && i0 < 32) {
+            const float tot = tree256_of(r, i0);
             if (i0 == 0) r[256] = tot;
         }
         __syncthreads();

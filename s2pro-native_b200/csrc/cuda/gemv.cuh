@@ -396,10 +396,7 @@ __device__ void gemv_stage_cta(const GemvStage& g, int row0, int cnt_total, unsi
                 const float gate = bf16_round(fold_row(r));
                 const float up = bf16_round(fold_row(r + cnt));
                 if (lane == 0) {
-                    /* src/slowar/kernels.cu:1216-1229: silu rounds to bf16 before the up-multiply */
-                    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-gate)));
-                    const float sil = bf16_round(__fmul_rn(gate, sig));
-                    g.y[r0 + r] = f2bf(__fmul_rn(sil, up));
+                    g.y[r0 + r] = f2bf(swiglu_f32(gate, up));
                 }
             }
         } else {

@@ -502,9 +502,7 @@ __device__ __noinline__ int gemv_fold(const MegaStage* gs, unsigned q0, unsigned
                     float gate = lane == 0 ? acc[0] : acc[1], up = lane == 0 ? acc[2] : acc[3];
                     if (WK == WK_INT8_CH) { gate = __fmul_rn(gate, rs_a); up = __fmul_rn(up, rs_b); }
                     gate = bf16_round(gate); up = bf16_round(up);
-                    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-gate)));
-                    const float sil = bf16_round(__fmul_rn(gate, sig));
-                    const __nv_bfloat16 v = f2bf(__fmul_rn(sil, up));
+                    const __nv_bfloat16 v = f2bf(swiglu_f32(gate, up));
                     if (y_ll) store_all(reinterpret_cast<uint32_t*>(d.y) + my_n, flag_word(v, my_tag));
                     else store_all(d.y + my_n, v);
                 } else {

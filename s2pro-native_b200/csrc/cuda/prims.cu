@@ -68,9 +68,6 @@ struct NormRowArgs {
     int settled;                 /* the gains are a model's: the kernel in front does not write them */
 };
 constexpr int NORM_MAX_WIDTH = 4096; /* two vectors per thread */
-__device__ __forceinline__ uint32_t add_bf16_pair(uint32_t a, uint32_t b) {
-    return (uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_lo(a), bf_lo(b)))) | ((uint32_t)__bfloat16_as_ushort(f2bf(__fadd_rn(bf_hi(a), bf_hi(b)))) << 16);
-}
 /* sum of squares over a row in shared memory: 256 strided chains, then the halving tree.  All threads of the CTA call it. */
 __device__ __forceinline__ float norm_inv(const __nv_bfloat16* xs, int width, float eps, float* red) {
     float ss = 0.f;
@@ -103,7 +100,7 @@ __global__ void __launch_bounds__(256) k_norm_row(NormRowArgs a) {
         uint4 q = src[v];
         if (add) {
             const uint4 p = add[v];
-            q = make_uint4(add_bf16_pair(q.x, p.x), add_bf16_pair(q.y, p.y), add_bf16_pair(q.z, p.z), add_bf16_pair(q.w, p.w));
+            q = make_uint4(add_bf16x2(q.x, p.x), add_bf16x2(q.y, p.y), add_bf16x2(q.z, p.z), add_bf16x2(q.w, p.w));
         }
         if (xo) xo[v] = q;
         reinterpret_cast<uint4*>(xs)[v] = q;
@@ -171,10 +168,10 @@ __global__ void __launch_bounds__(TICK_NORM_THREADS) k_norm_tick(NormRowArgs a) 
     uint2 x = reinterpret_cast<const uint2*>(a.src + row * S2P_DIM)[tid];
     if (a.part.partial && !a.part_logits) {
         const uint2 p = wide_part4_bf16<8>(a.part, tid * 4, r);
-        x = make_uint2(add_bf16_pair(x.x, p.x), add_bf16_pair(x.y, p.y));
+        x = make_uint2(add_bf16x2(x.x, p.x), add_bf16x2(x.y, p.y));
     } else if (a.add) {
         const uint2 p = reinterpret_cast<const uint2*>(a.add + (size_t)r * S2P_DIM)[tid];
-        x = make_uint2(add_bf16_pair(x.x, p.x), add_bf16_pair(x.y, p.y));
+        x = make_uint2(add_bf16x2(x.x, p.x), add_bf16x2(x.y, p.y));
     }
     if (a.x_out) reinterpret_cast<uint2*>(a.x_out + (size_t)r * S2P_DIM)[tid] = x;
     if (!a.w) return;
@@ -668,9 +665,7 @@ __global__ void __launch_bounds__(256) k_silu_mul(const __nv_bfloat16* __restric
         const int c = (int)(idx - r * ffn);
         const float g = bf2f(gu[(size_t)r * 2 * ffn + c]);
         const float u = bf2f(gu[(size_t)r * 2 * ffn + ffn + c]);
-        const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
-        const float sil = bf16_round(__fmul_rn(g, sig));
-        h[idx] = f2bf(__fmul_rn(sil, u));
+        h[idx] = f2bf(swiglu_f32(g, u));
     }
 }
 
@@ -691,9 +686,7 @@ __global__ void __launch_bounds__(256) k_silu_mul8(const uint4* gu, uint4* __res
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 const float g = k ? bf_hi(gw[j]) : bf_lo(gw[j]), up = k ? bf_hi(uw[j]) : bf_lo(uw[j]);
-                const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-g))); /* correctly rounded, as the division */
-                const float sil = bf16_round(__fmul_rn(g, sig));
-                r2[k] = __fmul_rn(sil, up);
+                r2[k] = swiglu_f32(g, up);
             }
             const __nv_bfloat162 pk = __halves2bfloat162(f2bf(r2[0]), f2bf(r2[1]));
             o[j] = *reinterpret_cast<const uint32_t*>(&pk);
@@ -797,7 +790,7 @@ __global__ void __launch_bounds__(VQ_THREADS) k_vq_embed_add(const __nv_bfloat16
     uint32_t* xw = &x.x;
 #pragma unroll
     for (int j = 0; j < 4; j++)
-        xw[j] = add_bf16_pair(xw[j], (uint32_t)__bfloat16_as_ushort(f2bf(acc[2 * j])) | ((uint32_t)__bfloat16_as_ushort(f2bf(acc[2 * j + 1])) << 16));
+        xw[j] = add_bf16x2(xw[j], (uint32_t)__bfloat16_as_ushort(f2bf(acc[2 * j])) | ((uint32_t)__bfloat16_as_ushort(f2bf(acc[2 * j + 1])) << 16));
     if (WIDE) *reinterpret_cast<uint4*>(at) = x;
     else
 #pragma unroll

@@ -137,7 +137,6 @@ __device__ void sampler_cta(const __nv_bfloat16* lrow, const __nv_bfloat16* eos_
     }
     S2P_CTA_SYNC();
     if (warp == 0) {
-    {
         int at = 0;
         int idx = lane < NW ? wt[lane * SMP_TOPK] : SMP_N_CAND;
         uint32_t key = idx < SMP_N_CAND ? sampler_key(cand[idx]) : 0u;
@@ -150,80 +149,79 @@ __device__ void sampler_cta(const __nv_bfloat16* lrow, const __nv_bfloat16* eos_
                 key = idx < SMP_N_CAND ? sampler_key(cand[idx]) : 0u;
             }
         }
-    }
-    __syncwarp();
-    int choice = 0;
-    if (!greedy) {
-        /* a rank per lane; the sums are the reference's, rank after rank */
-        const bool rank = lane < SMP_TOPK;
-        const float v = tv[rank ? lane : 0], m = tv[0];
-        auto sum_of = [](float x) {
-            float s = 0.f;
+        __syncwarp();
+        int choice = 0;
+        if (!greedy) {
+            /* a rank per lane; the sums are the reference's, rank after rank */
+            const bool rank = lane < SMP_TOPK;
+            const float v = tv[rank ? lane : 0], m = tv[0];
+            auto sum_of = [](float x) {
+                float s = 0.f;
 #pragma unroll
-            for (int j = 0; j < SMP_TOPK; j++) s = __fadd_rn(s, __shfl_sync(S2P_FULL_MASK, x, j));
-            return s;
-        };
-        const float e = expf(v - m);
-        const float share = __fdiv_rn(e, sum_of(e));
-        float cum = 0.f, upto = 0.f;
+                for (int j = 0; j < SMP_TOPK; j++) s = __fadd_rn(s, __shfl_sync(S2P_FULL_MASK, x, j));
+                return s;
+            };
+            const float e = expf(v - m);
+            const float share = __fdiv_rn(e, sum_of(e));
+            float cum = 0.f, upto = 0.f;
 #pragma unroll
-        for (int j = 0; j < SMP_TOPK; j++) {
-            cum = __fadd_rn(cum, __shfl_sync(S2P_FULL_MASK, share, j));
-            if (j == lane) upto = cum;
-        }
-        const bool masked = lane > 0 && upto > sh_topp;
-        const float t = sh_temp < 1e-5f ? 1e-5f : sh_temp;
-        const float m2 = __fdiv_rn(m, t);
-        float p2 = masked ? 0.f : expf(__fsub_rn(__fdiv_rn(v, t), m2));
-        p2 = __fdiv_rn(p2, sum_of(p2));
-
-        if (sp->seeded) {
-            const uint64_t step_seed = ((uint64_t)sp->seed31 * 19349663ULL) ^ (count0 * 73856093ULL);
-            const uint64_t hashed = (step_seed * 8589934591ULL) ^ ((uint64_t)lane * 479001599ULL);
-            float u = __fdiv_rn((float)(uint32_t)(hashed & 0xFFFFFFULL), 16777216.0f);
-            if (u < 1e-10f) u = 1e-10f;
-            const float g = -logf(-logf(u));
-            const float pert = __fadd_rn(logf(__fadd_rn(p2, 1e-10f)), g);
-            /* the first largest; what does not exceed -inf is never chosen, and rank 0 stands where nothing is */
-            const uint32_t key = rank && pert > -INFINITY ? sampler_key(pert) : 0u;
-            const uint32_t top = __reduce_max_sync(S2P_FULL_MASK, key);
-            choice = top ? __ffs(__ballot_sync(S2P_FULL_MASK, key == top)) - 1 : 0;
-        } else {
-            double r = 0.0;
-            if (lane == 0) r = (double)(xoshiro_next(sp->rng) >> 11) * 0x1.0p-53;
-            double cum2 = 0.0;
-            int lastnz = 0;
-            choice = -1;
-            for (int j = 0; j < SMP_TOPK; j++) { /* lane 0's result counts */
-                const float p = __shfl_sync(S2P_FULL_MASK, p2, j);
-                if (p <= 0.f) continue;
-                lastnz = j;
-                cum2 += (double)p;
-                if (choice < 0 && r < cum2) choice = j;
+            for (int j = 0; j < SMP_TOPK; j++) {
+                cum = __fadd_rn(cum, __shfl_sync(S2P_FULL_MASK, share, j));
+                if (j == lane) upto = cum;
             }
-            if (choice < 0) choice = lastnz;
+            const bool masked = lane > 0 && upto > sh_topp;
+            const float t = sh_temp < 1e-5f ? 1e-5f : sh_temp;
+            const float m2 = __fdiv_rn(m, t);
+            float p2 = masked ? 0.f : expf(__fsub_rn(__fdiv_rn(v, t), m2));
+            p2 = __fdiv_rn(p2, sum_of(p2));
+
+            if (sp->seeded) {
+                const uint64_t step_seed = ((uint64_t)sp->seed31 * 19349663ULL) ^ (count0 * 73856093ULL);
+                const uint64_t hashed = (step_seed * 8589934591ULL) ^ ((uint64_t)lane * 479001599ULL);
+                float u = __fdiv_rn((float)(uint32_t)(hashed & 0xFFFFFFULL), 16777216.0f);
+                if (u < 1e-10f) u = 1e-10f;
+                const float g = -logf(-logf(u));
+                const float pert = __fadd_rn(logf(__fadd_rn(p2, 1e-10f)), g);
+                /* the first largest; what does not exceed -inf is never chosen, and rank 0 stands where nothing is */
+                const uint32_t key = rank && pert > -INFINITY ? sampler_key(pert) : 0u;
+                const uint32_t top = __reduce_max_sync(S2P_FULL_MASK, key);
+                choice = top ? __ffs(__ballot_sync(S2P_FULL_MASK, key == top)) - 1 : 0;
+            } else {
+                double r = 0.0;
+                if (lane == 0) r = (double)(xoshiro_next(sp->rng) >> 11) * 0x1.0p-53;
+                double cum2 = 0.0;
+                int lastnz = 0;
+                choice = -1;
+                for (int j = 0; j < SMP_TOPK; j++) { /* lane 0's result counts */
+                    const float p = __shfl_sync(S2P_FULL_MASK, p2, j);
+                    if (p <= 0.f) continue;
+                    lastnz = j;
+                    cum2 += (double)p;
+                    if (choice < 0 && r < cum2) choice = j;
+                }
+                if (choice < 0) choice = lastnz;
+            }
+        }
+        if (tid == 0) {
+            const int ci = ti[choice];
+            if (ci == SMP_N_SEM) { /* EOS: semantic code forced to 0, sampler state untouched */
+                *out_tok = S2P_TOK_EOS;
+                *out_sem = 0;
+                *out_code0 = 0;
+                *out_eos = 1;
+                sm.fin_mode = 0;
+            } else {
+                const int64_t tok = (int64_t)S2P_TOK_SEMANTIC_START + ci;
+                *out_tok = tok;
+                *out_sem = ci;
+                *out_code0 = ci;
+                *out_eos = 0;
+                sm.fin_tok = tok;
+                sm.fin_mode = count0 < (uint64_t)window ? 1 : 2;
+                sp->count = count0 + 1;
+            }
         }
     }
-    if (tid == 0) {
-    const int ci = ti[choice];
-    if (ci == SMP_N_SEM) { /* EOS: semantic code forced to 0, sampler state untouched */
-        *out_tok = S2P_TOK_EOS;
-        *out_sem = 0;
-        *out_code0 = 0;
-        *out_eos = 1;
-        sm.fin_mode = 0;
-    } else {
-        const int64_t tok = (int64_t)S2P_TOK_SEMANTIC_START + ci;
-        *out_tok = tok;
-        *out_sem = ci;
-        *out_code0 = ci;
-        *out_eos = 0;
-        sm.fin_tok = tok;
-        sm.fin_mode = count0 < (uint64_t)window ? 1 : 2;
-        sp->count = count0 + 1;
-    }
-    } /* tid == 0 */
-    } /* warp == 0 */
     S2P_CTA_SYNC();
     /* history update, the shift done by the threads side by side from the staged window */
     if (sm.fin_mode == 1) {

@@ -142,8 +142,7 @@ __device__ __forceinline__ int sk_row(int t, int r, int ffn) {
 }
 /* silu(g) * u with the rounding steps of the unfused kernels (g, u: bf16 values held in f32) */
 __device__ __forceinline__ __nv_bfloat16 sk_swiglu(float g, float u) {
-    const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-g))); /* correctly rounded, as the division */
-    return f2bf(__fmul_rn(bf16_round(__fmul_rn(g, sig)), u));
+    return f2bf(swiglu_f32(g, u));
 }
 /* 32 accumulator columns of this warp's 32 TMEM lanes */
 __device__ __forceinline__ void sk_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {

@@ -32,6 +32,14 @@ class LinRef(C.Structure):
     _fields_ = [("kind", _I), ("w", _P), ("scales", _P), ("N", _I), ("K", _I), ("gshift", _I)]
 
 
+class NormIn(C.Structure):
+    _fields_ = [("src", _P), ("add", _P), ("gain", _P), ("x_out", _P), ("eps", _F), ("at", C.c_uint)]
+
+
+class TiledOut(C.Structure):
+    _fields_ = [("out", _P), ("lg", _I), ("kind", _I), ("int4", _I)]
+
+
 class VecRef(C.Structure):
     _fields_ = [("base", _P), ("index", _P), ("key", _P)]
 

@@ -3,16 +3,12 @@ import ctypes as C
 
 import pytest
 
-from _internal_abi import AttnArgs, QkvPostArgs
+from _internal_abi import AttnArgs, QkvPostArgs, TiledOut
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 P, I = C.c_void_p, C.c_int
 QH, KVH, HD = 32, 8, 128
-
-
-class TiledOut(C.Structure):
-    _fields_ = [("out", P), ("lg", I), ("kind", I), ("int4", I)]
 
 
 def p(t):

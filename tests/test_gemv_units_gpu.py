@@ -90,12 +90,8 @@ def test_every_kind_of_activation_gives_the_oracles_bits(mine, oracle, kind):
 @pytest.mark.parametrize("rows", [1, 2])
 @pytest.mark.parametrize("n,swiglu", [(6144, 0), (150, 0), (2 * 9728, 1), (2 * 77, 1)])
 def test_norm_in_the_linear_equals_the_two_kernels(testlib, kind, rows, n, swiglu):
-    from _internal_abi import LinRef
+    from _internal_abi import LinRef, NormIn
     P, I, L = C.c_void_p, C.c_int, C.POINTER(LinRef)
-
-    class NormIn(C.Structure):
-        _fields_ = [("src", P), ("add", P), ("gain", P), ("x_out", P), ("eps", C.c_float), ("at", C.c_uint)]
-
     testlib.gemv_rows.argtypes, testlib.gemv_rows_swiglu.argtypes = [L, P, P, I, I, P], [L, P, P, I, P]
     testlib.gemv_rows_norm.argtypes = [L, C.POINTER(NormIn), P, I, I, P]
     testlib.add_norm_to.argtypes = [P, P, P, P, P, I, P]
