@@ -142,7 +142,7 @@ __device__ void sampler_cta(const __nv_bfloat16* lrow, const __nv_bfloat16* eos_
         uint32_t key = idx < SMP_N_CAND ? sampler_key(cand[idx]) : 0u;
         for (int k = 0; k < SMP_TOPK; k++) {
             const int best = sampler_best(key, idx);
-            if (lane == 0) { tv[k] = best < SMP_N_CAND ? cand[best] : -INFINITY; ti[k] = best; }
+            if (lane == 0) { tv[k] = best < SMP_N_CAND ? cand[best] : -INFINITY; ti[k] = min(best, SMP_N_SEM); } /* nothing left: EOS, a row of NaN ends its stream */
             if (best < SMP_N_CAND && best == idx) {
                 at++;
                 idx = at < SMP_TOPK ? wt[lane * SMP_TOPK + at] : SMP_N_CAND;

@@ -70,9 +70,19 @@ def test_sequences_of_the_oracle(testlib, oracle, temperature, seed, window, spr
         assert d(lg) == (tok, sem.value, eos.value), t
 
 
-@pytest.mark.parametrize("temperature,seed", [(0.0, 0), (0.8, 42)])
-def test_rows_of_nan(testlib, temperature, seed):
-    """NaN is never chosen where there is something else, and takes nothing out of range."""
+@pytest.mark.parametrize("temperature,seed", [(0.0, 0), (0.8, 42), (0.8, 0)])
+@pytest.mark.parametrize("left", [2, 1, 0])
+def test_rows_of_nan(testlib, oracle, temperature, seed, left):
+    """NaN is never chosen where there is something else; where there is nothing else the frame is EOS, as the oracle's."""
+    from oracle import oracle_api as oa
     lg = np.full(4097, 0x7FC0, np.uint16)
-    lg[[17, 900]] = [0x3F80, 0x4000]  # 1 and 2
-    assert Device(testlib, temperature, 0.8, 1.1, 16, seed)(lg)[1] == 900 if temperature == 0 else Device(testlib, temperature, 0.8, 1.1, 16, seed)(lg)[1] in (17, 900)
+    lg[[17, 900][:left]] = [0x3F80, 0x4000][:left]  # 1 and 2
+    sp = C.create_string_buffer(oracle.s2po_sampler_size())
+    oracle.s2po_sampler_init(sp, temperature, 0.8, 1.1, 16, seed, 0)
+    sem, eos = C.c_int32(0), C.c_int32(0)
+    tok = oracle.s2po_sample(sp, oa.ptr(lg), int(lg[4096]), 4096, START, EOS, C.byref(sem), C.byref(eos))
+    got = Device(testlib, temperature, 0.8, 1.1, 16, seed)(lg)
+    if seed == 0 and temperature and left == 2:  # the oracle draws from another stream of random numbers
+        assert got[1] in (17, 900) and not got[2]
+    else:
+        assert got == (tok, sem.value, eos.value) and (got[2] == 0) == (left > 0)
