@@ -137,7 +137,7 @@ cudaError_t tick_begin(const TickBeginArgs* a, int rows, cudaStream_t st);
 cudaError_t tick_finish_keys(const unsigned long long* keys, int rows, int32_t* codes, cudaStream_t st);
 
 cudaError_t gemv_setup_all(void); /* once per device, before any stream capture */
-/* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: see launch_early (launch.cuh) */
+/* the exact-order linear, 1 <= M <= 16: an s2p_status; `early`: the weights are settled, they are read before the wait (gemv.cu, run_gemv_batch) */
 int gemv_rows(const LinRef* lin, const void* x, void* y, int M, int early, cudaStream_t st);
 /* h[M, N / 2] = silu(gate) * up for stacked [gate | up] rows, otherwise as gemv_rows with early.  Up to four rows the launch it
  * saves counts (tick of 1 row 3.53 -> 3.43 ms, 3 rows 5.61 -> 5.55, in the kernels of that time); in the kernels of more rows its epilogue costs
@@ -313,6 +313,7 @@ cudaError_t mega_launch(const MegaParams* p, int n_cta, cudaStream_t st);
 
 cudaError_t qkv_post(const QkvPostArgs* a, int rows, cudaStream_t st);
 cudaError_t attn_single(const AttnArgs* a, int rows, cudaStream_t st);
+int attn_prefill_rows_of_block(const AttnArgs* a, int rows); /* rows of the blocks that a slice of `rows` is cut into */
 /* the same, with the word that takes the code of a bounded wait that gave up; attn_single: the device's word for unwatched calls */
 cudaError_t attn_slice(const AttnArgs* a, int rows, int* status, cudaStream_t st);
 cudaError_t attn_prefill_set_wait_ns(unsigned long long ns); /* test hook: deadline of those waits */

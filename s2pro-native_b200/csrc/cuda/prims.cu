@@ -606,7 +606,7 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, int* status,
  * slower than 24, 10 and 14 than 12 and 16 (their warps load the schedulers unevenly).
  * Measured, us, before (waves of CTAs, all taken to see equally many tiles) and now: 512 rows at 0 109 -> 76, 430 78 -> 62, 1000 287 -> 216, 2048 912 ->
  * 806; behind a context, 77 after 1024 71 -> 70, 140 after 1000 90 -> 84, 2048 after 6052 5394 -> 5364. */
-static int attn_prefill_block(int rows, int pos0, int kv_heads, int sms, int block_rows) {
+static int attn_prefill_tiles(int rows, int pos0, int kv_heads, int sms, int block_rows) {
     const int nb = (rows + block_rows - 1) / block_rows;
     auto tiles = [&](int b) { return (pos0 + min(rows, (b + 1) * block_rows) + 127) / 128; };
     long long total = 0;
@@ -615,24 +615,27 @@ static int attn_prefill_block(int rows, int pos0, int kv_heads, int sms, int blo
     for (int k = 1; (k - 1) * sms < nb * kv_heads; k++) longest = max(longest, (long long)k * tiles(nb - 1 - (k - 1) * sms / kv_heads));
     return (int)min(longest, 1000000ll);
 }
-template <bool KV8>
-static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, int* status, cudaStream_t st) {
+int attn_prefill_rows_of_block(const AttnArgs* a, int rows) {
     static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {19200, 14700, 12100, 8700, 7200, 5650, 4700},
                      start_ns[7] = {2000, 2200, 6000, 3200, 5100, 4200, 4000};
     int best = 0;
     long long best_cost = 0;
     for (int v = 0; v < 7; v++) {
         const int ctas = (rows + block_rows[v] - 1) / block_rows[v] * a->kv_heads, sms = device_sm_count();
-        const long long cost = (long long)attn_prefill_block(rows, a->pos0, a->kv_heads, sms, block_rows[v]) * tile_ns[v] + (ctas + sms - 1) / sms * start_ns[v];
+        const long long cost = (long long)attn_prefill_tiles(rows, a->pos0, a->kv_heads, sms, block_rows[v]) * tile_ns[v] + (ctas + sms - 1) / sms * start_ns[v];
         if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
-    switch (best) {
-    case 0: return launch_attn_prefill<KV8, 4, 12, false>(a, rows, status, st);
-    case 1: return launch_attn_prefill<KV8, 4, 8, false>(a, rows, status, st);
-    case 2: return launch_attn_prefill<KV8, 4, 6, true>(a, rows, status, st);
-    case 3: return launch_attn_prefill<KV8, 2, 8, true>(a, rows, status, st);
-    case 4: return launch_attn_prefill<KV8, 2, 6, true>(a, rows, status, st);
-    case 5: return launch_attn_prefill<KV8, 2, 4, true>(a, rows, status, st);
+    return block_rows[best];
+}
+template <bool KV8>
+static cudaError_t launch_attn_prefill_rows(const AttnArgs* a, int rows, int* status, cudaStream_t st) {
+    switch (attn_prefill_rows_of_block(a, rows)) {
+    case 24: return launch_attn_prefill<KV8, 4, 12, false>(a, rows, status, st);
+    case 16: return launch_attn_prefill<KV8, 4, 8, false>(a, rows, status, st);
+    case 12: return launch_attn_prefill<KV8, 4, 6, true>(a, rows, status, st);
+    case 8: return launch_attn_prefill<KV8, 2, 8, true>(a, rows, status, st);
+    case 6: return launch_attn_prefill<KV8, 2, 6, true>(a, rows, status, st);
+    case 4: return launch_attn_prefill<KV8, 2, 4, true>(a, rows, status, st);
     default: return launch_attn_prefill<KV8, 2, 2, true>(a, rows, status, st);
     }
 }

@@ -7,11 +7,14 @@ from _internal_abi import AttnArgs
 
 pytestmark = pytest.mark.gpu
 QH, KVH, HD = 32, 8, 128
+# which block size each of them picks is asked for in test_attn_blocks_gpu.py
+SLICES = [(0, 2), (0, 129), (127, 2), (126, 5), (250, 73), (128, 128), (1000, 21), (0, 300), (40, 460), (3000, 450), (100, 50), (63, 150), (0, 209), (0, 700)]
+INFINITE_VALUES = [(0, 2), (3, 3), (126, 5), (0, 24), (120, 77), (0, 300), (0, 460), (0, 40), (0, 209), (0, 700)]
 
 
 @pytest.mark.parametrize("kv8", [0, 1])
 @pytest.mark.parametrize("shift", [0, 4])
-@pytest.mark.parametrize("pos0,rows", [(0, 2), (0, 129), (127, 2), (126, 5), (250, 73), (128, 128), (1000, 21), (0, 300), (40, 460), (3000, 450), (100, 50), (63, 150)])
+@pytest.mark.parametrize("pos0,rows", SLICES)
 def test_rows_of_a_slice_equal_single_rows(testlib, kv8, shift, pos0, rows):
     """All block sizes (their choice depends on the slice's length), ragged last blocks, tiles cut by the diagonal,
     and caches that are aligned to 4 bytes only."""
@@ -48,7 +51,7 @@ def test_rows_of_a_slice_equal_single_rows(testlib, kv8, shift, pos0, rows):
 
 
 @pytest.mark.parametrize("kv8", [0, 1])
-@pytest.mark.parametrize("pos0,rows", [(0, 2), (3, 3), (126, 5), (0, 24), (120, 77), (0, 300), (0, 460)])
+@pytest.mark.parametrize("pos0,rows", INFINITE_VALUES)
 def test_infinite_values_reach_only_the_rows_that_see_them(testlib, kv8, pos0, rows):
     """Every block size: infinities and NaN in the values of the slice's second half leave the rows before it as they are."""
     import torch
