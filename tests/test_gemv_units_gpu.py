@@ -40,6 +40,25 @@ def test_rows_equal_the_batch_kernels(mine, kind, n, k):
         assert torch.equal(got[:rows].view(torch.int16), want[:rows].view(torch.int16)) and (got[rows] == 7).all(), rows
 
 
+# sums that fit shared memory, and two shapes whose do not (the batch kernel's, for one row too)
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("f,k", [(77, 1024), (5, 409600), (70001, 1024)])
+def test_swiglu_rows_equal_the_separate_kernels(testlib, kind, f, k):
+    from _internal_abi import LinRef
+    testlib.gemv_rows_swiglu.argtypes = [C.POINTER(LinRef), C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]
+    w, s, gen = weights(kind, 2 * f, k, 32, f)
+    x = torch.randn(5, k, device="cuda", generator=gen).bfloat16()
+    gu, want = torch.empty((5, 2 * f), dtype=torch.bfloat16, device="cuda"), torch.empty((5, f), dtype=torch.bfloat16, device="cuda")
+    assert gemv(testlib, kind, gu, x, w, s, 5, 2 * f, k, 32) == 0 and testlib.s2pk_silu_mul(p(gu), p(want), 5, f, None) == 0
+    lin = LinRef(kind, w.data_ptr(), s.data_ptr(), 2 * f, k, 0 if kind == 0 else 5)
+    for rows in (1, 2, 3, 4):
+        got = torch.full((rows + 1, f), 7.0, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        assert testlib.gemv_rows_swiglu(C.byref(lin), p(x), p(got), rows, None) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(got[:rows].view(torch.int16), want[:rows].view(torch.int16)) and (got[rows] == 7).all(), rows
+
+
 @pytest.mark.parametrize("kind", [1, 2])
 @pytest.mark.parametrize("g,off", [(16, 0), (64, 2), (512, 0), (1024, 0), (2048, 6), (32, 2), (32, 14)])  # scales that 16-byte copies cannot take
 def test_groups_and_unaligned_scales(mine, kind, g, off):
