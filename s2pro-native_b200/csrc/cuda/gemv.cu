@@ -124,7 +124,7 @@ extern "C" cudaError_t gemv_setup_all(void) {
  * 4.6 / 7.0 / 8.5.)
  * Measured, ticks of the full model, ms, before (two activation rows to a packed fma, each widened to f32; 168 registers) and now: 3 rows INT4
  * 4.25 -> 4.06, 8 rows INT4 8.12 -> 6.55, 16 rows INT8 12.80 -> 10.81.  CTAs to an SM: of the shared form 5 (8 rows 7.23 with 4); of the other 4,
- * where up to four rows are slower by 1 % than with 3.  16 rows of 19456 x 2560 INT4 take 50 us, 16 T fma/s of the 28 that a loop of mixed fma
+ * where up to four rows are slower by 1 % than with 3.  16 rows of 19456 x 2560 INT4 take 46 us, 17 T fma/s of the 28 that a loop of mixed fma
  * alone reaches. */
 /* A SwiGLU over stacked [gate | up] rows (SW): half of a warp's rows are of either half, so gate and up of an output meet in
  * the warp; both round to bf16 first, as where a kernel of its own follows the linear. */
@@ -350,7 +350,8 @@ __global__ void __launch_bounds__(128, (BatchPlan<WK, MM, NS>::CTAS)) k_gemv_bat
 
 /* Launched to start while the kernel in front finishes, inside a tick and for callers alike (launch.cuh).  Inside a tick (`early`) the
  * weights are settled and asked for before the wait; a caller may have written them just before, so there the wait comes first and only
- * the launch itself overlaps: calls one after another of one row, INT4 19456 x 2560, 12.4 -> 10.4 us. */
+ * the launch itself overlaps: calls one after another of one row, INT4 19456 x 2560, 12.4 -> 10.4 us.  A lone call has nothing to overlap (24.5 us host to
+ * host, 27 with the kernel before). */
 template <int WK, int MM, int NS, bool SW>
 static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {
     constexpr int rows = 4 * (4 / NS); /* weight rows of a CTA */
