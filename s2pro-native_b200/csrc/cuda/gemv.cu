@@ -358,20 +358,35 @@ static cudaError_t run_gemv_batch(void* y, const void* x, const void* w, const v
     return launch_after(k_gemv_batch<WK, MM, NS, SW>, dim3((unsigned)((N + rows - 1) / rows), (unsigned)((M + MM - 1) / MM)), 128, 0, stream,
                        (__nv_bfloat16*)y, (const __nv_bfloat16*)x, w, scales, M, N, K, gshift, early);
 }
-/* Four warps share four rows where the CTAs of the shared form all fit the GPU at once, up to 2960 rows of weights, 3552 for two rows
- * (3552 x 2560 INT8, us, shared and not, one row 5.4 and 4.6, two 4.4 and 5.7, three 6.8 and 5.2); also where one warp each would leave a scheduler with
- * less than 2.5, which do not hide each other's latencies, provided that three quarters of the rounds' turns have a tile (a CTA waits for its slowest
- * warp).  (A SwiGLU's pairs of rows meet in a warp, which the tiles' sums of a shared row do not; the layers that have one have rows enough.) */
+/* Where four warps share four rows (a SwiGLU's pairs of rows meet in a warp, which the tiles' sums of a shared row do not; the layers that have one
+ * have rows enough).  us, each warp its own rows / shared:
+ *  - where the CTAs of the shared form all fit the GPU at once, up to 2960 rows of weights, 3552 for two rows (3552 x 2560 INT8, one row 4.6 / 5.4, two 5.7 / 4.4,
+ *    three 5.2 / 6.8), but for one and two rows of a single tile (2560 x 512 1.9 / 2.2);
+ *  - not where K has a tile or two, of which most of a CTA's warps get none: 4096 x 1024 INT8 one row 2.5 / 3.8, eight 4.6 / 5.7;
+ *  - where one warp each would leave a scheduler with less than 2.5, which do not hide each other's latencies, provided that three quarters of the rounds'
+ *    turns have a tile (a CTA waits for its slowest warp);
+ *  - five to eight rows where the other form puts a third CTA on some SMs and the shared one takes two waves at most: 4864 x 2560 eight rows INT8 13.3 / 10.6, INT4
+ *    12.9 / 10.1; 6144 x 2560, above, 13.4 / 13.5;
+ *  - two and five to eight rows of a long K, up to what was measured: 6144 x 9728 INT8 two 20.7 / 17.2, eight 43.0 / 37.7, 9728 x 9728 grouped eight 70 / 51; 19456 x 9728
+ *    two INT8 52 / 56. */
 static bool gemv_batch_fits_shared(int M, int N) { return (long long)((N + 3) / 4) * ((M + 7) / 8) <= (M == 2 ? 6ll : 5ll) * device_sm_count(); }
+static bool gemv_short(int M, int N, int K) { return gemv_batch_fits_shared(M, N) ? K == 512 && M <= 2 : K <= 2 * 512; }
+static bool gemv_batch_shared(int M, int N, int K) {
+    if (gemv_short(M, N, K)) return false;
+    if (gemv_batch_fits_shared(M, N)) return true;
+    const long long quads = (N + 3) / 4, warps = quads * ((M + 7) / 8), sms = device_sm_count();
+    const int T = K >> 9, turns = (T + 3) / 4 * 4;
+    if (warps < 10 * sms && 4 * T >= 3 * turns) return true;
+    if (M > 4 && M <= 8 && T >= 5 && quads > 8 * sms && quads <= 10 * sms) return true;
+    return (M == 2 || (M > 4 && M <= 8)) && T >= 8 && quads <= 17 * sms;
+}
 template <int WK, bool SW>
 cudaError_t launch_gemv_batch(void* y, const void* x, const void* w, const void* scales, int M, int N, int K,
                               int gshift, int early, cudaStream_t stream) {
     /* as few groups of activation rows as eight a group allow (each converts every code once), of one size */
     const int groups = (M + 7) / 8;
     const int mm = (M + groups - 1) / groups;
-    const long long warps = (long long)((N + 3) / 4) * groups, sched = 4ll * device_sm_count();
-    const int T = K >> 9, turns = (T + 3) / 4 * 4;
-    const bool shared = !SW && (gemv_batch_fits_shared(M, N) || (2 * warps < 5 * sched && 4 * T >= 3 * turns));
+    const bool shared = !SW && gemv_batch_shared(M, N, K);
 #define S2P_GB(MM)                                                                                            \
     do {                                                                                                      \
         if (shared) return run_gemv_batch<WK, MM, SW ? 1 : 4, SW>(y, x, w, scales, M, N, K, gshift, early, stream); \
@@ -663,12 +678,22 @@ template <int WK, bool SW> static int gemv_row_grid(int M, int N, int K, int gsh
  *  - from two warps of four rows to a scheduler, three and four rows (4097 x 2560, three rows INT4 5.9 / 6.3 (5.1 / 5.8); 6144 x 2560 7.4 / 6.5).  One and two rows only
  *    outside a tick: a caller's weights are not asked for before the wait, and more, smaller CTAs have more of them under way then (6144 x 2560 INT8 two
  *    rows 8.1 / 6.7 (7.0 / 6.4), 19456 x 2560 one row 13.1 / 11.5 (11.5 / 11.0), two 16.7 / 13.9 (15.3 / 13.7)).  One row of packed INT4 has too few
- *    instructions for that to matter (5.0 / 5.3, 10.6 / 10.5). */
+ *    instructions for that to matter (5.0 / 5.3, 10.6 / 10.5).  A long K turns both: one row is back with k_gemv_row while an SM has few enough rows
+ *    (6144 x 9728 INT8 13.7 / 17.1, grouped 14.1 / 18.2), two rows INT8 are with the shared form in a tick too (6144 x 6144 12.1 / 11.3);
+ *  - where some SMs get a fourth CTA of two rows and most do not, from 7104 to 9472 rows of weights: 7168 x 2560 INT4 7.6 / 8.6, 8192 8.0 / 9.1, grouped 8.7 / 9.2 and 9.1 / 9.6
+ *    (INT8 per channel 8.4 / 8.3, 9.0 / 9.2);
+ *  - a tile or two of K, whatever the rows: nothing to spread over an SM's warps (4096 x 512 INT8 two rows 3.1 / 2.0, 4096 x 1024 one row 3.3 / 2.5);
+ *  - three rows of INT8 per channel, whose chains the batch kernel holds with the fewest registers (4096 x 2560 6.7 / 5.4 (5.6 / 5.1), 4096 x 4096 9.0 / 7.4). */
 template <int WK, bool SW> static bool gemv_batch_faster(int M, int N, int K, int early) {
-    if (M > 4) return true;
+    if (M > 4 || (!SW && gemv_short(M, N, K))) return true;
     if (!SW && gemv_batch_fits_shared(M, N)) return K <= 12 * 512 || (WK == WK_INT4_PACK ? M != 2 : WK == WK_INT8_GRP && M == 4);
-    const bool many = (N + 3) / 4 >= 2 * 4 * device_sm_count();
-    return many && (M > 2 || (!early && (M == 2 || WK != WK_INT4_PACK)));
+    if (!SW && WK == WK_INT8_CH && M == 3 && K <= 12 * 512) return true;
+    const int quads = (N + 3) / 4, sms = device_sm_count();
+    const bool many = quads >= 2 * 4 * sms, deep = !SW && K >= 8 * 512;
+    if (!many || M > 2) return many;
+    if (deep && M == 1 && quads <= 12 * sms) return false;
+    if (!SW && !deep && M == 2 && WK != WK_INT8_CH && quads > 12 * sms && quads <= 16 * sms) return false;
+    return early ? deep && M == 2 && WK != WK_INT4_PACK : M == 2 || WK != WK_INT4_PACK;
 }
 template <int WK, bool SW>
 static cudaError_t launch_gemv_row(int grid, void* y, const void* x, const void* w, const void* scales, int M, int N, int K, int gshift, int early, cudaStream_t stream) {

@@ -52,3 +52,11 @@ def test_every_batch_size_gives_the_oracles_bits(mine, oracle, kind, n, k, all_r
 @pytest.mark.parametrize("n,k", [(2960, 512), (2961, 1024), (3552, 512), (3553, 1024), (1029, 6144), (1029, 6656), (4732, 512), (4733, 1024)])
 def test_both_sides_of_a_rule_give_the_oracles_bits(mine, oracle, kind, n, k):
     against_the_oracle(mine, oracle, kind, n, k, (1, 2, 3, 4, 5, 9))
+
+
+# a tile or two of K; three rows up to twelve tiles; two rows where some SMs get a fourth CTA; five to eight rows up to two waves of shared rows; eight tiles of K, up to 12 and 17 SMs' worth of quads
+@pytest.mark.parametrize("kind", ["int8", "int8_grouped", "int4"])
+@pytest.mark.parametrize("n,k,batches", [(2559, 512, (1, 2, 3, 8)), (4095, 1024, (1, 2, 3, 4, 8)), (2961, 1536, (1, 3)), (2961, 6144, (3,)), (2961, 6656, (3,)), (4736, 2560, (5, 8)), (4737, 2560, (5, 8)),
+                                         (5920, 2560, (6,)), (5921, 2560, (6,)), (7104, 4096, (1, 2)), (7105, 4096, (1,)), (7104, 512, (2,)), (7105, 1536, (2,)), (9472, 1536, (2,)), (9473, 1536, (2,)), (10064, 4096, (2, 7)), (10065, 4096, (2, 7))])
+def test_both_sides_of_the_rules_on_tiles_give_the_oracles_bits(mine, oracle, kind, n, k, batches):
+    against_the_oracle(mine, oracle, kind, n, k, batches)
