@@ -198,16 +198,21 @@ __global__ void __launch_bounds__(NT * 64, NT == 3 && KV8 ? 3 : 2) k_attn_decode
      * decide here how many of the `workers` per (row, kv head) take part: enough teams for about
      * ATTN_SPLITS_PER_TEAM splits each, so that the copies of one split overlap the arithmetic of
      * another, but never so few CTAs that SMs stay empty.  The others go straight to the arrival counter.
-     * Of the two counts around that share an INT8 cache's three CTAs to an SM take the higher: us, lower / higher, 8 x 8000 rows x positions 84 / 75,
-     * 16 x 6000 112 / 98, 64 x 1000 73 / 65, 64 x 3000 166 / 169, 128 x 1024 116 / 123.  With two CTAs to an SM it is the one whose CTAs take less
-     * time in all, a CTA the rounds of its busiest team and two more for its start and its partials: bf16 8 x 8000 97 / 93, 16 x 6000 120 / 114, 32 x 2000 72 / 77,
-     * 64 x 3000 183 / 191, 96 x 1000 100 / 116, 128 x 1024 134 / 147. */
+     * An INT8 cache's three CTAs to an SM take the share rounded up: us, rounded down / up, 8 x 8000 rows x positions 84 / 75, 64 x 1000 73 / 65, 64 x 3000 166 / 169,
+     * 128 x 1024 116 / 123.  A bf16 cache's two take, where the share fills the SMs, the one of both whose waves of CTAs, each the rounds of its busiest team
+     * and one more, are shorter: 20 x 2000 66 / 55, 24 x 2000 69 / 62, 96 x 1000 105 / 118, 128 x 1024 134 / 147 (and wrongly 64 x 3000
+     * 187 / 195).
+     * What fills the SMs stops short of a second wave, unless that leaves a quarter of the places empty.  Always rounded up / so: INT8 4 x 8000 51.1 / 46.1,
+     * 5 x 8000 69.4 / 51.3, 7 x 4000 43.6 / 37.8, 12 x 2000 36.4 / 32.1; 28 x 700 28.3 / 28.4 (always down 35.7).  (A search here over all counts costs every CTA more than it
+     * finds: 48 x 200 21.8 -> 23.0.) */
     constexpr bool THREES = KV8 && NT == 3;
-    constexpr int SHARE = NT * ATTN_SPLITS_PER_TEAM;
-    const int pairs = (int)(gridDim.x * gridDim.y), fill = ((THREES ? 3 : 2) * 148 + pairs - 1) / pairs;
-    auto time_of = [&](int e) { return e * ((n_active + e * NT - 1) / (e * NT) + 2); };
+    constexpr int SHARE = NT * ATTN_SPLITS_PER_TEAM, SLOTS = (THREES ? 3 : 2) * 148;
+    const int pairs = (int)(gridDim.x * gridDim.y);
+    int fill = SLOTS / pairs;
+    if (NT == 3 ? 4 * fill * pairs < 3 * SLOTS : fill * pairs < SLOTS) fill++; /* four teams: a row or two, one wave whatever the count */
+    auto time_of = [&](int e) { return (pairs * e + SLOTS - 1) / SLOTS * ((n_active + e * NT - 1) / (e * NT) + 1); };
     int share = (n_active + (THREES ? SHARE - 1 : 0)) / SHARE;
-    if (!THREES && share >= fill && share < workers && time_of(share + 1) < time_of(share)) share++;
+    if (!KV8 && share >= fill && share < workers && time_of(share + 1) < time_of(share)) share++;
     const int eff = min(workers, max(share, fill));
     const int first = wk < eff ? wk + eff * team : n_active, step = eff * NT;
 

@@ -57,6 +57,35 @@ def test_decode_attention(testlib, kind, rows, kv8, pos):
     assert same_rows(got, want, rows) and int(ctr.abs().max()) == 0
 
 
+# rows and lengths on either side of where the kernel takes one worker more: full SMs, three quarters of them, a share rounded up or by its waves
+@pytest.mark.parametrize("kv8", [0, 1])
+@pytest.mark.parametrize("rows,length", [(2, 1500), (3, 833), (4, 2000), (5, 4000), (7, 1800), (12, 769), (20, 2000), (28, 700), (37, 193), (42, 400), (96, 1000)])
+def test_the_number_of_workers_changes_no_bit(testlib, kv8, rows, length):
+    testlib.attn_decode.argtypes = [C.POINTER(AttnArgs), I, P]
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    max_seq = (length + 63) // 64 * 64
+    kv = torch.randint(-127, 128, (rows, 2, KVH, max_seq, HD), dtype=torch.int8, device="cuda", generator=g) if kv8 else torch.randn(rows, 2, KVH, max_seq, HD, device="cuda", generator=g).bfloat16()
+    sc = (torch.rand(rows, 2, KVH, max_seq, 4, device="cuda", generator=g) * 0.02 + 0.001).half()
+    q = torch.randn(rows, QH * HD, device="cuda", generator=g).bfloat16()
+    slots = max_seq // 64
+    part, ctr = torch.empty(rows * QH * slots * 130, device="cuda"), torch.zeros(rows * KVH, dtype=torch.int32, device="cuda")
+    at = torch.full((rows,), length - 1, dtype=torch.int32, device="cuda")
+    at[rows // 2] = 70  # a short row among them
+    a = AttnArgs()
+    a.q, a.q_heads, a.kv_heads, a.max_seq, a.kv8, a.head_dim = q.data_ptr(), QH, KVH, max_seq, kv8, HD
+    a.pos_arr, a.part, a.counters, a.n_split_slots = at.data_ptr(), part.data_ptr(), ctr.data_ptr(), slots
+    a.kv.base0, a.kv.row_stride, a.kv.v_off = kv.data_ptr(), kv[0].nbytes, kv[0, 0].nbytes
+    a.kv.sbase0, a.kv.srow_stride, a.kv.vs_off = sc.data_ptr(), sc[0].nbytes, sc[0, 0].nbytes
+    outs = []
+    for workers in (1, max(2, min(16, 2048 // (rows * KVH)))):
+        outs.append(torch.zeros_like(q))
+        a.out, a.workers = outs[-1].data_ptr(), workers
+        torch.cuda.synchronize()
+        assert testlib.attn_decode(C.byref(a), rows, None) == 0
+        torch.cuda.synchronize()
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16)) and outs[0].isfinite().all() and int(ctr.abs().max()) == 0
+
+
 @pytest.mark.parametrize("kind", [0, 2])
 @pytest.mark.parametrize("rows", [1, 32, 37, 38, 128])
 def test_fast_attention(testlib, kind, rows):
