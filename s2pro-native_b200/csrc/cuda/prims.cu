@@ -601,7 +601,8 @@ static cudaError_t launch_attn_prefill(const AttnArgs* a, int rows, int* status,
  * fill the GPU when the slice is short: the block size with the smallest estimate is taken, a start for each wave and so many tiles in sequence.  How
  * many: blocks of a slice see unequally many tiles and start longest first, so the schedule is about as long as the longest of
  * the longest block, the tiles over the SMs, and, where an SM gets k blocks, k times the shortest that can be a k-th one.
- * The times are measured ones for an INT8 cache (one block to an SM, 1 and 17 tiles); bf16 is within 10 %.  16 and 24 rows keep a scheduler busy
+ * The times are measured ones for an INT8 cache (one block to an SM, 1 and 17 tiles), moved by up to 4 % a tile to where the seven sizes cross in 366 slices
+ * of both caches (none slower for it; 300 after 1024 226 -> 205 bf16, 700 after 500 308 -> 270, 0.4 % above the fastest size on average).  16 and 24 rows keep a scheduler busy
  * with warps that do both products; up to 12 rows they are apart.  Sizes between these were no faster: 5 rows as 6, 18 and 20
  * slower than 24, 10 and 14 than 12 and 16 (their warps load the schedulers unevenly).
  * Measured, us, before (waves of CTAs, all taken to see equally many tiles) and now: 512 rows at 0 109 -> 76, 430 78 -> 62, 1000 287 -> 216, 2048 912 ->
@@ -616,8 +617,8 @@ static int attn_prefill_tiles(int rows, int pos0, int kv_heads, int sms, int blo
     return (int)min(longest, 1000000ll);
 }
 int attn_prefill_rows_of_block(const AttnArgs* a, int rows) {
-    static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {19200, 14700, 12100, 8700, 7200, 5650, 4700},
-                     start_ns[7] = {2000, 2200, 6000, 3200, 5100, 4200, 4000};
+    static const int block_rows[7] = {24, 16, 12, 8, 6, 4, 2}, tile_ns[7] = {18500, 15200, 12050, 8950, 7250, 5750, 4600},
+                     start_ns[7] = {3600, 2000, 6000, 3200, 5200, 5500, 4800};
     int best = 0;
     long long best_cost = 0;
     for (int v = 0; v < 7; v++) {
